@@ -164,6 +164,98 @@ void weight_matrix_packing(Tensor wt_outs, Tensor msk_outs, Tensor wt_in, Tensor
     }
 }
 
+// ---- the Python package's own calls (ops.py, quantize.py) -----------------------------------------------------------
+// What those modules check and launch, for arguments that pass every check: a decoding step is a chain of small launches,
+// and the same work done in Python (17 ctypes arguments, a device context, some thirty tensor properties) takes longer
+// than most of them run.  Nothing is diagnosed here: whenever a precondition does not hold, or the scratch buffer
+// of this stream does not exist yet, the caller is told so (-1 / None) and takes its own path, which raises or allocates.
+
+bool plain(const Tensor& t, const c10::Device& dev, c10::ScalarType type) {
+    return t.is_cuda() && t.device() == dev && t.scalar_type() == type && t.is_contiguous();
+}
+
+// `workspaces`: the Python package's dict (device index, raw stream) -> zero-initialised uint8 tensor
+int launch_checked(int64_t bits, bool matvec, int64_t path, void* out, const Tensor& matrix, const Tensor& x, int64_t rows,
+                   const Tensor& scales, const Tensor& zeros, int64_t group_size, const c10::optional<Tensor>& mask,
+                   const py::dict& workspaces) {
+    const auto dev = x.device();
+    if (bits != 4 && bits != 3 && bits != 2) return -1;
+    const int64_t in_size = x.size(-1);
+    if (!plain(x, dev, torch::kHalf) || !plain(matrix, dev, torch::kInt) || !plain(scales, dev, torch::kHalf) ||
+        !plain(zeros, dev, torch::kHalf) || matrix.dim() != 2 || scales.dim() != 2 || zeros.dim() != 2)
+        return -1;
+    const int64_t mtx_in = matrix.size(0), out_size = matrix.size(1);
+    const bool sparse = mask.has_value() && mask->defined();
+    if (sparse) {
+        if (bits != 4 || mtx_in * 16 != in_size || mtx_in % 2 || !plain(*mask, dev, torch::kInt) || mask->dim() != 2 ||
+            mask->size(0) != mtx_in / 2 || mask->size(1) != out_size)
+            return -1;
+    } else if ((mtx_in * 32) % bits || mtx_in * 32 / bits != in_size) {
+        return -1;
+    }
+    if (scales.size(1) != out_size || zeros.sizes() != scales.sizes()) return -1;
+    if (group_size == 0 || (group_size > 0 && group_size % 64)) return -1;
+    c10::cuda::OptionalCUDAGuard guard;
+    if (c10::cuda::current_device() != dev.index()) guard.set_device(dev);
+    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+    PyObject* const item = PyDict_GetItem(workspaces.ptr(), py::make_tuple((int)dev.index(), (uint64_t)(uintptr_t)stream).ptr());
+    if (!item) return -1;
+    const Tensor ws = py::cast<Tensor>(py::handle(item));
+    return i4mm_quant_matmul((int)bits, matvec ? 1 : 0, (int)path, out, matrix.data_ptr(), sparse ? mask->data_ptr() : nullptr,
+                             x.data_ptr(), scales.data_ptr(), zeros.data_ptr(), rows, in_size, out_size, scales.size(0), group_size,
+                             ws.data_ptr(), (size_t)ws.numel(), (void*)stream);
+}
+
+// ops._mult; route 0: by seq_len, 1: matmul, 2: matvec
+int try_mult(int64_t bits, int64_t route, int64_t path, const Tensor& outs, const Tensor& matrix, const Tensor& x, const Tensor& scales,
+             const Tensor& zeros, int64_t group_size, const c10::optional<Tensor>& mask, const py::dict& workspaces) {
+    if (x.dim() != 3 || outs.dim() != 3 || matrix.dim() != 2 || !plain(outs, x.device(), torch::kHalf)) return -1;
+    const int64_t batch = x.size(0), seq_len = x.size(1);
+    if (route == 2 && seq_len != 1) return -1;
+    if (outs.size(0) != batch || outs.size(1) != seq_len || outs.size(2) != matrix.size(1)) return -1;
+    return launch_checked(bits, route == 2 || (route == 0 && seq_len == 1), path, outs.data_ptr(), matrix, x, batch * seq_len,
+                          scales, zeros, group_size, mask, workspaces);
+}
+
+// QuantLinear.forward: the new output, or a status / -1
+py::object try_linear(int64_t bits, int64_t path, const Tensor& x, int64_t in_features, int64_t out_features, const Tensor& matrix,
+                      const Tensor& scales, const Tensor& zeros, int64_t group_size, const c10::optional<Tensor>& mask,
+                      const py::dict& workspaces) {
+    if (x.dim() < 1 || x.numel() == 0 || x.size(-1) != in_features || matrix.dim() != 2 || matrix.size(1) != out_features ||
+        !plain(x, x.device(), torch::kHalf))
+        return py::int_(-1);
+    auto sizes = x.sizes().vec();
+    sizes.back() = out_features;
+    Tensor out = at::empty(sizes, at::TensorOptions().dtype(torch::kHalf).device(x.device()));
+    const int status = launch_checked(bits, false, path, out.data_ptr(), matrix, x, x.numel() / in_features, scales, zeros, group_size,
+                                      mask, workspaces);
+    if (status != I4MM_OK) return py::int_(status);
+    return py::cast(out);
+}
+
+// ops.row_norm: the new output, or a status / -1
+py::object try_row_norm(int64_t mode, const Tensor& a, const c10::optional<Tensor>& b, const c10::optional<Tensor>& c) {
+    if (!a.is_cuda() || a.dim() != 2 || c10::cuda::current_device() != a.device().index()) return py::int_(-1);
+    const c10::optional<Tensor> operands[3] = {a, b, c};
+    const void* ptr[3] = {nullptr, nullptr, nullptr};
+    int64_t stride[3] = {0, 0, 0};
+    for (int i = 0; i < 3; ++i) {
+        if (!operands[i].has_value()) continue;
+        const Tensor& t = *operands[i];
+        if (!t.is_cuda() || t.device() != a.device() || t.scalar_type() != torch::kHalf || t.sizes() != a.sizes() || t.stride(1) != 1)
+            return py::int_(-1);
+        ptr[i] = t.data_ptr();
+        stride[i] = t.stride(0);
+    }
+    const int64_t rows = a.size(0), width = a.size(1);
+    const auto options = at::TensorOptions().dtype(torch::kHalf).device(a.device());
+    Tensor y = mode == 4 ? at::empty({2, rows, width}, options) : at::empty({rows, width}, options);
+    const int status = i4mm_row_norm((int)mode, y.data_ptr(), ptr[0], ptr[1], ptr[2], rows, width, stride[0], stride[1], stride[2],
+                                     (void*)c10::cuda::getCurrentCUDAStream(a.device().index()).stream());
+    if (status != I4MM_OK) return py::int_(status);
+    return py::cast(y);
+}
+
 // Not in the reference (its kernels have no waits): waits for every stream this module has launched on, on the
 // current device, and raises if a kernel gave up on one of its bounded device-side waits since the last check.
 // The multiply entries do not call it themselves, because it synchronises.
@@ -195,6 +287,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
           "declare that weight-side tensors are never written by the kernel preceding a multiply in the stream");
     m.def("check_device_status", &check_device_status,
           "raise if a kernel launched by this module gave up on a bounded device-side wait (synchronises)");
+
+    m.def("_try_mult", &try_mult, "ops._mult for arguments that pass its checks: status, or -1");
+    m.def("_try_linear", &try_linear, "QuantLinear.forward for arguments that pass its checks: output, status or -1");
+    m.def("_try_row_norm", &try_row_norm, "ops.row_norm for arguments that pass its checks: output, status or -1");
 
     m.def("weight_matrix_packing", &weight_matrix_packing, "int4_sparse_pack");
 

@@ -31,6 +31,22 @@ def set_static_weights(flag: bool) -> None:
     _static_weights = bool(flag)
 
 
+_native = None
+_ROUTES = {"auto": 0, "mtx": 1, "vec": 2}
+
+
+def native():
+    """The compiled module, whose `_try_*` functions make a call with valid arguments without Python's per-argument
+    costs; False if only the C ABI library has been built (the calls then go through ctypes)."""
+    global _native
+    if _native is None:
+        import os
+        from . import load_extension
+        from ._build import torch_ext_path
+        _native = load_extension() if os.path.exists(torch_ext_path()) else False
+    return _native
+
+
 class Int4MatmulError(RuntimeError):
     """A non-zero status from the C ABI other than a bad bit width."""
 
@@ -81,6 +97,15 @@ def check_device_status(device: torch.device | None = None) -> None:
 
 
 def _mult(bits: int, route: str, outs, matrix, multiplier, scales, zeros, group_size, sparse_mask, path: int) -> None:
+    if _static_weights:
+        path |= capi.PATH_STATIC_WEIGHTS
+    mod = native()
+    if mod:
+        status = mod._try_mult(bits, _ROUTES[route], path, outs, matrix, multiplier, scales, zeros, int(group_size), sparse_mask, _workspaces)
+        if status == capi.OK:
+            return
+        if status > 0:
+            raise Int4MatmulError(status, "int4matmul")
     if bits not in (4, 3, 2):
         raise ValueError("Unsupported bit width for " +
                          ("matvec" if multiplier.dim() == 3 and multiplier.shape[1] == 1 else "matmul"))
@@ -126,7 +151,7 @@ def _mult(bits: int, route: str, outs, matrix, multiplier, scales, zeros, group_
         stream = torch.cuda.current_stream(dev)
         ws = workspace(dev, stream)
         status = lib.i4mm_quant_matmul(
-            bits, 1 if matvec else 0, path | (capi.PATH_STATIC_WEIGHTS if _static_weights else 0), outs.data_ptr(), matrix.data_ptr(),
+            bits, 1 if matvec else 0, path, outs.data_ptr(), matrix.data_ptr(),
             sparse_mask.data_ptr() if sparse else None, multiplier.data_ptr(), scales.data_ptr(), zeros.data_ptr(),
             batch * seq_len, in_size, out_size, scales.shape[0], group_size,
             ws.data_ptr(), ws.numel(), stream.cuda_stream)
@@ -198,6 +223,13 @@ def row_norm(mode: int, a: torch.Tensor, b: torch.Tensor | None = None, c: torch
     """Row-wise glue of the layer-stack runner (`i4mm_row_norm`): v / rms(v) per row with
     v = a (mode 0), a + b + c (1), a + b / rms(b) (2), a * b (3).  Inputs fp16 (rows, width), last dim contiguous.
     Mode 4 returns (2, rows, width): mode 2's result, and mode 0 of that result, from one launch."""
+    mod = native()
+    if mod:
+        y = mod._try_row_norm(mode, a, b, c)
+        if not isinstance(y, int):
+            return y
+        if y > 0:
+            raise Int4MatmulError(y, "row_norm")
     rows, width = a.shape
     for t in (a, b, c):
         if t is not None and (t.dtype != torch.float16 or t.stride(-1) != 1 or tuple(t.shape) != (rows, width)):

@@ -78,7 +78,13 @@ class QuantLinear(torch.nn.Module):
         return cls(bits, n, s, group_size, matrix, qz["scales"].to(device), qz["zeros"].to(device), mask)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        from . import ops
+        from . import capi, ops
+        mod = ops.native()
+        if mod:
+            y = mod._try_linear(self.bits, capi.PATH_STATIC_WEIGHTS if ops._static_weights else capi.PATH_AUTO, x, self.in_features,
+                                self.out_features, self.matrix, self.scales, self.zeros, self.group_size, self.mask, ops._workspaces)
+            if not isinstance(y, int):
+                return y
         lead = x.shape[:-1]
         x3 = x.reshape(1, -1, self.in_features).to(torch.float16).contiguous()
         out = torch.empty((1, x3.shape[1], self.out_features), dtype=torch.float16, device=x.device)

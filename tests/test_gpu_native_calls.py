@@ -1,0 +1,94 @@
+"""The compiled fast path of the Python entries (ops, QuantLinear) against the same calls through ctypes: equal results for
+everything both accept, and the same exceptions for what the entries refuse."""
+import pytest
+import torch
+
+from int4matmul_kernels_b200 import ops, packing
+from int4matmul_kernels_b200.quantize import QuantLinear
+
+pytestmark = pytest.mark.gpu
+
+
+def both(monkeypatch, call):
+    """call() through the compiled module and through ctypes."""
+    assert ops.native()
+    fast = call()
+    with monkeypatch.context() as m:
+        m.setattr(ops, "_native", False)
+        slow = call()
+    return fast, slow
+
+
+def weights(bits, n, s, g, sparse=False):
+    w = packing.synthetic_weights(bits, n, s, g, sparse=sparse, seed=bits)
+    return w["matrix"], w["scales"], w["zeros"], w["mask"]
+
+
+@pytest.mark.parametrize("bits,sparse", [(4, False), (3, False), (2, False), (4, True)])
+@pytest.mark.parametrize("shape", [(256,), (1, 256), (5, 256), (2, 3, 256), (2, 1, 70, 256)])
+def test_quant_linear_shapes(monkeypatch, bits, sparse, shape):
+    m, s, z, k = weights(bits, 256, 192, 128, sparse)
+    layer = QuantLinear(bits, 256, 192, 128, m, s, z, k)
+    x = torch.randn(shape, generator=torch.Generator().manual_seed(1)).half().cuda()
+    for inp in (x, x.float(), torch.stack([x, x], dim=-1)[..., 0]):            # as it is, converted, strided
+        fast, slow = both(monkeypatch, lambda: layer(inp))
+        assert fast.shape == slow.shape == (*shape[:-1], 192) and torch.equal(fast, slow)
+
+
+def test_static_weights_flag_and_second_stream(monkeypatch):
+    m, s, z, _ = weights(4, 512, 128, 64)
+    x = torch.randn(1, 3, 512, generator=torch.Generator().manual_seed(2)).half().cuda()
+
+    def call():
+        out = torch.empty((1, 3, 128), dtype=torch.float16, device="cuda")
+        ops.quant_int4_linear_mult_mtx(out, m, x, s, z, 64, None)
+        return out
+    want, _ = both(monkeypatch, call)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    ops.set_static_weights(True)
+    try:
+        with torch.cuda.stream(side):
+            got = [call() for _ in range(3)]
+    finally:
+        ops.set_static_weights(False)
+    side.synchronize()
+    assert all(torch.equal(want, g) for g in got)
+
+
+@pytest.mark.parametrize("mode,n_in", [(0, 1), (1, 3), (2, 2), (3, 2), (4, 2)])
+def test_row_norm_operands(monkeypatch, mode, n_in):
+    big = torch.randn(4, 3 * 320, generator=torch.Generator().manual_seed(3)).half().cuda()
+    for args in ([big[:, i * 320:(i + 1) * 320] for i in range(n_in)], [big[:, :320].contiguous()] * n_in):
+        fast, slow = both(monkeypatch, lambda: ops.row_norm(mode, *args))
+        assert torch.equal(fast, slow)
+    for bad in (big[:, :320].float(), big[:, ::3], big[:2, :320]):
+        with pytest.raises((ValueError, ops.Int4MatmulError)):
+            ops.row_norm(2, big[:, :320], bad)
+
+
+def test_refusals_are_the_same(monkeypatch):
+    m, s, z, _ = weights(4, 256, 128, 128)
+    x = torch.zeros((1, 2, 256), dtype=torch.float16, device="cuda")
+    out = torch.zeros((1, 2, 128), dtype=torch.float16, device="cuda")
+    cases = [
+        lambda: ops.quant_matmul(5, out, m, x, s, z, 128, None),
+        lambda: ops.quant_matmul(4, out, m, x.float(), s, z, 128, None),
+        lambda: ops.quant_matmul(4, out, m, x.cpu(), s, z, 128, None),
+        lambda: ops.quant_matmul(4, out[..., ::2], m, x, s, z, 128, None),
+        lambda: ops.quant_matmul(4, out, m, x, s[:, :64].contiguous(), z, 128, None),
+        lambda: ops.quant_matmul(4, out, m, x, s, z, 96, None),
+        lambda: ops.quant_matmul(4, out, m, x, s, z, 64, None),                  # too few groups for this group size
+        lambda: ops.quant_matmul(3, out, m, x, s, z, 128, None),
+        lambda: ops.quant_matmul(2, out, m, x, s, z, 128, m),
+        lambda: ops.quant_int4_linear_mult_vec(out, m, x, s, z, 128, None),
+    ]
+    for call in cases:
+        seen = []
+        for native in (ops.native(), False):
+            with monkeypatch.context() as mp:
+                mp.setattr(ops, "_native", native)
+                with pytest.raises(Exception) as e:
+                    call()
+                seen.append((type(e.value), str(e.value)))
+        assert seen[0] == seen[1]
