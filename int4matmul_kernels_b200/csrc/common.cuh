@@ -73,6 +73,18 @@ struct GroupDiv {
     }
 };
 
+// ---- equal contiguous ranges of T work items over G workers ----------------------------------------------------
+// Non-negative quotient; 64-bit division is a ~500-cycle subroutine on the GPU, so the 32-bit one is used whenever the
+// operands allow it (practically always: unit counts are far below 2^32).
+__device__ __forceinline__ long long div_nn(long long a, long long b) {
+    if (((unsigned long long)a | (unsigned long long)b) >> 32) return a / b;
+    return (long long)((uint32_t)a / (uint32_t)b);
+}
+__device__ __forceinline__ long long range_lo(long long T, long long G, long long b) { return div_nn(T * b, G); }
+__device__ __forceinline__ int range_owner(long long T, long long G, long long t) {
+    return (int)(div_nn((t + 1) * G + T - 1, T) - 1);
+}
+
 // ---- where results go ----------------------------------------------------------------------------------------------
 // The ordinary entry writes one (rows, S) array.  The gathering entry writes this rank's S columns into the same place
 // of up to 8 arrays (its own and its peers' gathered (rows, ld) buffers, reached through peer-mapped pointers with

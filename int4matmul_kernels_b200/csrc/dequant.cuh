@@ -1,0 +1,100 @@
+// Dequantisation arithmetic shared by the kernels: packed fields planted into fp16 mantissas, then the reference's two
+// fp16 roundings (matmul.cuh:115-125) or, per weight, either coding.
+#pragma once
+
+#include "common.cuh"
+
+namespace i4mm {
+
+enum : int { MODE_FAST = 0, MODE_GENERAL = 1, MODE_SLOW = 2 };
+
+// (mask & a) | (~mask & b)
+__device__ __forceinline__ uint32_t bit_select(uint32_t mask, uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("lop3.b32 %0, %1, %2, %3, 0xCA;" : "=r"(d) : "r"(mask), "r"(a), "r"(b));
+    return d;
+}
+__device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
+
+// ---- per-column constants ---------------------------------------------------------------------------------
+struct ColK {
+    uint32_t s2, z2;
+    uint32_t zb;       // sparse fast mode: the integer zero-point (up to 127) replicated into 4 bytes
+};
+
+// v = (1024 + q_lo * 2^a, 1024 + q_hi * 2^b) -> the two fp16 weights.  mul / base undo the two shifts exactly.
+template <int BITS, int MODE>
+__device__ __forceinline__ uint32_t finish(uint32_t v, uint32_t mul, uint32_t base, uint32_t off, const ColK& c) {
+    if (MODE == MODE_FAST) return hmul2_u(hfma2_u(v, mul, off), c.s2);         // off = base - zero
+    const uint32_t q = hfma2_u(v, mul, base);                                  // exact integers
+    if (MODE == MODE_GENERAL) return hmul2_u(hsub2_u(q, c.z2), c.s2);
+    const __half2 qh = u32_as_h2(q);
+    const __half s = __ushort_as_half((unsigned short)(c.s2 & 0xFFFFu));
+    const __half z = __ushort_as_half((unsigned short)(c.z2 & 0xFFFFu));
+    const __half lo = dequant_dynamic<BITS>(__half2uint_rz(__low2half(qh)), s, z);
+    const __half hi = dequant_dynamic<BITS>(__half2uint_rz(__high2half(qh)), s, z);
+    return h2_as_u32(__halves2half2(lo, hi));
+}
+
+// half2 constants (hi << 16 | lo)
+constexpr uint32_t MUL_1_16 = 0x2C003C00u, BASE_1_16 = 0xD400E400u;      // (x1, x16): int4 nibble pairs
+constexpr uint32_t MUL_1_4 = 0x34003C00u, BASE_1_4 = 0xDC00E400u;        // (x1, x4):  int2 crumbs 0, 1
+constexpr uint32_t MUL_16_64 = 0x24002C00u, BASE_16_64 = 0xCC00D400u;    // (x16, x64): int2 crumbs 2, 3
+constexpr uint32_t MUL_1_8 = 0x30003C00u, BASE_1_8 = 0xD800E400u;        // (x1, x8):  int3 field pairs
+constexpr uint32_t MUL_1_1 = 0x3C003C00u, BASE_1_1 = 0xE400E400u;        // (x1, x1): sparse int4 through bytes
+
+// ---- 16:32 sparse: the next 8 positions of a 32-block ---------------------------------------------------------------
+// The next 8 kept nibbles are spread over the bytes of a register pair (even nibbles, odd nibbles); two PRMTs put them
+// at their positions.  The selectors of both PRMTs are one 32-bit word of a 256-entry table indexed by the byte of the
+// keep-mask (nibble j of the word belongs to position j).  A dropped position selects 8, for which PRMT replicates the
+// sign of a byte below 128: it yields 0x00, also when the same selector is applied to a constant of 0x7F bytes, which
+// so becomes the mask of the kept positions.  A 1 KB table: the same look-up in a table of 16-byte entries (selectors, masks and
+// popcount) takes ~10 shared-memory wavefronts per warp instead of ~3.5, because random entries of four banks collide.
+constexpr int kSparseLutEntries = 256;
+__device__ __forceinline__ uint32_t sparse_selectors(int keep) {
+    uint32_t sel = 0, rank = 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        uint32_t s = 8;
+        if (keep & (1 << j)) {
+            s = (rank >> 1) + 4u * (rank & 1u);
+            ++rank;
+        }
+        sel |= s << (4 * j);
+    }
+    return sel;
+}
+
+// A <- the four pairs of byte `step` (0..3, in this order) of keep-mask m; (hi : lo) is the stream of kept nibbles.
+template <int MODE>
+__device__ __forceinline__ void sparse_expand(uint32_t& lo, uint32_t& hi, uint32_t m, int step, const uint32_t* lut, const ColK& c,
+                                              uint32_t (&A)[4]) {
+    const uint32_t byte4 = (step == 0 ? m << 2 : m >> (8 * step - 2)) & 0x3FCu;          // 4 x the mask byte: table offset
+    const uint32_t sel = *reinterpret_cast<const uint32_t*>(reinterpret_cast<const char*>(lut) + byte4);
+    const uint32_t even = lo & 0x0F0F0F0Fu, odd = (lo >> 4) & 0x0F0F0F0Fu;
+    const uint32_t off = hsub2_u(BASE_1_1, c.z2);
+#pragma unroll
+    for (int q4 = 0; q4 < 2; ++q4) {
+        const uint32_t s = q4 ? sel >> 16 : sel;                                         // (PRMT reads the low 16 bits)
+        uint32_t d = prmt(even, odd, s);
+        const uint32_t keep = prmt(0x7F7F7F7Fu, 0x7F7F7F7Fu, s);
+        // fast mode: a dropped position gets the (integer) zero-point as its nibble, so it decodes to +0
+        if (MODE == MODE_FAST) d = bit_select(keep, d, c.zb);
+        A[2 * q4] = finish<4, MODE>(prmt(d, 0x64646464u, 0x5140), MUL_1_1, BASE_1_1, off, c);
+        A[2 * q4 + 1] = finish<4, MODE>(prmt(d, 0x64646464u, 0x7362), MUL_1_1, BASE_1_1, off, c);
+        if (MODE != MODE_FAST) {                                                         // exact zeros at dropped positions
+            const uint32_t k = keep * 2u + (keep & 0x01010101u);                         // 0x7F -> 0xFF
+            A[2 * q4] &= prmt(k, k, 0x1100);
+            A[2 * q4 + 1] &= prmt(k, k, 0x3322);
+        }
+    }
+    const uint32_t used = 4u * (uint32_t)__popc(byte4);                                  // bits of the stream, up to 32
+    lo = __funnelshift_rc(lo, hi, used);
+    hi = __funnelshift_rc(hi, 0u, used);
+}
+
+}  // namespace i4mm

@@ -34,14 +34,12 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "dequant.cuh"
 #include "ptx.cuh"
 
 namespace i4mm {
 
 namespace {
-
-
-enum : int { MODE_FAST = 0, MODE_GENERAL = 1, MODE_SLOW = 2 };
 
 
 struct UmmaParams {
@@ -64,64 +62,6 @@ struct UmmaParams {
     GroupDiv gdiv;
 };
 
-// (mask & a) | (~mask & b)
-__device__ __forceinline__ uint32_t bit_select(uint32_t mask, uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("lop3.b32 %0, %1, %2, %3, 0xCA;" : "=r"(d) : "r"(mask), "r"(a), "r"(b));
-    return d;
-}
-__device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t b, uint32_t c) {
-    uint32_t d;
-    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
-    return d;
-}
-
-// ---- per-column constants ---------------------------------------------------------------------------------
-struct ColK {
-    uint32_t s2, z2;
-    uint32_t zb;       // sparse fast mode: the integer zero-point replicated into 4 bytes
-};
-
-// v = (1024 + q_lo * 2^a, 1024 + q_hi * 2^b) -> the two fp16 weights.  mul / base undo the two shifts exactly.
-template <int BITS, int MODE>
-__device__ __forceinline__ uint32_t finish(uint32_t v, uint32_t mul, uint32_t base, uint32_t off, const ColK& c) {
-    if (MODE == MODE_FAST) return hmul2_u(hfma2_u(v, mul, off), c.s2);         // off = base - zero
-    const uint32_t q = hfma2_u(v, mul, base);                                  // exact integers
-    if (MODE == MODE_GENERAL) return hmul2_u(hsub2_u(q, c.z2), c.s2);
-    const __half2 qh = u32_as_h2(q);
-    const __half s = __ushort_as_half((unsigned short)(c.s2 & 0xFFFFu));
-    const __half z = __ushort_as_half((unsigned short)(c.z2 & 0xFFFFu));
-    const __half lo = dequant_dynamic<BITS>(__half2uint_rz(__low2half(qh)), s, z);
-    const __half hi = dequant_dynamic<BITS>(__half2uint_rz(__high2half(qh)), s, z);
-    return h2_as_u32(__halves2half2(lo, hi));
-}
-
-// half2 constants (hi << 16 | lo)
-constexpr uint32_t MUL_1_16 = 0x2C003C00u, BASE_1_16 = 0xD400E400u;      // (x1, x16): int4 nibble pairs
-constexpr uint32_t MUL_1_4 = 0x34003C00u, BASE_1_4 = 0xDC00E400u;        // (x1, x4):  int2 crumbs 0, 1
-constexpr uint32_t MUL_16_64 = 0x24002C00u, BASE_16_64 = 0xCC00D400u;    // (x16, x64): int2 crumbs 2, 3
-constexpr uint32_t MUL_1_8 = 0x30003C00u, BASE_1_8 = 0xD800E400u;        // (x1, x8):  int3 field pairs
-constexpr uint32_t MUL_1_1 = 0x3C003C00u, BASE_1_1 = 0xE400E400u;        // (x1, x1): sparse int4 through bytes
-
-// 256-entry table for the sparse expansion, indexed by one byte of the keep-mask (8 positions; see the sparse decode).
-// The next 8 kept nibbles are spread over the 8 bytes of a register pair (even nibbles, odd nibbles); for position p
-// with rank r among the kept ones the PRMT selector names byte r / 2 of the even or (4 +) of the odd register.
-//   x = selector of positions 0..3 | (4 * popcount) << 16 (PRMT reads only the low 16 bits of its selector)
-//   y = selector of positions 4..7      z, w = 0xFF in the bytes of the kept positions 0..3, 4..7
-constexpr int kSparseLutEntries = 256;
-__device__ __forceinline__ uint4 sparse_lut_entry(int mb) {
-    uint32_t sel[2] = {0, 0}, keep[2] = {0, 0}, rank = 0;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        if (mb & (1 << j)) {
-            sel[j >> 2] |= ((rank >> 1) + 4u * (rank & 1u)) << (4 * (j & 3));
-            keep[j >> 2] |= 0xFFu << (8 * (j & 3));
-            ++rank;
-        }
-    }
-    return make_uint4(sel[0] | ((4 * rank) << 16), sel[1], keep[0], keep[1]);
-}
-
 // ---- formats: one 64-k part of one column -> 32 registers of fp16 pairs -----------------------------------------
 // The pairs are in natural k order, except for dense int4 with PERM: there register 4r + j of packed word r holds
 // (k_j, k_{j+4}) of the word's eight k, which needs no byte shuffles; the activation tile is permuted to match
@@ -134,7 +74,7 @@ struct UFormat<4, false, PERM> {
     static constexpr int WROWS = 8, MROWS = 0;       // packed rows / mask rows per 64-k part
     static constexpr bool kPermutedK = PERM;
     template <int MODE>
-    __device__ static __forceinline__ void decode(uint32_t wbase, uint32_t, const ColK& c, uint32_t (&A)[32], const uint4*) {
+    __device__ static __forceinline__ void decode(uint32_t wbase, uint32_t, const ColK& c, uint32_t (&A)[32], const uint32_t*) {
         if (PERM) {
             // nibbles j and j + 4 of a word sit at the same offset of its two 16-bit halves: one LOP3 per pair plants both
             // into the mantissas of (1024, 1024); the odd nibbles come out multiplied by 16
@@ -168,7 +108,7 @@ struct UFormat<2, false, PERM> {
     static constexpr int WROWS = 4, MROWS = 0;
     static constexpr bool kPermutedK = false;
     template <int MODE>
-    __device__ static __forceinline__ void decode(uint32_t wbase, uint32_t, const ColK& c, uint32_t (&A)[32], const uint4*) {
+    __device__ static __forceinline__ void decode(uint32_t wbase, uint32_t, const ColK& c, uint32_t (&A)[32], const uint32_t*) {
         const uint32_t offa = hsub2_u(BASE_1_4, c.z2), offb = hsub2_u(BASE_16_64, c.z2);
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
@@ -191,7 +131,7 @@ struct UFormat<3, false, PERM> {
     static constexpr int WROWS = 6, MROWS = 0;
     static constexpr bool kPermutedK = false;
     template <int MODE>
-    __device__ static __forceinline__ void decode(uint32_t wbase, uint32_t, const ColK& c, uint32_t (&A)[32], const uint4*) {
+    __device__ static __forceinline__ void decode(uint32_t wbase, uint32_t, const ColK& c, uint32_t (&A)[32], const uint32_t*) {
         const uint32_t off = hsub2_u(BASE_1_8, c.z2);
 #pragma unroll
         for (int blk = 0; blk < 2; ++blk) {
@@ -222,36 +162,18 @@ struct UFormat<4, true, PERM> {
     static constexpr int WROWS = 4, MROWS = 2;
     static constexpr bool kPermutedK = false;
     template <int MODE>
-    __device__ static __forceinline__ void decode(uint32_t wbase, uint32_t mbase, const ColK& c, uint32_t (&A)[32], const uint4* lut) {
-        const uint32_t off = hsub2_u(BASE_1_1, c.z2);
+    __device__ static __forceinline__ void decode(uint32_t wbase, uint32_t mbase, const ColK& c, uint32_t (&A)[32], const uint32_t* lut) {
 #pragma unroll
         for (int blk = 0; blk < 2; ++blk) {
             // a 32-block of this column: the 64-bit word of its 16 kept nibbles (in increasing k) and its keep-mask
             uint32_t lo = ptx::lds32(wbase + (2 * blk) * 512), hi = ptx::lds32(wbase + (2 * blk + 1) * 512);
             const uint32_t m = ptx::lds32(mbase + blk * 512);
 #pragma unroll
-            for (int byte = 0; byte < 4; ++byte) {               // 8 positions per step
-                const uint4 e = lut[(m >> (8 * byte)) & 0xFFu];
-                const uint32_t even = lo & 0x0F0F0F0Fu;          // kept nibbles 0, 2, 4, 6 of the next eight, one per byte
-                const uint32_t odd = (lo >> 4) & 0x0F0F0F0Fu;    // kept nibbles 1, 3, 5, 7
-                uint32_t d[2] = {prmt(even, odd, e.x), prmt(even, odd, e.y)};   // positions 0..3, 4..7 as bytes
-                const uint32_t keep[2] = {e.z, e.w};
+            for (int step = 0; step < 4; ++step) {               // 8 positions each
+                uint32_t pairs[4];
+                sparse_expand<MODE>(lo, hi, m, step, lut, c, pairs);
 #pragma unroll
-                for (int q4 = 0; q4 < 2; ++q4) {
-                    // fast mode: a dropped position gets the (integer) zero-point as its nibble, so it decodes to +0
-                    if (MODE == MODE_FAST) d[q4] = bit_select(keep[q4], d[q4], c.zb);
-                    uint32_t a = finish<4, MODE>(prmt(d[q4], 0x64646464u, 0x5140), MUL_1_1, BASE_1_1, off, c);
-                    uint32_t b = finish<4, MODE>(prmt(d[q4], 0x64646464u, 0x7362), MUL_1_1, BASE_1_1, off, c);
-                    if (MODE != MODE_FAST) {                     // exact zeros at dropped positions
-                        a &= prmt(keep[q4], keep[q4], 0x1100);
-                        b &= prmt(keep[q4], keep[q4], 0x3322);
-                    }
-                    A[16 * blk + 4 * byte + 2 * q4] = a;
-                    A[16 * blk + 4 * byte + 2 * q4 + 1] = b;
-                }
-                const uint32_t sh = e.x >> 16;                   // 4 bits per kept position, up to 32
-                lo = __funnelshift_rc(lo, hi, sh);
-                hi = __funnelshift_rc(hi, 0u, sh);
+                for (int i = 0; i < 4; ++i) A[16 * blk + 4 * step + i] = pairs[i];
             }
         }
     }
@@ -336,17 +258,6 @@ struct Barriers {
     unsigned long long d_full, d_empty;
 };
 
-// Non-negative quotient; 64-bit division is a ~500-cycle subroutine on the GPU, so the 32-bit one is used whenever the
-// operands allow it (practically always: unit counts are far below 2^32).
-__device__ __forceinline__ long long div_nn(long long a, long long b) {
-    if (((unsigned long long)a | (unsigned long long)b) >> 32) return a / b;
-    return (long long)((uint32_t)a / (uint32_t)b);
-}
-__device__ __forceinline__ long long range_lo(long long T, long long G, long long b) { return div_nn(T * b, G); }
-__device__ __forceinline__ int range_owner(long long T, long long G, long long t) {
-    return (int)(div_nn((t + 1) * G + T - 1, T) - 1);
-}
-
 struct TensorMaps {
     CUtensorMap x;   // fp16 (rows, N):        box 64 k x NT rows, 128-byte swizzle; weight-streaming shapes: seen as
                      //                        (N / 64, rows, 64) with box kHalves x NT x 64, one copy per unit
@@ -381,7 +292,7 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const UmmaParams p, const __h
     constexpr int kABStages = ABStages<NT, PAIR>::value;
     extern __shared__ __align__(1024) unsigned char smem[];      // [B ring (1024-aligned tiles)][W ring]
     __shared__ __align__(8) Barriers bars;
-    __shared__ uint4 lut[SPARSE ? kSparseLutEntries : 1];
+    __shared__ uint32_t lut[SPARSE ? kSparseLutEntries : 1];
     __shared__ uint32_t tmem_base_smem;
     __shared__ volatile int s_abort;     // set by a warp that gives up on the accumulator (the MMA warp before it releases the epilogue
                                          // warps for the last time; an epilogue warp before its group's next named barrier)
@@ -426,7 +337,7 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const UmmaParams p, const __h
             }
             ptx::fence_mbar_init();
         }
-        if (SPARSE && warp < 8) lut[warp * 32 + lane] = sparse_lut_entry(warp * 32 + lane);   // (warps 0..7 are dequant warps in every configuration)
+        if (SPARSE && warp < 8) lut[warp * 32 + lane] = sparse_selectors(warp * 32 + lane);   // (warps 0..7 are dequant warps in every configuration)
         if (warp == kMma) {
             if (PAIR) {
                 ptx::tmem_alloc_pair(ptx::smem_u32(&tmem_base_smem), C::kTmemCols);
@@ -1013,10 +924,10 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const UmmaParams p, const __h
                         c.z2 = prmt(zz, zz, 0x1010);
                         c.zb = 0;
                     };
-                    // fast mode needs: scale sign clear, zero-point an integer in [0, 512] ([0, 255] for the sparse format)
+                    // fast mode needs: scale sign clear, zero-point an integer in [0, 512] ([0, 127] for the sparse format)
                     auto not_fast_bits = [&](const ColK& c) -> uint32_t {
                         const uint32_t zr = hadd2_u(hadd2_u(c.z2, kMagic1024), H2_N1024);
-                        constexpr uint32_t kAdd = SPARSE ? 0x2407u : 0x1FFFu;
+                        constexpr uint32_t kAdd = SPARSE ? 0x280Fu : 0x1FFFu;
                         const uint32_t zlo = c.z2 & 0xFFFFu;
                         return ((zlo | ((zlo & 0x7FFFu) + kAdd) | c.s2) & 0x8000u) | (zr ^ c.z2);
                     };
