@@ -12,7 +12,7 @@ void count_launch(int n) { g_launches.fetch_add((unsigned long long)n); }
 static thread_local int g_last_cuda_error = 0;        // what i4mm_last_cuda_error returns; every entry point records here
 void record_cuda_error(int e) { g_last_cuda_error = e; }
 int umma_last_shape();
-void umma_clear_last_shape();
+void set_last_shape(int shape);
 cudaError_t stream_launch(int bits, bool sparse, StreamParams p, int total_rows, int ctas, cudaStream_t stream);
 cudaError_t sparse_pack_launch(void* wt_out, void* msk_out, const void* wt_in, const void* msk_in,
                                int S, int N, void* violations, cudaStream_t stream);
@@ -21,6 +21,8 @@ cudaError_t rownorm_launch(int mode, void* y, const void* a, const void* b, cons
                            long long sa, long long sb, long long sc, cudaStream_t stream);
 int umma_launch(int bits, bool sparse, const StreamParams& p, int total_rows, int n_groups, int group_size, int cta_pairs,
                 int force_nt, int overlap, cudaStream_t stream, cudaError_t* cuda_err);
+bool rows_supported(int rows, int N, int S);
+cudaError_t rows_launch(int bits, bool sparse, const StreamParams& p, int overlap, cudaStream_t stream);
 bool umma_supported(int bits, bool sparse, int total_rows, int N, int S);
 }  // namespace i4mm
 
@@ -137,6 +139,12 @@ int multiply(int bits, int accumulate, int path, void* out, const i4mm::OutMap* 
     p.status = (int*)((char*)workspace + kStatusOffset);
 
     cudaStream_t st = (cudaStream_t)stream;
+    if (path == 0 && i4mm::rows_supported((int)rows, (int)N, (int)S)) {
+        i4mm::set_last_shape(16);
+        p.rows = (int)rows;
+        const cudaError_t e = i4mm::rows_launch(bits, sparse, p, overlap, st);
+        return e == cudaSuccess ? I4MM_OK : fail_cuda(e);
+    }
     bool use_umma = false;
     if (path >= 2 || gather) {
         if (!i4mm::umma_supported(bits, sparse, (int)rows, (int)N, (int)S)) return I4MM_ERR_UNSUPPORTED;
@@ -150,7 +158,7 @@ int multiply(int bits, int accumulate, int path, void* out, const i4mm::OutMap* 
         if (rc == I4MM_ERR_LAUNCH) return fail_cuda(ce);
         return rc;
     }
-    i4mm::umma_clear_last_shape();
+    i4mm::set_last_shape(0);
     const cudaError_t e = i4mm::stream_launch(bits, sparse, p, (int)rows, kMaxStreamCtas, st);
     if (e != cudaSuccess) return fail_cuda(e);
     return I4MM_OK;

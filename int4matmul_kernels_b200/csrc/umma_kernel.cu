@@ -1409,7 +1409,7 @@ int launch_fmt(UmmaParams& p, const __half* x, int n_groups, int pair_mode, int 
 }  // namespace
 
 int umma_last_shape() { return g_last_shape; }
-void umma_clear_last_shape() { g_last_shape = 0; }
+void set_last_shape(int shape) { g_last_shape = shape; }
 
 bool umma_supported(int bits, bool sparse, int total_rows, int N, int S) {
     (void)bits; (void)sparse; (void)S;
