@@ -77,19 +77,19 @@ size_t i4mm_workspace_bytes(void);
  *                        caller's `outs` (matvec_kernel.cu:351, 263, 381-382)
  *   accumulate == 0  ->  out is overwritten, as the reference's matmul route does (matmul_kernel.cu:299-332)
  *
- * rows = B*M may be any value >= 0 (rows == 0 returns I4MM_OK without a launch).  The entry picks the
- * weight-streaming kernel for few rows and the tcgen05 tensor-core kernel for many; `path` forces one:
- *   0 = automatic (the tcgen05 kernel when the driver's tensor-map encoder is found), 1 = streaming (mma.sync,
+ * rows = B*M may be any value >= 0 (rows == 0 returns I4MM_OK without a launch).  The entry picks the few-row kernel
+ * for up to 8 rows of a small matrix and the tcgen05 tensor-core kernel for everything else; `path` forces one:
+ *   0 = automatic (the streaming kernel where the driver's tensor-map encoder is not found), 1 = streaming (mma.sync,
  *   split-K over the whole GPU), 2 = tcgen05 / TMEM pipeline (128 rows or more run as CTA pairs, two SMs per
  *   MMA), 3 = tcgen05 with single CTAs only.
  *   With path 2 or 3, `path | (T << 8)` also fixes the rows per tile (the MMA's N) to T in {16, 32, 64, 128, 160, 192,
  *   224, 256} instead of choosing it by shape (T >= 128 with path 2 runs as CTA pairs; T <= 64 needs rows <= T):
  *   for tests and tuning, results do not depend on it beyond fp32 summation order.
  *   `path | I4MM_PATH_STATIC_WEIGHTS` is the caller's promise that matrix, mask, scales and zeros are not written by
- *   the kernel that precedes this call in the stream (weights of a loaded model never are).  The tcgen05 kernel is then
- *   launched so that its set-up and its first weight copies overlap the tail of that kernel (programmatic dependent
- *   launch); it still waits for that kernel before it reads x, reads or writes out, or touches the workspace.  Without
- *   the flag every launch is ordered after the whole preceding kernel, as the reference's launches are.
+ *   the kernel that precedes this call in the stream (weights of a loaded model never are).  Launches may begin while
+ *   that kernel is still finishing (programmatic dependent launch); with the promise the first weight copies go out
+ *   then, while x, out and the workspace are touched only once that kernel is complete.  Without it nothing at all is
+ *   read before, as with the reference's launches.
  */
 #define I4MM_PATH_STATIC_WEIGHTS 0x100000
 int i4mm_quant_matmul(int bits, int accumulate, int path,

@@ -24,9 +24,10 @@ _static_weights = False
 def set_static_weights(flag: bool) -> None:
     """Declare that the weight-side tensors (matrix, mask, scales, zeros) passed to the multiply entries are never
     written by the kernel that precedes the call in the stream, as is the case for the weights of a loaded model.
-    Launches may then begin (set-up, first weight copies) while that kernel is still finishing; activations, outputs
-    and scratch are still only touched once it is complete.  Off by default: the reference orders every launch after
-    the whole preceding kernel, and a caller that rewrites weights right before a call relies on that."""
+    Launches begin while that kernel is still finishing; with the promise their first weight copies go out then, while
+    activations, outputs and scratch are still only touched once it is complete.  Off by default (nothing is read early):
+    the reference orders every launch after the whole preceding kernel, and a caller that rewrites weights right before a
+    call relies on that."""
     global _static_weights
     _static_weights = bool(flag)
 
