@@ -21,7 +21,7 @@ cudaError_t rownorm_launch(int mode, void* y, const void* a, const void* b, cons
                            long long sa, long long sb, long long sc, cudaStream_t stream);
 int umma_launch(int bits, bool sparse, const StreamParams& p, int total_rows, int n_groups, int group_size, int cta_pairs,
                 int force_nt, int overlap, cudaStream_t stream, cudaError_t* cuda_err);
-bool rows_supported(int rows, int N, int S);
+bool rows_supported(int bits, bool accumulate, int rows, int N, int S);
 cudaError_t rows_launch(int bits, bool sparse, const StreamParams& p, int overlap, cudaStream_t stream);
 bool umma_supported(int bits, bool sparse, int total_rows, int N, int S);
 }  // namespace i4mm
@@ -139,7 +139,7 @@ int multiply(int bits, int accumulate, int path, void* out, const i4mm::OutMap* 
     p.status = (int*)((char*)workspace + kStatusOffset);
 
     cudaStream_t st = (cudaStream_t)stream;
-    if (path == 0 && i4mm::rows_supported((int)rows, (int)N, (int)S)) {
+    if (path == 0 && i4mm::rows_supported(bits, accumulate != 0, (int)rows, (int)N, (int)S)) {
         i4mm::set_last_shape(16);
         p.rows = (int)rows;
         const cudaError_t e = i4mm::rows_launch(bits, sparse, p, overlap, st);

@@ -561,17 +561,29 @@ cudaError_t rows_launch_fmt(const RowsParams& p, int sms, int dev, cudaStream_t 
 
 }  // namespace
 
-// Which calls take this kernel by default.  Its fixed cost per launch is about half of the tcgen05 kernel's, its rate is
-// lower, so the line is drawn by the number of weights.  One pass with its zero-fill, us, back to back, tcgen05 kernel ->
-// this one, one row: int4 2048^2 12.3 -> 7.6, 1024 x 8192 12.3 -> 8.2, 5120^2 14.4 -> 12.4, 5120 x 8192 16.4 -> 14.7,
-// 8192^2 18.6 -> 20.2, 16384^2 42.5 -> 53.6; int3 5120^2 14.5 -> 12.4, 8192^2 20.5 -> 20.6; int2 5120^2 14.4 -> 10.3,
-// 8192^2 18.5 -> 18.5; 16:32 5120^2 16.5 -> 14.4, 8192 x 5120 20.5 -> 20.5.  More rows cost the lanes more activation
-// copies and reads: int4 5120^2 with 4 rows 12.1 -> 12.6, with 8 rows 14.9 -> 15.1; 16:32 with 8 rows 16.5 -> 17.5.
+// Which calls take this kernel by default; every figure is us on one B200, tcgen05 kernel -> this one.
+// Alone, its fixed cost per launch is about half of the other's and its rate is lower: adding one row to a zero-filled
+// output, int4 2048^2 12.4 -> 8.2, 5120^2 14.6 -> 12.3, 5120 x 8192 16.5 -> 15.2, but 16384^2 42.5 -> 53.6; int3 5120^2
+// 15.5 -> 12.3; int2 15.0 -> 11.1; 16:32 17.0 -> 14.4.  So the adding route's line is the number of weights.  From more than 2
+// column tiles per SM on, K cannot be cut any more and SMs are left with uneven numbers of tiles: 1024 x 30720 16.5 -> 14.3,
+// 1024 x 37888 14.4 -> 14.4, 1024 x 40960 18.4 -> 19.4 (16:32 21.9 -> 25.2), 16:32 2304 x 20480 20.6 -> 22.5.
+// A call that overwrites stands between others in a model's layer, and there a change of kernel from one matrix to the next costs
+// 2..5 us (the next kernel's launch no longer overlaps).  min(N, S) is the layer's width for its every matrix, so a bound on it keeps
+// a layer on one kernel: four matrices and their row norms, one row, int4 5120 wide with only the 5120^2 one on this kernel
+// 86.5 -> 91.5 and 4096 (11008) 72.3 -> 73.8, but 3072 (5120), all four on it, 56.5 -> 49.9 and 2048 (5632) 53.3 -> 44.2.  int2 is the
+// exception (its decode is cheapest here): 5120 83.0 -> 84.5 but 4096 (11008) 69.6 -> 65.1.  With 4 rows int4 4096 79.1 -> 81.6, 2048
+// 58.7 -> 50.4; with 8 rows 3072 69.2 -> 73.7, 2048 67.0 -> 61.3 (5..8 rows have larger stages and fewer of them).
+// Very long columns: the last part adds the sums of hundreds of parts one after the other, 4 rows 131072 x 64 77 -> 62 but 262144 x 64
+// 79 -> 120, 8 rows 65536 x 64 98 -> 63 but 131072 x 64 99 -> 121.
 // (The bounds also keep step and tile numbers far inside 32 bits.)
-constexpr long long kMostWeightsOneRow = 48ll << 20, kMostWeightsFewRows = 16ll << 20;
+constexpr long long kMi = 1ll << 20;
 
-bool rows_supported(int rows, int N, int S) {
-    return rows >= 1 && rows <= kMaxRows && (long long)N * S <= (rows == 1 ? kMostWeightsOneRow : kMostWeightsFewRows);
+bool rows_supported(int bits, bool accumulate, int rows, int N, int S) {
+    const long long weights = (long long)N * S;
+    const int width = N < S ? N : S;
+    if (rows == 1) return weights <= (S > 148 * 2 * kTileCols ? 36 : 48) * kMi && (accumulate || bits == 2 || width <= 3072);
+    if (rows < 1 || rows > kMaxRows || weights > 16 * kMi) return false;
+    return rows <= 4 ? N <= 131072 && (bits == 2 || width <= 3072) : N <= 65536 && width <= 2560;
 }
 
 cudaError_t rows_launch(int bits, bool sparse, const StreamParams& sp, int overlap, cudaStream_t stream) {

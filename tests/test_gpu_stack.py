@@ -73,6 +73,21 @@ def test_row_norm_launched_behind_a_multiply_reads_its_finished_output(rows):
     ops.check_device_status()
 
 
+@pytest.mark.parametrize("seed", [1, 2])
+def test_one_row_through_13b_layers_takes_one_kernel(seed):
+    """Every matrix of a 5120-wide layer takes the tcgen05 kernel for one row (one of them on the few-row kernel between
+    the others costs 5 us a layer): the same bits as with the kernel forced."""
+    def forced(w, x):
+        out = torch.empty((1, x.shape[0], w.s), dtype=torch.float16, device=x.device)
+        ops.quant_int4_linear_mult_mtx(out, w.matrix, x.unsqueeze(0).contiguous(), w.scales, w.zeros, w.group_size, None, path=2)
+        return out[0]
+    stack = sharding.DecoderStack(sharding.StackConfig(layers=2), 0, 1, torch.device("cuda"))
+    x = torch.randn((1, 5120), generator=torch.Generator().manual_seed(seed)).half().cuda()
+    y = stack.forward(x)
+    stack.multiply = forced
+    assert torch.equal(y, stack.forward(x))
+
+
 class _SynchronisedStack(sharding.DecoderStack):
     """The stack with a device synchronisation after every launch: the reference for what a pass must compute."""
 
