@@ -89,7 +89,9 @@ size_t i4mm_workspace_bytes(void);
  *   the kernel that precedes this call in the stream (weights of a loaded model never are).  Launches may begin while
  *   that kernel is still finishing (programmatic dependent launch); with the promise the first weight copies go out
  *   then, while x, out and the workspace are touched only once that kernel is complete.  Without it nothing at all is
- *   read before, as with the reference's launches.
+ *   read before, as with the reference's launches.  The kernels of this library let their successor begin only once
+ *   everything before them is complete, so the promise is about one kernel; a row norm that carries the same flag is the
+ *   exception (see i4mm_row_norm).
  */
 #define I4MM_PATH_STATIC_WEIGHTS 0x100000
 int i4mm_quant_matmul(int bits, int accumulate, int path,
@@ -201,6 +203,9 @@ int i4mm_check_mask(const void* mask, int64_t N, int64_t S, void* violations, vo
  * a, b, c fp16 (rows, width) with row strides in elements (column slices of a gathered buffer are fine);
  * y fp16 (rows, width) contiguous ((2, rows, width) in mode 4); width even; pointers 4-byte aligned.  No counterpart in the reference
  * (it has no model code): it replaces the handful of eager elementwise kernels between two quantized linears.
+ * `mode | I4MM_PATH_STATIC_WEIGHTS` extends the promise of that name: the kernel that precedes the row norm (and those before
+ * it, as long as they are row norms with this flag too) does not write weight-side tensors of the multiply after it either.
+ * That multiply, if it carries the promise itself, may then copy weights while the kernel before the row norm is running.
  */
 int i4mm_row_norm(int mode, void* y, const void* a, const void* b, const void* c, int64_t rows, int64_t width,
                   int64_t stride_a, int64_t stride_b, int64_t stride_c, void* stream);

@@ -18,7 +18,7 @@ cudaError_t sparse_pack_launch(void* wt_out, void* msk_out, const void* wt_in, c
                                int S, int N, void* violations, cudaStream_t stream);
 cudaError_t check_mask_launch(const void* mask, size_t count, void* violations, cudaStream_t stream);
 cudaError_t rownorm_launch(int mode, void* y, const void* a, const void* b, const void* c, long long rows, int width,
-                           long long sa, long long sb, long long sc, cudaStream_t stream);
+                           long long sa, long long sb, long long sc, int early, cudaStream_t stream);
 int umma_launch(int bits, bool sparse, const StreamParams& p, int total_rows, int n_groups, int group_size, int cta_pairs,
                 int force_nt, int overlap, cudaStream_t stream, cudaError_t* cuda_err);
 bool rows_supported(int bits, bool accumulate, int rows, int N, int S);
@@ -216,6 +216,8 @@ int i4mm_device_status(void* workspace, void* stream) {
 
 int i4mm_row_norm(int mode, void* y, const void* a, const void* b, const void* c, int64_t rows, int64_t width,
                   int64_t stride_a, int64_t stride_b, int64_t stride_c, void* stream) {
+    const int early = mode > 0 && (mode & I4MM_PATH_STATIC_WEIGHTS) ? 1 : 0;
+    if (early) mode &= ~I4MM_PATH_STATIC_WEIGHTS;
     if (mode < 0 || mode > 4 || rows < 0 || width <= 0 || width % 2 != 0 || width > (1 << 30) || rows > (1ll << 31) - 1)
         return I4MM_ERR_SHAPE;
     if (rows == 0) return I4MM_OK;
@@ -225,7 +227,7 @@ int i4mm_row_norm(int mode, void* y, const void* a, const void* b, const void* c
          reinterpret_cast<uintptr_t>(c)) & 3u)
         return I4MM_ERR_ALIGN;
     const cudaError_t e = i4mm::rownorm_launch(mode, y, a, b, c, rows, (int)width, stride_a, stride_b, stride_c,
-                                               (cudaStream_t)stream);
+                                               early, (cudaStream_t)stream);
     if (e != cudaSuccess) return fail_cuda(e);
     return I4MM_OK;
 }

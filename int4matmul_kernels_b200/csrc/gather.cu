@@ -30,10 +30,10 @@ struct PeerFlags {
 // kernel can be replayed from a CUDA graph: every rank runs the same sequence of calls, hence the same epochs.
 __global__ void gather_sync_kernel(PeerFlags pf, unsigned int* epochs, int* status, int world, int rank, int slot, int slots) {
     __shared__ unsigned int s_epoch;
-    // launched with programmatic stream serialization: the kernel after this one may be scheduled at once (it waits for
-    // this one itself before it reads anything), and nothing happens here before the multiply has completed
-    i4mm::ptx::grid_launch_dependents();
+    // launched with programmatic stream serialization: nothing happens here before the multiply has completed, and the
+    // kernel after this one may be scheduled from then on
     i4mm::ptx::grid_dependency_wait();
+    i4mm::ptx::grid_launch_dependents();
     if (threadIdx.x == 0) s_epoch = ++epochs[slot];
     __syncthreads();
     const unsigned int epoch = s_epoch;

@@ -110,7 +110,10 @@ __device__ __forceinline__ bool elect_one() {
 // A kernel launched with the programmatic-stream-serialization attribute may start while the kernel before it in the
 // stream is still running.  wait: returns once that kernel has completed and its writes are visible (at once when the
 // launch had no such attribute).  launch_dependents: the next kernel in the stream may be scheduled as soon as every
-// CTA of this grid has said so or exited.
+// CTA of this grid has said so or exited.  Said after the wait, it tells the next kernel that everything before this one is
+// complete: what that kernel reads early (weights, by its caller's promise) then only has to be left alone by this
+// one.  Said before the wait, it would let the next kernel, and with a chain of such kernels a far later one, run beside a
+// kernel several launches back that still writes those weights.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

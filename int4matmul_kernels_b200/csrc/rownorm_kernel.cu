@@ -20,6 +20,16 @@ namespace {
 // nothing else writes that memory during the kernel, which lets it move loads above griddepcontrol.wait (observed: the
 // modes with an inner norm read the multiply's output before it was complete).
 
+// Launched with programmatic stream serialization: nothing is read or written here before the kernel before this one has
+// completed.  The kernel after this one may be scheduled from then on, or with `early` at once: a multiply with the
+// static-weights promise then copies weights while the kernel before this one still runs, which only the caller can allow
+// (five row norms among the four multiplies of a 13B-class layer, one row, promise given: 79 us so, 76 with early).
+__device__ __forceinline__ void begin(int early) {
+    if (early) ptx::grid_launch_dependents();
+    ptx::grid_dependency_wait();
+    if (!early) ptx::grid_launch_dependents();
+}
+
 __device__ __forceinline__ float block_sum(float v, float* red) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
@@ -34,13 +44,9 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 template <int MODE>
 __global__ void __launch_bounds__(256) rownorm_kernel(__half* y, const __half* a,
                                                       const __half* b, const __half* c,
-                                                      int width, long long sa, long long sb, long long sc) {
+                                                      int width, long long sa, long long sb, long long sc, int early) {
     __shared__ float red[32];
-    // Launched with programmatic stream serialization: the kernel after this one may be scheduled at once (a multiply
-    // then sets itself up and starts copying weights meanwhile), and nothing is read or written here before the kernel
-    // before this one has completed.
-    ptx::grid_launch_dependents();
-    ptx::grid_dependency_wait();
+    begin(early);
     const long long row = blockIdx.x;
     const __half2* a2 = reinterpret_cast<const __half2*>(a + row * sa);
     const __half2* b2 = MODE != 0 ? reinterpret_cast<const __half2*>(b + row * sb) : nullptr;
@@ -87,10 +93,9 @@ template <int MODE>
 __global__ void __launch_bounds__(kCachedThreads) rownorm_cached_kernel(__half* y, const __half* a,
                                                                         const __half* b, const __half* c,
                                                                         int width, long long sa, long long sb, long long sc,
-                                                                        long long second_output) {
+                                                                        long long second_output, int early) {
     __shared__ float red[32];
-    ptx::grid_launch_dependents();        // as in rownorm_kernel
-    ptx::grid_dependency_wait();
+    begin(early);
     constexpr bool kHasB = MODE != 0, kHasC = MODE == 1, kInnerNorm = MODE == 2 || MODE == 4;
     const long long row = blockIdx.x;
     const __half2* a2 = reinterpret_cast<const __half2*>(a + row * sa);
@@ -150,7 +155,7 @@ __global__ void __launch_bounds__(kCachedThreads) rownorm_cached_kernel(__half* 
 }  // namespace
 
 cudaError_t rownorm_launch(int mode, void* y, const void* a, const void* b, const void* c, long long rows, int width,
-                           long long sa, long long sb, long long sc, cudaStream_t stream) {
+                           long long sa, long long sb, long long sc, int early, cudaStream_t stream) {
     if (rows <= 0) return cudaSuccess;
     __half* yy = (__half*)y;
     const __half *aa = (const __half*)a, *bb = (const __half*)b, *cc = (const __half*)c;
@@ -168,28 +173,28 @@ cudaError_t rownorm_launch(int mode, void* y, const void* a, const void* b, cons
     if (width <= kCachedWidth) {
         cfg.blockDim = dim3(kCachedThreads, 1, 1);
         switch (mode) {
-            case 0: e = cudaLaunchKernelEx(&cfg, rownorm_cached_kernel<0>, yy, aa, bb, cc, width, sa, sb, sc, second); break;
-            case 1: e = cudaLaunchKernelEx(&cfg, rownorm_cached_kernel<1>, yy, aa, bb, cc, width, sa, sb, sc, second); break;
-            case 2: e = cudaLaunchKernelEx(&cfg, rownorm_cached_kernel<2>, yy, aa, bb, cc, width, sa, sb, sc, second); break;
-            case 3: e = cudaLaunchKernelEx(&cfg, rownorm_cached_kernel<3>, yy, aa, bb, cc, width, sa, sb, sc, second); break;
-            default: e = cudaLaunchKernelEx(&cfg, rownorm_cached_kernel<4>, yy, aa, bb, cc, width, sa, sb, sc, second); break;
+            case 0: e = cudaLaunchKernelEx(&cfg, rownorm_cached_kernel<0>, yy, aa, bb, cc, width, sa, sb, sc, second, early); break;
+            case 1: e = cudaLaunchKernelEx(&cfg, rownorm_cached_kernel<1>, yy, aa, bb, cc, width, sa, sb, sc, second, early); break;
+            case 2: e = cudaLaunchKernelEx(&cfg, rownorm_cached_kernel<2>, yy, aa, bb, cc, width, sa, sb, sc, second, early); break;
+            case 3: e = cudaLaunchKernelEx(&cfg, rownorm_cached_kernel<3>, yy, aa, bb, cc, width, sa, sb, sc, second, early); break;
+            default: e = cudaLaunchKernelEx(&cfg, rownorm_cached_kernel<4>, yy, aa, bb, cc, width, sa, sb, sc, second, early); break;
         }
         if (e == cudaSuccess) count_launch();
         return e;
     }
     if (mode == 4) {                                              // wide rows: the two steps as two launches
-        e = cudaLaunchKernelEx(&cfg, rownorm_kernel<2>, yy, aa, bb, cc, width, sa, sb, sc);
+        e = cudaLaunchKernelEx(&cfg, rownorm_kernel<2>, yy, aa, bb, cc, width, sa, sb, sc, early);
         if (e != cudaSuccess) return e;
         count_launch();
-        e = cudaLaunchKernelEx(&cfg, rownorm_kernel<0>, yy + second, (const __half*)yy, bb, cc, width, (long long)width, sb, sc);
+        e = cudaLaunchKernelEx(&cfg, rownorm_kernel<0>, yy + second, (const __half*)yy, bb, cc, width, (long long)width, sb, sc, early);
         if (e == cudaSuccess) count_launch();
         return e;
     }
     switch (mode) {
-        case 0: e = cudaLaunchKernelEx(&cfg, rownorm_kernel<0>, yy, aa, bb, cc, width, sa, sb, sc); break;
-        case 1: e = cudaLaunchKernelEx(&cfg, rownorm_kernel<1>, yy, aa, bb, cc, width, sa, sb, sc); break;
-        case 2: e = cudaLaunchKernelEx(&cfg, rownorm_kernel<2>, yy, aa, bb, cc, width, sa, sb, sc); break;
-        default: e = cudaLaunchKernelEx(&cfg, rownorm_kernel<3>, yy, aa, bb, cc, width, sa, sb, sc); break;
+        case 0: e = cudaLaunchKernelEx(&cfg, rownorm_kernel<0>, yy, aa, bb, cc, width, sa, sb, sc, early); break;
+        case 1: e = cudaLaunchKernelEx(&cfg, rownorm_kernel<1>, yy, aa, bb, cc, width, sa, sb, sc, early); break;
+        case 2: e = cudaLaunchKernelEx(&cfg, rownorm_kernel<2>, yy, aa, bb, cc, width, sa, sb, sc, early); break;
+        default: e = cudaLaunchKernelEx(&cfg, rownorm_kernel<3>, yy, aa, bb, cc, width, sa, sb, sc, early); break;
     }
     if (e == cudaSuccess) count_launch();
     return e;

@@ -279,7 +279,6 @@ __global__ void __launch_bounds__(kRowsThreads, kCtasPerSm) rows_kernel(const Ro
     unsigned char* const ring = smem_raw + SM::kRed + warp * (D * ST::kBytes);
     const uint32_t ring_addr = ptx::smem_u32(ring);
 
-    ptx::grid_launch_dependents();
     // Without the promise that weight-side tensors are not written by the kernel before this one, nothing is read early
     if (!p.overlap) ptx::grid_dependency_wait();
 
@@ -376,6 +375,7 @@ __global__ void __launch_bounds__(kRowsThreads, kCtasPerSm) rows_kernel(const Ro
 #pragma unroll 1
         for (int j = 0; j < D; ++j) { fetch_weights(j); fetch_x(j); fetch_advance(); ptx::cp_async_commit(); }
     }
+    ptx::grid_launch_dependents();                           // not before the wait: see ptx.cuh
     if (SPARSE) {
         for (int i = threadIdx.x; i < 256; i += kRowsThreads) lut_mem[i] = sparse_selectors(i);
         __syncthreads();

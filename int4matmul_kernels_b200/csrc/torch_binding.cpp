@@ -233,7 +233,7 @@ py::object try_linear(int64_t bits, int64_t path, const Tensor& x, int64_t in_fe
     return py::cast(out);
 }
 
-// ops.row_norm: the new output, or a status / -1
+// ops.row_norm (mode may carry I4MM_PATH_STATIC_WEIGHTS): the new output, or a status / -1
 py::object try_row_norm(int64_t mode, const Tensor& a, const c10::optional<Tensor>& b, const c10::optional<Tensor>& c) {
     if (!a.is_cuda() || a.dim() != 2 || c10::cuda::current_device() != a.device().index()) return py::int_(-1);
     const c10::optional<Tensor> operands[3] = {a, b, c};
@@ -249,7 +249,7 @@ py::object try_row_norm(int64_t mode, const Tensor& a, const c10::optional<Tenso
     }
     const int64_t rows = a.size(0), width = a.size(1);
     const auto options = at::TensorOptions().dtype(torch::kHalf).device(a.device());
-    Tensor y = mode == 4 ? at::empty({2, rows, width}, options) : at::empty({rows, width}, options);
+    Tensor y = (mode & ~(int64_t)I4MM_PATH_STATIC_WEIGHTS) == 4 ? at::empty({2, rows, width}, options) : at::empty({rows, width}, options);
     const int status = i4mm_row_norm((int)mode, y.data_ptr(), ptr[0], ptr[1], ptr[2], rows, width, stride[0], stride[1], stride[2],
                                      (void*)c10::cuda::getCurrentCUDAStream(a.device().index()).stream());
     if (status != I4MM_OK) return py::int_(status);

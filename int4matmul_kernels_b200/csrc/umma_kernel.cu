@@ -358,9 +358,6 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const UmmaParams p, const __h
         ptx::tc_fence_after_sync();
     }
     const uint32_t tmem_base = tmem_base_smem;       // not valid in the weight producer's warp, which never uses it
-    // The next kernel of the stream may be scheduled from here on (it takes an SM only when a CTA of this grid has left
-    // it); if it is one of these kernels, its set-up and its first weight copies then overlap this grid's tail.
-    if (threadIdx.x == 0) ptx::grid_launch_dependents();
 
     // ---- this CTA's share of the (tile, unit) space; one unit = H x 64 k.  Whole tiles unless the split-K variant ----
     const long long U = p.U;
@@ -437,6 +434,7 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const UmmaParams p, const __h
         // a barrier per unit, as for the other formats, costs this warp more per unit than the unit may take.)
         for (uint32_t o = lane * 16; o < (uint32_t)(kABStages * kBStageBytes); o += 32 * 16) ptx::sts128(b_ring + o, make_uint4(0, 0, 0, 0));
         ptx::grid_dependency_wait();      // the activations may be the output of the kernel before this one in the stream
+        if (lane == 0) ptx::grid_launch_dependents();      // as below
         constexpr int D = C::kXStaging;
         const int total = (int)(t_hi - t_lo);
         const int nrows = min(NT, p.rows);                              // (one row tile: these shapes have at most NT rows)
@@ -490,6 +488,10 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const UmmaParams p, const __h
             // the activations may be the output of the kernel before this one in the stream (the weight-side tensors
             // are not: see the launch attribute in launch_nt)
             ptx::grid_dependency_wait();
+            // The next kernel of the stream may be scheduled from here on (it takes an SM only when a CTA of this grid has
+            // left it); if it is one of these kernels, its set-up and its first weight copies then overlap this grid's tail.
+            // Not before the wait: see ptx.cuh.
+            ptx::grid_launch_dependents();
             for (long long t = t_lo; t < t_hi && ok;) {
                 const long long tile = div_nn(t, U);
                 const int u0 = (int)(t - tile * U);
@@ -1036,10 +1038,10 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const UmmaParams p, const __h
 // (no __restrict__ here or on umma_kernel's activations: both kernels may start while the kernel that writes what they
 // read is still running, and a restrict-qualified pointer would allow the compiler to load above griddepcontrol.wait)
 __global__ void kparts_reduce_kernel(float* parts, const OutMap om, int rows, int S, int kparts) {
-    // (launched with programmatic stream serialization: the next kernel may be scheduled at once, this one touches
-    // nothing before the kernel that wrote the parts has completed)
-    ptx::grid_launch_dependents();
+    // (launched with programmatic stream serialization: touches nothing before the kernel that wrote the parts has
+    // completed, and lets the next kernel be scheduled from then on)
     ptx::grid_dependency_wait();
+    ptx::grid_launch_dependents();
     const int s8 = S / 8;
     const long long n8 = (long long)rows * s8;
     const size_t stride = (size_t)rows * S;

@@ -23,11 +23,11 @@ _static_weights = False
 
 def set_static_weights(flag: bool) -> None:
     """Declare that the weight-side tensors (matrix, mask, scales, zeros) passed to the multiply entries are never
-    written by the kernel that precedes the call in the stream, as is the case for the weights of a loaded model.
-    Launches begin while that kernel is still finishing; with the promise their first weight copies go out then, while
-    activations, outputs and scratch are still only touched once it is complete.  Off by default (nothing is read early):
-    the reference orders every launch after the whole preceding kernel, and a caller that rewrites weights right before a
-    call relies on that."""
+    written by the kernel that precedes the call in the stream, nor, where that is a `row_norm`, by the one before it, as is
+    the case for the weights of a loaded model.  Launches begin while that kernel is still finishing; with the promise
+    their first weight copies go out then, while activations, outputs and scratch are still only touched once it is complete.
+    Off by default (nothing is read early): the reference orders every launch after the whole preceding kernel, and a
+    caller that rewrites weights right before a call relies on that."""
     global _static_weights
     _static_weights = bool(flag)
 
@@ -224,9 +224,10 @@ def row_norm(mode: int, a: torch.Tensor, b: torch.Tensor | None = None, c: torch
     """Row-wise glue of the layer-stack runner (`i4mm_row_norm`): v / rms(v) per row with
     v = a (mode 0), a + b + c (1), a + b / rms(b) (2), a * b (3).  Inputs fp16 (rows, width), last dim contiguous.
     Mode 4 returns (2, rows, width): mode 2's result, and mode 0 of that result, from one launch."""
-    mod = native()
+    early = capi.PATH_STATIC_WEIGHTS if _static_weights else 0
+    mod = native() if 0 <= mode <= 4 else False
     if mod:
-        y = mod._try_row_norm(mode, a, b, c)
+        y = mod._try_row_norm(mode | early, a, b, c)
         if not isinstance(y, int):
             return y
         if y > 0:
@@ -235,10 +236,12 @@ def row_norm(mode: int, a: torch.Tensor, b: torch.Tensor | None = None, c: torch
     for t in (a, b, c):
         if t is not None and (t.dtype != torch.float16 or t.stride(-1) != 1 or tuple(t.shape) != (rows, width)):
             raise ValueError("row_norm inputs must be fp16 (rows, width) with a contiguous last dim")
+    if not 0 <= mode <= 4:
+        raise Int4MatmulError(capi.ERR_SHAPE, "row_norm")
     y = torch.empty((2, rows, width) if mode == 4 else (rows, width), dtype=torch.float16, device=a.device)
     stream = torch.cuda.current_stream(a.device)
     status = capi.load().i4mm_row_norm(
-        mode, y.data_ptr(), a.data_ptr(), b.data_ptr() if b is not None else None, c.data_ptr() if c is not None else None,
+        mode | early, y.data_ptr(), a.data_ptr(), b.data_ptr() if b is not None else None, c.data_ptr() if c is not None else None,
         rows, width, a.stride(0), b.stride(0) if b is not None else 0, c.stride(0) if c is not None else 0, stream.cuda_stream)
     if status != capi.OK:
         raise Int4MatmulError(status, "row_norm")

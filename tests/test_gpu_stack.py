@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 import torch
 
-from int4matmul_kernels_b200 import ops, packing, sharding
+from int4matmul_kernels_b200 import capi, ops, packing, sharding
 from oracle import reference_oracle as oracle
 
 from helpers import assert_parity
@@ -32,6 +32,9 @@ def test_row_norm_modes_match_the_fp32_expression(rows, width):
         # fp32 math on both sides, different summation order inside the row reduction: within 1 fp16 ulp
         ulp = oracle.fp16_ulp_distance(y.cpu().numpy(), w.to(torch.float16).cpu().numpy())
         assert ulp.max() <= 1, f"mode {mode}: {ulp.max()} ulp"
+    for bad in (-1, 5, 4 | capi.PATH_STATIC_WEIGHTS):
+        with pytest.raises(ops.Int4MatmulError):
+            ops.row_norm(bad, a, b)
     # mode 4 = mode 2 and mode 0 of its result from one launch: the same bits as the two launches
     both = ops.row_norm(4, a, b)
     assert both.shape == (2, rows, width)
