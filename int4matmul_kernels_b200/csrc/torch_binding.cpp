@@ -167,93 +167,144 @@ void weight_matrix_packing(Tensor wt_outs, Tensor msk_outs, Tensor wt_in, Tensor
 // ---- the Python package's own calls (ops.py, quantize.py) -----------------------------------------------------------
 // What those modules check and launch, for arguments that pass every check: a decoding step is a chain of small launches,
 // and the same work done in Python (17 ctypes arguments, a device context, some thirty tensor properties) takes longer
-// than most of them run.  Nothing is diagnosed here: whenever a precondition does not hold, or the scratch buffer
-// of this stream does not exist yet, the caller is told so (-1 / None) and takes its own path, which raises or allocates.
+// than most of them run.  Nothing is diagnosed here: whenever a precondition does not hold (an argument that is no tensor
+// or no integer, memory that cannot be had, ...), or the scratch buffer of this stream does not exist yet, the caller is told so
+// (-1) and takes its own path, which raises, converts or allocates.  The arguments are therefore plain Python objects: a typed
+// signature would raise an error of its own first.
+
+// (an undefined tensor stands for None)
+bool as_tensor(const py::object& o, Tensor& t) {
+    if (!THPVariable_Check(o.ptr())) return false;
+    t = THPVariable_Unpack(o.ptr());
+    return true;
+}
+bool as_optional_tensor(const py::object& o, Tensor& t) { return o.is_none() || as_tensor(o, t); }
+
+bool as_int(const py::object& o, int64_t& v) {
+    if (!PyIndex_Check(o.ptr())) return false;
+    v = PyNumber_AsSsize_t(o.ptr(), PyExc_OverflowError);
+    if (v == -1 && PyErr_Occurred()) {
+        PyErr_Clear();
+        return false;
+    }
+    return true;
+}
 
 bool plain(const Tensor& t, const c10::Device& dev, c10::ScalarType type) {
     return t.is_cuda() && t.device() == dev && t.scalar_type() == type && t.is_contiguous();
 }
 
+// the weight side of a call, as the caller has it
+struct Weights {
+    Tensor matrix, scales, zeros, mask;
+    int64_t bits = 0, group_size = 0;
+    bool read(const py::object& bits_, const py::object& matrix_, const py::object& scales_, const py::object& zeros_,
+              const py::object& group_size_, const py::object& mask_) {
+        return as_int(bits_, bits) && as_int(group_size_, group_size) && as_tensor(matrix_, matrix) && as_tensor(scales_, scales) &&
+               as_tensor(zeros_, zeros) && as_optional_tensor(mask_, mask);
+    }
+};
+
 // `workspaces`: the Python package's dict (device index, raw stream) -> zero-initialised uint8 tensor
-int launch_checked(int64_t bits, bool matvec, int64_t path, void* out, const Tensor& matrix, const Tensor& x, int64_t rows,
-                   const Tensor& scales, const Tensor& zeros, int64_t group_size, const c10::optional<Tensor>& mask,
-                   const py::dict& workspaces) {
+int launch_checked(const Weights& w, bool matvec, int64_t path, void* out, const Tensor& x, int64_t rows, const py::dict& workspaces) {
     const auto dev = x.device();
-    if (bits != 4 && bits != 3 && bits != 2) return -1;
+    if (w.bits != 4 && w.bits != 3 && w.bits != 2) return -1;
     const int64_t in_size = x.size(-1);
-    if (!plain(x, dev, torch::kHalf) || !plain(matrix, dev, torch::kInt) || !plain(scales, dev, torch::kHalf) ||
-        !plain(zeros, dev, torch::kHalf) || matrix.dim() != 2 || scales.dim() != 2 || zeros.dim() != 2)
+    if (!plain(x, dev, torch::kHalf) || !plain(w.matrix, dev, torch::kInt) || !plain(w.scales, dev, torch::kHalf) ||
+        !plain(w.zeros, dev, torch::kHalf) || w.matrix.dim() != 2 || w.scales.dim() != 2 || w.zeros.dim() != 2)
         return -1;
-    const int64_t mtx_in = matrix.size(0), out_size = matrix.size(1);
-    const bool sparse = mask.has_value() && mask->defined();
+    const int64_t mtx_in = w.matrix.size(0), out_size = w.matrix.size(1);
+    const bool sparse = w.mask.defined();
     if (sparse) {
-        if (bits != 4 || mtx_in * 16 != in_size || mtx_in % 2 || !plain(*mask, dev, torch::kInt) || mask->dim() != 2 ||
-            mask->size(0) != mtx_in / 2 || mask->size(1) != out_size)
+        if (w.bits != 4 || mtx_in * 16 != in_size || mtx_in % 2 || !plain(w.mask, dev, torch::kInt) || w.mask.dim() != 2 ||
+            w.mask.size(0) != mtx_in / 2 || w.mask.size(1) != out_size)
             return -1;
-    } else if ((mtx_in * 32) % bits || mtx_in * 32 / bits != in_size) {
+    } else if ((mtx_in * 32) % w.bits || mtx_in * 32 / w.bits != in_size) {
         return -1;
     }
-    if (scales.size(1) != out_size || zeros.sizes() != scales.sizes()) return -1;
-    if (group_size == 0 || (group_size > 0 && group_size % 64)) return -1;
+    if (w.scales.size(1) != out_size || w.zeros.sizes() != w.scales.sizes()) return -1;
+    if (w.group_size == 0 || (w.group_size > 0 && w.group_size % 64)) return -1;
     c10::cuda::OptionalCUDAGuard guard;
     if (c10::cuda::current_device() != dev.index()) guard.set_device(dev);
     const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
     PyObject* const item = PyDict_GetItem(workspaces.ptr(), py::make_tuple((int)dev.index(), (uint64_t)(uintptr_t)stream).ptr());
     if (!item) return -1;
     const Tensor ws = py::cast<Tensor>(py::handle(item));
-    return i4mm_quant_matmul((int)bits, matvec ? 1 : 0, (int)path, out, matrix.data_ptr(), sparse ? mask->data_ptr() : nullptr,
-                             x.data_ptr(), scales.data_ptr(), zeros.data_ptr(), rows, in_size, out_size, scales.size(0), group_size,
-                             ws.data_ptr(), (size_t)ws.numel(), (void*)stream);
+    return i4mm_quant_matmul((int)w.bits, matvec ? 1 : 0, (int)path, out, w.matrix.data_ptr(), sparse ? w.mask.data_ptr() : nullptr,
+                             x.data_ptr(), w.scales.data_ptr(), w.zeros.data_ptr(), rows, in_size, out_size, w.scales.size(0),
+                             w.group_size, ws.data_ptr(), (size_t)ws.numel(), (void*)stream);
 }
 
 // ops._mult; route 0: by seq_len, 1: matmul, 2: matvec
-int try_mult(int64_t bits, int64_t route, int64_t path, const Tensor& outs, const Tensor& matrix, const Tensor& x, const Tensor& scales,
-             const Tensor& zeros, int64_t group_size, const c10::optional<Tensor>& mask, const py::dict& workspaces) {
-    if (x.dim() != 3 || outs.dim() != 3 || matrix.dim() != 2 || !plain(outs, x.device(), torch::kHalf)) return -1;
-    const int64_t batch = x.size(0), seq_len = x.size(1);
-    if (route == 2 && seq_len != 1) return -1;
-    if (outs.size(0) != batch || outs.size(1) != seq_len || outs.size(2) != matrix.size(1)) return -1;
-    return launch_checked(bits, route == 2 || (route == 0 && seq_len == 1), path, outs.data_ptr(), matrix, x, batch * seq_len,
-                          scales, zeros, group_size, mask, workspaces);
+int try_mult(const py::object& bits, int64_t route, int64_t path, const py::object& outs_, const py::object& matrix, const py::object& x_,
+             const py::object& scales, const py::object& zeros, const py::object& group_size, const py::object& mask,
+             const py::dict& workspaces) {
+    Weights w;
+    Tensor outs, x;
+    if (!w.read(bits, matrix, scales, zeros, group_size, mask) || !as_tensor(outs_, outs) || !as_tensor(x_, x)) return -1;
+    try {
+        if (x.dim() != 3 || outs.dim() != 3 || w.matrix.dim() != 2 || !plain(outs, x.device(), torch::kHalf)) return -1;
+        const int64_t batch = x.size(0), seq_len = x.size(1);
+        if (route == 2 && seq_len != 1) return -1;
+        if (outs.size(0) != batch || outs.size(1) != seq_len || outs.size(2) != w.matrix.size(1)) return -1;
+        return launch_checked(w, route == 2 || (route == 0 && seq_len == 1), path, outs.data_ptr(), x, batch * seq_len, workspaces);
+    } catch (const c10::Error&) {
+        return -1;                                          // (nothing was launched: everything that throws comes before that)
+    }
 }
 
 // QuantLinear.forward: the new output, or a status / -1
-py::object try_linear(int64_t bits, int64_t path, const Tensor& x, int64_t in_features, int64_t out_features, const Tensor& matrix,
-                      const Tensor& scales, const Tensor& zeros, int64_t group_size, const c10::optional<Tensor>& mask,
-                      const py::dict& workspaces) {
-    if (x.dim() < 1 || x.numel() == 0 || x.size(-1) != in_features || matrix.dim() != 2 || matrix.size(1) != out_features ||
-        !plain(x, x.device(), torch::kHalf))
+py::object try_linear(const py::object& bits, int64_t path, const py::object& x_, const py::object& in_features_,
+                      const py::object& out_features_, const py::object& matrix, const py::object& scales, const py::object& zeros,
+                      const py::object& group_size, const py::object& mask, const py::dict& workspaces) {
+    Weights w;
+    Tensor x;
+    int64_t in_features = 0, out_features = 0;
+    if (!w.read(bits, matrix, scales, zeros, group_size, mask) || !as_tensor(x_, x) || !as_int(in_features_, in_features) ||
+        !as_int(out_features_, out_features))
         return py::int_(-1);
-    auto sizes = x.sizes().vec();
-    sizes.back() = out_features;
-    Tensor out = at::empty(sizes, at::TensorOptions().dtype(torch::kHalf).device(x.device()));
-    const int status = launch_checked(bits, false, path, out.data_ptr(), matrix, x, x.numel() / in_features, scales, zeros, group_size,
-                                      mask, workspaces);
-    if (status != I4MM_OK) return py::int_(status);
-    return py::cast(out);
+    try {
+        if (x.dim() < 1 || x.numel() == 0 || x.size(-1) != in_features || w.matrix.dim() != 2 || w.matrix.size(1) != out_features ||
+            !plain(x, x.device(), torch::kHalf))
+            return py::int_(-1);
+        auto sizes = x.sizes().vec();
+        sizes.back() = out_features;
+        Tensor out = at::empty(sizes, at::TensorOptions().dtype(torch::kHalf).device(x.device()));
+        const int status = launch_checked(w, false, path, out.data_ptr(), x, x.numel() / in_features, workspaces);
+        if (status != I4MM_OK) return py::int_(status);
+        return py::cast(out);
+    } catch (const c10::Error&) {
+        return py::int_(-1);
+    }
 }
 
 // ops.row_norm (mode may carry I4MM_PATH_STATIC_WEIGHTS): the new output, or a status / -1
-py::object try_row_norm(int64_t mode, const Tensor& a, const c10::optional<Tensor>& b, const c10::optional<Tensor>& c) {
-    if (!a.is_cuda() || a.dim() != 2 || c10::cuda::current_device() != a.device().index()) return py::int_(-1);
-    const c10::optional<Tensor> operands[3] = {a, b, c};
-    const void* ptr[3] = {nullptr, nullptr, nullptr};
-    int64_t stride[3] = {0, 0, 0};
-    for (int i = 0; i < 3; ++i) {
-        if (!operands[i].has_value()) continue;
-        const Tensor& t = *operands[i];
-        if (!t.is_cuda() || t.device() != a.device() || t.scalar_type() != torch::kHalf || t.sizes() != a.sizes() || t.stride(1) != 1)
-            return py::int_(-1);
-        ptr[i] = t.data_ptr();
-        stride[i] = t.stride(0);
+py::object try_row_norm(int64_t mode, const py::object& a_, const py::object& b, const py::object& c) {
+    Tensor a, operands[3];
+    if (!as_tensor(a_, a) || !as_optional_tensor(b, operands[1]) || !as_optional_tensor(c, operands[2])) return py::int_(-1);
+    operands[0] = a;
+    try {
+        if (!a.is_cuda() || a.dim() != 2 || c10::cuda::current_device() != a.device().index()) return py::int_(-1);
+        const void* ptr[3] = {nullptr, nullptr, nullptr};
+        int64_t stride[3] = {0, 0, 0};
+        for (int i = 0; i < 3; ++i) {
+            const Tensor& t = operands[i];
+            if (!t.defined()) continue;
+            if (!t.is_cuda() || t.device() != a.device() || t.scalar_type() != torch::kHalf || t.sizes() != a.sizes() || t.stride(1) != 1)
+                return py::int_(-1);
+            ptr[i] = t.data_ptr();
+            stride[i] = t.stride(0);
+        }
+        const int64_t rows = a.size(0), width = a.size(1);
+        const auto options = at::TensorOptions().dtype(torch::kHalf).device(a.device());
+        Tensor y = (mode & ~(int64_t)I4MM_PATH_STATIC_WEIGHTS) == 4 ? at::empty({2, rows, width}, options) : at::empty({rows, width}, options);
+        const int status = i4mm_row_norm((int)mode, y.data_ptr(), ptr[0], ptr[1], ptr[2], rows, width, stride[0], stride[1], stride[2],
+                                         (void*)c10::cuda::getCurrentCUDAStream(a.device().index()).stream());
+        if (status != I4MM_OK) return py::int_(status);
+        return py::cast(y);
+    } catch (const c10::Error&) {
+        return py::int_(-1);
     }
-    const int64_t rows = a.size(0), width = a.size(1);
-    const auto options = at::TensorOptions().dtype(torch::kHalf).device(a.device());
-    Tensor y = (mode & ~(int64_t)I4MM_PATH_STATIC_WEIGHTS) == 4 ? at::empty({2, rows, width}, options) : at::empty({rows, width}, options);
-    const int status = i4mm_row_norm((int)mode, y.data_ptr(), ptr[0], ptr[1], ptr[2], rows, width, stride[0], stride[1], stride[2],
-                                     (void*)c10::cuda::getCurrentCUDAStream(a.device().index()).stream());
-    if (status != I4MM_OK) return py::int_(status);
-    return py::cast(y);
 }
 
 // Not in the reference (its kernels have no waits): waits for every stream this module has launched on, on the

@@ -82,7 +82,7 @@ class QuantLinear(torch.nn.Module):
         mod = ops.native()
         if mod:
             y = mod._try_linear(self.bits, capi.PATH_STATIC_WEIGHTS if ops._static_weights else capi.PATH_AUTO, x, self.in_features,
-                                self.out_features, self.matrix, self.scales, self.zeros, self.group_size, self.mask, ops._workspaces)
+                                self.out_features, self.matrix, self.scales, self.zeros, int(self.group_size), self.mask, ops._workspaces)
             if not isinstance(y, int):
                 return y
         lead = x.shape[:-1]

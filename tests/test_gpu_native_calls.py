@@ -1,5 +1,6 @@
 """The compiled fast path of the Python entries (ops, QuantLinear) against the same calls through ctypes: equal results for
 everything both accept, and the same exceptions for what the entries refuse."""
+import numpy as np
 import pytest
 import torch
 
@@ -82,6 +83,18 @@ def test_refusals_are_the_same(monkeypatch):
         lambda: ops.quant_matmul(3, out, m, x, s, z, 128, None),
         lambda: ops.quant_matmul(2, out, m, x, s, z, 128, m),
         lambda: ops.quant_int4_linear_mult_vec(out, m, x, s, z, 128, None),
+        # arguments of another kind: the entry's own diagnosis, not that of the compiled function's signature
+        lambda: ops.quant_matmul(4, out, m, None, s, z, 128, None),
+        lambda: ops.quant_matmul(4, None, m, x, s, z, 128, None),
+        lambda: ops.quant_matmul(4, out, m, x.cpu().numpy(), s, z, 128, None),
+        lambda: ops.quant_matmul(4, out, m, x, None, z, 128, None),
+        lambda: ops.quant_matmul(4, out, m, x, s, z, None, None),
+        lambda: ops.quant_matmul(4, out, m, x, s, z, 128, False),
+        lambda: QuantLinear(4, 256, 128, None, m, s, z)(x),
+        lambda: QuantLinear(4, 256, 128, 128, m, s, z)(None),
+        lambda: ops.row_norm(2, x[0]),
+        lambda: ops.row_norm(0, None),
+        lambda: ops.row_norm(2, x[0], 1.0),
     ]
     for call in cases:
         seen = []
@@ -92,3 +105,12 @@ def test_refusals_are_the_same(monkeypatch):
                     call()
                 seen.append((type(e.value), str(e.value)))
         assert seen[0] == seen[1]
+
+
+@pytest.mark.parametrize("kind", [float, int, np.int64, torch.tensor])
+def test_group_size_of_any_kind_that_int_takes(monkeypatch, kind):
+    m, s, z, _ = weights(4, 256, 128, 128)
+    layer = QuantLinear(4, 256, 128, kind(128), m, s, z)
+    x = torch.randn((3, 256), generator=torch.Generator().manual_seed(4)).half().cuda()
+    fast, slow = both(monkeypatch, lambda: layer(x))
+    assert torch.equal(fast, slow) and torch.equal(fast, QuantLinear(4, 256, 128, 128, m, s, z)(x))
