@@ -3,6 +3,8 @@
 #include "../../include/int4matmul_b200.h"
 
 #include <atomic>
+#include <condition_variable>
+#include <mutex>
 
 #include "common.cuh"
 
@@ -76,6 +78,49 @@ size_t i4mm_workspace_bytes(void) { return kCounterBytes + kPartialBytes; }
 
 namespace {
 
+// A multiply whose K range is cut into parts is two launches, and what the first leaves in the workspace belongs to the second.
+// Host threads that share a stream (and so its workspace) therefore take turns here, one whole multiply each; threads on other
+// workspaces do not wait.  (A caller's interpreter lock does not do this: it is given up during the call.)
+class WorkspaceTurn {
+public:
+    explicit WorkspaceTurn(const void* ws) : ws_(ws) {
+        std::unique_lock<std::mutex> lock(mutex_);
+        while (taken(ws)) {
+            ++waiting_;
+            cv_.wait(lock);
+            --waiting_;
+        }
+        next_ = first_;
+        first_ = this;
+    }
+    ~WorkspaceTurn() {
+        std::lock_guard<std::mutex> lock(mutex_);
+        WorkspaceTurn** at = &first_;
+        while (*at != this) at = &(*at)->next_;
+        *at = next_;
+        if (waiting_) cv_.notify_all();
+    }
+    WorkspaceTurn(const WorkspaceTurn&) = delete;
+    WorkspaceTurn& operator=(const WorkspaceTurn&) = delete;
+
+private:
+    static bool taken(const void* ws) {
+        for (const WorkspaceTurn* t = first_; t; t = t->next_)
+            if (t->ws_ == ws) return true;
+        return false;
+    }
+    static std::mutex mutex_;
+    static std::condition_variable cv_;
+    static WorkspaceTurn* first_;                         // the calls in progress (each on its thread's stack)
+    static int waiting_;
+    const void* ws_;
+    WorkspaceTurn* next_ = nullptr;
+};
+std::mutex WorkspaceTurn::mutex_;
+std::condition_variable WorkspaceTurn::cv_;
+WorkspaceTurn* WorkspaceTurn::first_ = nullptr;
+int WorkspaceTurn::waiting_ = 0;
+
 // The multiply behind both entries.  gather == nullptr: results go to `out` (rows, S).
 int multiply(int bits, int accumulate, int path, void* out, const i4mm::OutMap* gather, const void* matrix, const void* mask,
              const void* x, const void* scales, const void* zeros, int64_t rows, int64_t N, int64_t S, int64_t n_groups,
@@ -138,6 +183,7 @@ int multiply(int bits, int accumulate, int path, void* out, const i4mm::OutMap* 
     p.partials = (float*)((char*)workspace + kCounterBytes);
     p.status = (int*)((char*)workspace + kStatusOffset);
 
+    const WorkspaceTurn turn(workspace);
     cudaStream_t st = (cudaStream_t)stream;
     if (path == 0 && i4mm::rows_supported(bits, accumulate != 0, (int)rows, (int)N, (int)S)) {
         i4mm::set_last_shape(16);

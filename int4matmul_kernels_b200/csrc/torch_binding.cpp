@@ -171,6 +171,7 @@ void weight_matrix_packing(Tensor wt_outs, Tensor msk_outs, Tensor wt_in, Tensor
 // or no integer, memory that cannot be had, ...), or the scratch buffer of this stream does not exist yet, the caller is told so
 // (-1) and takes its own path, which raises, converts or allocates.  The arguments are therefore plain Python objects: a typed
 // signature would raise an error of its own first.
+// A launch may block when the stream's queue is full, so the interpreter's lock is given up over it, as ctypes does.
 
 // (an undefined tensor stands for None)
 bool as_tensor(const py::object& o, Tensor& t) {
@@ -230,6 +231,8 @@ int launch_checked(const Weights& w, bool matvec, int64_t path, void* out, const
     PyObject* const item = PyDict_GetItem(workspaces.ptr(), py::make_tuple((int)dev.index(), (uint64_t)(uintptr_t)stream).ptr());
     if (!item) return -1;
     const Tensor ws = py::cast<Tensor>(py::handle(item));
+    // (every tensor is held by a reference of this call's own)
+    py::gil_scoped_release release;
     return i4mm_quant_matmul((int)w.bits, matvec ? 1 : 0, (int)path, out, w.matrix.data_ptr(), sparse ? w.mask.data_ptr() : nullptr,
                              x.data_ptr(), w.scales.data_ptr(), w.zeros.data_ptr(), rows, in_size, out_size, w.scales.size(0),
                              w.group_size, ws.data_ptr(), (size_t)ws.numel(), (void*)stream);
@@ -298,8 +301,12 @@ py::object try_row_norm(int64_t mode, const py::object& a_, const py::object& b,
         const int64_t rows = a.size(0), width = a.size(1);
         const auto options = at::TensorOptions().dtype(torch::kHalf).device(a.device());
         Tensor y = (mode & ~(int64_t)I4MM_PATH_STATIC_WEIGHTS) == 4 ? at::empty({2, rows, width}, options) : at::empty({rows, width}, options);
-        const int status = i4mm_row_norm((int)mode, y.data_ptr(), ptr[0], ptr[1], ptr[2], rows, width, stride[0], stride[1], stride[2],
-                                         (void*)c10::cuda::getCurrentCUDAStream(a.device().index()).stream());
+        const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(a.device().index()).stream();
+        int status;
+        {
+            py::gil_scoped_release release;
+            status = i4mm_row_norm((int)mode, y.data_ptr(), ptr[0], ptr[1], ptr[2], rows, width, stride[0], stride[1], stride[2], (void*)stream);
+        }
         if (status != I4MM_OK) return py::int_(status);
         return py::cast(y);
     } catch (const c10::Error&) {

@@ -1,5 +1,8 @@
 """The compiled fast path of the Python entries (ops, QuantLinear) against the same calls through ctypes: equal results for
 everything both accept, and the same exceptions for what the entries refuse."""
+import threading
+import time
+
 import numpy as np
 import pytest
 import torch
@@ -114,3 +117,55 @@ def test_group_size_of_any_kind_that_int_takes(monkeypatch, kind):
     x = torch.randn((3, 256), generator=torch.Generator().manual_seed(4)).half().cuda()
     fast, slow = both(monkeypatch, lambda: layer(x))
     assert torch.equal(fast, slow) and torch.equal(fast, QuantLinear(4, 256, 128, 128, m, s, z)(x))
+
+
+def test_other_threads_run_while_a_launch_waits_for_room_in_the_queue():
+    m, s, z, _ = weights(4, 256, 128, 128)
+    layer = QuantLinear(4, 256, 128, 128, m, s, z)
+    x = torch.zeros((1, 256), dtype=torch.float16, device="cuda")
+    layer(x)
+    ops.row_norm(0, x)
+    torch.cuda.synchronize()
+    ticks, stop = [], threading.Event()
+
+    def tick():
+        while not stop.is_set():
+            ticks.append(time.monotonic())
+            time.sleep(0.005)
+    thread = threading.Thread(target=tick)
+    thread.start()
+    try:
+        for call in (lambda: layer(x), lambda: ops.row_norm(0, x)):
+            torch.cuda._sleep(2_000_000_000)                                    # about a second during which nothing is taken from the queue
+            for _ in range(3000):
+                call()
+            torch.cuda.synchronize()
+    finally:
+        stop.set()
+        thread.join()
+    gap = max(b - a for a, b in zip(ticks, ticks[1:]))
+    assert gap < 0.5, gap
+
+
+def test_threads_that_share_a_stream_do_not_mix_their_launches():
+    """Multiplies cut into K parts are two launches with sums in the stream's scratch between them."""
+    problems = []
+    for i, rows in enumerate((40, 48, 64, 8)):
+        m, s, z, _ = weights(4, 4096, 512, 128)
+        layer = QuantLinear(4, 4096, 512, 128, m, s, z)
+        x = torch.randn((rows, 4096), generator=torch.Generator().manual_seed(i)).half().cuda()
+        problems.append((layer, x, layer(x)))
+    torch.cuda.synchronize()
+    bad = []
+
+    def run(layer, x, want):
+        outs = [layer(x) for _ in range(300)]
+        torch.cuda.synchronize()
+        bad.extend(i for i, o in enumerate(outs) if not torch.equal(o, want))
+    threads = [threading.Thread(target=run, args=p) for p in problems]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad, len(bad)
+    ops.check_device_status()
