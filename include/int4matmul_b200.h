@@ -52,9 +52,10 @@ int i4mm_version(void);
 /* Kernels this library has launched in this process so far, over all entry points (a multiply is one launch,
  * or two where it cuts K into parts and reduces them).  For accounting in benchmarks; no reference counterpart. */
 unsigned long long i4mm_launch_count(void);
-/* What the last i4mm_quant_matmul call of this host thread launched on the tcgen05 path: rows per tile (the MMA's N:
- * 16, 32, 64, 128, 160, 192, 224 or 256) + 1000 if it ran as CTA pairs + 10000 * K parts; 16 after a call that took
- * the few-row kernel (up to 8 rows of a small matrix, path 0); 0 after a call that took the streaming path.  For tests that must know which kernel instance they exercised; no reference counterpart. */
+/* What the last i4mm_quant_matmul call of this host thread launched: on the tcgen05 path the rows per tile (the MMA's N:
+ * 16, 32, 64, 128, 160, 192, 224 or 256) + 1000 if it ran as CTA pairs + 10000 * K parts; 8 after a call that took the
+ * few-row kernel (up to 8 rows of a small matrix, path 0); 0 after a call that took the streaming path.  For tests that
+ * must know which kernel instance they exercised; no reference counterpart. */
 int i4mm_last_launch_shape(void);
 
 /*

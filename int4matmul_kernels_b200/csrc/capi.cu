@@ -186,7 +186,7 @@ int multiply(int bits, int accumulate, int path, void* out, const i4mm::OutMap* 
     const WorkspaceTurn turn(workspace);
     cudaStream_t st = (cudaStream_t)stream;
     if (path == 0 && i4mm::rows_supported(bits, accumulate != 0, (int)rows, (int)N, (int)S)) {
-        i4mm::set_last_shape(16);
+        i4mm::set_last_shape(8);
         p.rows = (int)rows;
         const cudaError_t e = i4mm::rows_launch(bits, sparse, p, overlap, st);
         return e == cudaSuccess ? I4MM_OK : fail_cuda(e);
