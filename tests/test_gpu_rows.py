@@ -8,7 +8,7 @@ import torch
 from int4matmul_kernels_b200 import capi, ops
 from oracle import reference_oracle as oracle
 
-from helpers import assert_parity, run_problem
+from helpers import assert_parity, run_problem, to_dev
 from test_gpu_stream import FORMATS, fmt_id, one_hot_problem
 
 pytestmark = pytest.mark.gpu
@@ -52,6 +52,31 @@ def test_which_calls_take_it(fmt, adds, rows, n, s, few):
     getattr(ops, f"quant_int{bits}_linear_mult_{'vec' if adds else 'mtx'}")(out, matrix, x, scales, zeros, -1, mask)
     assert took_few_rows() == (few == "all" or few == f"int{bits}") == expected_few_rows(bits, rows, n, s, adds)
     assert (out == torch.tensor((n // 2 if sparse else n) * 2.0 ** -10, dtype=torch.float16)).all()
+
+
+@pytest.mark.parametrize("fmt", FORMATS, ids=fmt_id)
+@pytest.mark.parametrize("m", [1, 3, 8])
+@pytest.mark.parametrize("n", [64, 192, 384])
+@pytest.mark.parametrize("tiles_per_sm", [4, 8])
+def test_ctas_that_walk_several_column_tiles(fmt, m, n, tiles_per_sm):
+    """More column tiles than CTAs fit on the GPU, with fewer 128-k steps per tile than a CTA has warps: copies run ahead
+    over tile borders and the sums' memory is used again."""
+    bits, sparse = fmt
+    s = 64 * (tiles_per_sm * torch.cuda.get_device_properties(0).multi_processor_count + tiles_per_sm // 4 * 2 - 1)
+    p = oracle.make_packed_problem(bits, n, s, m, 64, sparse=sparse, seed=n + m)
+    rng = np.random.default_rng(1)
+    cols = np.unique(np.concatenate([np.arange(192), s - 1 - np.arange(192), rng.integers(0, s, 400)]))
+    w = {k: to_dev(p[k]) if p[k] is not None else None for k in ("matrix", "mask", "scales", "zeros", "x")}
+    outs = []
+    for path in (capi.PATH_AUTO, capi.PATH_STATIC_WEIGHTS, capi.PATH_AUTO):
+        outs.append(torch.empty((1, m, s), dtype=torch.float16, device="cuda"))
+        getattr(ops, f"quant_int{bits}_linear_mult_mtx")(outs[-1], w["matrix"], w["x"], w["scales"], w["zeros"], 64, w["mask"], path=path)
+        assert took_few_rows() == expected_few_rows(bits, m, n, s, False)
+    torch.cuda.synchronize()
+    assert expected_few_rows(bits, m, n, s, False) or (m > 1 and n * s > 2 ** 24)
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    want, bound = oracle.expected_columns(bits, p["matrix"], p["mask"], p["scales"], p["zeros"], 64, p["x"], cols)
+    assert_parity(outs[0].cpu().numpy()[..., cols], want, bound, f"{fmt} m={m} {n}x{s}")
 
 
 @pytest.mark.parametrize("fmt", FORMATS, ids=fmt_id)
