@@ -73,8 +73,8 @@ template <bool PERM>
 struct UFormat<4, false, PERM> {
     static constexpr int WROWS = 8, MROWS = 0;       // packed rows / mask rows per 64-k part
     static constexpr bool kPermutedK = PERM;
-    template <int MODE>
-    __device__ static __forceinline__ void decode(uint32_t wbase, uint32_t, const ColK& c, uint32_t (&A)[32], const uint32_t*) {
+    template <int MODE, class Entry>
+    __device__ static __forceinline__ void decode(uint32_t wbase, uint32_t, const ColK& c, uint32_t (&A)[32], const Entry*) {
         if (PERM) {
             // nibbles j and j + 4 of a word sit at the same offset of its two 16-bit halves: one LOP3 per pair plants both
             // into the mantissas of (1024, 1024); the odd nibbles come out multiplied by 16
@@ -107,8 +107,8 @@ template <bool PERM>
 struct UFormat<2, false, PERM> {
     static constexpr int WROWS = 4, MROWS = 0;
     static constexpr bool kPermutedK = false;
-    template <int MODE>
-    __device__ static __forceinline__ void decode(uint32_t wbase, uint32_t, const ColK& c, uint32_t (&A)[32], const uint32_t*) {
+    template <int MODE, class Entry>
+    __device__ static __forceinline__ void decode(uint32_t wbase, uint32_t, const ColK& c, uint32_t (&A)[32], const Entry*) {
         const uint32_t offa = hsub2_u(BASE_1_4, c.z2), offb = hsub2_u(BASE_16_64, c.z2);
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
@@ -130,8 +130,8 @@ template <bool PERM>
 struct UFormat<3, false, PERM> {
     static constexpr int WROWS = 6, MROWS = 0;
     static constexpr bool kPermutedK = false;
-    template <int MODE>
-    __device__ static __forceinline__ void decode(uint32_t wbase, uint32_t, const ColK& c, uint32_t (&A)[32], const uint32_t*) {
+    template <int MODE, class Entry>
+    __device__ static __forceinline__ void decode(uint32_t wbase, uint32_t, const ColK& c, uint32_t (&A)[32], const Entry*) {
         const uint32_t off = hsub2_u(BASE_1_8, c.z2);
 #pragma unroll
         for (int blk = 0; blk < 2; ++blk) {
@@ -161,8 +161,8 @@ template <bool PERM>
 struct UFormat<4, true, PERM> {
     static constexpr int WROWS = 4, MROWS = 2;
     static constexpr bool kPermutedK = false;
-    template <int MODE>
-    __device__ static __forceinline__ void decode(uint32_t wbase, uint32_t mbase, const ColK& c, uint32_t (&A)[32], const uint32_t* lut) {
+    template <int MODE, class Entry>
+    __device__ static __forceinline__ void decode(uint32_t wbase, uint32_t mbase, const ColK& c, uint32_t (&A)[32], const Entry* lut) {
 #pragma unroll
         for (int blk = 0; blk < 2; ++blk) {
             // a 32-block of this column: the 64-bit word of its 16 kept nibbles (in increasing k) and its keep-mask
@@ -190,6 +190,21 @@ struct WStage {     // one stage of the packed-weight ring: one unit = H parts o
 
 constexpr int kMaxWStages = 16;
 constexpr int kMaxABStages = 6;
+
+// Look-up table of the 16:32 expansion.  Entries of 4 bytes are the better ones everywhere (96 rows 5120 x 20480: 52.0 us, 56.3 with
+// 16 bytes) but with tiles of 64 rows, where two CTAs on an SM keep the ALU pipe full and what counts is instructions (48 rows
+// 5120 x 20480: 64.2 and 55.6, 20480 x 5120: 47.8 and 44.7).
+// kFastBound: the fast mode takes zero-points up to 127 / 255, whose fp16 bits + kFastBound = 0x7FFF.
+template <bool SPARSE, int NT>
+struct SparseTable {
+    using Entry = uint32_t;
+    static constexpr uint32_t kFastBound = 0x280Fu;
+};
+template <>
+struct SparseTable<true, 64> {
+    using Entry = uint4;
+    static constexpr uint32_t kFastBound = 0x2407u;
+};
 
 template <int NT, bool PAIR>
 struct Cfg {
@@ -292,7 +307,7 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const UmmaParams p, const __h
     constexpr int kABStages = ABStages<NT, PAIR>::value;
     extern __shared__ __align__(1024) unsigned char smem[];      // [B ring (1024-aligned tiles)][W ring]
     __shared__ __align__(8) Barriers bars;
-    __shared__ uint32_t lut[SPARSE ? kSparseLutEntries : 1];
+    __shared__ typename SparseTable<SPARSE, NT>::Entry lut[SPARSE ? kSparseLutEntries : 1];
     __shared__ uint32_t tmem_base_smem;
     __shared__ volatile int s_abort;     // set by a warp that gives up on the accumulator (the MMA warp before it releases the epilogue
                                          // warps for the last time; an epilogue warp before its group's next named barrier)
@@ -337,7 +352,7 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const UmmaParams p, const __h
             }
             ptx::fence_mbar_init();
         }
-        if (SPARSE && warp < 8) lut[warp * 32 + lane] = sparse_selectors(warp * 32 + lane);   // (warps 0..7 are dequant warps in every configuration)
+        if (SPARSE && warp < 8) sparse_table_entry(lut[warp * 32 + lane], warp * 32 + lane);   // (warps 0..7 are dequant warps in every configuration)
         if (warp == kMma) {
             if (PAIR) {
                 ptx::tmem_alloc_pair(ptx::smem_u32(&tmem_base_smem), C::kTmemCols);
@@ -926,10 +941,10 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const UmmaParams p, const __h
                         c.z2 = prmt(zz, zz, 0x1010);
                         c.zb = 0;
                     };
-                    // fast mode needs: scale sign clear, zero-point an integer in [0, 512] ([0, 127] for the sparse format)
+                    // fast mode needs: scale sign clear, zero-point an integer in [0, 512] (sparse format: see SparseTable)
                     auto not_fast_bits = [&](const ColK& c) -> uint32_t {
                         const uint32_t zr = hadd2_u(hadd2_u(c.z2, kMagic1024), H2_N1024);
-                        constexpr uint32_t kAdd = SPARSE ? 0x280Fu : 0x1FFFu;
+                        constexpr uint32_t kAdd = SPARSE ? SparseTable<SPARSE, NT>::kFastBound : 0x1FFFu;
                         const uint32_t zlo = c.z2 & 0xFFFFu;
                         return ((zlo | ((zlo & 0x7FFFu) + kAdd) | c.s2) & 0x8000u) | (zr ^ c.z2);
                     };

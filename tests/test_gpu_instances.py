@@ -9,7 +9,7 @@ from int4matmul_kernels_b200 import capi, ops
 from oracle import reference_oracle as oracle
 
 from helpers import assert_parity, device_problem, run_problem, to_dev
-from test_gpu_stream import FORMATS, fmt_id
+from test_gpu_stream import FORMATS, fmt_id, one_hot_problem
 
 pytestmark = pytest.mark.gpu
 
@@ -188,3 +188,51 @@ def test_overlapped_launches_keep_stream_order_for_activations_and_outputs(m):
     want, _, bound = oracle.expected(probs[0])
     assert_parity(out.cpu().numpy(), want, bound, f"first link m={m}")
     ops.check_device_status()
+
+
+def modes_along_k(p, seed):
+    """Groups of integer, fractional, byte-sized (up to 255), larger and exponent-coded weights in turn, along K and from one
+    column tile to the next, with stretches of plain ones between them."""
+    rng = np.random.default_rng(seed)
+    groups, s = p["zeros"].shape
+    for g in range(groups):
+        for c in range(0, s, 64):
+            at = (g, slice(c, c + 64))
+            kind = (0, 0, 0, 1, 2, 2, 2, 2, 0, 3, 0, 4, 4, 2, 1, 0)[(g + 5 * (c // 128) + (c // 64) % 2) % 16]
+            if kind == 1:
+                p["zeros"][at] = (p["zeros"][at].astype(np.float32) + rng.uniform(-0.5, 0.5, 64)).astype(np.float16)
+            elif kind == 2:
+                p["zeros"][at] = rng.integers(128, 256, 64)
+            elif kind == 3:
+                p["zeros"][at] = rng.integers(256, 900, 64)
+            elif kind == 4:
+                p["scales"][at] = -p["scales"][at]
+    return p
+
+
+@pytest.mark.parametrize("fmt", FORMATS, ids=fmt_id)
+@pytest.mark.parametrize("path,m", [(capi.PATH_AUTO, 1), (capi.PATH_AUTO, 8), (PAIR, 8), (PAIR, 24), (PAIR, 50), (SINGLE, 128),
+                                    (PAIR, 128), (SINGLE, 192), (PAIR, 192), (SINGLE, 256), (PAIR, 256)])
+def test_dequantisation_modes_that_change_along_k(fmt, path, m):
+    bits, sparse = fmt
+    n, s, g = 4096 + 192, 128 * 5, 64
+    p = modes_along_k(oracle.make_problem(bits, n, s, m, g, sparse=sparse, seed=m), m)
+    nt = next(t for t in (16, 32, 64, 128, 192, 256) if t >= m)
+    got = run_problem(p, path=path if path == capi.PATH_AUTO else forced(path, nt))
+    assert last_shape() % 10000 == (8 if path == capi.PATH_AUTO else nt + (1000 if path == PAIR and nt >= 128 else 0))
+    want, _, bound = oracle.expected(p, outs_in=np.zeros((1, 1, s), np.float16) if m == 1 else None)
+    assert_parity(got, want, bound, f"{fmt} m={m} path={path}")
+
+
+@pytest.mark.parametrize("path", [capi.PATH_AUTO, PAIR], ids=["auto", "pair"])
+@pytest.mark.parametrize("zeros", [(100, 128), (128, 256), (250, 260)])
+def test_sparse_weights_with_byte_sized_zero_points_are_bit_exact(path, zeros):
+    """x = rows of the identity: the outputs are the fp16 weights, dropped ones exact zeros."""
+    p = one_hot_problem(4, True, 256, 128, 64, 11, "integer")
+    p["zeros"] = np.random.default_rng(2).integers(*zeros, p["zeros"].shape).astype(np.float16)
+    w16 = oracle.dequant_w16(4, p["q"], p["scales"], p["zeros"], 64, p["keep"])
+    eye = p["x"][0]
+    for rows in (8, 256):
+        for lo in range(0, 256, rows):
+            got = run_problem(dict(p, x=np.ascontiguousarray(eye[lo:lo + rows])[None], m=rows), path=path)[0]
+            assert np.array_equal(got.view(np.uint16), w16[lo:lo + rows].view(np.uint16))
