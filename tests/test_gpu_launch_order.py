@@ -9,8 +9,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("bits,sparse", [(4, False), (3, False), (4, True)])
-@pytest.mark.parametrize("m", [1, 8, 24, 64, 200])
-def test_weights_written_by_the_preceding_kernel_are_seen(bits, sparse, m):
+@pytest.mark.parametrize("m,path", [(1, 0), (1, 2), (8, 0), (8, 2), (24, 0), (64, 0), (200, 0)])
+def test_weights_written_by_the_preceding_kernel_are_seen(bits, sparse, m, path):
     n, s = 2048, 1536
     w = [packing.synthetic_weights(bits, n, s, 128, sparse=sparse, seed=i) for i in range(2)]
     # scales from a row-norm launch: that kernel lets its successor start before it has written anything
@@ -24,7 +24,8 @@ def test_weights_written_by_the_preceding_kernel_are_seen(bits, sparse, m):
         if sync:
             torch.cuda.synchronize()
         out = torch.empty((1, m, s), dtype=torch.float16, device="cuda")
-        getattr(ops, f"quant_int{bits}_linear_mult_mtx")(out, matrix, x, scales, w[i]["zeros"], 128, w[i]["mask"])
+        getattr(ops, f"quant_int{bits}_linear_mult_mtx")(out, matrix, x, scales, w[i]["zeros"], 128, w[i]["mask"], path=path)
+        assert (capi.load().i4mm_last_launch_shape() == 8) == (path == 0 and m <= 8)      # few-row kernel
         return out
     want = [step(i, True) for i in range(2)]
     torch.cuda.synchronize()
