@@ -61,8 +61,8 @@ DEFAULT_WORKLOAD = "int4_matmul_m2048_5120x20480"
 MATVEC_WORKLOAD = "int4_matvec_16384"            # the other half of the metric: timed by the default run as well
 
 # DRAM bytes per launch of the dominant kernel (dram__bytes_read.sum + dram__bytes_write.sum of one ncu capture of
-# the unsharded workload), with the first 12 hex digits of the SHA-256 of csrc/umma_kernel.cu as it was when the
-# capture was made: the figure is printed only while the kernel source still is that file, else `traffic` is null.
+# the unsharded workload), with the first 12 hex digits of the SHA-256 of the kernel's source files (kernel_source_tag) as they
+# were when the capture was made: the figure is printed only while they still are those files, else `traffic` is null.
 NCU_TRAFFIC_BYTES = {
     "int4_matmul_m2048_5120x20480": (224119296 + 67726080, "3e9726a8cb99"),
     "int4_matvec_16384": (143103744 + 4355072, "3e9726a8cb99"),
@@ -146,9 +146,16 @@ def cpu_problem(w, seed=0):
 
 def kernel_source_tag():
     import hashlib
-    path = os.path.join(ROOT, "int4matmul_kernels_b200", "csrc", "umma_kernel.cu")
-    with open(path, "rb") as f:
-        return hashlib.sha256(f.read()).hexdigest()[:12]
+    digest = hashlib.sha256()
+    for name in ("umma_kernel.cu", "dequant.cuh", "common.cuh", "ptx.cuh"):
+        with open(os.path.join(ROOT, "int4matmul_kernels_b200", "csrc", name), "rb") as f:
+            digest.update(f.read())
+    return digest.hexdigest()[:12]
+
+
+def kernel_name(launch_shape):
+    """The kernel behind an i4mm_last_launch_shape() value."""
+    return "rows_kernel (mma.sync)" if launch_shape == 8 else "umma_kernel (tcgen05)" if launch_shape else "stream_kernel (mma.sync)"
 
 
 def ncu_traffic(name, world):
@@ -417,6 +424,18 @@ def run_stack(args):
         dist.all_reduce(t, op=dist.ReduceOp.MAX)
         ms_e2e = float(t.item())
 
+    # which kernels a pass runs (one more pass, outside the timed region)
+    kernels, linear = set(), stack._linear
+
+    def recorded_linear(*a):
+        parts = linear(*a)
+        kernels.add(kernel_name(capi.load().i4mm_last_launch_shape()))
+        return parts
+    stack._linear = recorded_linear
+    stack.forward(h0)
+    del stack._linear
+    torch.cuda.synchronize()
+
     # ---- parity, outside the timed region: layer 0's q|k|v multiply of this rank's shard against the CPU oracle on
     # sampled columns, and (several GPUs) the gathered buffer: this rank's block bit-equal to its own product, the
     # whole buffer identical on every rank ----
@@ -497,7 +516,7 @@ def run_stack(args):
                         l2=f"{cfg.layers * wpl // 2 / 1e9:.1f} GB of weights per pass (>> L2)",
                         timed_as="one CUDA graph of the K steps" if graph is not None else "K direct launches"),
             roofline=dict(bound=kind, achieved=achieved, peak=peak, unit=unit, frac=achieved / peak, traffic=None,
-                          peak_source=peaks["source"], kernel="umma_kernel (tcgen05)",
+                          peak_source=peaks["source"], kernel=" + ".join(sorted(kernels)),
                           note="whole pass incl. normalisation kernels and all-gathers, per GPU; sustained peak for tensor"),
             parity=parity, cpu_baseline=None,
             e2e=dict(value=units / (ms_e2e / args.steps / 1e3), unit=unit, h2d_bytes_per_step=h_host.numel() * 2,
@@ -612,7 +631,6 @@ def run_workload(args, name, w, ctx):
             out_all.zero_()
         ops.quant_matmul(w["bits"], outs[i % n_out], L["matrix"], x, L["scales"], L["zeros"], w["g"], L["mask"], path=args.path)
 
-    use_umma = args.path != 1                       # automatic = the tcgen05 kernel for every row count
     for i in range(max(args.warmup, 3)):
         step(i)
     torch.cuda.synchronize()
@@ -706,7 +724,7 @@ def run_workload(args, name, w, ctx):
         achieved, peak, runit = tfs, peaks["tf_burst"], "TFLOP/s"
     roofline = dict(bound=kind, achieved=achieved, peak=peak, unit=runit, frac=achieved / peak,
                     traffic=ncu_traffic(name, world), peak_source=peaks["source"],
-                    us_per_launch=us_launch, kernel="umma_kernel (tcgen05)" if use_umma else "stream_kernel (mma.sync)",
+                    us_per_launch=us_launch, kernel=kernel_name(shape),
                     launch_shape=shape, frac_of_nominal=achieved / (8000.0 if kind == "hbm" else 2250.0),
                     frac_of_sustained_bf16=(tfs / peaks["tf_sustained"]) if kind == "tensor" else None)
     if 16 <= w["m"] <= 256:
