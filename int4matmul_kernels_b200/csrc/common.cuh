@@ -122,7 +122,7 @@ struct StreamParams {
     int CT;                  // ceil(S / 128)
     int accumulate;          // out = half(float(out) + acc) instead of overwrite
     GroupDiv gdiv;
-    OutMap om;               // tcgen05 kernel only: destinations of the result (dst[0] == out for the ordinary entry)
+    OutMap om;               // tcgen05 and few-row kernels: destinations of the result (dst[0] == out for the ordinary entry)
 };
 
 // Counts kernel launches of this library in this process (read through i4mm_launch_count); defined in capi.cu.

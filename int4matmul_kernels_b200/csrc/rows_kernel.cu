@@ -568,11 +568,12 @@ cudaError_t rows_launch_fmt(const RowsParams& p, int sms, int dev, cudaStream_t 
 // column tiles per SM on, K cannot be cut any more and SMs are left with uneven numbers of tiles: 1024 x 30720 16.5 -> 14.3,
 // 1024 x 37888 14.4 -> 14.4, 1024 x 40960 18.4 -> 19.4 (16:32 21.9 -> 25.2), 16:32 2304 x 20480 20.6 -> 22.5.
 // A call that overwrites stands between others in a model's layer, and there a change of kernel from one matrix to the next costs
-// 2..5 us (the next kernel's launch no longer overlaps).  min(N, S) is the layer's width for its every matrix, so a bound on it keeps
-// a layer on one kernel: four matrices and their row norms, one row, int4 5120 wide with only the 5120^2 one on this kernel
-// 86.5 -> 91.5 and 4096 (11008) 72.3 -> 73.8, but 3072 (5120), all four on it, 56.5 -> 49.9 and 2048 (5632) 53.3 -> 44.2.  int2 is the
-// exception (its decode is cheapest here): 5120 83.0 -> 84.5 but 4096 (11008) 69.6 -> 65.1.  With 4 rows int4 4096 79.1 -> 81.6, 2048
-// 58.7 -> 50.4; with 8 rows 3072 69.2 -> 73.7, 2048 67.0 -> 61.3 (5..8 rows have larger stages and fewer of them).
+// 2..5 us.  min(N, S) is the layer's width for its every matrix, so a bound on it keeps a layer on one kernel.  Four matrices and
+// their row norms, width (inner width), all on the tcgen05 kernel -> those of up to 48 Mi weights (2..8 rows: 16 Mi) on this one:
+// one int4 row 5120 (13824) 84.6 -> 89.7, 4096 (11008) 69.3 -> 71.9, 3584 (9472) 61.5 -> 63.3, but 3072 (8192) 56.8 -> 50.1, 2048 (5632)
+// 49.7 -> 38.1.  int2 is the exception, its decode is cheapest here: 5120 82.9 -> 83.4, 4096 68.9 -> 63.7.  4 rows int4 4096 74.8 -> 79.9,
+// 3072 62.1 -> 63.7, 2560 (6912) 57.7 -> 56.9, 2048 54.9 -> 46.3; 8 rows (larger stages, fewer of them) 3072 71.4 -> 73.1, 2560 65.4 ->
+// 64.6, 2048 63.5 -> 56.0.  (Alone and back to back, 4096^2 would still be faster here: one row 10.9 -> 8.4.)
 // Very long columns: the last part adds the sums of hundreds of parts one after the other, 4 rows 131072 x 64 77 -> 62 but 262144 x 64
 // 79 -> 120, 8 rows 65536 x 64 98 -> 63 but 131072 x 64 99 -> 121.
 // (The bounds also keep step and tile numbers far inside 32 bits.)
