@@ -12,7 +12,7 @@ from __future__ import annotations
 
 import torch
 
-from . import packing
+from . import capi, ops, packing
 
 
 def quantize_groupwise(weight: torch.Tensor, bits: int = 4, group_size: int = 128, sparse: bool = False):
@@ -78,7 +78,6 @@ class QuantLinear(torch.nn.Module):
         return cls(bits, n, s, group_size, matrix, qz["scales"].to(device), qz["zeros"].to(device), mask)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        from . import capi, ops
         mod = ops.native()
         if mod:
             y = mod._try_linear(self.bits, capi.PATH_STATIC_WEIGHTS if ops._static_weights else capi.PATH_AUTO, x, self.in_features,

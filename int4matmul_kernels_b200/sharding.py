@@ -17,7 +17,7 @@ from typing import Callable, Optional
 import torch
 import torch.distributed as dist
 
-from . import packing
+from . import capi, ops, packing
 
 
 def column_range(s: int, rank: int, world: int) -> tuple[int, int]:
@@ -66,7 +66,6 @@ class QuantWeights:
 
 def cuda_multiply(w: QuantWeights, x: torch.Tensor) -> torch.Tensor:
     """x (rows, N) fp16 CUDA -> (rows, w.s) fp16 through the library (overwrite semantics)."""
-    from . import ops
     out = torch.empty((1, x.shape[0], w.s), dtype=torch.float16, device=x.device)
     fn = getattr(ops, f"quant_int{w.bits}_linear_mult_mtx")
     fn(out, w.matrix, x.view(1, x.shape[0], x.shape[1]), w.scales, w.zeros, w.group_size, w.mask)
@@ -91,7 +90,6 @@ class PeerGather:
 
     def __init__(self, shapes: dict, rank: int, world: int, device, group=None):
         import ctypes
-        from . import capi
         self.lib = capi.load()
         self.rank, self.world, self.device = rank, world, torch.device(device)
         self.names = list(shapes)
@@ -126,14 +124,12 @@ class PeerGather:
             dist.barrier(group=group)           # nobody writes before everybody has mapped
 
     def _check(self, status: int, what: str) -> None:
-        from . import capi, ops
         if status != capi.OK:
             raise ops.Int4MatmulError(status, what)
 
     def multiply(self, name: str, w: QuantWeights, x: torch.Tensor, parts: int = 1) -> list:
         """x (rows, N) times this rank's shard `w`, written into every rank's gathered buffer `name`, then the hand-shake.
         Returns the `parts` gathered matrices as column slices (rows, S_part) of the local buffer."""
-        from . import capi, ops
         rows_max, ld = self.shapes[name]
         rows = x.shape[0]
         if rows > rows_max or w.s * self.world != ld:
@@ -300,7 +296,6 @@ class DecoderStack:
         """v / rms(v) per row with v = a (mode 0), a + b + c (1), a + b / rms(b) (2), a * b (3), in fp32.
         One fused kernel on CUDA tensors; the same expression in torch ops on CPU tensors (host-logic tests)."""
         if a.is_cuda:
-            from . import ops
             return ops.row_norm(mode, a, b, c)
 
         def rn(f):
@@ -314,7 +309,6 @@ class DecoderStack:
         """(combine(2, a, b), combine(0, of that)): a layer's output and the next layer's normalised input; one launch
         on CUDA tensors."""
         if a.is_cuda:
-            from . import ops
             both = ops.row_norm(4, a, b)
             return both[0], both[1]
         h = cls.combine(2, a, b)
