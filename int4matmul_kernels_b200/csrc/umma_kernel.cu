@@ -30,6 +30,7 @@
 #include <cuda.h>
 #include <dlfcn.h>
 
+#include <cstddef>
 #include <atomic>
 #include <mutex>
 #include <type_traits>
@@ -38,6 +39,10 @@
 #include "dequant.cuh"
 #include "ptx.cuh"
 
+namespace i4mm {
+int g_tune[16] = {0, 2};
+}
+extern "C" void i4mm_tune(int i, int v) { i4mm::g_tune[i] = v; }
 namespace i4mm {
 
 namespace {
@@ -211,7 +216,7 @@ template <int NT, bool PAIR>
 struct Cfg {
     // packed-weight ring (128 k per stage).  Few rows: the kernel streams weights from HBM, and the ring has to
     // cover the DRAM latency; many rows: weights are a trickle next to the activation tiles
-    static constexpr bool kStream = NT <= 64;                         // weight-streaming shapes: one CTA per SM with everything doubled
+    static constexpr bool kStream = NT <= 32;                         // weight-streaming shapes: one CTA per SM with everything doubled
     // NT = 128..192: an MMA of N <= 192 takes 512..768 cycles per 128 k, the dequantisation of its weights with two
     // warpgroups ~1400, so these shapes get four warpgroups as well, and a deeper weight ring
     // (single CTAs have the shared memory for the 4 A / activation stages that four warpgroups need only at NT = 128)
@@ -227,13 +232,14 @@ struct Cfg {
     // complete, expect_tx + the copy's issue another ~190): at 128 k per stage that alone is ~27 us for 16384 x 16384
     // weights on 148 SMs, so the weight-streaming shapes use 256-k units.
     static constexpr int kHalves = kStream ? 4 : 2;
-    static constexpr int kWStages = kStream ? (NT <= 32 ? 9 : 6) : kDequantBound ? 6 : 3;
+    static constexpr int kWStages = kStream ? (NT <= 16 ? 9 : 6) : NT <= 64 ? 8 : kDequantBound ? 6 : 3;
     // staging slots (units of look-ahead) for activation rows that are reordered on their way into the A / activation
     // stages (umma_kernel's PERM)
     static constexpr int kXStaging = 4;
     static constexpr int kWG = kStream ? 3 : kDequantBound ? 4 : 2;   // dequant warpgroups (4 warps each), taking units in turn
     static constexpr int kABStages = kStream ? 3 : NT == 128 ? 4 : 3;   // ring of (A in tensor memory, activation tile in shared memory) pairs, one unit per stage
     static constexpr bool kWGuard = kWStages % kWG != 0;
+    static constexpr bool kEpiWarps = NT >= 128 || kStream;           // a warpgroup of its own for the epilogue (else dequant warpgroup 0 does it)
     static constexpr bool kEpiTransposed = NT >= 128;                 // epilogue stores go through a shared-memory transposition tile
     static constexpr bool kEpiHandoff = kStream;                      // the MMA warp waits for the accumulator and wakes the epilogue warps (named barrier)
     static constexpr bool kDeferArrive = kStream;                     // a dequant warp announces an A stage only before its next wait (hides the tcgen05.wait::st latency)
@@ -244,16 +250,19 @@ struct Cfg {
     // thread's loop (wait ~190 cycles, expect_tx + copies ~250) delivers a 16 KB stage per ~500-700 cycles, about
     // 4-5 TB/s over the whole GPU, which is less than the memory system can stream.
     static constexpr int kWProducers = kStream ? 2 : 1;
-    static constexpr int kWarps = 4 * kWG + 4 * kEpiGroups + 3 + (kWProducers - 1);  // + weight producer(s), activation producer, MMA issuer
+    static constexpr int kWarps = 4 * kWG + (kEpiWarps ? 4 * kEpiGroups : 0) + 3 + (kWProducers - 1);  // + weight producer(s), activation producer, MMA issuer
     static constexpr int kThreads = kWarps * 32;
     static constexpr int kDCols = NT < 32 ? 32 : NT;                  // accumulator columns
     static constexpr int kACol0 = kDCols;                             // A stages follow: 32 columns per 64 k
     static constexpr int kAStageCols = 32 * kHalves;
     static constexpr int kColsUsed = kDCols + kAStageCols * kABStages;
     static constexpr int kTmemCols = kColsUsed <= 256 ? 256 : 512;
-    static constexpr bool kSplit = kStream;                           // split-K over CTAs with a scratch reduction
-    static constexpr int kSlotElems = NT * 128;                   // 64-bit words of one CTA's partial tile in the scratch
-    static constexpr int kMinBlocks = 1;
+    // split-K over CTAs with a scratch reduction.  The code handles tiles of up to 128 rows, but the reducing CTA reads
+    // its partners' partial tiles in dependent L2 round trips (rows x partners / 8 of them): measured at 128 rows that
+    // costs 15-30 K cycles per tile and loses more than the better balance gains, so only the few-row shapes split.
+    static constexpr bool kSplit = NT <= 32;
+    static constexpr int kSlotElems = kDCols * 128;                   // 64-bit words of one CTA's partial tile in the scratch
+    static constexpr int kMinBlocks = kStream ? 1 : NT <= 64 ? 2 : 1;
 };
 
 // A / activation stages.  A CTA of a pair holds only half of each activation tile, which leaves shared memory for as
@@ -279,16 +288,314 @@ struct TensorMaps {
     CUtensorMap z;
 };
 
+// The dequant warps: every unit of [t_lo, t_hi) that is this warpgroup's turn.  after_segment(...) is called by warpgroup 0
+// of the configurations without epilogue warps.  Returns the number of segments, or -1 after a wait that timed out.
+template <class F, int NT, bool PAIR, class Entry, class AfterSegment>
+__device__ __forceinline__ int dequant_units(const UmmaParams& p, uint32_t bars, uint32_t w_ring, uint32_t tmem_base, long long t_lo, long long t_hi,
+                                             const Entry* lut, const AfterSegment& after_segment) {
+    using C = Cfg<NT, PAIR>;
+    constexpr bool SPARSE = F::MROWS != 0;
+    constexpr int H = C::kHalves, kABStages = ABStages<NT, PAIR>::value;
+    using WS = WStage<F, H>;
+    const int lane = threadIdx.x & 31, warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0);
+    const long long U = p.U;
+    auto bar = [&](size_t first, uint32_t i) { return bars + (uint32_t)first + 8 * i; };
+                const int wg = warp >> 2;                                           // warpgroup: takes every kWG-th weight stage
+                const int col = (warp & 3) * 32 + lane;                             // weight column in the tile = tensor-memory lane
+                const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
+                uint32_t si0 = 0, seg = 0;                                           // si0: weight stages consumed before this segment
+                int pending = -1;                                                    // A stage written but not yet announced (Cfg::kDeferArrive)
+                // the stores into tensor memory are complete -> the stage may be read by the MMAs
+                auto announce = [&](uint32_t stage) {
+                    ptx::tc_wait_st();
+                    ptx::tc_fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) {
+                        if (PAIR) ptx::mbar_arrive_cluster(ptx::map_to_cta(bar(offsetof(Barriers, ab_full), stage), 0));
+                        else ptx::mbar_arrive(bar(offsetof(Barriers, ab_full), stage));
+                    }
+                };
+                bool ok = true;
+                for (long long t = t_lo; t < t_hi && ok;) {
+                    const long long tile = div_nn(t, U);
+                    const int u0 = (int)(t - tile * U);
+                    const int u1 = (int)min(U, u0 + (t_hi - t));
+                    // this warpgroup's units of the segment: those whose stage index is congruent to wg modulo kWG
+                    for (int u = u0 + (int)(((uint32_t)wg + (uint32_t)C::kWG - si0 % (uint32_t)C::kWG) % (uint32_t)C::kWG); u < u1; u += C::kWG) {
+                        const uint32_t si = si0 + (uint32_t)(u - u0);
+                        const uint32_t ws = si % C::kWStages, wph = (si / C::kWStages) & 1u;     // constants: multiply-shift, no division
+                        if (C::kWGuard && !ptx::mbar_wait(bar(offsetof(Barriers, w_empty), ws), wph ^ 1u)) {   // see Cfg::kWStages
+                            if (lane == 0) atomicExch(p.status, 35);
+                            ok = false;
+                            break;
+                        }
+                        if (!ptx::mbar_wait(bar(offsetof(Barriers, w_full), ws), wph)) {
+                            if (lane == 0) atomicExch(p.status, 31);
+                            ok = false;
+                            break;
+                        }
+                        const uint32_t st = w_ring + ws * WS::kBytes;
+                        const uint32_t g0 = p.gdiv((uint32_t)H * (uint32_t)u);
+                        const uint32_t as = si % kABStages, aph = (si / kABStages) & 1u;
+                        // polled before the first part is decoded, so that the answer costs no latency when it is needed
+                        const bool free_early = ptx::mbar_test_wait(bar(offsetof(Barriers, ab_free), as), aph ^ 1u);
+                        // scale and zero-point of this thread's column in row `row` of the stage's group box, both halves of a register
+                        auto load_group = [&](uint32_t row, ColK& c) {
+                            const uint32_t sz = ptx::lds32(st + WS::kS + row * 256 + (col & ~1) * 2) >> (16 * (col & 1));
+                            const uint32_t zz = ptx::lds32(st + WS::kZ + row * 256 + (col & ~1) * 2) >> (16 * (col & 1));
+                            c.s2 = prmt(sz, sz, 0x1010);
+                            c.z2 = prmt(zz, zz, 0x1010);
+                            c.zb = 0;
+                        };
+                        // fast mode needs: scale sign clear, zero-point an integer in [0, 512] (sparse format: see SparseTable)
+                        auto not_fast_bits = [&](const ColK& c) -> uint32_t {
+                            const uint32_t zr = hadd2_u(hadd2_u(c.z2, kMagic1024), H2_N1024);
+                            constexpr uint32_t kAdd = SPARSE ? SparseTable<SPARSE, NT>::kFastBound : 0x1FFFu;
+                            const uint32_t zlo = c.z2 & 0xFFFFu;
+                            return ((zlo | ((zlo & 0x7FFFu) + kAdd) | c.s2) & 0x8000u) | (zr ^ c.z2);
+                        };
+                        // after the last read of the weight stage
+                        auto release_weights = [&]() {
+                            __syncwarp();
+                            if (lane == 0) ptx::mbar_arrive(bar(offsetof(Barriers, w_empty), ws));
+                        };
+                        // before the first store into the A stage
+                        auto acquire_a_stage = [&]() -> bool {
+                            if (C::kDeferArrive && pending >= 0) announce(pending);       // before any wait: the MMAs must be able to go on
+                            // the A stage (and its activation tile) is free once the MMAs of its previous use have completed
+                            if (!free_early && !ptx::mbar_wait(bar(offsetof(Barriers, ab_free), as), aph ^ 1u)) {
+                                if (lane == 0) atomicExch(p.status, 32);
+                                return false;
+                            }
+                            ptx::tc_fence_after_sync();
+                            return true;
+                        };
+                        // The parts are decoded in the fast mode by straight-line code, without a mode decision in between;
+                        // whether every group of the unit really is in the fast mode (for every column of the warp) is
+                        // voted once, when the last group has been read and before the weight stage is released.  If not,
+                        // the unit is decoded again with a decision per part (the stores are simply overwritten).
+                        bool redo = false;
+                        {
+                            ColK c;
+                            uint32_t cur_row = 0xFFFFFFFFu, nf = 0;
+#pragma unroll
+                            for (int h = 0; h < H; ++h) {
+                                // scale and zero-point change only where the group does (warp-uniform)
+                                const uint32_t row = (h == 0) ? 0u : (p.gdiv((uint32_t)H * (uint32_t)u + (uint32_t)h) - g0);   // 0 .. H - 1
+                                if (row != cur_row) {
+                                    cur_row = row;
+                                    load_group(row, c);
+                                    nf |= not_fast_bits(c);
+                                    if (SPARSE) c.zb = __half2uint_rz(__ushort_as_half((unsigned short)(c.z2 & 0xFFFFu))) * 0x01010101u;
+                                }
+                                if (h == H - 1 && __any_sync(0xFFFFFFFFu, nf != 0)) {
+                                    redo = true;
+                                    break;
+                                }
+                                uint32_t A[32];
+                                F::template decode<MODE_FAST>(st + WS::kW + h * (F::WROWS * 512) + col * 4, st + WS::kMask + h * (F::MROWS * 512) + col * 4, c, A, lut);
+                                if (h == H - 1) release_weights();
+                                if (h == 0 && !acquire_a_stage()) { ok = false; break; }
+                                ptx::tmem_st32(lane_addr + C::kACol0 + as * C::kAStageCols + h * 32, A);
+                            }
+                        }
+                        if (redo && ok) {
+                            // some group needs the general or the per-weight mode (rolled loop: three decode bodies in the
+                            // instruction cache, not three per part)
+                            ptx::tc_wait_st();
+                            ColK c;
+                            uint32_t cur_row = 0xFFFFFFFFu;
+#pragma unroll 1
+                            for (int h = 0; h < H; ++h) {
+                                const uint32_t row = (h == 0) ? 0u : (p.gdiv((uint32_t)H * (uint32_t)u + (uint32_t)h) - g0);
+                                if (row != cur_row) {
+                                    cur_row = row;
+                                    load_group(row, c);
+                                }
+                                const uint32_t wb = st + WS::kW + h * (F::WROWS * 512) + col * 4;
+                                const uint32_t mb = st + WS::kMask + h * (F::MROWS * 512) + col * 4;
+                                uint32_t A[32];
+                                if (!__any_sync(0xFFFFFFFFu, not_fast_bits(c) != 0)) {
+                                    if (SPARSE) c.zb = __half2uint_rz(__ushort_as_half((unsigned short)(c.z2 & 0xFFFFu))) * 0x01010101u;
+                                    F::template decode<MODE_FAST>(wb, mb, c, A, lut);
+                                } else {
+                                    c.zb = 0;
+                                    const bool lin = __hge(__ushort_as_half((unsigned short)(c.s2 & 0xFFFFu)), __ushort_as_half(0));
+                                    if (__all_sync(0xFFFFFFFFu, lin)) F::template decode<MODE_GENERAL>(wb, mb, c, A, lut);
+                                    else F::template decode<MODE_SLOW>(wb, mb, c, A, lut);
+                                }
+                                if (h == H - 1) release_weights();
+                                ptx::tmem_st32(lane_addr + C::kACol0 + as * C::kAStageCols + h * 32, A);
+                            }
+                        }
+                        if (!ok) break;
+                        // (not deferred for the warpgroup's first stage: the pipeline is still filling and the MMA warp is waiting)
+                        if (C::kDeferArrive && si >= (uint32_t)C::kWG) pending = (int)as;
+                        else announce((int)as);
+                    }
+                    if (!ok) break;
+                    if (C::kDeferArrive && pending >= 0) { announce(pending); pending = -1; }
+                    if (!C::kEpiWarps && wg == 0) ok = after_segment(seg, tile, u0, u1);
+                    ++seg;
+                    si0 += (uint32_t)(u1 - u0);
+                    t += u1 - u0;
+                }
+    return ok ? (int)seg : -1;
+}
+
+// The same as a function of its own for the few-row shapes, where this loop is what bounds the kernel: inside the kernel
+// its registers and instructions changed with every change to the other roles.
+template <class F, int NT, class Entry>
+__device__ __noinline__ int dequant_role(const UmmaParams& p, uint32_t bars, uint32_t w_ring, uint32_t tmem_base, long long t_lo, long long t_hi, const Entry* lut) {
+    return dequant_units<F, NT, false>(p, bars, w_ring, tmem_base, t_lo, t_hi, lut, [](uint32_t, long long, int, int) { return true; });
+}
+
+// The weight-streaming shapes (one row tile).  Split-K: the CTAs b_lo .. b_hi share this tile.  b_lo, which owns its
+// first units and reaches them last, adds the others' partial tiles to its own accumulator in CTA order - a fixed
+// order, so results are reproducible; the others wait for nobody.  A partial element is one 64-bit word (fp32
+// value | tag 1 in the high half), written with a single store, so no fence, counter or second round trip is
+// needed; the reader clears what it has read, which leaves the scratch all-zero for the next launch.  One slot per
+// CTA is enough: a CTA has at most one tile that it shares and does not sum.
+// A CTA's last tile is left to all of its warpgroups, `part` of `parts` rows each, since the dequant warps have
+// nothing else to do by then: what counts there is the number of dependent round trips to L2 (~0.7 us each), and so
+// the number of loads in flight.
+// A function of its own, so that its registers do not weigh on the dequantisation loop (inlined: 16384 x 16384, one row,
+// 37.7 -> 44.7 us).
+template <int NT, bool LAST>
+__device__ __noinline__ bool split_epilogue(const UmmaParams& p, uint32_t tmem_base, uint32_t d_full, uint32_t d_empty, const volatile int* s_abort,
+                                            uint32_t seg, long long t0, int units, int part, int parts, bool handed) {
+    // outputs, old outputs and the scratch may still be in use by the kernel before this one in the stream
+    ptx::grid_dependency_wait();
+    const int warp = (int)(threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const long long U = p.U, G = gridDim.x, n_tiles = p.CT, tile = div_nn(t0, U);
+    const int u0 = (int)(t0 - tile * U), u1 = u0 + units;
+    const int ct = (int)tile, col = (warp & 3) * 32 + lane, scol = ct * 128 + col;
+    const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
+    const bool col_ok = scol < p.S;
+    const int me = (int)blockIdx.x, r0 = p.rows * part / parts, r1 = p.rows * (part + 1) / parts;
+    int b_lo = me, b_hi = me;
+    if (u0 != 0 || u1 != (int)U) {
+        const long long T = n_tiles * U, lo_t = tile * U;
+        b_lo = range_owner(T, G, lo_t);
+        b_hi = range_owner(T, G, lo_t + U - 1);
+    }
+    unsigned long long* const partials64 = reinterpret_cast<unsigned long long*>(p.partials);
+    auto slot_of = [&](int bb) { return partials64 + (size_t)bb * NT * 128 + col; };
+    bool accumulator_ready = false;
+    auto wait_accumulator = [&]() -> bool {
+        if (accumulator_ready) return true;
+        accumulator_ready = true;
+        if (handed) {
+            ptx::named_bar_sync(2, 128 + 32);      // released by the MMA warp once the accumulator is complete
+            if (*s_abort) return false;
+        } else if (!ptx::mbar_wait(d_full, seg & 1u)) {
+            if (lane == 0) atomicExch(p.status, 33);
+            return false;
+        }
+        ptx::tc_fence_after_sync();
+        return true;
+    };
+    auto release_accumulator = [&]() {                 // (a last tile's is not waited for)
+        if (parts > 1) return;
+        ptx::tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(d_empty);
+    };
+    if (me != b_lo) {
+        if (!wait_accumulator()) return false;
+        unsigned long long* const mine = slot_of(me);
+#pragma unroll 1
+        for (int j0 = r0; j0 < r1; j0 += 16) {
+            uint32_t v[16];
+            ptx::tmem_ld16(lane_addr + j0, v);
+            ptx::tc_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+                if (j0 + j < r1) ptx::st_relaxed_gpu_u64(mine + (j0 + j) * 128, (1ull << 32) | v[j]);
+        }
+        release_accumulator();
+        return true;
+    }
+    __half* const out0 = p.om.dst[0] + (col_ok ? p.om.col(scol) : 0);
+    bool waiting_ok = true;
+    // rows rb .. rb + n - 1 (n <= RB), the partners PB at a time: RB x PB loads in flight
+    auto finish_rows = [&](auto rb_tag, auto pb_tag, int rb, int n) -> bool {
+        constexpr int RB = decltype(rb_tag)::value, PB = decltype(pb_tag)::value;
+        float sum[RB];
+        __half old[RB];
+#pragma unroll
+        for (int i = 0; i < RB; ++i) {
+            sum[i] = 0.f;
+            if (p.accumulate && i < n && col_ok) old[i] = out0[(size_t)(rb + i) * p.om.ld];
+        }
+#pragma unroll 1
+        for (int q = b_lo + 1; LAST && q <= b_hi; q += PB) {
+            unsigned long long w[PB][RB];
+#pragma unroll
+            for (int j = 0; j < PB; ++j)
+#pragma unroll
+                for (int i = 0; i < RB; ++i)
+                    if (q + j <= b_hi && i < n) w[j][i] = ptx::ld_relaxed_gpu_u64(slot_of(q + j) + (rb + i) * 128);
+#pragma unroll
+            for (int j = 0; j < PB; ++j)
+#pragma unroll
+                for (int i = 0; i < RB; ++i)
+                    if (q + j <= b_hi && i < n) {
+                        unsigned long long* const at = slot_of(q + j) + (rb + i) * 128;
+                        for (uint32_t spins = 0; (uint32_t)(w[j][i] >> 32) != 1u && waiting_ok; ++spins) {
+                            if (spins >= ptx::kSpinLimit) {            // a contributor never delivered: report, stop waiting
+                                atomicExch(p.status, 34);
+                                waiting_ok = false;
+                                break;
+                            }
+                            __nanosleep(20);
+                            w[j][i] = ptx::ld_relaxed_gpu_u64(at);
+                        }
+                        sum[i] += __uint_as_float((uint32_t)w[j][i]);
+                        ptx::st_relaxed_gpu_u64(at, 0ull);
+                    }
+        }
+        if (!wait_accumulator()) return false;
+        uint32_t v[RB];
+        ptx::tmem_ld(lane_addr + rb, v);
+        ptx::tc_wait_ld();
+        if (rb + n >= r1) release_accumulator();
+#pragma unroll
+        for (int i = 0; i < RB; ++i) {
+            if (i < n && col_ok) {
+                float f = __uint_as_float(v[i]) + sum[i];
+                const size_t at = (size_t)(rb + i) * p.om.ld;
+                if (p.accumulate) f += __half2float(old[i]);
+                const __half h = __float2half_rn(f);
+                out0[at] = h;
+                for (int d = 1; d < p.om.n_dst; ++d) p.om.dst[d][at + (out0 - p.om.dst[0])] = h;
+            }
+        }
+        return true;
+    };
+    if (r1 - r0 <= 4) {
+        if (r1 > r0 && !finish_rows(std::integral_constant<int, 4>(), std::integral_constant<int, 4>(), r0, r1 - r0)) return false;
+    } else {
+#pragma unroll 1
+        for (int rb = r0; rb < r1; rb += 8)
+            if (!finish_rows(std::integral_constant<int, 8>(), std::integral_constant<int, 2>(), rb, min(8, r1 - rb))) return false;
+    }
+    if (handed && !wait_accumulator()) return false;               // (no rows: the MMA warp's barrier still counts these warps)
+    if (p.om.n_dst > 1) __threadfence_system();                // as below
+    return true;
+}
+
 // PAIR: launched as clusters of two CTAs (two SMs) that run every MMA together (cta_group::2, M = 256): the pair's
 // tile is 256 weight columns x NT rows, each CTA dequantises its own 128 columns and loads only half of the rows of
 // the activation tile, which halves the L2 -> shared-memory traffic that bounds the many-row shapes.
 // PERM (up to 8 rows of dense int4 only): the cheaper k order of UFormat, with the activations reordered to match.
 template <int BITS, bool SPARSE, int NT, bool PAIR, bool PERM = false>
 __global__ void __launch_bounds__(Cfg<NT, PAIR>::kThreads, Cfg<NT, PAIR>::kMinBlocks)
-umma_kernel(const __grid_constant__ TensorMaps tm, const UmmaParams p, const __half* x) {
+umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaParams p, const __half* x) {
     using C = Cfg<NT, PAIR>;
     using F = UFormat<BITS, SPARSE, PERM>;
     static_assert(!PERM || (C::kStream && F::kPermutedK), "the permuted k order is for dense int4 weight streaming");
+    constexpr bool kSpread = C::kStream && !PERM;                  // the last tile's epilogue is every warpgroup's (split_epilogue)
     constexpr int H = C::kHalves;                                    // 64-k parts per unit
     using WS = WStage<F, H>;
     static_assert(!PAIR || (NT >= 128 && !C::kEpiHandoff), "CTA pairs are for the many-row shapes");
@@ -299,7 +606,7 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const UmmaParams p, const __h
     // single CTAs at NT = 256 have no shared memory left for a second transposition tile: the second epilogue group idles
     constexpr int kEpiGroups = (C::kEpiGroups == 2 && (PAIR || NT < 256)) ? 2 : 1;
     constexpr int kEpiWarp0 = 4 * C::kWG;                           // first epilogue warp (a multiple of 4: lane quarter = warp % 4)
-    constexpr int kWProducer = kEpiWarp0 + 4 * C::kEpiGroups, kBProducer = kWProducer + 1, kMma = kWProducer + 2;
+    constexpr int kWProducer = kEpiWarp0 + (C::kEpiWarps ? 4 * C::kEpiGroups : 0), kBProducer = kWProducer + 1, kMma = kWProducer + 2;
     constexpr int kWProducer2 = kWProducer + 3;                     // only when Cfg::kWProducers == 2
     constexpr int kABStages = ABStages<NT, PAIR>::value;
     extern __shared__ __align__(1024) unsigned char smem[];      // [B ring (1024-aligned tiles)][W ring]
@@ -612,138 +919,7 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const UmmaParams p, const __h
         // Accumulator of one finished segment -> fp16 rows of `out`, or a partial tile for the split-K reduction.
         // Run by 4 warps whose index modulo 4 selects the 32 tensor-memory lanes (= weight columns) they may read.
         bool dependency_waited = false;
-        // The weight-streaming shapes (one row tile).  Split-K: the CTAs b_lo .. b_hi share this tile.  b_lo, which owns its
-        // first units and reaches them last, adds the others' partial tiles to its own accumulator in CTA order - a fixed
-        // order, so results are reproducible; the others wait for nobody.  A partial element is one 64-bit word (fp32
-        // value | tag 1 in the high half), written with a single store, so no fence, counter or second round trip is
-        // needed; the reader clears what it has read, which leaves the scratch all-zero for the next launch.  One slot per
-        // CTA is enough: a CTA has at most one tile that it shares and does not sum.
-        // A CTA's last tile is left to all of its warpgroups, `part` of `parts` rows each, since the dequant warps have
-        // nothing else to do by then: what counts there is the number of dependent round trips to L2 (~0.7 us each), and so
-        // the number of loads in flight.
-        auto epilogue_split = [&](auto last, uint32_t seg, long long tile, int u0, int u1, int part, int parts, bool handed) -> bool {
-            if (!dependency_waited) {
-                // outputs, old outputs and the scratch may still be in use by the kernel before this one in the stream
-                ptx::grid_dependency_wait();
-                dependency_waited = true;
-            }
-            const int ct = tile_ct(tile), col = (warp & 3) * 32 + lane, scol = ct * 128 + col;
-            const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
-            const bool col_ok = scol < p.S;
-            const int me = (int)b, r0 = p.rows * part / parts, r1 = p.rows * (part + 1) / parts;
-            int b_lo = me, b_hi = me;
-            if (u0 != 0 || u1 != (int)U) {
-                const long long T = n_tiles * U, lo_t = tile * U;
-                b_lo = range_owner(T, G, lo_t);
-                b_hi = range_owner(T, G, lo_t + U - 1);
-            }
-            unsigned long long* const partials64 = reinterpret_cast<unsigned long long*>(p.partials);
-            auto slot_of = [&](int bb) { return partials64 + (size_t)bb * C::kSlotElems + col; };
-            bool accumulator_ready = false;
-            auto wait_accumulator = [&]() -> bool {
-                if (accumulator_ready) return true;
-                accumulator_ready = true;
-                if (handed) {
-                    ptx::named_bar_sync(2, 128 + 32);      // released by the MMA warp once the accumulator is complete
-                    if (s_abort) return false;
-                } else if (!ptx::mbar_wait(ptx::smem_u32(&bars.d_full), seg & 1u)) {
-                    if (lane == 0) atomicExch(p.status, 33);
-                    return false;
-                }
-                ptx::tc_fence_after_sync();
-                return true;
-            };
-            auto release_accumulator = [&]() {                 // (a last tile's is not waited for)
-                if (parts > 1) return;
-                ptx::tc_fence_before_sync();
-                __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&bars.d_empty));
-            };
-            if (me != b_lo) {
-                if (!wait_accumulator()) return false;
-                unsigned long long* const mine = slot_of(me);
-#pragma unroll 1
-                for (int j0 = r0; j0 < r1; j0 += 16) {
-                    uint32_t v[16];
-                    ptx::tmem_ld16(lane_addr + j0, v);
-                    ptx::tc_wait_ld();
-#pragma unroll
-                    for (int j = 0; j < 16; ++j)
-                        if (j0 + j < r1) ptx::st_relaxed_gpu_u64(mine + (j0 + j) * 128, (1ull << 32) | v[j]);
-                }
-                release_accumulator();
-                return true;
-            }
-            __half* const out0 = p.om.dst[0] + (col_ok ? p.om.col(scol) : 0);
-            bool waiting_ok = true;
-            // rows rb .. rb + n - 1 (n <= RB), the partners PB at a time: RB x PB loads in flight
-            auto finish_rows = [&](auto rb_tag, auto pb_tag, int rb, int n) -> bool {
-                constexpr int RB = decltype(rb_tag)::value, PB = decltype(pb_tag)::value;
-                float sum[RB];
-                __half old[RB];
-#pragma unroll
-                for (int i = 0; i < RB; ++i) {
-                    sum[i] = 0.f;
-                    if (p.accumulate && i < n && col_ok) old[i] = out0[(size_t)(rb + i) * p.om.ld];
-                }
-#pragma unroll 1
-                for (int q = b_lo + 1; decltype(last)::value && q <= b_hi; q += PB) {
-                    unsigned long long w[PB][RB];
-#pragma unroll
-                    for (int j = 0; j < PB; ++j)
-#pragma unroll
-                        for (int i = 0; i < RB; ++i)
-                            if (q + j <= b_hi && i < n) w[j][i] = ptx::ld_relaxed_gpu_u64(slot_of(q + j) + (rb + i) * 128);
-#pragma unroll
-                    for (int j = 0; j < PB; ++j)
-#pragma unroll
-                        for (int i = 0; i < RB; ++i)
-                            if (q + j <= b_hi && i < n) {
-                                unsigned long long* const at = slot_of(q + j) + (rb + i) * 128;
-                                for (uint32_t spins = 0; (uint32_t)(w[j][i] >> 32) != 1u && waiting_ok; ++spins) {
-                                    if (spins >= ptx::kSpinLimit) {            // a contributor never delivered: report, stop waiting
-                                        atomicExch(p.status, 34);
-                                        waiting_ok = false;
-                                        break;
-                                    }
-                                    __nanosleep(20);
-                                    w[j][i] = ptx::ld_relaxed_gpu_u64(at);
-                                }
-                                sum[i] += __uint_as_float((uint32_t)w[j][i]);
-                                ptx::st_relaxed_gpu_u64(at, 0ull);
-                            }
-                }
-                if (!wait_accumulator()) return false;
-                uint32_t v[RB];
-                ptx::tmem_ld(lane_addr + rb, v);
-                ptx::tc_wait_ld();
-                if (rb + n >= r1) release_accumulator();
-#pragma unroll
-                for (int i = 0; i < RB; ++i) {
-                    if (i < n && col_ok) {
-                        float f = __uint_as_float(v[i]) + sum[i];
-                        const size_t at = (size_t)(rb + i) * p.om.ld;
-                        if (p.accumulate) f += __half2float(old[i]);
-                        const __half h = __float2half_rn(f);
-                        out0[at] = h;
-                        for (int d = 1; d < p.om.n_dst; ++d) p.om.dst[d][at + (out0 - p.om.dst[0])] = h;
-                    }
-                }
-                return true;
-            };
-            if (r1 - r0 <= 4) {
-                if (r1 > r0 && !finish_rows(std::integral_constant<int, 4>(), std::integral_constant<int, 4>(), r0, r1 - r0)) return false;
-            } else {
-#pragma unroll 1
-                for (int rb = r0; rb < r1; rb += 8)
-                    if (!finish_rows(std::integral_constant<int, 8>(), std::integral_constant<int, 2>(), rb, min(8, r1 - rb))) return false;
-            }
-            if (handed && !wait_accumulator()) return false;               // (no rows: the MMA warp's barrier still counts these warps)
-            if (p.om.n_dst > 1) __threadfence_system();                // as below
-            return true;
-        };
-        // Whole tiles, or one K part of a tile
-        auto epilogue_whole = [&](uint32_t seg, long long tile, int u0, int u1) -> bool {
+        auto epilogue = [&](uint32_t seg, long long tile, int u0, int u1) -> bool {
             if (!dependency_waited) {
                 // outputs, old outputs and the scratch may still be in use by the kernel before this one in the stream
                 ptx::grid_dependency_wait();
@@ -752,10 +928,26 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const UmmaParams p, const __h
             const int mt = tile_mt(tile), ct = tile_ct(tile);
             const int col = (warp & 3) * 32 + lane;
             const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
+            const bool complete = (u0 == 0) && (u1 == (int)U);
             const int scol = ct * 128 + col;
             const bool col_ok = scol < p.S;
             const int row0 = mt * NT;
             const int nrows = min(NT, p.rows - row0);
+            // Split-K: the CTAs b_lo .. b_hi share this tile.  b_lo (which owns the tile's first units and reaches them
+            // last) adds the others' partial tiles to its own accumulator in CTA order - a fixed order, so results are
+            // reproducible.  A partial element is one 64-bit word (fp32 value | tag 1 in the high half), written with a
+            // single store, so no fence, counter or second round trip is needed; the reader clears what it has read,
+            // which leaves the scratch all-zero for the next launch.  Every other CTA's share of the tile is the first
+            // segment of its range, so one slot per CTA is enough.
+            int b_lo = 0, b_hi = -1;
+            unsigned long long* slot = nullptr;
+            unsigned long long* const partials64 = reinterpret_cast<unsigned long long*>(p.partials);
+            if (C::kSplit && !complete) {
+                const long long T = n_tiles * U, lo_t = tile * U;
+                b_lo = range_owner(T, G, lo_t);
+                b_hi = range_owner(T, G, lo_t + U - 1);
+                if ((int)b != b_lo) slot = partials64 + (size_t)(PAIR ? b * 2 + rank : b) * C::kSlotElems;
+            }
             // K parts: fp32 rows j0 .. of this lane's column into the (part, row, S) scratch; the reduce kernel sums the parts
             auto put_kpart = [&](auto& v, int j0) {
                 constexpr int CNT = (int)(sizeof(v) / sizeof(uint32_t));
@@ -765,14 +957,74 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const UmmaParams p, const __h
                     if (j0 + j < nrows)
                         p.partials[((size_t)kpart * p.rows + row0 + j0 + j) * p.S + scol] = __uint_as_float(v[j]);
             };
-            {
+            // leaves accumulator rows j0 .. j0 + n - 1 of this lane's column in this CTA's slot
+            auto put_partial = [&](auto& v, int j0) {
+                constexpr int CNT = (int)(sizeof(v) / sizeof(uint32_t));
+#pragma unroll
+                for (int j = 0; j < CNT; ++j)
+                    if (j0 + j < nrows) ptx::st_relaxed_gpu_u64(slot + (j0 + j) * 128 + col, (1ull << 32) | v[j]);
+            };
+            // adds the other CTAs' partial rows j0 .. j0 + n - 1 to v, in CTA order, and clears them
+            auto add_partials = [&](auto& v, int j0) {
+                constexpr int CNT = (int)(sizeof(v) / sizeof(uint32_t));
+                bool waiting_ok = true;
+                for (int bb = b_lo + 1; bb <= b_hi; ++bb) {
+                    unsigned long long* src = partials64 + (size_t)(PAIR ? bb * 2 + (int)rank : bb) * C::kSlotElems + col;
+#pragma unroll
+                    for (int jb = 0; jb < CNT; jb += 8) {
+                        if (j0 + jb >= nrows) break;                       // warp-uniform
+                        unsigned long long w[8];
+#pragma unroll
+                        for (int i = 0; i < 8; ++i)
+                            if (j0 + jb + i < nrows) w[i] = ptx::ld_relaxed_gpu_u64(src + (j0 + jb + i) * 128);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            if (j0 + jb + i < nrows) {
+                                for (uint32_t spins = 0; (uint32_t)(w[i] >> 32) != 1u && waiting_ok; ++spins) {
+                                    if (spins >= ptx::kSpinLimit) {        // a contributor never delivered: report, stop waiting
+                                        atomicExch(p.status, 34);
+                                        waiting_ok = false;
+                                        break;
+                                    }
+                                    __nanosleep(64);
+                                    w[i] = ptx::ld_relaxed_gpu_u64(src + (j0 + jb + i) * 128);
+                                }
+                                v[jb + i] = __float_as_uint(__uint_as_float(v[jb + i]) + __uint_as_float((uint32_t)w[i]));
+                                ptx::st_relaxed_gpu_u64(src + (j0 + jb + i) * 128, 0ull);
+                            }
+                        }
+                    }
+                }
+            };
+            // The weight-streaming shapes fetch the other CTAs' partial tiles BEFORE the own accumulator is complete (the
+            // partners delivered them early in their run, as their first segment, and these warps have nothing else to
+            // do): their sum, in CTA order, then only has to be added, and the dependent round trips to L2 are off the tail.
+            constexpr int kPre = (C::kSplit && C::kEpiHandoff) ? C::kDCols : 1;
+            uint32_t pre[kPre];
+            bool prefetched = false;
+            if (C::kSplit && C::kEpiHandoff && !slot && b_hi > b_lo) {
+#pragma unroll
+                for (int j = 0; j < kPre; ++j) pre[j] = 0u;
+                if (kPre >= 16) {
+#pragma unroll
+                    for (int j0 = 0; j0 < kPre; j0 += 16) add_partials(reinterpret_cast<uint32_t(&)[16]>(pre[j0 < kPre ? j0 : 0]), j0);
+                }
+                prefetched = true;
+            }
+            if (C::kEpiHandoff) {
+                ptx::named_bar_sync(2, 128 + 32);          // released by the MMA warp once the accumulator is complete
+                if (s_abort) return false;
+            } else {
                 bool got = ptx::mbar_wait(ptx::smem_u32(&bars.d_full), seg & 1u);
                 if (!got && lane == 0) atomicExch(p.status, 33);
-                // the four warps of an epilogue group meet at named barriers further down: a give-up has to be
-                // the whole group's decision, or the warps that went on would wait there for ever
-                if (!got) s_abort = 1;
-                ptx::named_bar_sync(1 + 3 * ((warp - kEpiWarp0) >> 2), 128);
-                if (s_abort) return false;
+                if (C::kEpiTransposed) {
+                    // the four warps of an epilogue group meet at named barriers further down: a give-up has to be
+                    // the whole group's decision, or the warps that went on would wait there for ever
+                    if (!got) s_abort = 1;
+                    ptx::named_bar_sync(1 + 3 * ((warp - kEpiWarp0) >> 2), 128);
+                    got = s_abort == 0;
+                }
+                if (!got) return false;
             }
             ptx::tc_fence_after_sync();
             // matvec route with more than 64 rows (a batch of one-row products): the caller's old values of rows
@@ -784,7 +1036,7 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const UmmaParams p, const __h
                     if (j0 + j < nrows)
                         v[j] = __float_as_uint(__uint_as_float(v[j]) + __half2float(p.om.dst[0][(size_t)(row0 + j0 + j) * p.om.ld + p.om.col(scol)]));
             };
-            {
+            if (C::kEpiTransposed) {
                 // 16 accumulator columns (= 16 output rows) at a time: transposed through a 4 KB shared-memory tile so that
                 // the global stores are 16-byte rows instead of one 2-byte element per lane
                 const int eg = (warp - kEpiWarp0) >> 2;                     // epilogue warpgroup: its share of the accumulator columns
@@ -808,6 +1060,13 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const UmmaParams p, const __h
                             __syncwarp();
                             if (lane == 0) ptx::mbar_arrive_cluster(ptx::map_to_cta(ptx::smem_u32(&bars.d_empty), 0));
                         }
+                        if (C::kSplit) {
+                            if (slot) {
+                                put_partial(v, j0);
+                                continue;
+                            }
+                            if (b_hi > b_lo) add_partials(v, j0);
+                        }
                         if (p.kparts > 1) {
                             put_kpart(v, j0);
                             continue;
@@ -820,7 +1079,7 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const UmmaParams p, const __h
                     }
                     ptx::named_bar_sync(bar_id, 128);
 #pragma unroll 1
-                    for (int idx = t128; idx < (p.kparts > 1 ? 0 : kShare * 16); idx += 128) {   // 16-byte chunks: row = idx / 16, chunk = idx % 16
+                    for (int idx = t128; idx < ((slot || p.kparts > 1) ? 0 : kShare * 16); idx += 128) {   // 16-byte chunks: row = idx / 16, chunk = idx % 16
                         const int m = eg * kShare + (idx >> 4), c8 = (idx & 15) * 8;
                         if (m < nrows && ct * 128 + c8 < p.S) {
                             const uint4 q = ptx::lds128(stage + (idx >> 4) * 256 + c8 * 2);
@@ -843,6 +1102,13 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const UmmaParams p, const __h
                             else ptx::mbar_arrive(ptx::smem_u32(&bars.d_empty));
                         }
                     }
+                    if (C::kSplit) {
+                        if (slot) {
+                            put_partial(v, j0);
+                            continue;
+                        }
+                        if (b_hi > b_lo) add_partials(v, j0);
+                    }
                     if (p.kparts > 1) {
                         put_kpart(v, j0);
                         continue;
@@ -864,6 +1130,51 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const UmmaParams p, const __h
                     }
                     ptx::named_bar_sync(bar_id, 128);
                 }
+            } else {
+            constexpr int CH = NT >= 64 ? 32 : 16;          // accumulator columns per tensor-memory load
+#pragma unroll 1
+            for (int j0 = 0; j0 < NT; j0 += CH) {
+                uint32_t v[CH];
+                if (CH == 32) ptx::tmem_ld32(lane_addr + j0, reinterpret_cast<uint32_t(&)[32]>(v));
+                else ptx::tmem_ld16(lane_addr + j0, reinterpret_cast<uint32_t(&)[16]>(v));
+                ptx::tc_wait_ld();
+                if (j0 + CH >= NT) {                       // the last columns are in registers: the accumulator is free again
+                    ptx::tc_fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&bars.d_empty));
+                }
+                if (slot) {
+                    put_partial(v, j0);
+                    continue;
+                }
+                if (C::kSplit && b_hi > b_lo) {
+                    if (prefetched) {
+#pragma unroll
+                        for (int j = 0; j < CH; ++j)
+                            v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(pre[(j0 + j) < kPre ? j0 + j : 0]));
+                    } else {
+                        add_partials(v, j0);
+                    }
+                }
+                if (p.kparts > 1) {
+                    put_kpart(v, j0);
+                    continue;
+                }
+                if (col_ok) {
+                    const long long dcol = p.om.col(scol);
+#pragma unroll
+                    for (int j = 0; j < CH; ++j) {
+                        const int m = j0 + j;
+                        if (m < nrows) {
+                            float f = __uint_as_float(v[j]);
+                            const size_t at = (size_t)(row0 + m) * p.om.ld + dcol;
+                            if (p.accumulate) f += __half2float(p.om.dst[0][at]);
+                            const __half h = __float2half_rn(f);
+                            for (int d = 0; d < p.om.n_dst; ++d) p.om.dst[d][at] = h;
+                        }
+                    }
+                }
+            }
             }
             // Stores into other GPUs' buffers: every storing thread makes its own stores visible system-wide before the
             // CTA can finish, so that the hand-shake kernel's flag (written by another SM, possibly over another link)
@@ -872,169 +1183,47 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const UmmaParams p, const __h
             return true;
         };
 
-        uint32_t seg = 0;
-        bool aborted = false;
-        if (warp >= kEpiWarp0 + 4 * kEpiGroups) {
+        bool aborted = false;                                     // (kSpread)
+        uint32_t last_seg = 0;
+        if (C::kEpiWarps && warp >= kEpiWarp0 + 4 * kEpiGroups) {
             // (an epilogue warpgroup that this configuration does not use)
-        } else if (warp >= kEpiWarp0) {
+        } else if (C::kEpiWarps && warp >= kEpiWarp0) {
             // ----- dedicated epilogue warps: one pass per segment -----
+            uint32_t seg = 0;
             for (long long t = t_lo; t < t_hi;) {
                 const long long tile = div_nn(t, U);
                 const int u0 = (int)(t - tile * U);
                 const int u1 = (int)min(U, u0 + (t_hi - t));
-                if (C::kSplit) {
-                    if (t + (u1 - u0) >= t_hi) break;                  // the last tile is everybody's: below
-                    if (!epilogue_split(std::false_type(), seg, tile, u0, u1, 0, 1, true)) { aborted = true; break; }
-                } else if (!epilogue_whole(seg, tile, u0, u1)) break;
+                if constexpr (kSpread) {
+                    if (t + (u1 - u0) >= t_hi) {                       // the last tile is everybody's: below
+                        last_seg = seg;
+                        break;
+                    }
+                    if (!split_epilogue<NT, false>(p, tmem_base, ptx::smem_u32(&bars.d_full), ptx::smem_u32(&bars.d_empty), &s_abort, seg, t, u1 - u0, 0, 1, true)) {
+                        aborted = true;
+                        break;
+                    }
+                } else if (!epilogue(seg, tile, u0, u1)) break;
                 ++seg;
                 t += u1 - u0;
             }
         } else {
             // ----- dequant warps -----
-            const int wg = warp >> 2;                                           // warpgroup: takes every kWG-th weight stage
-            const int col = (warp & 3) * 32 + lane;                             // weight column in the tile = tensor-memory lane
-            const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
-            uint32_t si0 = 0;                                                    // si0: weight stages consumed before this segment
-            int pending = -1;                                                    // A stage written but not yet announced (Cfg::kDeferArrive)
-            // the stores into tensor memory are complete -> the stage may be read by the MMAs
-            auto announce = [&](int stage) {
-                ptx::tc_wait_st();
-                ptx::tc_fence_before_sync();
-                __syncwarp();
-                if (lane == 0) {
-                    if (PAIR) ptx::mbar_arrive_cluster(ptx::map_to_cta(ptx::smem_u32(&bars.ab_full[stage]), 0));
-                    else ptx::mbar_arrive(ptx::smem_u32(&bars.ab_full[stage]));
-                }
-            };
-            bool ok = true;
-            for (long long t = t_lo; t < t_hi && ok;) {
-                const long long tile = div_nn(t, U);
-                const int u0 = (int)(t - tile * U);
-                const int u1 = (int)min(U, u0 + (t_hi - t));
-                // this warpgroup's units of the segment: those whose stage index is congruent to wg modulo kWG
-                for (int u = u0 + (int)(((uint32_t)wg + (uint32_t)C::kWG - si0 % (uint32_t)C::kWG) % (uint32_t)C::kWG); u < u1; u += C::kWG) {
-                    const uint32_t si = si0 + (uint32_t)(u - u0);
-                    const uint32_t ws = si % C::kWStages, wph = (si / C::kWStages) & 1u;     // constants: multiply-shift, no division
-                    if (C::kWGuard && !ptx::mbar_wait(ptx::smem_u32(&bars.w_empty[ws]), wph ^ 1u)) {   // see Cfg::kWStages
-                        if (lane == 0) atomicExch(p.status, 35);
-                        ok = false;
-                        break;
-                    }
-                    if (!ptx::mbar_wait(ptx::smem_u32(&bars.w_full[ws]), wph)) {
-                        if (lane == 0) atomicExch(p.status, 31);
-                        ok = false;
-                        break;
-                    }
-                    const uint32_t st = w_ring + ws * WS::kBytes;
-                    const uint32_t g0 = p.gdiv((uint32_t)H * (uint32_t)u);
-                    const uint32_t as = si % kABStages, aph = (si / kABStages) & 1u;
-                    // polled before the first part is decoded, so that the answer costs no latency when it is needed
-                    const bool free_early = ptx::mbar_test_wait(ptx::smem_u32(&bars.ab_free[as]), aph ^ 1u);
-                    // scale and zero-point of this thread's column in row `row` of the stage's group box, both halves of a register
-                    auto load_group = [&](uint32_t row, ColK& c) {
-                        const uint32_t sz = ptx::lds32(st + WS::kS + row * 256 + (col & ~1) * 2) >> (16 * (col & 1));
-                        const uint32_t zz = ptx::lds32(st + WS::kZ + row * 256 + (col & ~1) * 2) >> (16 * (col & 1));
-                        c.s2 = prmt(sz, sz, 0x1010);
-                        c.z2 = prmt(zz, zz, 0x1010);
-                        c.zb = 0;
-                    };
-                    // fast mode needs: scale sign clear, zero-point an integer in [0, 512] (sparse format: see SparseTable)
-                    auto not_fast_bits = [&](const ColK& c) -> uint32_t {
-                        const uint32_t zr = hadd2_u(hadd2_u(c.z2, kMagic1024), H2_N1024);
-                        constexpr uint32_t kAdd = SPARSE ? SparseTable<SPARSE, NT>::kFastBound : 0x1FFFu;
-                        const uint32_t zlo = c.z2 & 0xFFFFu;
-                        return ((zlo | ((zlo & 0x7FFFu) + kAdd) | c.s2) & 0x8000u) | (zr ^ c.z2);
-                    };
-                    // after the last read of the weight stage
-                    auto release_weights = [&]() {
-                        __syncwarp();
-                        if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&bars.w_empty[ws]));
-                    };
-                    // before the first store into the A stage
-                    auto acquire_a_stage = [&]() -> bool {
-                        if (C::kDeferArrive && pending >= 0) announce(pending);       // before any wait: the MMAs must be able to go on
-                        // the A stage (and its activation tile) is free once the MMAs of its previous use have completed
-                        if (!free_early && !ptx::mbar_wait(ptx::smem_u32(&bars.ab_free[as]), aph ^ 1u)) {
-                            if (lane == 0) atomicExch(p.status, 32);
-                            return false;
-                        }
-                        ptx::tc_fence_after_sync();
-                        return true;
-                    };
-                    // The parts are decoded in the fast mode by straight-line code, without a mode decision in between;
-                    // whether every group of the unit really is in the fast mode (for every column of the warp) is
-                    // voted once, when the last group has been read and before the weight stage is released.  If not,
-                    // the unit is decoded again with a decision per part (the stores are simply overwritten).
-                    bool redo = false;
-                    {
-                        ColK c;
-                        uint32_t cur_row = 0xFFFFFFFFu, nf = 0;
-#pragma unroll
-                        for (int h = 0; h < H; ++h) {
-                            // scale and zero-point change only where the group does (warp-uniform)
-                            const uint32_t row = (h == 0) ? 0u : (p.gdiv((uint32_t)H * (uint32_t)u + (uint32_t)h) - g0);   // 0 .. H - 1
-                            if (row != cur_row) {
-                                cur_row = row;
-                                load_group(row, c);
-                                nf |= not_fast_bits(c);
-                                if (SPARSE) c.zb = __half2uint_rz(__ushort_as_half((unsigned short)(c.z2 & 0xFFFFu))) * 0x01010101u;
-                            }
-                            if (h == H - 1 && __any_sync(0xFFFFFFFFu, nf != 0)) {
-                                redo = true;
-                                break;
-                            }
-                            uint32_t A[32];
-                            F::template decode<MODE_FAST>(st + WS::kW + h * (F::WROWS * 512) + col * 4, st + WS::kMask + h * (F::MROWS * 512) + col * 4, c, A, lut);
-                            if (h == H - 1) release_weights();
-                            if (h == 0 && !acquire_a_stage()) { ok = false; break; }
-                            ptx::tmem_st32(lane_addr + C::kACol0 + as * C::kAStageCols + h * 32, A);
-                        }
-                    }
-                    if (redo && ok) {
-                        // some group needs the general or the per-weight mode (rolled loop: three decode bodies in the
-                        // instruction cache, not three per part)
-                        ptx::tc_wait_st();
-                        ColK c;
-                        uint32_t cur_row = 0xFFFFFFFFu;
-#pragma unroll 1
-                        for (int h = 0; h < H; ++h) {
-                            const uint32_t row = (h == 0) ? 0u : (p.gdiv((uint32_t)H * (uint32_t)u + (uint32_t)h) - g0);
-                            if (row != cur_row) {
-                                cur_row = row;
-                                load_group(row, c);
-                            }
-                            const uint32_t wb = st + WS::kW + h * (F::WROWS * 512) + col * 4;
-                            const uint32_t mb = st + WS::kMask + h * (F::MROWS * 512) + col * 4;
-                            uint32_t A[32];
-                            if (!__any_sync(0xFFFFFFFFu, not_fast_bits(c) != 0)) {
-                                if (SPARSE) c.zb = __half2uint_rz(__ushort_as_half((unsigned short)(c.z2 & 0xFFFFu))) * 0x01010101u;
-                                F::template decode<MODE_FAST>(wb, mb, c, A, lut);
-                            } else {
-                                c.zb = 0;
-                                const bool lin = __hge(__ushort_as_half((unsigned short)(c.s2 & 0xFFFFu)), __ushort_as_half(0));
-                                if (__all_sync(0xFFFFFFFFu, lin)) F::template decode<MODE_GENERAL>(wb, mb, c, A, lut);
-                                else F::template decode<MODE_SLOW>(wb, mb, c, A, lut);
-                            }
-                            if (h == H - 1) release_weights();
-                            ptx::tmem_st32(lane_addr + C::kACol0 + as * C::kAStageCols + h * 32, A);
-                        }
-                    }
-                    if (!ok) break;
-                    // (not deferred for the warpgroup's first stage: the pipeline is still filling and the MMA warp is waiting)
-                    if (C::kDeferArrive && si >= (uint32_t)C::kWG) pending = (int)as;
-                    else announce((int)as);
-                }
-                if (!ok) { aborted = true; break; }
-                if (C::kDeferArrive && pending >= 0) { announce(pending); pending = -1; }
-                if (t + (u1 - u0) < t_hi) ++seg;
-                si0 += (uint32_t)(u1 - u0);
-                t += u1 - u0;
+            if constexpr (kSpread) {
+                const int segs = dequant_role<F, NT>(p, ptx::smem_u32(&bars), w_ring, tmem_base, t_lo, t_hi, lut);
+                aborted = segs < 0;
+                last_seg = (uint32_t)(segs - 1);
+            } else {
+                dequant_units<F, NT, PAIR>(p, ptx::smem_u32(&bars), w_ring, tmem_base, t_lo, t_hi, lut, epilogue);
             }
         }
-        if (C::kSplit && !aborted && t_lo < t_hi) {
+        if constexpr (kSpread) {
             // the CTA's last tile (or its part of one): every warpgroup takes some of the rows
-            const long long tile = div_nn(t_hi - 1, U), u_lo = max(t_lo, tile * U) - tile * U;
-            epilogue_split(std::true_type(), seg, tile, (int)u_lo, (int)(t_hi - tile * U), (warp >> 2) % (C::kWG + 1), C::kWG + 1, warp >= kEpiWarp0);
+            if (!aborted && t_lo < t_hi && (p.rows > 4 || warp >= kEpiWarp0)) {
+                const long long t0 = max(t_lo, div_nn(t_hi - 1, U) * U);
+                split_epilogue<NT, true>(p, tmem_base, ptx::smem_u32(&bars.d_full), ptx::smem_u32(&bars.d_empty), &s_abort, last_seg, t0, (int)(t_hi - t0),
+                                         p.rows > 4 ? warp >> 2 : 0, p.rows > 4 ? C::kWG + 1 : 1, warp >= kEpiWarp0);
+            }
         }
     }
 
@@ -1412,7 +1601,7 @@ int launch_fmt(UmmaParams& p, const __half* x, int n_groups, int pair_mode, int 
         case 16:
             // up to 8 rows of dense int4: the k order that needs no byte shuffles (more rows would cost the one warp
             // that reorders the activations more per unit than the unit takes)
-            if (BITS == 4 && !SPARSE && p.rows <= 8) return launch_nt<BITS, SPARSE, 16, false, BITS == 4 && !SPARSE>(p, x, n_groups, stream, cuda_err);
+            if (BITS == 4 && !SPARSE && p.rows <= g_tune[1]) return launch_nt<BITS, SPARSE, 16, false, BITS == 4 && !SPARSE>(p, x, n_groups, stream, cuda_err);
             return launch_nt<BITS, SPARSE, 16, false>(p, x, n_groups, stream, cuda_err);
         case 32: return launch_nt<BITS, SPARSE, 32, false>(p, x, n_groups, stream, cuda_err);
         case 64: return launch_nt<BITS, SPARSE, 64, false>(p, x, n_groups, stream, cuda_err);
