@@ -30,7 +30,6 @@
 #include <cuda.h>
 #include <dlfcn.h>
 
-#include <cstddef>
 #include <atomic>
 #include <mutex>
 #include <type_traits>
@@ -39,10 +38,6 @@
 #include "dequant.cuh"
 #include "ptx.cuh"
 
-namespace i4mm {
-int g_tune[16] = {0, 2};
-}
-extern "C" void i4mm_tune(int i, int v) { i4mm::g_tune[i] = v; }
 namespace i4mm {
 
 namespace {
@@ -288,179 +283,18 @@ struct TensorMaps {
     CUtensorMap z;
 };
 
-// The dequant warps: every unit of [t_lo, t_hi) that is this warpgroup's turn.  after_segment(...) is called by warpgroup 0
-// of the configurations without epilogue warps.  Returns the number of segments, or -1 after a wait that timed out.
-template <class F, int NT, bool PAIR, class Entry, class AfterSegment>
-__device__ __forceinline__ int dequant_units(const UmmaParams& p, uint32_t bars, uint32_t w_ring, uint32_t tmem_base, long long t_lo, long long t_hi,
-                                             const Entry* lut, const AfterSegment& after_segment) {
-    using C = Cfg<NT, PAIR>;
-    constexpr bool SPARSE = F::MROWS != 0;
-    constexpr int H = C::kHalves, kABStages = ABStages<NT, PAIR>::value;
-    using WS = WStage<F, H>;
-    const int lane = threadIdx.x & 31, warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0);
-    const long long U = p.U;
-    auto bar = [&](size_t first, uint32_t i) { return bars + (uint32_t)first + 8 * i; };
-                const int wg = warp >> 2;                                           // warpgroup: takes every kWG-th weight stage
-                const int col = (warp & 3) * 32 + lane;                             // weight column in the tile = tensor-memory lane
-                const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
-                uint32_t si0 = 0, seg = 0;                                           // si0: weight stages consumed before this segment
-                int pending = -1;                                                    // A stage written but not yet announced (Cfg::kDeferArrive)
-                // the stores into tensor memory are complete -> the stage may be read by the MMAs
-                auto announce = [&](uint32_t stage) {
-                    ptx::tc_wait_st();
-                    ptx::tc_fence_before_sync();
-                    __syncwarp();
-                    if (lane == 0) {
-                        if (PAIR) ptx::mbar_arrive_cluster(ptx::map_to_cta(bar(offsetof(Barriers, ab_full), stage), 0));
-                        else ptx::mbar_arrive(bar(offsetof(Barriers, ab_full), stage));
-                    }
-                };
-                bool ok = true;
-                for (long long t = t_lo; t < t_hi && ok;) {
-                    const long long tile = div_nn(t, U);
-                    const int u0 = (int)(t - tile * U);
-                    const int u1 = (int)min(U, u0 + (t_hi - t));
-                    // this warpgroup's units of the segment: those whose stage index is congruent to wg modulo kWG
-                    for (int u = u0 + (int)(((uint32_t)wg + (uint32_t)C::kWG - si0 % (uint32_t)C::kWG) % (uint32_t)C::kWG); u < u1; u += C::kWG) {
-                        const uint32_t si = si0 + (uint32_t)(u - u0);
-                        const uint32_t ws = si % C::kWStages, wph = (si / C::kWStages) & 1u;     // constants: multiply-shift, no division
-                        if (C::kWGuard && !ptx::mbar_wait(bar(offsetof(Barriers, w_empty), ws), wph ^ 1u)) {   // see Cfg::kWStages
-                            if (lane == 0) atomicExch(p.status, 35);
-                            ok = false;
-                            break;
-                        }
-                        if (!ptx::mbar_wait(bar(offsetof(Barriers, w_full), ws), wph)) {
-                            if (lane == 0) atomicExch(p.status, 31);
-                            ok = false;
-                            break;
-                        }
-                        const uint32_t st = w_ring + ws * WS::kBytes;
-                        const uint32_t g0 = p.gdiv((uint32_t)H * (uint32_t)u);
-                        const uint32_t as = si % kABStages, aph = (si / kABStages) & 1u;
-                        // polled before the first part is decoded, so that the answer costs no latency when it is needed
-                        const bool free_early = ptx::mbar_test_wait(bar(offsetof(Barriers, ab_free), as), aph ^ 1u);
-                        // scale and zero-point of this thread's column in row `row` of the stage's group box, both halves of a register
-                        auto load_group = [&](uint32_t row, ColK& c) {
-                            const uint32_t sz = ptx::lds32(st + WS::kS + row * 256 + (col & ~1) * 2) >> (16 * (col & 1));
-                            const uint32_t zz = ptx::lds32(st + WS::kZ + row * 256 + (col & ~1) * 2) >> (16 * (col & 1));
-                            c.s2 = prmt(sz, sz, 0x1010);
-                            c.z2 = prmt(zz, zz, 0x1010);
-                            c.zb = 0;
-                        };
-                        // fast mode needs: scale sign clear, zero-point an integer in [0, 512] (sparse format: see SparseTable)
-                        auto not_fast_bits = [&](const ColK& c) -> uint32_t {
-                            const uint32_t zr = hadd2_u(hadd2_u(c.z2, kMagic1024), H2_N1024);
-                            constexpr uint32_t kAdd = SPARSE ? SparseTable<SPARSE, NT>::kFastBound : 0x1FFFu;
-                            const uint32_t zlo = c.z2 & 0xFFFFu;
-                            return ((zlo | ((zlo & 0x7FFFu) + kAdd) | c.s2) & 0x8000u) | (zr ^ c.z2);
-                        };
-                        // after the last read of the weight stage
-                        auto release_weights = [&]() {
-                            __syncwarp();
-                            if (lane == 0) ptx::mbar_arrive(bar(offsetof(Barriers, w_empty), ws));
-                        };
-                        // before the first store into the A stage
-                        auto acquire_a_stage = [&]() -> bool {
-                            if (C::kDeferArrive && pending >= 0) announce(pending);       // before any wait: the MMAs must be able to go on
-                            // the A stage (and its activation tile) is free once the MMAs of its previous use have completed
-                            if (!free_early && !ptx::mbar_wait(bar(offsetof(Barriers, ab_free), as), aph ^ 1u)) {
-                                if (lane == 0) atomicExch(p.status, 32);
-                                return false;
-                            }
-                            ptx::tc_fence_after_sync();
-                            return true;
-                        };
-                        // The parts are decoded in the fast mode by straight-line code, without a mode decision in between;
-                        // whether every group of the unit really is in the fast mode (for every column of the warp) is
-                        // voted once, when the last group has been read and before the weight stage is released.  If not,
-                        // the unit is decoded again with a decision per part (the stores are simply overwritten).
-                        bool redo = false;
-                        {
-                            ColK c;
-                            uint32_t cur_row = 0xFFFFFFFFu, nf = 0;
-#pragma unroll
-                            for (int h = 0; h < H; ++h) {
-                                // scale and zero-point change only where the group does (warp-uniform)
-                                const uint32_t row = (h == 0) ? 0u : (p.gdiv((uint32_t)H * (uint32_t)u + (uint32_t)h) - g0);   // 0 .. H - 1
-                                if (row != cur_row) {
-                                    cur_row = row;
-                                    load_group(row, c);
-                                    nf |= not_fast_bits(c);
-                                    if (SPARSE) c.zb = __half2uint_rz(__ushort_as_half((unsigned short)(c.z2 & 0xFFFFu))) * 0x01010101u;
-                                }
-                                if (h == H - 1 && __any_sync(0xFFFFFFFFu, nf != 0)) {
-                                    redo = true;
-                                    break;
-                                }
-                                uint32_t A[32];
-                                F::template decode<MODE_FAST>(st + WS::kW + h * (F::WROWS * 512) + col * 4, st + WS::kMask + h * (F::MROWS * 512) + col * 4, c, A, lut);
-                                if (h == H - 1) release_weights();
-                                if (h == 0 && !acquire_a_stage()) { ok = false; break; }
-                                ptx::tmem_st32(lane_addr + C::kACol0 + as * C::kAStageCols + h * 32, A);
-                            }
-                        }
-                        if (redo && ok) {
-                            // some group needs the general or the per-weight mode (rolled loop: three decode bodies in the
-                            // instruction cache, not three per part)
-                            ptx::tc_wait_st();
-                            ColK c;
-                            uint32_t cur_row = 0xFFFFFFFFu;
-#pragma unroll 1
-                            for (int h = 0; h < H; ++h) {
-                                const uint32_t row = (h == 0) ? 0u : (p.gdiv((uint32_t)H * (uint32_t)u + (uint32_t)h) - g0);
-                                if (row != cur_row) {
-                                    cur_row = row;
-                                    load_group(row, c);
-                                }
-                                const uint32_t wb = st + WS::kW + h * (F::WROWS * 512) + col * 4;
-                                const uint32_t mb = st + WS::kMask + h * (F::MROWS * 512) + col * 4;
-                                uint32_t A[32];
-                                if (!__any_sync(0xFFFFFFFFu, not_fast_bits(c) != 0)) {
-                                    if (SPARSE) c.zb = __half2uint_rz(__ushort_as_half((unsigned short)(c.z2 & 0xFFFFu))) * 0x01010101u;
-                                    F::template decode<MODE_FAST>(wb, mb, c, A, lut);
-                                } else {
-                                    c.zb = 0;
-                                    const bool lin = __hge(__ushort_as_half((unsigned short)(c.s2 & 0xFFFFu)), __ushort_as_half(0));
-                                    if (__all_sync(0xFFFFFFFFu, lin)) F::template decode<MODE_GENERAL>(wb, mb, c, A, lut);
-                                    else F::template decode<MODE_SLOW>(wb, mb, c, A, lut);
-                                }
-                                if (h == H - 1) release_weights();
-                                ptx::tmem_st32(lane_addr + C::kACol0 + as * C::kAStageCols + h * 32, A);
-                            }
-                        }
-                        if (!ok) break;
-                        // (not deferred for the warpgroup's first stage: the pipeline is still filling and the MMA warp is waiting)
-                        if (C::kDeferArrive && si >= (uint32_t)C::kWG) pending = (int)as;
-                        else announce((int)as);
-                    }
-                    if (!ok) break;
-                    if (C::kDeferArrive && pending >= 0) { announce(pending); pending = -1; }
-                    if (!C::kEpiWarps && wg == 0) ok = after_segment(seg, tile, u0, u1);
-                    ++seg;
-                    si0 += (uint32_t)(u1 - u0);
-                    t += u1 - u0;
-                }
-    return ok ? (int)seg : -1;
-}
-
-// The same as a function of its own for the few-row shapes, where this loop is what bounds the kernel: inside the kernel
-// its registers and instructions changed with every change to the other roles.
-template <class F, int NT, class Entry>
-__device__ __noinline__ int dequant_role(const UmmaParams& p, uint32_t bars, uint32_t w_ring, uint32_t tmem_base, long long t_lo, long long t_hi, const Entry* lut) {
-    return dequant_units<F, NT, false>(p, bars, w_ring, tmem_base, t_lo, t_hi, lut, [](uint32_t, long long, int, int) { return true; });
-}
-
-// The weight-streaming shapes (one row tile).  Split-K: the CTAs b_lo .. b_hi share this tile.  b_lo, which owns its
-// first units and reaches them last, adds the others' partial tiles to its own accumulator in CTA order - a fixed
-// order, so results are reproducible; the others wait for nobody.  A partial element is one 64-bit word (fp32
-// value | tag 1 in the high half), written with a single store, so no fence, counter or second round trip is
-// needed; the reader clears what it has read, which leaves the scratch all-zero for the next launch.  One slot per
-// CTA is enough: a CTA has at most one tile that it shares and does not sum.
-// A CTA's last tile is left to all of its warpgroups, `part` of `parts` rows each, since the dequant warps have
-// nothing else to do by then: what counts there is the number of dependent round trips to L2 (~0.7 us each), and so
-// the number of loads in flight.
-// A function of its own, so that its registers do not weigh on the dequantisation loop (inlined: 16384 x 16384, one row,
-// 37.7 -> 44.7 us).
+// The weight-streaming shapes but for PERM's (one row tile).  Split-K: the CTAs b_lo .. b_hi share this tile.  b_lo, which
+// owns its first units and reaches them last, adds the others' partial tiles to its own accumulator in CTA order - a fixed
+// order, so results are reproducible; the others wait for nobody.  A partial element is one 64-bit word (fp32 value | tag 1
+// in the high half), written with a single store, so no fence, counter or second round trip is needed; the reader clears
+// what it has read, which leaves the scratch all-zero for the next launch.  One slot per CTA is enough: a CTA has at most one
+// tile that it shares and does not sum.
+// What bounds it is the number of dependent round trips to L2 (~0.7 us each) between the last MMA and the end of the launch.
+// So a CTA's last tile is left to all of its warpgroups, `part` of `parts` rows each (the dequant warps have nothing else to do
+// by then), and every thread has 16 loads in flight.  With one warpgroup that read 8 rows of one partner at a time, 16384 x 5120
+// int4 took 25.2 us with 16 rows and 35.7 with 32; now 20.4 and 24.0 (one row, where there is one load: 17.0 both).
+// A function of its own, so that its registers do not weigh on the dequantisation loop.
+// t0, units: the CTA's units of the tile.  handed: the caller is the epilogue warpgroup, which the MMA warp releases.
 template <int NT, bool LAST>
 __device__ __noinline__ bool split_epilogue(const UmmaParams& p, uint32_t tmem_base, uint32_t d_full, uint32_t d_empty, const volatile int* s_abort,
                                             uint32_t seg, long long t0, int units, int part, int parts, bool handed) {
@@ -588,14 +422,14 @@ __device__ __noinline__ bool split_epilogue(const UmmaParams& p, uint32_t tmem_b
 // PAIR: launched as clusters of two CTAs (two SMs) that run every MMA together (cta_group::2, M = 256): the pair's
 // tile is 256 weight columns x NT rows, each CTA dequantises its own 128 columns and loads only half of the rows of
 // the activation tile, which halves the L2 -> shared-memory traffic that bounds the many-row shapes.
-// PERM (up to 8 rows of dense int4 only): the cheaper k order of UFormat, with the activations reordered to match.
+// PERM (up to 3 rows of dense int4 only): the cheaper k order of UFormat, with the activations reordered to match.
 template <int BITS, bool SPARSE, int NT, bool PAIR, bool PERM = false>
 __global__ void __launch_bounds__(Cfg<NT, PAIR>::kThreads, Cfg<NT, PAIR>::kMinBlocks)
 umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaParams p, const __half* x) {
     using C = Cfg<NT, PAIR>;
     using F = UFormat<BITS, SPARSE, PERM>;
     static_assert(!PERM || (C::kStream && F::kPermutedK), "the permuted k order is for dense int4 weight streaming");
-    constexpr bool kSpread = C::kStream && !PERM;                  // the last tile's epilogue is every warpgroup's (split_epilogue)
+    constexpr bool kSpread = C::kStream && !PERM;                    // every warpgroup takes part in the last tile's epilogue
     constexpr int H = C::kHalves;                                    // 64-k parts per unit
     using WS = WStage<F, H>;
     static_assert(!PAIR || (NT >= 128 && !C::kEpiHandoff), "CTA pairs are for the many-row shapes");
@@ -1183,22 +1017,18 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
             return true;
         };
 
-        bool aborted = false;                                     // (kSpread)
-        uint32_t last_seg = 0;
+        uint32_t seg = 0;
+        bool aborted = false;                                              // a wait timed out (kSpread)
         if (C::kEpiWarps && warp >= kEpiWarp0 + 4 * kEpiGroups) {
             // (an epilogue warpgroup that this configuration does not use)
         } else if (C::kEpiWarps && warp >= kEpiWarp0) {
             // ----- dedicated epilogue warps: one pass per segment -----
-            uint32_t seg = 0;
             for (long long t = t_lo; t < t_hi;) {
                 const long long tile = div_nn(t, U);
                 const int u0 = (int)(t - tile * U);
                 const int u1 = (int)min(U, u0 + (t_hi - t));
                 if constexpr (kSpread) {
-                    if (t + (u1 - u0) >= t_hi) {                       // the last tile is everybody's: below
-                        last_seg = seg;
-                        break;
-                    }
+                    if (t + (u1 - u0) >= t_hi) break;                  // the last tile is everybody's: below
                     if (!split_epilogue<NT, false>(p, tmem_base, ptx::smem_u32(&bars.d_full), ptx::smem_u32(&bars.d_empty), &s_abort, seg, t, u1 - u0, 0, 1, true)) {
                         aborted = true;
                         break;
@@ -1209,20 +1039,153 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
             }
         } else {
             // ----- dequant warps -----
-            if constexpr (kSpread) {
-                const int segs = dequant_role<F, NT>(p, ptx::smem_u32(&bars), w_ring, tmem_base, t_lo, t_hi, lut);
-                aborted = segs < 0;
-                last_seg = (uint32_t)(segs - 1);
-            } else {
-                dequant_units<F, NT, PAIR>(p, ptx::smem_u32(&bars), w_ring, tmem_base, t_lo, t_hi, lut, epilogue);
+            const int wg = warp >> 2;                                           // warpgroup: takes every kWG-th weight stage
+            const int col = (warp & 3) * 32 + lane;                             // weight column in the tile = tensor-memory lane
+            const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
+            uint32_t si0 = 0;                                                    // si0: weight stages consumed before this segment
+            int pending = -1;                                                    // A stage written but not yet announced (Cfg::kDeferArrive)
+            // the stores into tensor memory are complete -> the stage may be read by the MMAs
+            auto announce = [&](int stage) {
+                ptx::tc_wait_st();
+                ptx::tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) {
+                    if (PAIR) ptx::mbar_arrive_cluster(ptx::map_to_cta(ptx::smem_u32(&bars.ab_full[stage]), 0));
+                    else ptx::mbar_arrive(ptx::smem_u32(&bars.ab_full[stage]));
+                }
+            };
+            bool ok = true;
+            for (long long t = t_lo; t < t_hi && ok;) {
+                const long long tile = div_nn(t, U);
+                const int u0 = (int)(t - tile * U);
+                const int u1 = (int)min(U, u0 + (t_hi - t));
+                // this warpgroup's units of the segment: those whose stage index is congruent to wg modulo kWG
+                for (int u = u0 + (int)(((uint32_t)wg + (uint32_t)C::kWG - si0 % (uint32_t)C::kWG) % (uint32_t)C::kWG); u < u1; u += C::kWG) {
+                    const uint32_t si = si0 + (uint32_t)(u - u0);
+                    const uint32_t ws = si % C::kWStages, wph = (si / C::kWStages) & 1u;     // constants: multiply-shift, no division
+                    if (C::kWGuard && !ptx::mbar_wait(ptx::smem_u32(&bars.w_empty[ws]), wph ^ 1u)) {   // see Cfg::kWStages
+                        if (lane == 0) atomicExch(p.status, 35);
+                        ok = false;
+                        break;
+                    }
+                    if (!ptx::mbar_wait(ptx::smem_u32(&bars.w_full[ws]), wph)) {
+                        if (lane == 0) atomicExch(p.status, 31);
+                        ok = false;
+                        break;
+                    }
+                    const uint32_t st = w_ring + ws * WS::kBytes;
+                    const uint32_t g0 = p.gdiv((uint32_t)H * (uint32_t)u);
+                    const uint32_t as = si % kABStages, aph = (si / kABStages) & 1u;
+                    // polled before the first part is decoded, so that the answer costs no latency when it is needed
+                    const bool free_early = ptx::mbar_test_wait(ptx::smem_u32(&bars.ab_free[as]), aph ^ 1u);
+                    // scale and zero-point of this thread's column in row `row` of the stage's group box, both halves of a register
+                    auto load_group = [&](uint32_t row, ColK& c) {
+                        const uint32_t sz = ptx::lds32(st + WS::kS + row * 256 + (col & ~1) * 2) >> (16 * (col & 1));
+                        const uint32_t zz = ptx::lds32(st + WS::kZ + row * 256 + (col & ~1) * 2) >> (16 * (col & 1));
+                        c.s2 = prmt(sz, sz, 0x1010);
+                        c.z2 = prmt(zz, zz, 0x1010);
+                        c.zb = 0;
+                    };
+                    // fast mode needs: scale sign clear, zero-point an integer in [0, 512] (sparse format: see SparseTable)
+                    auto not_fast_bits = [&](const ColK& c) -> uint32_t {
+                        const uint32_t zr = hadd2_u(hadd2_u(c.z2, kMagic1024), H2_N1024);
+                        constexpr uint32_t kAdd = SPARSE ? SparseTable<SPARSE, NT>::kFastBound : 0x1FFFu;
+                        const uint32_t zlo = c.z2 & 0xFFFFu;
+                        return ((zlo | ((zlo & 0x7FFFu) + kAdd) | c.s2) & 0x8000u) | (zr ^ c.z2);
+                    };
+                    // after the last read of the weight stage
+                    auto release_weights = [&]() {
+                        __syncwarp();
+                        if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&bars.w_empty[ws]));
+                    };
+                    // before the first store into the A stage
+                    auto acquire_a_stage = [&]() -> bool {
+                        if (C::kDeferArrive && pending >= 0) announce(pending);       // before any wait: the MMAs must be able to go on
+                        // the A stage (and its activation tile) is free once the MMAs of its previous use have completed
+                        if (!free_early && !ptx::mbar_wait(ptx::smem_u32(&bars.ab_free[as]), aph ^ 1u)) {
+                            if (lane == 0) atomicExch(p.status, 32);
+                            return false;
+                        }
+                        ptx::tc_fence_after_sync();
+                        return true;
+                    };
+                    // The parts are decoded in the fast mode by straight-line code, without a mode decision in between;
+                    // whether every group of the unit really is in the fast mode (for every column of the warp) is
+                    // voted once, when the last group has been read and before the weight stage is released.  If not,
+                    // the unit is decoded again with a decision per part (the stores are simply overwritten).
+                    bool redo = false;
+                    {
+                        ColK c;
+                        uint32_t cur_row = 0xFFFFFFFFu, nf = 0;
+#pragma unroll
+                        for (int h = 0; h < H; ++h) {
+                            // scale and zero-point change only where the group does (warp-uniform)
+                            const uint32_t row = (h == 0) ? 0u : (p.gdiv((uint32_t)H * (uint32_t)u + (uint32_t)h) - g0);   // 0 .. H - 1
+                            if (row != cur_row) {
+                                cur_row = row;
+                                load_group(row, c);
+                                nf |= not_fast_bits(c);
+                                if (SPARSE) c.zb = __half2uint_rz(__ushort_as_half((unsigned short)(c.z2 & 0xFFFFu))) * 0x01010101u;
+                            }
+                            if (h == H - 1 && __any_sync(0xFFFFFFFFu, nf != 0)) {
+                                redo = true;
+                                break;
+                            }
+                            uint32_t A[32];
+                            F::template decode<MODE_FAST>(st + WS::kW + h * (F::WROWS * 512) + col * 4, st + WS::kMask + h * (F::MROWS * 512) + col * 4, c, A, lut);
+                            if (h == H - 1) release_weights();
+                            if (h == 0 && !acquire_a_stage()) { ok = false; break; }
+                            ptx::tmem_st32(lane_addr + C::kACol0 + as * C::kAStageCols + h * 32, A);
+                        }
+                    }
+                    if (redo && ok) {
+                        // some group needs the general or the per-weight mode (rolled loop: three decode bodies in the
+                        // instruction cache, not three per part)
+                        ptx::tc_wait_st();
+                        ColK c;
+                        uint32_t cur_row = 0xFFFFFFFFu;
+#pragma unroll 1
+                        for (int h = 0; h < H; ++h) {
+                            const uint32_t row = (h == 0) ? 0u : (p.gdiv((uint32_t)H * (uint32_t)u + (uint32_t)h) - g0);
+                            if (row != cur_row) {
+                                cur_row = row;
+                                load_group(row, c);
+                            }
+                            const uint32_t wb = st + WS::kW + h * (F::WROWS * 512) + col * 4;
+                            const uint32_t mb = st + WS::kMask + h * (F::MROWS * 512) + col * 4;
+                            uint32_t A[32];
+                            if (!__any_sync(0xFFFFFFFFu, not_fast_bits(c) != 0)) {
+                                if (SPARSE) c.zb = __half2uint_rz(__ushort_as_half((unsigned short)(c.z2 & 0xFFFFu))) * 0x01010101u;
+                                F::template decode<MODE_FAST>(wb, mb, c, A, lut);
+                            } else {
+                                c.zb = 0;
+                                const bool lin = __hge(__ushort_as_half((unsigned short)(c.s2 & 0xFFFFu)), __ushort_as_half(0));
+                                if (__all_sync(0xFFFFFFFFu, lin)) F::template decode<MODE_GENERAL>(wb, mb, c, A, lut);
+                                else F::template decode<MODE_SLOW>(wb, mb, c, A, lut);
+                            }
+                            if (h == H - 1) release_weights();
+                            ptx::tmem_st32(lane_addr + C::kACol0 + as * C::kAStageCols + h * 32, A);
+                        }
+                    }
+                    if (!ok) break;
+                    // (not deferred for the warpgroup's first stage: the pipeline is still filling and the MMA warp is waiting)
+                    if (C::kDeferArrive && si >= (uint32_t)C::kWG) pending = (int)as;
+                    else announce((int)as);
+                }
+                if (!ok) { aborted = true; break; }
+                if (C::kDeferArrive && pending >= 0) { announce(pending); pending = -1; }
+                if (!C::kEpiWarps && wg == 0) ok = epilogue(seg, tile, u0, u1);
+                if (!kSpread || t + (u1 - u0) < t_hi) ++seg;
+                si0 += (uint32_t)(u1 - u0);
+                t += u1 - u0;
             }
         }
         if constexpr (kSpread) {
-            // the CTA's last tile (or its part of one): every warpgroup takes some of the rows
-            if (!aborted && t_lo < t_hi && (p.rows > 4 || warp >= kEpiWarp0)) {
+            const bool all = p.rows > 1;
+            if (!aborted && t_lo < t_hi && (all || warp >= kEpiWarp0)) {
                 const long long t0 = max(t_lo, div_nn(t_hi - 1, U) * U);
-                split_epilogue<NT, true>(p, tmem_base, ptx::smem_u32(&bars.d_full), ptx::smem_u32(&bars.d_empty), &s_abort, last_seg, t0, (int)(t_hi - t0),
-                                         p.rows > 4 ? warp >> 2 : 0, p.rows > 4 ? C::kWG + 1 : 1, warp >= kEpiWarp0);
+                split_epilogue<NT, true>(p, tmem_base, ptx::smem_u32(&bars.d_full), ptx::smem_u32(&bars.d_empty), &s_abort, seg, t0, (int)(t_hi - t0),
+                                         all ? warp >> 2 : 0, all ? C::kWG + 1 : 1, warp >= kEpiWarp0);
             }
         }
     }
@@ -1599,9 +1562,10 @@ int launch_fmt(UmmaParams& p, const __half* x, int n_groups, int pair_mode, int 
     }
     switch (nt) {
         case 16:
-            // up to 8 rows of dense int4: the k order that needs no byte shuffles (more rows would cost the one warp
-            // that reorders the activations more per unit than the unit takes)
-            if (BITS == 4 && !SPARSE && p.rows <= g_tune[1]) return launch_nt<BITS, SPARSE, 16, false, BITS == 4 && !SPARSE>(p, x, n_groups, stream, cuda_err);
+            // up to 3 rows of dense int4: the k order that needs no byte shuffles.  More rows cost the one warp that reorders the
+            // activations more per unit than the unit takes (16384 x 16384, this order / the natural one: 1 row 37.8 / 40.8 us,
+            // 3 rows 41.0 / 41.2, 4 rows 44.7 / 41.5, 8 rows 55.5 / 42.2)
+            if (BITS == 4 && !SPARSE && p.rows <= 3) return launch_nt<BITS, SPARSE, 16, false, BITS == 4 && !SPARSE>(p, x, n_groups, stream, cuda_err);
             return launch_nt<BITS, SPARSE, 16, false>(p, x, n_groups, stream, cuda_err);
         case 32: return launch_nt<BITS, SPARSE, 32, false>(p, x, n_groups, stream, cuda_err);
         case 64: return launch_nt<BITS, SPARSE, 64, false>(p, x, n_groups, stream, cuda_err);
