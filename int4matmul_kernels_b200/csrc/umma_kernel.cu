@@ -294,10 +294,11 @@ struct TensorMaps {
 // by then), and every thread has 16 loads in flight.  With one warpgroup that read 8 rows of one partner at a time, 16384 x 5120
 // int4 took 25.2 us with 16 rows and 35.7 with 32; now 20.4 and 24.0 (one row, where there is one load: 17.0 both).
 // A function of its own, so that its registers do not weigh on the dequantisation loop.
-// t0, units: the CTA's units of the tile.  handed: the caller is the epilogue warpgroup, which the MMA warp releases.
+// t0, units: the CTA's units of the tile.  bar_id, bar_threads: the named barrier at which the MMA warp says that the accumulator
+// is complete (once per call, also where this part has no rows).
 template <int NT, bool LAST>
-__device__ __noinline__ bool split_epilogue(const UmmaParams& p, uint32_t tmem_base, uint32_t d_full, uint32_t d_empty, const volatile int* s_abort,
-                                            uint32_t seg, long long t0, int units, int part, int parts, bool handed) {
+__device__ __noinline__ bool split_epilogue(const UmmaParams& p, uint32_t tmem_base, uint32_t d_empty, const volatile int* s_abort, long long t0,
+                                            int units, int part, int parts, uint32_t bar_id, uint32_t bar_threads) {
     // outputs, old outputs and the scratch may still be in use by the kernel before this one in the stream
     ptx::grid_dependency_wait();
     const int warp = (int)(threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -319,13 +320,9 @@ __device__ __noinline__ bool split_epilogue(const UmmaParams& p, uint32_t tmem_b
     auto wait_accumulator = [&]() -> bool {
         if (accumulator_ready) return true;
         accumulator_ready = true;
-        if (handed) {
-            ptx::named_bar_sync(2, 128 + 32);      // released by the MMA warp once the accumulator is complete
-            if (*s_abort) return false;
-        } else if (!ptx::mbar_wait(d_full, seg & 1u)) {
-            if (lane == 0) atomicExch(p.status, 33);
-            return false;
-        }
+        __syncwarp();
+        ptx::named_bar_sync(bar_id, bar_threads);      // released by the MMA warp once the accumulator is complete
+        if (*s_abort) return false;
         ptx::tc_fence_after_sync();
         return true;
     };
@@ -414,7 +411,7 @@ __device__ __noinline__ bool split_epilogue(const UmmaParams& p, uint32_t tmem_b
         for (int rb = r0; rb < r1; rb += 8)
             if (!finish_rows(std::integral_constant<int, 8>(), std::integral_constant<int, 2>(), rb, min(8, r1 - rb))) return false;
     }
-    if (handed && !wait_accumulator()) return false;               // (no rows: the MMA warp's barrier still counts these warps)
+    if (!wait_accumulator()) return false;                         // (no rows: the barrier still counts these warps)
     if (p.om.n_dst > 1) __threadfence_system();                // as below
     return true;
 }
@@ -536,6 +533,12 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
         t_lo = range_lo(n_tiles, G, b) * U;
         t_hi = range_lo(n_tiles, G, b + 1) * U;
     }
+
+    // Every warpgroup takes part in the last tile's epilogue (one row is one load per thread: the epilogue warps' alone).  They
+    // meet the MMA warp at a named barrier of their own: a parity wait on d_full by the dequant warps, which may be several
+    // short tiles ahead of the MMAs, could take an earlier tile's phase for the last one's.
+    const bool spread_last = kSpread && p.rows > 1 && t_lo < t_hi;
+    constexpr uint32_t kSpreadThreads = (C::kWG + 1) * 128 + 32;
 
     if (warp == kWProducer || (C::kWProducers == 2 && warp == kWProducer2)) {
         // =========================== packed weights (+ scales / zeros): one thread per producer warp ===========================
@@ -679,12 +682,13 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
         {
             const uint32_t idesc = PAIR ? ptx::idesc_f16_m256(NT) : ptx::idesc_f16_m128(NT);
             uint32_t si = 0, seg = 0;
-            bool ok = true;
+            bool ok = true, last = false;
             if (PAIR && rank != 0) t_lo = t_hi;              // the leader issues for both CTAs
             for (long long t = t_lo; t < t_hi && ok;) {
                 const long long tile = div_nn(t, U);
                 const int u0 = (int)(t - tile * U);
                 const int u1 = (int)min(U, u0 + (t_hi - t));
+                last = t + (u1 - u0) >= t_hi;
                 if (!ptx::mbar_wait(ptx::smem_u32(&bars.d_empty), (seg & 1u) ^ 1u)) {
                     if (lane == 0) atomicExch(p.status, 21);
                     ok = false;
@@ -737,7 +741,8 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                         break;
                     }
                     ptx::tc_fence_before_sync();
-                    ptx::named_bar_arrive(2, 128 + 32);
+                    if (spread_last && last) ptx::named_bar_arrive(5, kSpreadThreads);
+                    else ptx::named_bar_arrive(2, 128 + 32);
                 }
                 ++seg;
                 t += u1 - u0;
@@ -745,7 +750,8 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
             if (C::kEpiHandoff && !ok) {
                 s_abort = 1;
                 __threadfence_block();
-                ptx::named_bar_arrive(2, 128 + 32);
+                if (!spread_last || !last) ptx::named_bar_arrive(2, 128 + 32);
+                if (spread_last) ptx::named_bar_arrive(5, kSpreadThreads);      // the last tile's: by every role once, whatever happened
             }
         }
     } else {
@@ -1029,7 +1035,7 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                 const int u1 = (int)min(U, u0 + (t_hi - t));
                 if constexpr (kSpread) {
                     if (t + (u1 - u0) >= t_hi) break;                  // the last tile is everybody's: below
-                    if (!split_epilogue<NT, false>(p, tmem_base, ptx::smem_u32(&bars.d_full), ptx::smem_u32(&bars.d_empty), &s_abort, seg, t, u1 - u0, 0, 1, true)) {
+                    if (!split_epilogue<NT, false>(p, tmem_base, ptx::smem_u32(&bars.d_empty), &s_abort, t, u1 - u0, 0, 1, 2, 128 + 32)) {
                         aborted = true;
                         break;
                     }
@@ -1175,17 +1181,18 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                 if (!ok) { aborted = true; break; }
                 if (C::kDeferArrive && pending >= 0) { announce(pending); pending = -1; }
                 if (!C::kEpiWarps && wg == 0) ok = epilogue(seg, tile, u0, u1);
-                if (!kSpread || t + (u1 - u0) < t_hi) ++seg;
+                ++seg;
                 si0 += (uint32_t)(u1 - u0);
                 t += u1 - u0;
             }
         }
         if constexpr (kSpread) {
-            const bool all = p.rows > 1;
-            if (!aborted && t_lo < t_hi && (all || warp >= kEpiWarp0)) {
+            if (aborted) {
+                if (spread_last) ptx::named_bar_arrive(5, kSpreadThreads);
+            } else if (spread_last || (warp >= kEpiWarp0 && t_lo < t_hi)) {
                 const long long t0 = max(t_lo, div_nn(t_hi - 1, U) * U);
-                split_epilogue<NT, true>(p, tmem_base, ptx::smem_u32(&bars.d_full), ptx::smem_u32(&bars.d_empty), &s_abort, seg, t0, (int)(t_hi - t0),
-                                         all ? warp >> 2 : 0, all ? C::kWG + 1 : 1, warp >= kEpiWarp0);
+                split_epilogue<NT, true>(p, tmem_base, ptx::smem_u32(&bars.d_empty), &s_abort, t0, (int)(t_hi - t0), spread_last ? warp >> 2 : 0,
+                                         spread_last ? C::kWG + 1 : 1, spread_last ? 5 : 2, spread_last ? kSpreadThreads : 128 + 32);
             }
         }
     }
