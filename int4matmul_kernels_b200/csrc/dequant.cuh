@@ -14,6 +14,12 @@ __device__ __forceinline__ uint32_t bit_select(uint32_t mask, uint32_t a, uint32
     asm("lop3.b32 %0, %1, %2, %3, 0xCA;" : "=r"(d) : "r"(mask), "r"(a), "r"(b));
     return d;
 }
+// (a & b) ^ c
+__device__ __forceinline__ uint32_t and_xor(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t d;
+    asm("lop3.b32 %0, %1, %2, %3, 0x6A;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
 __device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t b, uint32_t c) {
     uint32_t d;
     asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
@@ -51,8 +57,7 @@ constexpr uint32_t MUL_1_1 = 0x3C003C00u, BASE_1_1 = 0xE400E400u;        // (x1,
 // The next 8 kept nibbles are spread over the bytes of a register pair (even nibbles, odd nibbles); two PRMTs put them
 // at their positions.  The selectors of both PRMTs are one 32-bit word of a 256-entry table indexed by the byte of the
 // keep-mask (nibble j of the word belongs to position j).  A dropped position selects 8, for which PRMT replicates the
-// sign of a byte below 128: it yields 0x00, also when the same selector is applied to a constant of 0x7F bytes, which
-// so becomes the mask of the kept positions.  A 1 KB table: the same look-up in a table of 16-byte entries (selectors, masks and
+// sign of a byte below 128 (a nibble, XORed with a zero-point below 128): it yields 0x00.  A 1 KB table: the same look-up in a table of 16-byte entries (selectors, masks and
 // popcount) takes ~10 shared-memory wavefronts per warp instead of ~3.5, because random entries of four banks collide.
 constexpr int kSparseLutEntries = 256;
 __device__ __forceinline__ uint32_t sparse_selectors(int keep) {
@@ -75,18 +80,21 @@ __device__ __forceinline__ void sparse_expand(uint32_t& lo, uint32_t& hi, uint32
                                               uint32_t (&A)[4]) {
     const uint32_t byte4 = (step == 0 ? m << 2 : m >> (8 * step - 2)) & 0x3FCu;          // 4 x the mask byte: table offset
     const uint32_t sel = *reinterpret_cast<const uint32_t*>(reinterpret_cast<const char*>(lut) + byte4);
-    const uint32_t even = lo & 0x0F0F0F0Fu, odd = (lo >> 4) & 0x0F0F0F0Fu;
+    // Fast mode: a dropped position gets the (integer) zero-point as its nibble, so it decodes to +0.  The nibbles go through
+    // the PRMT with the zero-point XORed in, which the extraction's LOP3 does for nothing, so that a dropped position's 0x00 and
+    // a kept one's nibble both come right by one XOR afterwards (a mask of the kept positions and a select were two
+    // instructions of five per 4 positions: one row 16384 x 16384 57.3 -> 54.4 us, 2048 rows 5120 x 20480 350.5 -> 340.4)
+    const uint32_t flip = MODE == MODE_FAST ? c.zb : 0u;
+    const uint32_t even = and_xor(lo, 0x0F0F0F0Fu, flip), odd = and_xor(lo >> 4, 0x0F0F0F0Fu, flip);
     const uint32_t off = hsub2_u(BASE_1_1, c.z2);
 #pragma unroll
     for (int q4 = 0; q4 < 2; ++q4) {
         const uint32_t s = q4 ? sel >> 16 : sel;                                         // (PRMT reads the low 16 bits)
-        uint32_t d = prmt(even, odd, s);
-        const uint32_t keep = prmt(0x7F7F7F7Fu, 0x7F7F7F7Fu, s);
-        // fast mode: a dropped position gets the (integer) zero-point as its nibble, so it decodes to +0
-        if (MODE == MODE_FAST) d = bit_select(keep, d, c.zb);
+        const uint32_t d = prmt(even, odd, s) ^ flip;
         A[2 * q4] = finish<4, MODE>(prmt(d, 0x64646464u, 0x5140), MUL_1_1, BASE_1_1, off, c);
         A[2 * q4 + 1] = finish<4, MODE>(prmt(d, 0x64646464u, 0x7362), MUL_1_1, BASE_1_1, off, c);
         if (MODE != MODE_FAST) {                                                         // exact zeros at dropped positions
+            const uint32_t keep = prmt(0x7F7F7F7Fu, 0x7F7F7F7Fu, s);
             const uint32_t k = keep * 2u + (keep & 0x01010101u);                         // 0x7F -> 0xFF
             A[2 * q4] &= prmt(k, k, 0x1100);
             A[2 * q4 + 1] &= prmt(k, k, 0x3322);
