@@ -8,7 +8,7 @@
 //                     packed weight rows, the keep mask and the groups' scales / zeros of one unit (128 k; 256 k for
 //                     the weight-streaming shapes) into a shared-memory ring
 //   activation prod.  one thread: the activation tile (NT rows x one unit of k as 128-byte-swizzled sub-tiles of 64 k);
-//                     for dense int4 weight streaming the whole warp, which reorders k inside the tile (see UFormat)
+//                     for dense int4 with up to 3 rows the whole warp, which reorders k inside the tile (see UFormat)
 //   dequant warps     warpgroups of 4 warps take the units in turn; thread i of a group owns weight column i: reads
 //                     its packed words from shared memory, rebuilds fp16((q - zero) * scale) in registers and
 //                     writes them into its own tensor-memory lane with tcgen05.st (one packed int32 = 8 consecutive
@@ -16,8 +16,9 @@
 //   MMA warp          one elected thread issues 8 (16) x tcgen05.mma (M = 128, N = NT, K = 16) per unit, A from tensor
 //                     memory, B from the swizzled shared-memory tile, and commits to mbarriers that recycle the
 //                     stages; the accumulator never leaves tensor memory until the tile is done
-//   epilogue          4 warps read the accumulator (tcgen05.ld), convert to fp16 and store; a warpgroup of its own
-//                     except for 33..64 rows, where dequant warpgroup 0 does it
+//   epilogue          reads the accumulator (tcgen05.ld), converts to fp16 and stores: one warpgroup of its own for up to 32
+//                     rows (a CTA's last tile: from 2 rows on the dequant warpgroups as well, see last_epilogue), dequant
+//                     warpgroup 0 for 33..64, two warpgroups of their own (half of the columns each) above
 //
 // Configurations (Cfg<NT, PAIR>): NT <= 32 rows stream the weights once from HBM - one CTA per SM, 3 dequant warpgroups,
 // 9 weight stages and 3 A / activation stages of 256 k, and the (tile, unit) space cut into equal ranges per CTA
@@ -283,96 +284,165 @@ struct TensorMaps {
     CUtensorMap z;
 };
 
-// The weight-streaming shapes but for PERM's (one row tile).  Split-K: the CTAs b_lo .. b_hi share this tile.  b_lo, which
-// owns its first units and reaches them last, adds the others' partial tiles to its own accumulator in CTA order - a fixed
+// Rows 0 .. n - 1 of one column to every destination (out0: the first row in the first one).  Without a branch per row: a store
+// behind a loop over the destinations costs ~100 cycles.
+template <int RB>
+__device__ __forceinline__ void store_rows(const OutMap& om, __half* out0, long long ld, int n_dst, const __half (&h)[RB], int n) {
+#pragma unroll
+    for (int i = 0; i < RB; ++i)
+        if (i < n) out0[(size_t)i * ld] = h[i];
+    for (int d = 1; d < n_dst; ++d) {
+        __half* const out = om.dst[d] + (out0 - om.dst[0]);
+#pragma unroll
+        for (int i = 0; i < RB; ++i)
+            if (i < n) out[(size_t)i * ld] = h[i];
+    }
+}
+
+// The epilogue of the weight-streaming shapes (one row tile) but for PERM's.  Split-K: the CTAs b_lo .. b_hi share a tile.  b_lo,
+// which owns its first units and reaches them last, adds the others' partial tiles to its own accumulator in CTA order - a fixed
 // order, so results are reproducible; the others wait for nobody.  A partial element is one 64-bit word (fp32 value | tag 1
 // in the high half), written with a single store, so no fence, counter or second round trip is needed; the reader clears
 // what it has read, which leaves the scratch all-zero for the next launch.  One slot per CTA is enough: a CTA has at most one
-// tile that it shares and does not sum.
-// What bounds it is the number of dependent round trips to L2 (~0.7 us each) between the last MMA and the end of the launch.
-// So a CTA's last tile is left to all of its warpgroups, `part` of `parts` rows each (the dequant warps have nothing else to do
-// by then), and every thread has 16 loads in flight.  With one warpgroup that read 8 rows of one partner at a time, 16384 x 5120
-// int4 took 25.2 us with 16 rows and 35.7 with 32; now 20.4 and 24.0 (one row, where there is one load: 17.0 both).
-// A function of its own, so that its registers do not weigh on the dequantisation loop.
-// t0, units: the CTA's units of the tile.  bar_id, bar_threads: the named barrier at which the MMA warp says that the accumulator
-// is complete (once per call, also where this part has no rows).
-template <int NT, bool LAST>
-__device__ __noinline__ bool split_epilogue(const UmmaParams& p, uint32_t tmem_base, uint32_t d_empty, const volatile int* s_abort, long long t0,
-                                            int units, int part, int parts, uint32_t bar_id, uint32_t bar_threads) {
+// tile that it shares and does not sum.  A tile that a CTA sums is its last one, so there are two functions.
+
+// A tile before a CTA's last one, by the epilogue warps: a whole tile, or (share: this lane's column of the CTA's slot) the CTA's share
+// of a tile that another CTA sums.  The next tile's MMAs wait for it.  Not inlined and with its arguments by value: with `p` by
+// reference a call cost ~1 us (1024 x 32768 int4, 5 rows, three tiles a CTA: 16.2 us, now 13.4), and inlined it slowed the decode
+// loop (13824 x 5120 int4, 4 rows: 17.4 us, now 16.8).
+// out0: the column's first output; rows / out_rows: rows of the launch, and those that this lane stores.
+__device__ __noinline__ bool early_epilogue(const OutMap& om, int n_dst, long long ld, __half* out0, int rows, int out_rows, int accumulate,
+                                            unsigned long long* share, uint32_t tmem_base, uint32_t d_empty, uint32_t s_abort) {
+    const uint32_t lane_addr = tmem_base + ((threadIdx.x & 96u) << 16);
+    auto release = [&]() {
+        ptx::tc_fence_before_sync();
+        __syncwarp();
+        if ((threadIdx.x & 31) == 0) ptx::mbar_arrive(d_empty);
+    };
+    __half old[8];
+    auto load_old = [&](int rb) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            old[i] = __ushort_as_half(0);
+            if (accumulate && rb + i < out_rows) old[i] = out0[(size_t)(rb + i) * ld];
+        }
+    };
+    if (!share) load_old(0);
+    ptx::named_bar_sync(2, 128 + 32);              // released by the MMA warp once the accumulator is complete
+    if (ptx::lds32(s_abort)) return false;
+    ptx::tc_fence_after_sync();
+    if (share) {
+#pragma unroll 1
+        for (int rb = 0; rb < rows; rb += 16) {
+            uint32_t v[16];
+            ptx::tmem_ld16(lane_addr + rb, v);
+            ptx::tc_wait_ld();
+            if (rb + 16 >= rows) release();
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+                if (rb + i < rows) ptx::st_relaxed_gpu_u64(share + (rb + i) * 128, (1ull << 32) | v[i]);
+        }
+        return true;
+    }
+    auto finish_rows = [&](auto rb_tag, int rb) {
+        constexpr int RB = decltype(rb_tag)::value;
+        uint32_t v[RB];
+        ptx::tmem_ld(lane_addr + rb, v);
+        ptx::tc_wait_ld();
+        if (rb + RB >= rows) release();
+        __half h[RB];
+#pragma unroll
+        for (int i = 0; i < RB; ++i) {
+            const float f = __uint_as_float(v[i]);
+            h[i] = __float2half_rn(accumulate ? f + __half2float(old[i]) : f);
+        }
+        store_rows<RB>(om, out0 + (size_t)rb * ld, ld, n_dst, h, out_rows - rb);
+    };
+    if (rows <= 4) {
+        finish_rows(std::integral_constant<int, 4>(), 0);
+    } else {
+#pragma unroll 1
+        for (int rb = 0; rb < rows; rb += 8) {
+            if (rb > 0) load_old(rb);
+            finish_rows(std::integral_constant<int, 8>(), rb);
+        }
+    }
+    if (n_dst > 1) __threadfence_system();         // as in umma_kernel's epilogue
+    return true;
+}
+
+// A CTA's last tile: units t0 .. t0 + units - 1.  What bounds it is the number of dependent round trips to L2 (~0.7 us each) between
+// the last MMA and the end of the launch, so the tile can be left to all of the CTA's warpgroups (the dequant warps have nothing
+// else to do by then), `part` of `parts` rows each; a thread has RB x PB partial words in flight, up to 16: with 4 rows and 4
+// partners or 8 rows and 2 partners.  One warpgroup that read 8 rows of one partner at a time took 25.2 us with 16 rows of 16384 x 5120
+// int4 and 35.7 with 32; now 19.6 and 22.6.  (When: see spread_last.)
+// bar_id, bar_threads: the named barrier at which the MMA warp says that the accumulator is complete (once per call, also where this
+// part has no rows).  Inlined, with one pass over at most 8 rows: a call cost ~1 us here as well.
+template <int NT>
+__device__ __forceinline__ bool last_epilogue(const UmmaParams& p, uint32_t tmem_base, const volatile int* s_abort, long long t0, int units,
+                                              int part, int parts, uint32_t bar_id, uint32_t bar_threads) {
     // outputs, old outputs and the scratch may still be in use by the kernel before this one in the stream
     ptx::grid_dependency_wait();
     const int warp = (int)(threadIdx.x >> 5), lane = threadIdx.x & 31;
-    const long long U = p.U, G = gridDim.x, n_tiles = p.CT, tile = div_nn(t0, U);
+    const long long U = p.U, G = gridDim.x, tile = div_nn(t0, U);
     const int u0 = (int)(t0 - tile * U), u1 = u0 + units;
-    const int ct = (int)tile, col = (warp & 3) * 32 + lane, scol = ct * 128 + col;
+    const int col = (warp & 3) * 32 + lane, scol = (int)tile * 128 + col;
     const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
     const bool col_ok = scol < p.S;
-    const int me = (int)blockIdx.x, r0 = p.rows * part / parts, r1 = p.rows * (part + 1) / parts;
+    const int me = (int)blockIdx.x, r0 = p.rows * part / parts, n = p.rows * (part + 1) / parts - r0;      // n <= 8
     int b_lo = me, b_hi = me;
     if (u0 != 0 || u1 != (int)U) {
-        const long long T = n_tiles * U, lo_t = tile * U;
+        const long long T = p.CT * U, lo_t = tile * U;
         b_lo = range_owner(T, G, lo_t);
         b_hi = range_owner(T, G, lo_t + U - 1);
     }
     unsigned long long* const partials64 = reinterpret_cast<unsigned long long*>(p.partials);
     auto slot_of = [&](int bb) { return partials64 + (size_t)bb * NT * 128 + col; };
-    bool accumulator_ready = false;
     auto wait_accumulator = [&]() -> bool {
-        if (accumulator_ready) return true;
-        accumulator_ready = true;
         __syncwarp();
         ptx::named_bar_sync(bar_id, bar_threads);      // released by the MMA warp once the accumulator is complete
         if (*s_abort) return false;
         ptx::tc_fence_after_sync();
         return true;
     };
-    auto release_accumulator = [&]() {                 // (a last tile's is not waited for)
-        if (parts > 1) return;
-        ptx::tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(d_empty);
-    };
     if (me != b_lo) {
         if (!wait_accumulator()) return false;
-        unsigned long long* const mine = slot_of(me);
-#pragma unroll 1
-        for (int j0 = r0; j0 < r1; j0 += 16) {
-            uint32_t v[16];
-            ptx::tmem_ld16(lane_addr + j0, v);
-            ptx::tc_wait_ld();
+        unsigned long long* const mine = slot_of(me) + r0 * 128;
+        uint32_t v[8];
+        ptx::tmem_ld(lane_addr + r0, v);
+        ptx::tc_wait_ld();
 #pragma unroll
-            for (int j = 0; j < 16; ++j)
-                if (j0 + j < r1) ptx::st_relaxed_gpu_u64(mine + (j0 + j) * 128, (1ull << 32) | v[j]);
-        }
-        release_accumulator();
+        for (int i = 0; i < 8; ++i)
+            if (i < n) ptx::st_relaxed_gpu_u64(mine + i * 128, (1ull << 32) | v[i]);
         return true;
     }
-    __half* const out0 = p.om.dst[0] + (col_ok ? p.om.col(scol) : 0);
+    __half* const out0 = p.om.dst[0] + (col_ok ? p.om.col(scol) : 0) + (size_t)r0 * p.om.ld;
     bool waiting_ok = true;
-    // rows rb .. rb + n - 1 (n <= RB), the partners PB at a time: RB x PB loads in flight
-    auto finish_rows = [&](auto rb_tag, auto pb_tag, int rb, int n) -> bool {
+    // all of this part's rows (n <= RB), the partners PB at a time: RB x PB loads in flight
+    auto finish_rows = [&](auto rb_tag, auto pb_tag) -> bool {
         constexpr int RB = decltype(rb_tag)::value, PB = decltype(pb_tag)::value;
         float sum[RB];
         __half old[RB];
 #pragma unroll
         for (int i = 0; i < RB; ++i) {
             sum[i] = 0.f;
-            if (p.accumulate && i < n && col_ok) old[i] = out0[(size_t)(rb + i) * p.om.ld];
+            old[i] = __ushort_as_half(0);
+            if (p.accumulate && i < n && col_ok) old[i] = out0[(size_t)i * p.om.ld];
         }
 #pragma unroll 1
-        for (int q = b_lo + 1; LAST && q <= b_hi; q += PB) {
+        for (int q = b_lo + 1; q <= b_hi; q += PB) {
             unsigned long long w[PB][RB];
 #pragma unroll
             for (int j = 0; j < PB; ++j)
 #pragma unroll
                 for (int i = 0; i < RB; ++i)
-                    if (q + j <= b_hi && i < n) w[j][i] = ptx::ld_relaxed_gpu_u64(slot_of(q + j) + (rb + i) * 128);
+                    if (q + j <= b_hi && i < n) w[j][i] = ptx::ld_relaxed_gpu_u64(slot_of(q + j) + (r0 + i) * 128);
 #pragma unroll
             for (int j = 0; j < PB; ++j)
 #pragma unroll
                 for (int i = 0; i < RB; ++i)
                     if (q + j <= b_hi && i < n) {
-                        unsigned long long* const at = slot_of(q + j) + (rb + i) * 128;
+                        unsigned long long* const at = slot_of(q + j) + (r0 + i) * 128;
                         for (uint32_t spins = 0; (uint32_t)(w[j][i] >> 32) != 1u && waiting_ok; ++spins) {
                             if (spins >= ptx::kSpinLimit) {            // a contributor never delivered: report, stop waiting
                                 atomicExch(p.status, 34);
@@ -388,31 +458,24 @@ __device__ __noinline__ bool split_epilogue(const UmmaParams& p, uint32_t tmem_b
         }
         if (!wait_accumulator()) return false;
         uint32_t v[RB];
-        ptx::tmem_ld(lane_addr + rb, v);
+        ptx::tmem_ld(lane_addr + r0, v);
         ptx::tc_wait_ld();
-        if (rb + n >= r1) release_accumulator();
+        __half h[RB];
 #pragma unroll
         for (int i = 0; i < RB; ++i) {
-            if (i < n && col_ok) {
-                float f = __uint_as_float(v[i]) + sum[i];
-                const size_t at = (size_t)(rb + i) * p.om.ld;
-                if (p.accumulate) f += __half2float(old[i]);
-                const __half h = __float2half_rn(f);
-                out0[at] = h;
-                for (int d = 1; d < p.om.n_dst; ++d) p.om.dst[d][at + (out0 - p.om.dst[0])] = h;
-            }
+            float f = __uint_as_float(v[i]) + sum[i];
+            if (p.accumulate) f += __half2float(old[i]);
+            h[i] = __float2half_rn(f);
         }
+        store_rows<RB>(p.om, out0, p.om.ld, p.om.n_dst, h, col_ok ? n : 0);
         return true;
     };
-    if (r1 - r0 <= 4) {
-        if (r1 > r0 && !finish_rows(std::integral_constant<int, 4>(), std::integral_constant<int, 4>(), r0, r1 - r0)) return false;
+    if (n <= 4) {
+        if (!finish_rows(std::integral_constant<int, 4>(), std::integral_constant<int, 4>())) return false;
     } else {
-#pragma unroll 1
-        for (int rb = r0; rb < r1; rb += 8)
-            if (!finish_rows(std::integral_constant<int, 8>(), std::integral_constant<int, 2>(), rb, min(8, r1 - rb))) return false;
+        if (!finish_rows(std::integral_constant<int, 8>(), std::integral_constant<int, 2>())) return false;
     }
-    if (!wait_accumulator()) return false;                         // (no rows: the barrier still counts these warps)
-    if (p.om.n_dst > 1) __threadfence_system();                // as below
+    if (p.om.n_dst > 1) __threadfence_system();                // as in umma_kernel's epilogue
     return true;
 }
 
@@ -534,11 +597,20 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
         t_hi = range_lo(n_tiles, G, b + 1) * U;
     }
 
-    // Every warpgroup takes part in the last tile's epilogue (one row is one load per thread: the epilogue warps' alone).  They
-    // meet the MMA warp at a named barrier of their own: a parity wait on d_full by the dequant warps, which may be several
-    // short tiles ahead of the MMAs, could take an earlier tile's phase for the last one's.
-    const bool spread_last = kSpread && p.rows > 1 && t_lo < t_hi;
+    // Every warpgroup takes part in the epilogue of the last tile (not with one row, which is one load per thread: the epilogue warps'
+    // alone).  They meet the MMA warp at a named barrier of their own: a parity wait on d_full by the dequant warps, which may be
+    // several short tiles ahead of the MMAs, could take an earlier tile's phase for the last one's.
+    // Up to 6 rows of a tile that this CTA sums are the epilogue warps' alone if no partner's share is the partner's whole range (it
+    // delivered early, or there is none): these warps then have everything before the last MMA, while the dequant warps would start
+    // after it.  us, all warpgroups / epilogue warps: 1024 x 32768 int4 4 rows 13.7 / 12.6, 5 rows 14.4 / 13.4, 8 rows 14.2 / 13.4,
+    // but 3072 x 12288 8 rows 12.9 / 13.7; with shares that are whole ranges 512 x 8192 8 rows 7.5 / 9.0.
+    bool spread_last = false;
+    if (kSpread && p.rows > 1 && t_lo < t_hi) {
+        const long long first = div_nn(t_hi - 1, U) * U;               // the last tile's first unit
+        spread_last = p.rows > 6 || t_lo > first || range_lo(n_tiles * U, G, b + 2) <= first + U;
+    }
     constexpr uint32_t kSpreadThreads = (C::kWG + 1) * 128 + 32;
+    static_assert(!kSpread || NT <= 8 * (C::kWG + 1), "last_epilogue takes at most 8 rows a warpgroup");
 
     if (warp == kWProducer || (C::kWProducers == 2 && warp == kWProducer2)) {
         // =========================== packed weights (+ scales / zeros): one thread per producer warp ===========================
@@ -1034,8 +1106,13 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                 const int u0 = (int)(t - tile * U);
                 const int u1 = (int)min(U, u0 + (t_hi - t));
                 if constexpr (kSpread) {
-                    if (t + (u1 - u0) >= t_hi) break;                  // the last tile is everybody's: below
-                    if (!split_epilogue<NT, false>(p, tmem_base, ptx::smem_u32(&bars.d_empty), &s_abort, t, u1 - u0, 0, 1, 2, 128 + 32)) {
+                    if (t + (u1 - u0) >= t_hi) break;                  // the last tile: below
+                    ptx::grid_dependency_wait();                       // as in `epilogue`
+                    const int col = (int)threadIdx.x & 127, scol = (int)tile * 128 + col;
+                    const bool col_ok = scol < p.S;
+                    if (!early_epilogue(p.om, p.om.n_dst, p.om.ld, p.om.dst[0] + (col_ok ? p.om.col(scol) : 0), p.rows, col_ok ? p.rows : 0, p.accumulate,
+                                        u0 == 0 ? nullptr : reinterpret_cast<unsigned long long*>(p.partials) + (size_t)blockIdx.x * NT * 128 + col,
+                                        tmem_base, ptx::smem_u32(&bars.d_empty), ptx::smem_u32(const_cast<int*>(&s_abort)))) {
                         aborted = true;
                         break;
                     }
@@ -1191,8 +1268,8 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                 if (spread_last) ptx::named_bar_arrive(5, kSpreadThreads);
             } else if (spread_last || (warp >= kEpiWarp0 && t_lo < t_hi)) {
                 const long long t0 = max(t_lo, div_nn(t_hi - 1, U) * U);
-                split_epilogue<NT, true>(p, tmem_base, ptx::smem_u32(&bars.d_empty), &s_abort, t0, (int)(t_hi - t0), spread_last ? warp >> 2 : 0,
-                                         spread_last ? C::kWG + 1 : 1, spread_last ? 5 : 2, spread_last ? kSpreadThreads : 128 + 32);
+                last_epilogue<NT>(p, tmem_base, &s_abort, t0, (int)(t_hi - t0), spread_last ? warp >> 2 : 0, spread_last ? C::kWG + 1 : 1,
+                                  spread_last ? 5 : 2, spread_last ? kSpreadThreads : 128 + 32);
             }
         }
     }

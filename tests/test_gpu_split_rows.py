@@ -1,5 +1,7 @@
-"""GPU parity tests of the few-row tcgen05 shapes (2..32 rows) where column tiles are shared: the owner of a tile sums its partners'
-shares with every warpgroup, some rows each."""
+"""GPU parity tests of the few-row tcgen05 shapes (1..32 rows) where column tiles are shared: the owner of a tile sums its partners'
+shares, with its epilogue warps alone or with every warpgroup, some rows each (dense int4 with up to 3 rows runs in another k order)."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -7,17 +9,19 @@ import torch
 from int4matmul_kernels_b200 import capi, ops
 from oracle import reference_oracle as oracle
 
-from helpers import assert_parity, run_problem
+from helpers import assert_parity, run_problem, to_dev
 from test_gpu_stream import FORMATS, fmt_id
 
 pytestmark = pytest.mark.gpu
 P = capi.PATH_TCGEN05
 
 
-# one 256-k unit per CTA and as many partners as units (16384 x 64); a last unit that is only partly there; tiles cut in two or
-# three with a CTA in the middle (19 and 75 tiles of 8 units); whole tiles after shared ones (300 tiles); S % 128 = 64
+# By the CTAs of 148 SMs: one 256-k unit per CTA and as many partners as units (16384 x 64); a last unit that is only partly there
+# (8256 x 320); tiles shared by 7 or 8 CTAs, of which most hold one unit (19 tiles of 8 units); by 2 or 3, with a CTA in the middle
+# (75 tiles of 8 units); whole tiles after shared ones (300 tiles of 2 units); S % 128 = 64.  Up to 6 rows of tiles whose other shares
+# all came early in their CTAs' ranges are summed by the epilogue warps alone (two of the 75 and the 300 tiles)
 @pytest.mark.parametrize("n,s,g", [(16384, 64, 128), (8256, 320, 192), (2048, 2432, -1), (2048, 9536, 64), (512, 38400, 128)])
-@pytest.mark.parametrize("m", [2, 3, 4, 5, 9, 16, 17, 31, 32])
+@pytest.mark.parametrize("m", [1, 2, 3, 4, 5, 6, 7, 8, 9, 16, 17, 31, 32])
 @pytest.mark.parametrize("fmt", FORMATS, ids=fmt_id)
 def test_shared_tiles(fmt, m, n, s, g):
     bits, sparse = fmt
@@ -42,3 +46,45 @@ def test_matvec_route_adds_into_outs(fmt, batch):
     got = run_problem(p, path=P, outs_in=base)
     want, _, bound = oracle.expected(p, outs_in=base)
     assert_parity(got, want, bound, f"accumulate {fmt}")
+
+
+@pytest.mark.parametrize("fmt", FORMATS, ids=fmt_id)
+@pytest.mark.parametrize("batch", [1, 2, 4, 16, 32])
+def test_matvec_route_adds_into_outs_of_several_tiles_per_cta(fmt, batch):
+    """Tiles that a CTA sums before its last one (300 tiles of 2 units) read the old outputs as well."""
+    bits, sparse = fmt
+    n, s = 512, 38400
+    p = oracle.make_packed_problem(bits, n, s, 1, 64, sparse=sparse, batch=batch, seed=41)
+    base = np.random.default_rng(3).standard_normal((batch, 1, s)).astype(np.float16)
+    got = run_problem(p, path=P, outs_in=base, route="vec")
+    cols = np.unique(np.concatenate([np.arange(0, s, 128), np.arange(127, s, 128)]))         # both edges of every tile
+    want, bound = oracle.expected_columns(bits, p["matrix"], p["mask"], p["scales"], p["zeros"], 64, p["x"], cols,
+                                          outs_in=np.ascontiguousarray(base[..., cols]))
+    assert_parity(got[..., cols], want, bound, f"accumulate {fmt}")
+
+
+# shared tiles; whole tiles and shared ones; a few-row kernel's call (path 0) and K parts (48 rows), which store on their own
+@pytest.mark.parametrize("n,s", [(8256, 320), (512, 38400), (2048, 1024)])
+@pytest.mark.parametrize("m", [1, 2, 5, 16, 17, 32, 48])
+@pytest.mark.parametrize("path", [capi.PATH_AUTO, P])
+@pytest.mark.parametrize("fmt", [(4, False), (4, True)], ids=fmt_id)
+def test_several_destinations_hold_the_same_bits(fmt, path, m, n, s):
+    """Three ordinary local buffers as the gathering entry's destinations, with rows longer than S: each holds what one call with one
+    destination gives, and nothing else is written."""
+    bits, sparse = fmt
+    p = oracle.make_packed_problem(bits, n, s, m, 64, sparse=sparse, seed=n + m)
+    w = {k: to_dev(p[k]) if p[k] is not None else None for k in ("matrix", "mask", "scales", "zeros", "x")}
+    want = torch.empty((1, m, s), dtype=torch.float16, device="cuda")
+    getattr(ops, f"quant_int{bits}_linear_mult_mtx")(want, w["matrix"], w["x"], w["scales"], w["zeros"], 64, w["mask"], path=path)
+    lib, ld, stream = capi.load(), s + 64, torch.cuda.current_stream()
+    shape = lib.i4mm_last_launch_shape()
+    bufs = [torch.full((m, ld), 7.0, dtype=torch.float16, device="cuda") for _ in range(3)]
+    ws = ops.workspace(torch.device("cuda", torch.cuda.current_device()), stream)
+    status = lib.i4mm_quant_matmul_gather(bits, path, (ctypes.c_void_p * 3)(*[b.data_ptr() for b in bufs]), 3, ld, 1, 0, 1,
+                                          w["matrix"].data_ptr(), w["mask"].data_ptr() if sparse else None, w["x"].data_ptr(),
+                                          w["scales"].data_ptr(), w["zeros"].data_ptr(), m, n, s, p["scales"].shape[0], 64,
+                                          ws.data_ptr(), ws.numel(), stream.cuda_stream)
+    assert status == capi.OK and lib.i4mm_last_launch_shape() == shape
+    torch.cuda.synchronize()
+    for b in bufs:
+        assert torch.equal(b[:, :s], want[0]) and (b[:, s:] == 7.0).all()
