@@ -253,9 +253,9 @@ struct Cfg {
     static constexpr int kAStageCols = 32 * kHalves;
     static constexpr int kColsUsed = kDCols + kAStageCols * kABStages;
     static constexpr int kTmemCols = kColsUsed <= 256 ? 256 : 512;
-    // split-K over CTAs with a scratch reduction.  The code handles tiles of up to 128 rows, but the reducing CTA reads
-    // its partners' partial tiles in dependent L2 round trips (rows x partners / 8 of them): measured at 128 rows that
-    // costs 15-30 K cycles per tile and loses more than the better balance gains, so only the few-row shapes split.
+    // split-K over CTAs with a scratch reduction: the few-row shapes.  (It was measured at 128 rows with a sum by one warpgroup, one
+    // partner at a time: 15-30 K cycles per tile, which lost more than the better balance gained.  Not measured since the sum is
+    // spread over the warpgroups; more rows cut K into parts, see choose_kparts.)
     static constexpr bool kSplit = NT <= 32;
     static constexpr int kSlotElems = kDCols * 128;                   // 64-bit words of one CTA's partial tile in the scratch
     static constexpr int kMinBlocks = kStream ? 1 : NT <= 64 ? 2 : 1;
@@ -845,12 +845,8 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
             const bool col_ok = scol < p.S;
             const int row0 = mt * NT;
             const int nrows = min(NT, p.rows - row0);
-            // Split-K: the CTAs b_lo .. b_hi share this tile.  b_lo (which owns the tile's first units and reaches them
-            // last) adds the others' partial tiles to its own accumulator in CTA order - a fixed order, so results are
-            // reproducible.  A partial element is one 64-bit word (fp32 value | tag 1 in the high half), written with a
-            // single store, so no fence, counter or second round trip is needed; the reader clears what it has read,
-            // which leaves the scratch all-zero for the next launch.  Every other CTA's share of the tile is the first
-            // segment of its range, so one slot per CTA is enough.
+            // Split-K here is that of the permuted k order (PERM: dense int4, up to 3 rows).  Same protocol and order of the sum as
+            // last_epilogue, but one warpgroup alone reads the partners' shares, one partner at a time.
             int b_lo = 0, b_hi = -1;
             unsigned long long* slot = nullptr;
             unsigned long long* const partials64 = reinterpret_cast<unsigned long long*>(p.partials);
@@ -858,7 +854,7 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                 const long long T = n_tiles * U, lo_t = tile * U;
                 b_lo = range_owner(T, G, lo_t);
                 b_hi = range_owner(T, G, lo_t + U - 1);
-                if ((int)b != b_lo) slot = partials64 + (size_t)(PAIR ? b * 2 + rank : b) * C::kSlotElems;
+                if ((int)b != b_lo) slot = partials64 + (size_t)b * C::kSlotElems;
             }
             // K parts: fp32 rows j0 .. of this lane's column into the (part, row, S) scratch; the reduce kernel sums the parts
             auto put_kpart = [&](auto& v, int j0) {
@@ -876,22 +872,21 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                 for (int j = 0; j < CNT; ++j)
                     if (j0 + j < nrows) ptx::st_relaxed_gpu_u64(slot + (j0 + j) * 128 + col, (1ull << 32) | v[j]);
             };
-            // adds the other CTAs' partial rows j0 .. j0 + n - 1 to v, in CTA order, and clears them
-            auto add_partials = [&](auto& v, int j0) {
-                constexpr int CNT = (int)(sizeof(v) / sizeof(uint32_t));
+            // adds the other CTAs' partial rows to v, in CTA order, and clears them
+            auto add_partials = [&](uint32_t (&v)[16]) {
                 bool waiting_ok = true;
                 for (int bb = b_lo + 1; bb <= b_hi; ++bb) {
-                    unsigned long long* src = partials64 + (size_t)(PAIR ? bb * 2 + (int)rank : bb) * C::kSlotElems + col;
+                    unsigned long long* src = partials64 + (size_t)bb * C::kSlotElems + col;
 #pragma unroll
-                    for (int jb = 0; jb < CNT; jb += 8) {
-                        if (j0 + jb >= nrows) break;                       // warp-uniform
+                    for (int jb = 0; jb < 16; jb += 8) {
+                        if (jb >= nrows) break;                            // warp-uniform
                         unsigned long long w[8];
 #pragma unroll
                         for (int i = 0; i < 8; ++i)
-                            if (j0 + jb + i < nrows) w[i] = ptx::ld_relaxed_gpu_u64(src + (j0 + jb + i) * 128);
+                            if (jb + i < nrows) w[i] = ptx::ld_relaxed_gpu_u64(src + (jb + i) * 128);
 #pragma unroll
                         for (int i = 0; i < 8; ++i) {
-                            if (j0 + jb + i < nrows) {
+                            if (jb + i < nrows) {
                                 for (uint32_t spins = 0; (uint32_t)(w[i] >> 32) != 1u && waiting_ok; ++spins) {
                                     if (spins >= ptx::kSpinLimit) {        // a contributor never delivered: report, stop waiting
                                         atomicExch(p.status, 34);
@@ -899,29 +894,23 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                                         break;
                                     }
                                     __nanosleep(64);
-                                    w[i] = ptx::ld_relaxed_gpu_u64(src + (j0 + jb + i) * 128);
+                                    w[i] = ptx::ld_relaxed_gpu_u64(src + (jb + i) * 128);
                                 }
                                 v[jb + i] = __float_as_uint(__uint_as_float(v[jb + i]) + __uint_as_float((uint32_t)w[i]));
-                                ptx::st_relaxed_gpu_u64(src + (j0 + jb + i) * 128, 0ull);
+                                ptx::st_relaxed_gpu_u64(src + (jb + i) * 128, 0ull);
                             }
                         }
                     }
                 }
             };
-            // The weight-streaming shapes fetch the other CTAs' partial tiles BEFORE the own accumulator is complete (the
-            // partners delivered them early in their run, as their first segment, and these warps have nothing else to
-            // do): their sum, in CTA order, then only has to be added, and the dependent round trips to L2 are off the tail.
-            constexpr int kPre = (C::kSplit && C::kEpiHandoff) ? C::kDCols : 1;
-            uint32_t pre[kPre];
-            bool prefetched = false;
-            if (C::kSplit && C::kEpiHandoff && !slot && b_hi > b_lo) {
+            // The other CTAs' partial tiles are fetched BEFORE the own accumulator is complete (the partners delivered them
+            // early in their run, as their first segment, and these warps have nothing else to do): their sum, in CTA order,
+            // then only has to be added, and the dependent round trips to L2 are off the tail.
+            uint32_t pre[16];
+            if (C::kSplit && !slot && b_hi > b_lo) {
 #pragma unroll
-                for (int j = 0; j < kPre; ++j) pre[j] = 0u;
-                if (kPre >= 16) {
-#pragma unroll
-                    for (int j0 = 0; j0 < kPre; j0 += 16) add_partials(reinterpret_cast<uint32_t(&)[16]>(pre[j0 < kPre ? j0 : 0]), j0);
-                }
-                prefetched = true;
+                for (int j = 0; j < 16; ++j) pre[j] = 0u;
+                add_partials(pre);
             }
             if (C::kEpiHandoff) {
                 ptx::named_bar_sync(2, 128 + 32);          // released by the MMA warp once the accumulator is complete
@@ -972,13 +961,6 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                             __syncwarp();
                             if (lane == 0) ptx::mbar_arrive_cluster(ptx::map_to_cta(ptx::smem_u32(&bars.d_empty), 0));
                         }
-                        if (C::kSplit) {
-                            if (slot) {
-                                put_partial(v, j0);
-                                continue;
-                            }
-                            if (b_hi > b_lo) add_partials(v, j0);
-                        }
                         if (p.kparts > 1) {
                             put_kpart(v, j0);
                             continue;
@@ -991,7 +973,7 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                     }
                     ptx::named_bar_sync(bar_id, 128);
 #pragma unroll 1
-                    for (int idx = t128; idx < ((slot || p.kparts > 1) ? 0 : kShare * 16); idx += 128) {   // 16-byte chunks: row = idx / 16, chunk = idx % 16
+                    for (int idx = t128; idx < (p.kparts > 1 ? 0 : kShare * 16); idx += 128) {   // 16-byte chunks: row = idx / 16, chunk = idx % 16
                         const int m = eg * kShare + (idx >> 4), c8 = (idx & 15) * 8;
                         if (m < nrows && ct * 128 + c8 < p.S) {
                             const uint4 q = ptx::lds128(stage + (idx >> 4) * 256 + c8 * 2);
@@ -1013,13 +995,6 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                             if (PAIR) ptx::mbar_arrive_cluster(ptx::map_to_cta(ptx::smem_u32(&bars.d_empty), 0));
                             else ptx::mbar_arrive(ptx::smem_u32(&bars.d_empty));
                         }
-                    }
-                    if (C::kSplit) {
-                        if (slot) {
-                            put_partial(v, j0);
-                            continue;
-                        }
-                        if (b_hi > b_lo) add_partials(v, j0);
                     }
                     if (p.kparts > 1) {
                         put_kpart(v, j0);
@@ -1055,17 +1030,14 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                     __syncwarp();
                     if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&bars.d_empty));
                 }
-                if (slot) {
-                    put_partial(v, j0);
-                    continue;
-                }
-                if (C::kSplit && b_hi > b_lo) {
-                    if (prefetched) {
+                if (C::kSplit) {                           // (NT = 16: one pass)
+                    if (slot) {
+                        put_partial(v, j0);
+                        continue;
+                    }
+                    if (b_hi > b_lo) {
 #pragma unroll
-                        for (int j = 0; j < CH; ++j)
-                            v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(pre[(j0 + j) < kPre ? j0 + j : 0]));
-                    } else {
-                        add_partials(v, j0);
+                        for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(pre[j]));
                     }
                 }
                 if (p.kparts > 1) {
@@ -1542,10 +1514,9 @@ int launch_nt(const UmmaParams& p_in, const __half* x, int n_groups, cudaStream_
         }
         long long clusters = max_clusters[dev];
         const long long tiles2 = (long long)p.MTILES * ((p.CT + 1) / 2);
-        if (!C::kSplit && !p.accumulate)
+        if (!p.accumulate)
             p.kparts = choose_kparts(clusters, tiles2, p.U, p.rows, p.S);
-        const long long work = p.kparts > 1 ? tiles2 * p.kparts : tiles2 * (C::kSplit ? p.U : 1);
-        if (C::kSplit && clusters > kPartialWords / C::kSlotElems / 2) clusters = kPartialWords / C::kSlotElems / 2;
+        const long long work = tiles2 * p.kparts;
         if (clusters > work || p.kparts > 1) clusters = work;
         cfg.gridDim = dim3((unsigned)(2 * clusters), 1, 1);
         e = cudaLaunchKernelEx(&cfg, kern, tm, p, x);
