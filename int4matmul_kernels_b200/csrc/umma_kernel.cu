@@ -257,7 +257,7 @@ struct Cfg {
     // partner at a time: 15-30 K cycles per tile, which lost more than the better balance gained.  Not measured since the sum is
     // spread over the warpgroups; more rows cut K into parts, see choose_kparts.)
     static constexpr bool kSplit = NT <= 32;
-    static constexpr int kSlotElems = kDCols * 128;                   // 64-bit words of one CTA's partial tile in the scratch
+    static constexpr int kSlotElems = NT * 128;                       // 64-bit words of one CTA's partial tile in the scratch
     static constexpr int kMinBlocks = kStream ? 1 : NT <= 64 ? 2 : 1;
 };
 
@@ -284,8 +284,8 @@ struct TensorMaps {
     CUtensorMap z;
 };
 
-// Rows 0 .. n - 1 of one column to every destination (out0: the first row in the first one).  Without a branch per row: a store
-// behind a loop over the destinations costs ~100 cycles.
+// Rows 0 .. n - 1 of one column to every destination (out0: the first row in the first one).  The first destination's stores are
+// predicated, without the branch and the loop over destinations per row (5120 x 20480 int4, 32 rows: 24.9 -> 23.5 us).
 template <int RB>
 __device__ __forceinline__ void store_rows(const OutMap& om, __half* out0, long long ld, int n_dst, const __half (&h)[RB], int n) {
 #pragma unroll
@@ -299,7 +299,7 @@ __device__ __forceinline__ void store_rows(const OutMap& om, __half* out0, long 
     }
 }
 
-// The epilogue of the weight-streaming shapes (one row tile) but for PERM's.  Split-K: the CTAs b_lo .. b_hi share a tile.  b_lo,
+// The epilogue of the weight-streaming shapes (one row tile).  Split-K: the CTAs b_lo .. b_hi share a tile.  b_lo,
 // which owns its first units and reaches them last, adds the others' partial tiles to its own accumulator in CTA order - a fixed
 // order, so results are reproducible; the others wait for nobody.  A partial element is one 64-bit word (fp32 value | tag 1
 // in the high half), written with a single store, so no fence, counter or second round trip is needed; the reader clears
@@ -308,8 +308,8 @@ __device__ __forceinline__ void store_rows(const OutMap& om, __half* out0, long 
 
 // A tile before a CTA's last one, by the epilogue warps: a whole tile, or (share: this lane's column of the CTA's slot) the CTA's share
 // of a tile that another CTA sums.  The next tile's MMAs wait for it.  Not inlined and with its arguments by value: with `p` by
-// reference a call cost ~1 us (1024 x 32768 int4, 5 rows, three tiles a CTA: 16.2 us, now 13.4), and inlined it slowed the decode
-// loop (13824 x 5120 int4, 4 rows: 17.4 us, now 16.8).
+// reference a call cost ~1 us (1024 x 32768 int4, 5 rows, two or three tiles a CTA: 16.2 us, now 12.9), and inlined it slowed the
+// decode loop (13824 x 5120 int4, 4 rows: 17.4 us, now 16.5).
 // out0: the column's first output; rows / out_rows: rows of the launch, and those that this lane stores.
 __device__ __noinline__ bool early_epilogue(const OutMap& om, int n_dst, long long ld, __half* out0, int rows, int out_rows, int accumulate,
                                             unsigned long long* share, uint32_t tmem_base, uint32_t d_empty, uint32_t s_abort) {
@@ -374,8 +374,8 @@ __device__ __noinline__ bool early_epilogue(const OutMap& om, int n_dst, long lo
 // A CTA's last tile: units t0 .. t0 + units - 1.  What bounds it is the number of dependent round trips to L2 (~0.7 us each) between
 // the last MMA and the end of the launch, so the tile can be left to all of the CTA's warpgroups (the dequant warps have nothing
 // else to do by then), `part` of `parts` rows each; a thread has RB x PB partial words in flight, up to 16: with 4 rows and 4
-// partners or 8 rows and 2 partners.  One warpgroup that read 8 rows of one partner at a time took 25.2 us with 16 rows of 16384 x 5120
-// int4 and 35.7 with 32; now 19.6 and 22.6.  (When: see spread_last.)
+// partners or 8 rows and 2 partners.  One warpgroup that read 8 rows of one partner at a time took 25.9 us with 16 rows of 16384 x 5120
+// int4 and 34.4 with 32; now 20.8 and 23.2.  (When: see spread_last.)
 // bar_id, bar_threads: the named barrier at which the MMA warp says that the accumulator is complete (once per call, also where this
 // part has no rows).  Inlined, with one pass over at most 8 rows: a call cost ~1 us here as well.
 template <int NT>
@@ -397,7 +397,7 @@ __device__ __forceinline__ bool last_epilogue(const UmmaParams& p, uint32_t tmem
         b_hi = range_owner(T, G, lo_t + U - 1);
     }
     unsigned long long* const partials64 = reinterpret_cast<unsigned long long*>(p.partials);
-    auto slot_of = [&](int bb) { return partials64 + (size_t)bb * NT * 128 + col; };
+    auto slot_of = [&](int bb) { return partials64 + (size_t)bb * Cfg<NT, false>::kSlotElems + col; };
     auto wait_accumulator = [&]() -> bool {
         __syncwarp();
         ptx::named_bar_sync(bar_id, bar_threads);      // released by the MMA warp once the accumulator is complete
@@ -489,7 +489,6 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
     using C = Cfg<NT, PAIR>;
     using F = UFormat<BITS, SPARSE, PERM>;
     static_assert(!PERM || (C::kStream && F::kPermutedK), "the permuted k order is for dense int4 weight streaming");
-    constexpr bool kSpread = C::kStream && !PERM;                    // every warpgroup takes part in the last tile's epilogue
     constexpr int H = C::kHalves;                                    // 64-k parts per unit
     using WS = WStage<F, H>;
     static_assert(!PAIR || (NT >= 128 && !C::kEpiHandoff), "CTA pairs are for the many-row shapes");
@@ -602,15 +601,16 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
     // several short tiles ahead of the MMAs, could take an earlier tile's phase for the last one's.
     // Up to 6 rows of a tile that this CTA sums are the epilogue warps' alone if no partner's share is the partner's whole range (it
     // delivered early, or there is none): these warps then have everything before the last MMA, while the dequant warps would start
-    // after it.  us, all warpgroups / epilogue warps: 1024 x 32768 int4 4 rows 13.7 / 12.6, 5 rows 14.4 / 13.4, 8 rows 14.2 / 13.4,
-    // but 3072 x 12288 8 rows 12.9 / 13.7; with shares that are whole ranges 512 x 8192 8 rows 7.5 / 9.0.
+    // after it.  us, all warpgroups / epilogue warps: 1024 x 32768 int4 4 rows 13.7 / 12.6, 5 rows 14.4 / 13.3, 8 rows 14.4 / 13.4,
+    // but 3072 x 12288 5 rows 12.7 / 13.5, 8 rows 12.7 / 13.7; with shares that are whole ranges 512 x 8192 8 rows 7.1 / 8.5.  (With
+    // two passes in last_epilogue; by this rule and one pass 1024 x 32768 12.2, 12.9, 13.8, 3072 x 12288 12.7, 12.2, 512 x 8192 6.9.)
     bool spread_last = false;
-    if (kSpread && p.rows > 1 && t_lo < t_hi) {
+    if (C::kStream && p.rows > 1 && t_lo < t_hi) {
         const long long first = div_nn(t_hi - 1, U) * U;               // the last tile's first unit
         spread_last = p.rows > 6 || t_lo > first || range_lo(n_tiles * U, G, b + 2) <= first + U;
     }
     constexpr uint32_t kSpreadThreads = (C::kWG + 1) * 128 + 32;
-    static_assert(!kSpread || NT <= 8 * (C::kWG + 1), "last_epilogue takes at most 8 rows a warpgroup");
+    static_assert(!C::kStream || NT <= 8 * (C::kWG + 1), "last_epilogue takes at most 8 rows a warpgroup");
 
     if (warp == kWProducer || (C::kWProducers == 2 && warp == kWProducer2)) {
         // =========================== packed weights (+ scales / zeros): one thread per producer warp ===========================
@@ -828,10 +828,10 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
         }
     } else {
         // =========================== dequant warpgroups; epilogue warps ===========================
-        // Accumulator of one finished segment -> fp16 rows of `out`, or a partial tile for the split-K reduction.
-        // Run by 4 warps whose index modulo 4 selects the 32 tensor-memory lanes (= weight columns) they may read.
+        // Accumulator of one finished tile (or K part of one) of the shapes for more than 32 rows -> fp16 rows of `out`, or fp32 rows in
+        // the scratch.  (Up to 32 rows: early_epilogue, last_epilogue.)  Run by 4 warps whose index modulo 4 selects the 32 tensor-memory lanes (= weight columns) they may read.
         bool dependency_waited = false;
-        auto epilogue = [&](uint32_t seg, long long tile, int u0, int u1) -> bool {
+        auto epilogue = [&](uint32_t seg, long long tile) -> bool {
             if (!dependency_waited) {
                 // outputs, old outputs and the scratch may still be in use by the kernel before this one in the stream
                 ptx::grid_dependency_wait();
@@ -840,22 +840,10 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
             const int mt = tile_mt(tile), ct = tile_ct(tile);
             const int col = (warp & 3) * 32 + lane;
             const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
-            const bool complete = (u0 == 0) && (u1 == (int)U);
             const int scol = ct * 128 + col;
             const bool col_ok = scol < p.S;
             const int row0 = mt * NT;
             const int nrows = min(NT, p.rows - row0);
-            // Split-K here is that of the permuted k order (PERM: dense int4, up to 3 rows).  Same protocol and order of the sum as
-            // last_epilogue, but one warpgroup alone reads the partners' shares, one partner at a time.
-            int b_lo = 0, b_hi = -1;
-            unsigned long long* slot = nullptr;
-            unsigned long long* const partials64 = reinterpret_cast<unsigned long long*>(p.partials);
-            if (C::kSplit && !complete) {
-                const long long T = n_tiles * U, lo_t = tile * U;
-                b_lo = range_owner(T, G, lo_t);
-                b_hi = range_owner(T, G, lo_t + U - 1);
-                if ((int)b != b_lo) slot = partials64 + (size_t)b * C::kSlotElems;
-            }
             // K parts: fp32 rows j0 .. of this lane's column into the (part, row, S) scratch; the reduce kernel sums the parts
             auto put_kpart = [&](auto& v, int j0) {
                 constexpr int CNT = (int)(sizeof(v) / sizeof(uint32_t));
@@ -865,68 +853,16 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                     if (j0 + j < nrows)
                         p.partials[((size_t)kpart * p.rows + row0 + j0 + j) * p.S + scol] = __uint_as_float(v[j]);
             };
-            // leaves accumulator rows j0 .. j0 + n - 1 of this lane's column in this CTA's slot
-            auto put_partial = [&](auto& v, int j0) {
-                constexpr int CNT = (int)(sizeof(v) / sizeof(uint32_t));
-#pragma unroll
-                for (int j = 0; j < CNT; ++j)
-                    if (j0 + j < nrows) ptx::st_relaxed_gpu_u64(slot + (j0 + j) * 128 + col, (1ull << 32) | v[j]);
-            };
-            // adds the other CTAs' partial rows to v, in CTA order, and clears them
-            auto add_partials = [&](uint32_t (&v)[16]) {
-                bool waiting_ok = true;
-                for (int bb = b_lo + 1; bb <= b_hi; ++bb) {
-                    unsigned long long* src = partials64 + (size_t)bb * C::kSlotElems + col;
-#pragma unroll
-                    for (int jb = 0; jb < 16; jb += 8) {
-                        if (jb >= nrows) break;                            // warp-uniform
-                        unsigned long long w[8];
-#pragma unroll
-                        for (int i = 0; i < 8; ++i)
-                            if (jb + i < nrows) w[i] = ptx::ld_relaxed_gpu_u64(src + (jb + i) * 128);
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) {
-                            if (jb + i < nrows) {
-                                for (uint32_t spins = 0; (uint32_t)(w[i] >> 32) != 1u && waiting_ok; ++spins) {
-                                    if (spins >= ptx::kSpinLimit) {        // a contributor never delivered: report, stop waiting
-                                        atomicExch(p.status, 34);
-                                        waiting_ok = false;
-                                        break;
-                                    }
-                                    __nanosleep(64);
-                                    w[i] = ptx::ld_relaxed_gpu_u64(src + (jb + i) * 128);
-                                }
-                                v[jb + i] = __float_as_uint(__uint_as_float(v[jb + i]) + __uint_as_float((uint32_t)w[i]));
-                                ptx::st_relaxed_gpu_u64(src + (jb + i) * 128, 0ull);
-                            }
-                        }
-                    }
-                }
-            };
-            // The other CTAs' partial tiles are fetched BEFORE the own accumulator is complete (the partners delivered them
-            // early in their run, as their first segment, and these warps have nothing else to do): their sum, in CTA order,
-            // then only has to be added, and the dependent round trips to L2 are off the tail.
-            uint32_t pre[16];
-            if (C::kSplit && !slot && b_hi > b_lo) {
-#pragma unroll
-                for (int j = 0; j < 16; ++j) pre[j] = 0u;
-                add_partials(pre);
+            bool got = ptx::mbar_wait(ptx::smem_u32(&bars.d_full), seg & 1u);
+            if (!got && lane == 0) atomicExch(p.status, 33);
+            if (C::kEpiTransposed) {
+                // the four warps of an epilogue group meet at named barriers further down: a give-up has to be
+                // the whole group's decision, or the warps that went on would wait there for ever
+                if (!got) s_abort = 1;
+                ptx::named_bar_sync(1 + 3 * ((warp - kEpiWarp0) >> 2), 128);
+                got = s_abort == 0;
             }
-            if (C::kEpiHandoff) {
-                ptx::named_bar_sync(2, 128 + 32);          // released by the MMA warp once the accumulator is complete
-                if (s_abort) return false;
-            } else {
-                bool got = ptx::mbar_wait(ptx::smem_u32(&bars.d_full), seg & 1u);
-                if (!got && lane == 0) atomicExch(p.status, 33);
-                if (C::kEpiTransposed) {
-                    // the four warps of an epilogue group meet at named barriers further down: a give-up has to be
-                    // the whole group's decision, or the warps that went on would wait there for ever
-                    if (!got) s_abort = 1;
-                    ptx::named_bar_sync(1 + 3 * ((warp - kEpiWarp0) >> 2), 128);
-                    got = s_abort == 0;
-                }
-                if (!got) return false;
-            }
+            if (!got) return false;
             ptx::tc_fence_after_sync();
             // matvec route with more than 64 rows (a batch of one-row products): the caller's old values of rows
             // j0 .. of this lane's column are added to the unrounded sums, so that there is still one rounding
@@ -1030,16 +966,6 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                     __syncwarp();
                     if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&bars.d_empty));
                 }
-                if (C::kSplit) {                           // (NT = 16: one pass)
-                    if (slot) {
-                        put_partial(v, j0);
-                        continue;
-                    }
-                    if (b_hi > b_lo) {
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(pre[j]));
-                    }
-                }
                 if (p.kparts > 1) {
                     put_kpart(v, j0);
                     continue;
@@ -1068,7 +994,7 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
         };
 
         uint32_t seg = 0;
-        bool aborted = false;                                              // a wait timed out (kSpread)
+        bool aborted = false;                                              // a wait timed out (weight-streaming shapes)
         if (C::kEpiWarps && warp >= kEpiWarp0 + 4 * kEpiGroups) {
             // (an epilogue warpgroup that this configuration does not use)
         } else if (C::kEpiWarps && warp >= kEpiWarp0) {
@@ -1077,18 +1003,18 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                 const long long tile = div_nn(t, U);
                 const int u0 = (int)(t - tile * U);
                 const int u1 = (int)min(U, u0 + (t_hi - t));
-                if constexpr (kSpread) {
+                if constexpr (C::kStream) {
                     if (t + (u1 - u0) >= t_hi) break;                  // the last tile: below
                     ptx::grid_dependency_wait();                       // as in `epilogue`
                     const int col = (int)threadIdx.x & 127, scol = (int)tile * 128 + col;
                     const bool col_ok = scol < p.S;
                     if (!early_epilogue(p.om, p.om.n_dst, p.om.ld, p.om.dst[0] + (col_ok ? p.om.col(scol) : 0), p.rows, col_ok ? p.rows : 0, p.accumulate,
-                                        u0 == 0 ? nullptr : reinterpret_cast<unsigned long long*>(p.partials) + (size_t)blockIdx.x * NT * 128 + col,
+                                        u0 == 0 ? nullptr : reinterpret_cast<unsigned long long*>(p.partials) + (size_t)b * C::kSlotElems + col,
                                         tmem_base, ptx::smem_u32(&bars.d_empty), ptx::smem_u32(const_cast<int*>(&s_abort)))) {
                         aborted = true;
                         break;
                     }
-                } else if (!epilogue(seg, tile, u0, u1)) break;
+                } else if (!epilogue(seg, tile)) break;
                 ++seg;
                 t += u1 - u0;
             }
@@ -1229,13 +1155,13 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                 }
                 if (!ok) { aborted = true; break; }
                 if (C::kDeferArrive && pending >= 0) { announce(pending); pending = -1; }
-                if (!C::kEpiWarps && wg == 0) ok = epilogue(seg, tile, u0, u1);
+                if (!C::kEpiWarps && wg == 0) ok = epilogue(seg, tile);
                 ++seg;
                 si0 += (uint32_t)(u1 - u0);
                 t += u1 - u0;
             }
         }
-        if constexpr (kSpread) {
+        if constexpr (C::kStream) {
             if (aborted) {
                 if (spread_last) ptx::named_bar_arrive(5, kSpreadThreads);
             } else if (spread_last || (warp >= kEpiWarp0 && t_lo < t_hi)) {
@@ -1617,9 +1543,11 @@ int launch_fmt(UmmaParams& p, const __half* x, int n_groups, int pair_mode, int 
     }
     switch (nt) {
         case 16:
-            // up to 3 rows of dense int4: the k order that needs no byte shuffles.  More rows cost the one warp that reorders the
-            // activations more per unit than the unit takes (16384 x 16384, this order / the natural one: 1 row 37.8 / 40.8 us,
-            // 3 rows 41.0 / 41.2, 4 rows 44.7 / 41.5, 8 rows 55.5 / 42.2)
+            // Up to 3 rows of dense int4: the k order that needs no byte shuffles.  More rows cost the one warp that reorders the
+            // activations more per unit than the unit takes, the sooner the more units a CTA has (us, this order / the natural one:
+            // 16384 x 16384 1 row 37.4 / 39.5, 3 rows 39.1 / 40.0, 4 rows 41.9 / 40.0, 5 rows 45.0 / 40.3; 13824 x 5120 3 rows 15.6 / 16.5,
+            // 4 rows 16.0 / 16.4, 5 rows 16.8 / 16.9; 5120 x 20480 3 rows 19.8 / 20.6, 4 rows 20.6 / 20.4; 1024 x 32768 5 rows 12.3 / 12.9;
+            // the other way round only where a tile is one or two units: 512 x 8192 3 rows 6.7 / 6.5)
             if (BITS == 4 && !SPARSE && p.rows <= 3) return launch_nt<BITS, SPARSE, 16, false, BITS == 4 && !SPARSE>(p, x, n_groups, stream, cuda_err);
             return launch_nt<BITS, SPARSE, 16, false>(p, x, n_groups, stream, cuda_err);
         case 32: return launch_nt<BITS, SPARSE, 32, false>(p, x, n_groups, stream, cuda_err);
