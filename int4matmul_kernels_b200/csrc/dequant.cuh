@@ -57,8 +57,9 @@ constexpr uint32_t MUL_1_1 = 0x3C003C00u, BASE_1_1 = 0xE400E400u;        // (x1,
 // The next 8 kept nibbles are spread over the bytes of a register pair (even nibbles, odd nibbles); two PRMTs put them
 // at their positions.  The selectors of both PRMTs are one 32-bit word of a 256-entry table indexed by the byte of the
 // keep-mask (nibble j of the word belongs to position j).  A dropped position selects 8, for which PRMT replicates the
-// sign of a byte below 128 (a nibble, XORed with a zero-point below 128): it yields 0x00.  A 1 KB table: the same look-up in a table of 16-byte entries (selectors, masks and
-// popcount) takes ~10 shared-memory wavefronts per warp instead of ~3.5, because random entries of four banks collide.
+// sign of a byte below 128 (a nibble, XORed with a zero-point below 128): it yields 0x00.  A 1 KB table: the same look-up in a
+// table of 16-byte entries (selectors, masks and popcount) takes ~10 shared-memory wavefronts per warp instead of ~3.5, because
+// random entries of four banks collide.
 constexpr int kSparseLutEntries = 256;
 __device__ __forceinline__ uint32_t sparse_selectors(int keep) {
     uint32_t sel = 0, rank = 0;
@@ -83,7 +84,8 @@ __device__ __forceinline__ void sparse_expand(uint32_t& lo, uint32_t& hi, uint32
     // Fast mode: a dropped position gets the (integer) zero-point as its nibble, so it decodes to +0.  The nibbles go through
     // the PRMT with the zero-point XORed in, which the extraction's LOP3 does for nothing, so that a dropped position's 0x00 and
     // a kept one's nibble both come right by one XOR afterwards (a mask of the kept positions and a select were two
-    // instructions of five per 4 positions: one row 16384 x 16384 57.3 -> 54.4 us, 2048 rows 5120 x 20480 350.5 -> 340.4)
+    // instructions of five per 4 positions: one row 16384 x 16384 57.3 -> 54.4 us, 2048 rows 5120 x 20480 350.5 -> 340.4; few-row
+    // kernel 2048 x 5632 1 row 8.4 -> 8.1, 8 rows 11.6 -> 11.4, of 24 sizes only 2048 x 2048 with 5..8 rows is slower, 8.0 -> 8.1)
     const uint32_t flip = MODE == MODE_FAST ? c.zb : 0u;
     const uint32_t even = and_xor(lo, 0x0F0F0F0Fu, flip), odd = and_xor(lo >> 4, 0x0F0F0F0Fu, flip);
     const uint32_t off = hsub2_u(BASE_1_1, c.z2);

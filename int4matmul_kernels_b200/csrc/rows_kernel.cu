@@ -561,21 +561,24 @@ cudaError_t rows_launch_fmt(const RowsParams& p, int sms, int dev, cudaStream_t 
 
 }  // namespace
 
-// Which calls take this kernel by default; every figure is us on one B200, tcgen05 kernel -> this one.
-// Alone, its fixed cost per launch is about half of the other's and its rate is lower: adding one row to a zero-filled
-// output, int4 2048^2 12.4 -> 8.2, 5120^2 14.6 -> 12.3, 5120 x 8192 16.5 -> 15.2, but 16384^2 42.5 -> 53.6; int3 5120^2
-// 15.5 -> 12.3; int2 15.0 -> 11.1; 16:32 17.0 -> 14.4.  So the adding route's line is the number of weights.  From more than 2
-// column tiles per SM on, K cannot be cut any more and SMs are left with uneven numbers of tiles: 1024 x 30720 16.5 -> 14.3,
-// 1024 x 37888 14.4 -> 14.4, 1024 x 40960 18.4 -> 19.4 (16:32 21.9 -> 25.2), 16:32 2304 x 20480 20.6 -> 22.5.
+// Which calls take this kernel by default; every figure is us on one B200, tcgen05 kernel -> this one, calls back to back.
+// Alone, its fixed cost per launch is about half of the other's and its rate is lower: one row int4 2048^2 7.7 -> 4.8, 4096 x 12288
+// 13.7 -> 13.1, 5120 x 9728 13.7 -> 14.9; int2 5120^2 10.3 -> 9.7.  So the adding route's line is the number of weights.  From more than
+// 2 column tiles per SM on, K cannot be cut any more and SMs are left with uneven numbers of tiles: 1024 x 30720 11.5 -> 10.8,
+// 1024 x 36864 12.1 -> 10.9, 1024 x 40960 12.7 -> 14.5 (16:32 17.2 -> 17.7).
 // A call that overwrites stands between others in a model's layer, and there a change of kernel from one matrix to the next costs
 // 2..5 us.  min(N, S) is the layer's width for its every matrix, so a bound on it keeps a layer on one kernel.  Four matrices and
 // their row norms, width (inner width), all on the tcgen05 kernel -> those of up to 48 Mi weights (2..8 rows: 16 Mi) on this one:
-// one int4 row 5120 (13824) 84.6 -> 89.7, 4096 (11008) 69.3 -> 71.9, 3584 (9472) 61.5 -> 63.3, but 3072 (8192) 56.8 -> 50.1, 2048 (5632)
-// 49.7 -> 38.1.  int2 is the exception, its decode is cheapest here: 5120 82.9 -> 83.4, 4096 68.9 -> 63.7.  4 rows int4 4096 74.8 -> 79.9,
-// 3072 62.1 -> 63.7, 2560 (6912) 57.7 -> 56.9, 2048 54.9 -> 46.3; 8 rows (larger stages, fewer of them) 3072 71.4 -> 73.1, 2560 65.4 ->
-// 64.6, 2048 63.5 -> 56.0.  (Alone and back to back, 4096^2 would still be faster here: one row 10.9 -> 8.4.)
-// Very long columns: the last part adds the sums of hundreds of parts one after the other, 4 rows 131072 x 64 77 -> 62 but 262144 x 64
-// 79 -> 120, 8 rows 65536 x 64 98 -> 63 but 131072 x 64 99 -> 121.
+// one int4 row 5120 (13824) 76.3 -> 76.8, 4096 (11008) 62.5 -> 60.4, 3584 (9472) 54.1 -> 52.4, 3072 (8192) 50.7 -> 43.5, 2048 (5632)
+// 42.8 -> 32.0; int2, whose decode is cheapest here, 5120 76.2 -> 74.5, 4096 62.6 -> 55.9.  4 rows int4 4096 66.7 -> 66.2, 3072 53.5 ->
+// 52.8, 2560 (6912) 49.2 -> 47.5, 2048 45.5 -> 40.2; 8 rows (larger stages, fewer of them) 3072 55.7 -> 57.9, 2560 51.3 -> 51.0, 2304
+// (6144) 49.1 -> 51.4, 2048 49.1 -> 48.6, 1536 (4096) 43.1 -> 39.8.
+// Very long columns: the last part adds the sums of hundreds of parts one after the other, 4 rows 65536 x 64 38.8 -> 30.1, 131072 x 64
+// 40.9 -> 57.6, 8 rows 32768 x 64 38.0 -> 31.8, 65536 x 64 42.9 -> 58.0.
+// The lines were drawn when one warpgroup of the tcgen05 kernel summed a shared tile (77, 99 us for the last two sizes above).  Against
+// the present one they hold for layers and lie too far out elsewhere: 4 and 8 rows of long columns (16384 x 1024 12.6 -> 14.4 and
+// 14.1 -> 23.5, 65536 x 256 25.1 -> 35.6 and 27.3 -> 65.8), one row alone of int3 and 16:32 from about 16 Mi weights on (5120^2 10.7 ->
+// 11.8 and 11.9 -> 12.8), of all but int2 from about 40 Mi, and 1984 x 19008 (11.9 -> 14.9).
 // (The bounds also keep step and tile numbers far inside 32 bits.)
 constexpr long long kMi = 1ll << 20;
 
