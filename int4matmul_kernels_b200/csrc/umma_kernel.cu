@@ -76,14 +76,14 @@ struct UFormat<4, false, PERM> {
     static constexpr int WROWS = 8, MROWS = 0;       // packed rows / mask rows per 64-k part
     static constexpr bool kPermutedK = PERM;
     template <int MODE, class Entry>
-    __device__ static __forceinline__ void decode(uint32_t wbase, uint32_t, const ColK& c, uint32_t (&A)[32], const Entry*) {
+    __device__ static __forceinline__ void decode(uint32_t wbase, uint32_t, int half, const ColK& c, uint32_t* A, const Entry*) {
         if (PERM) {
             // nibbles j and j + 4 of a word sit at the same offset of its two 16-bit halves: one LOP3 per pair plants both
             // into the mantissas of (1024, 1024); the odd nibbles come out multiplied by 16
             const uint32_t off1 = hsub2_u(BASE_1_1, c.z2), off16 = hsub2_u(H2_N64, c.z2);
 #pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                const uint32_t w = ptx::lds32(wbase + r * 512);
+            for (int r = 0; r < 4; ++r) {
+                const uint32_t w = ptx::lds32(wbase + (4 * half + r) * 512);
                 const uint32_t w8 = w >> 8;
                 A[4 * r + 0] = finish<4, MODE>(and_or(w, 0x000F000Fu, kMagic1024), MUL_1_1, BASE_1_1, off1, c);      // k0, k4
                 A[4 * r + 1] = finish<4, MODE>(and_or(w, 0x00F000F0u, kMagic1024), H2_1_16, H2_N64, off16, c);       // k1, k5
@@ -94,8 +94,8 @@ struct UFormat<4, false, PERM> {
         }
         const uint32_t off = hsub2_u(BASE_1_16, c.z2);
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            const uint32_t w = ptx::lds32(wbase + r * 512);
+        for (int r = 0; r < 4; ++r) {
+            const uint32_t w = ptx::lds32(wbase + (4 * half + r) * 512);
             const uint32_t y0 = prmt(w, w, 0x1010), y1 = prmt(w, w, 0x3232);   // low / high 16 bits in both lanes
             A[4 * r + 0] = finish<4, MODE>(and_or(y0, 0x00F0000Fu, kMagic1024), MUL_1_16, BASE_1_16, off, c);        // k0, k1
             A[4 * r + 1] = finish<4, MODE>(and_or(y0 >> 8, 0x00F0000Fu, kMagic1024), MUL_1_16, BASE_1_16, off, c);   // k2, k3
@@ -110,11 +110,11 @@ struct UFormat<2, false, PERM> {
     static constexpr int WROWS = 4, MROWS = 0;
     static constexpr bool kPermutedK = false;
     template <int MODE, class Entry>
-    __device__ static __forceinline__ void decode(uint32_t wbase, uint32_t, const ColK& c, uint32_t (&A)[32], const Entry*) {
+    __device__ static __forceinline__ void decode(uint32_t wbase, uint32_t, int half, const ColK& c, uint32_t* A, const Entry*) {
         const uint32_t offa = hsub2_u(BASE_1_4, c.z2), offb = hsub2_u(BASE_16_64, c.z2);
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const uint32_t w = ptx::lds32(wbase + r * 512);
+        for (int r = 0; r < 2; ++r) {
+            const uint32_t w = ptx::lds32(wbase + (2 * half + r) * 512);
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const uint32_t y = h ? prmt(w, w, 0x3232) : prmt(w, w, 0x1010);   // crumbs 8h .. 8h+7 in both lanes
@@ -133,28 +133,24 @@ struct UFormat<3, false, PERM> {
     static constexpr int WROWS = 6, MROWS = 0;
     static constexpr bool kPermutedK = false;
     template <int MODE, class Entry>
-    __device__ static __forceinline__ void decode(uint32_t wbase, uint32_t, const ColK& c, uint32_t (&A)[32], const Entry*) {
+    __device__ static __forceinline__ void decode(uint32_t wbase, uint32_t, int blk, const ColK& c, uint32_t* A, const Entry*) {
         const uint32_t off = hsub2_u(BASE_1_8, c.z2);
+        const uint32_t w0 = ptx::lds32(wbase + (3 * blk) * 512), w1 = ptx::lds32(wbase + (3 * blk + 1) * 512), w2 = ptx::lds32(wbase + (3 * blk + 2) * 512);
+        // the 96-bit stream in 12-bit chunks: chunk j holds fields 4j .. 4j+3 = pairs (2j, 2j+1)
+        uint32_t ch[8];
+        ch[0] = w0;
+        ch[1] = w0 >> 12;
+        ch[2] = __funnelshift_r(w0, w1, 24);
+        ch[3] = w1 >> 4;
+        ch[4] = w1 >> 16;
+        ch[5] = __funnelshift_r(w1, w2, 28);
+        ch[6] = w2 >> 8;
+        ch[7] = w2 >> 20;
 #pragma unroll
-        for (int blk = 0; blk < 2; ++blk) {
-            const uint32_t w0 = ptx::lds32(wbase + (3 * blk) * 512), w1 = ptx::lds32(wbase + (3 * blk + 1) * 512),
-                           w2 = ptx::lds32(wbase + (3 * blk + 2) * 512);
-            // the 96-bit stream in 12-bit chunks: chunk j holds fields 4j .. 4j+3 = pairs (2j, 2j+1)
-            uint32_t ch[8];
-            ch[0] = w0;
-            ch[1] = w0 >> 12;
-            ch[2] = __funnelshift_r(w0, w1, 24);
-            ch[3] = w1 >> 4;
-            ch[4] = w1 >> 16;
-            ch[5] = __funnelshift_r(w1, w2, 28);
-            ch[6] = w2 >> 8;
-            ch[7] = w2 >> 20;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const uint32_t y = prmt(ch[j], ch[j], 0x1010);
-                A[16 * blk + 2 * j + 0] = finish<3, MODE>(and_or(y, 0x00380007u, kMagic1024), MUL_1_8, BASE_1_8, off, c);
-                A[16 * blk + 2 * j + 1] = finish<3, MODE>(and_or(y >> 6, 0x00380007u, kMagic1024), MUL_1_8, BASE_1_8, off, c);
-            }
+        for (int j = 0; j < 8; ++j) {
+            const uint32_t y = prmt(ch[j], ch[j], 0x1010);
+            A[2 * j + 0] = finish<3, MODE>(and_or(y, 0x00380007u, kMagic1024), MUL_1_8, BASE_1_8, off, c);
+            A[2 * j + 1] = finish<3, MODE>(and_or(y >> 6, 0x00380007u, kMagic1024), MUL_1_8, BASE_1_8, off, c);
         }
     }
 };
@@ -164,22 +160,32 @@ struct UFormat<4, true, PERM> {
     static constexpr int WROWS = 4, MROWS = 2;
     static constexpr bool kPermutedK = false;
     template <int MODE, class Entry>
-    __device__ static __forceinline__ void decode(uint32_t wbase, uint32_t mbase, const ColK& c, uint32_t (&A)[32], const Entry* lut) {
+    __device__ static __forceinline__ void decode(uint32_t wbase, uint32_t mbase, int blk, const ColK& c, uint32_t* A, const Entry* lut) {
+        // a 32-block of this column: the 64-bit word of its 16 kept nibbles (in increasing k) and its keep-mask
+        uint32_t lo = ptx::lds32(wbase + (2 * blk) * 512), hi = ptx::lds32(wbase + (2 * blk + 1) * 512);
+        const uint32_t m = ptx::lds32(mbase + blk * 512);
 #pragma unroll
-        for (int blk = 0; blk < 2; ++blk) {
-            // a 32-block of this column: the 64-bit word of its 16 kept nibbles (in increasing k) and its keep-mask
-            uint32_t lo = ptx::lds32(wbase + (2 * blk) * 512), hi = ptx::lds32(wbase + (2 * blk + 1) * 512);
-            const uint32_t m = ptx::lds32(mbase + blk * 512);
+        for (int step = 0; step < 4; ++step) {               // 8 positions each
+            uint32_t pairs[4];
+            sparse_expand<MODE>(lo, hi, m, step, lut, c, pairs);
 #pragma unroll
-            for (int step = 0; step < 4; ++step) {               // 8 positions each
-                uint32_t pairs[4];
-                sparse_expand<MODE>(lo, hi, m, step, lut, c, pairs);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) A[16 * blk + 4 * step + i] = pairs[i];
-            }
+            for (int i = 0; i < 4; ++i) A[4 * step + i] = pairs[i];
         }
     }
 };
+
+template <class F, int MODE, class Entry>
+__device__ __forceinline__ void decode_part(uint32_t wbase, uint32_t mbase, const ColK& c, uint32_t (&A)[32], const Entry* lut) {
+#pragma unroll
+    for (int half = 0; half < 2; ++half) F::template decode<MODE>(wbase, mbase, half, c, A + 16 * half, lut);
+}
+
+// Bits that are set where a column's group is not in the fast mode, for two groups at once: s, z their scales and zero-points, zi = z + 1024;
+// BOUND + the fp16 bits of the largest zero-point = 0x7FFF
+template <uint32_t BOUND>
+__device__ __forceinline__ uint32_t not_fast_bits(uint32_t s, uint32_t z, uint32_t zi) {
+    return ((z | s | ((z & 0x7FFF7FFFu) + BOUND * 0x10001u)) & 0x80008000u) | (hadd2_u(zi, H2_N1024) ^ z);
+}
 
 template <class F, int H>
 struct WStage {     // one stage of the packed-weight ring: one unit = H parts of 64 k
@@ -200,7 +206,7 @@ constexpr int kMaxABStages = 6;
 template <bool SPARSE, int NT>
 struct SparseTable {
     using Entry = uint32_t;
-    static constexpr uint32_t kFastBound = 0x280Fu;
+    static constexpr uint32_t kFastBound = SPARSE ? 0x280Fu : 0x1FFFu;
 };
 template <>
 struct SparseTable<true, 64> {
@@ -238,7 +244,6 @@ struct Cfg {
     static constexpr bool kEpiWarps = NT >= 128 || kStream;           // a warpgroup of its own for the epilogue (else dequant warpgroup 0 does it)
     static constexpr bool kEpiTransposed = NT >= 128;                 // epilogue stores go through a shared-memory transposition tile
     static constexpr bool kEpiHandoff = kStream;                      // the MMA warp waits for the accumulator and wakes the epilogue warps (named barrier)
-    static constexpr bool kDeferArrive = kStream;                     // a dequant warp announces an A stage only before its next wait (hides the tcgen05.wait::st latency)
     // many rows: two epilogue warpgroups, each draining half of the accumulator's columns, so that the next tile's
     // MMAs wait half as long for the accumulator
     static constexpr int kEpiGroups = NT >= 128 ? 2 : 1;
@@ -1024,7 +1029,6 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
             const int col = (warp & 3) * 32 + lane;                             // weight column in the tile = tensor-memory lane
             const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
             uint32_t si0 = 0;                                                    // si0: weight stages consumed before this segment
-            int pending = -1;                                                    // A stage written but not yet announced (Cfg::kDeferArrive)
             // the stores into tensor memory are complete -> the stage may be read by the MMAs
             auto announce = [&](int stage) {
                 ptx::tc_wait_st();
@@ -1040,121 +1044,194 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                 const long long tile = div_nn(t, U);
                 const int u0 = (int)(t - tile * U);
                 const int u1 = (int)min(U, u0 + (t_hi - t));
+                // a unit of this warpgroup: its place in the rings, and the wait for its weights
+                struct Unit {
+                    uint32_t si, ws, st, g0, as, aph;       // stage index, weight stage and its address, first group, A stage and its phase
+                };
+                auto next_unit = [&](int u, Unit& n) -> bool {
+                    n.si = si0 + (uint32_t)(u - u0);
+                    n.ws = n.si % C::kWStages;                                              // constants: multiply-shift, no division
+                    const uint32_t wph = (n.si / C::kWStages) & 1u;
+                    if (C::kWGuard && !ptx::mbar_wait(ptx::smem_u32(&bars.w_empty[n.ws]), wph ^ 1u)) {   // see Cfg::kWStages
+                        if (lane == 0) atomicExch(p.status, 35);
+                        return false;
+                    }
+                    if (!ptx::mbar_wait(ptx::smem_u32(&bars.w_full[n.ws]), wph)) {
+                        if (lane == 0) atomicExch(p.status, 31);
+                        return false;
+                    }
+                    n.st = w_ring + n.ws * WS::kBytes;
+                    n.g0 = p.gdiv((uint32_t)H * (uint32_t)u);
+                    n.as = n.si % kABStages;
+                    n.aph = (n.si / kABStages) & 1u;
+                    return true;
+                };
+                // row of part h's group in the stage's boxes of scales and zero-points
+                auto group_row = [&](int u, uint32_t g0, int h) -> uint32_t {
+                    return h == 0 ? 0u : p.gdiv((uint32_t)H * (uint32_t)u + (uint32_t)h) - g0;   // 0 .. H - 1
+                };
+                // after the last read of the weight stage
+                auto release_weights = [&](uint32_t ws) {
+                    __syncwarp();
+                    if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&bars.w_empty[ws]));
+                };
+                // before the first store into the A stage: it (and its activation tile) is free once the MMAs of its previous use have completed
+                auto acquire_a_stage = [&](const Unit& n, bool free_early) -> bool {
+                    if (!free_early && !ptx::mbar_wait(ptx::smem_u32(&bars.ab_free[n.as]), n.aph ^ 1u)) {
+                        if (lane == 0) atomicExch(p.status, 32);
+                        return false;
+                    }
+                    ptx::tc_fence_after_sync();
+                    return true;
+                };
+                auto words = [&](const Unit& n, int h) -> uint32_t { return n.st + WS::kW + h * (F::WROWS * 512) + col * 4; };
+                auto masks = [&](const Unit& n, int h) -> uint32_t { return n.st + WS::kMask + h * (F::MROWS * 512) + col * 4; };
+                auto a_cols = [&](const Unit& n, int h) -> uint32_t { return lane_addr + C::kACol0 + n.as * C::kAStageCols + h * 32; };
+                // Fast mode: scale signs clear, zero-points integers in [0, 512] (sparse format: see SparseTable), for every column of the
+                // warp in every group of the unit.
+                constexpr uint32_t kBound = SparseTable<SPARSE, NT>::kFastBound;
                 // this warpgroup's units of the segment: those whose stage index is congruent to wg modulo kWG
                 for (int u = u0 + (int)(((uint32_t)wg + (uint32_t)C::kWG - si0 % (uint32_t)C::kWG) % (uint32_t)C::kWG); u < u1; u += C::kWG) {
-                    const uint32_t si = si0 + (uint32_t)(u - u0);
-                    const uint32_t ws = si % C::kWStages, wph = (si / C::kWStages) & 1u;     // constants: multiply-shift, no division
-                    if (C::kWGuard && !ptx::mbar_wait(ptx::smem_u32(&bars.w_empty[ws]), wph ^ 1u)) {   // see Cfg::kWStages
-                        if (lane == 0) atomicExch(p.status, 35);
-                        ok = false;
-                        break;
-                    }
-                    if (!ptx::mbar_wait(ptx::smem_u32(&bars.w_full[ws]), wph)) {
-                        if (lane == 0) atomicExch(p.status, 31);
-                        ok = false;
-                        break;
-                    }
-                    const uint32_t st = w_ring + ws * WS::kBytes;
-                    const uint32_t g0 = p.gdiv((uint32_t)H * (uint32_t)u);
-                    const uint32_t as = si % kABStages, aph = (si / kABStages) & 1u;
-                    // polled before the first part is decoded, so that the answer costs no latency when it is needed
-                    const bool free_early = ptx::mbar_test_wait(ptx::smem_u32(&bars.ab_free[as]), aph ^ 1u);
-                    // scale and zero-point of this thread's column in row `row` of the stage's group box, both halves of a register
-                    auto load_group = [&](uint32_t row, ColK& c) {
-                        const uint32_t sz = ptx::lds32(st + WS::kS + row * 256 + (col & ~1) * 2) >> (16 * (col & 1));
-                        const uint32_t zz = ptx::lds32(st + WS::kZ + row * 256 + (col & ~1) * 2) >> (16 * (col & 1));
-                        c.s2 = prmt(sz, sz, 0x1010);
-                        c.z2 = prmt(zz, zz, 0x1010);
-                        c.zb = 0;
-                    };
-                    // fast mode needs: scale sign clear, zero-point an integer in [0, 512] (sparse format: see SparseTable)
-                    auto not_fast_bits = [&](const ColK& c) -> uint32_t {
-                        const uint32_t zr = hadd2_u(hadd2_u(c.z2, kMagic1024), H2_N1024);
-                        constexpr uint32_t kAdd = SPARSE ? SparseTable<SPARSE, NT>::kFastBound : 0x1FFFu;
-                        const uint32_t zlo = c.z2 & 0xFFFFu;
-                        return ((zlo | ((zlo & 0x7FFFu) + kAdd) | c.s2) & 0x8000u) | (zr ^ c.z2);
-                    };
-                    // after the last read of the weight stage
-                    auto release_weights = [&]() {
-                        __syncwarp();
-                        if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&bars.w_empty[ws]));
-                    };
-                    // before the first store into the A stage
-                    auto acquire_a_stage = [&]() -> bool {
-                        if (C::kDeferArrive && pending >= 0) announce(pending);       // before any wait: the MMAs must be able to go on
-                        // the A stage (and its activation tile) is free once the MMAs of its previous use have completed
-                        if (!free_early && !ptx::mbar_wait(ptx::smem_u32(&bars.ab_free[as]), aph ^ 1u)) {
-                            if (lane == 0) atomicExch(p.status, 32);
-                            return false;
-                        }
-                        ptx::tc_fence_after_sync();
-                        return true;
-                    };
-                    // The parts are decoded in the fast mode by straight-line code, without a mode decision in between;
-                    // whether every group of the unit really is in the fast mode (for every column of the warp) is
-                    // voted once, when the last group has been read and before the weight stage is released.  If not,
-                    // the unit is decoded again with a decision per part (the stores are simply overwritten).
-                    bool redo = false;
-                    {
-                        ColK c;
-                        uint32_t cur_row = 0xFFFFFFFFu, nf = 0;
+                    Unit n;
+                    if (!next_unit(u, n)) { ok = false; break; }
+                    uint32_t A[32];
+                    if constexpr (C::kStream) {
+                        // Few rows are bound by this loop: by its instructions (per unit ~700 a scheduler with the other roles', and the half-precision
+                        // pipe alone is busy for 650 cycles) and by the waits between its steps.  So the mode is voted before anything is
+                        // decoded, for two groups at a time, the parts are straight-line code without a branch in between, and a unit is
+                        // announced as soon as it is written.  (With a branch per part on a new group, the vote at the last part, the other modes'
+                        // 32 registers beside it, and the announcement put off to the warpgroup's next unit: one row 16384 x 16384 int4 37.2 us,
+                        // 16:32 52.4, int3 40.5, int2 37.3; now 35.9, 51.5, 39.1, 33.8.  General mode, which decoded twice: 66, 111, 79, 71; now
+                        // 53, 86, 62, 63; every second group in the exponent coding: 176, 208, 180, 142; now 181, 194, 179, 126.  Not better: the parts
+                        // as a loop of two iterations (36.8, 52.9, 41.6, 36.4); two warpgroups with 128 registers; an MMA warp, an accumulator and
+                        // half-stages for each warpgroup.  The shapes below, which wait for other things, do not gain: NT = 64 loses 2..6 %.)
+                        uint32_t sp[H / 2], zp[H / 2], zi[H / 2], nf = 0;           // two parts' scales, zero-points, zero-points + 1024
 #pragma unroll
-                        for (int h = 0; h < H; ++h) {
-                            // scale and zero-point change only where the group does (warp-uniform)
-                            const uint32_t row = (h == 0) ? 0u : (p.gdiv((uint32_t)H * (uint32_t)u + (uint32_t)h) - g0);   // 0 .. H - 1
-                            if (row != cur_row) {
-                                cur_row = row;
-                                load_group(row, c);
-                                nf |= not_fast_bits(c);
-                                if (SPARSE) c.zb = __half2uint_rz(__ushort_as_half((unsigned short)(c.z2 & 0xFFFFu))) * 0x01010101u;
-                            }
-                            if (h == H - 1 && __any_sync(0xFFFFFFFFu, nf != 0)) {
-                                redo = true;
-                                break;
-                            }
-                            uint32_t A[32];
-                            F::template decode<MODE_FAST>(st + WS::kW + h * (F::WROWS * 512) + col * 4, st + WS::kMask + h * (F::MROWS * 512) + col * 4, c, A, lut);
-                            if (h == H - 1) release_weights();
-                            if (h == 0 && !acquire_a_stage()) { ok = false; break; }
-                            ptx::tmem_st32(lane_addr + C::kACol0 + as * C::kAStageCols + h * 32, A);
+                        for (int h = 0; h < H; h += 2) {
+                            const uint32_t a0 = n.st + WS::kS + col * 2 + group_row(u, n.g0, h) * 256, a1 = n.st + WS::kS + col * 2 + group_row(u, n.g0, h + 1) * 256;
+                            sp[h / 2] = prmt(ptx::lds_u16(a0), ptx::lds_u16(a1), 0x5410);
+                            zp[h / 2] = prmt(ptx::lds_u16(a0 + H * 256), ptx::lds_u16(a1 + H * 256), 0x5410);
                         }
-                    }
-                    if (redo && ok) {
-                        // some group needs the general or the per-weight mode (rolled loop: three decode bodies in the
-                        // instruction cache, not three per part)
-                        ptx::tc_wait_st();
-                        ColK c;
-                        uint32_t cur_row = 0xFFFFFFFFu;
+#pragma unroll
+                        for (int i = 0; i < H / 2; ++i) {
+                            zi[i] = hadd2_u(zp[i], kMagic1024);                    // (integer zero-points: their value in the low bits)
+                            nf |= not_fast_bits<kBound>(sp[i], zp[i], zi[i]);
+                        }
+                        // A unit that is not in the fast mode, with a decision per part: rolled (one body of each mode in the instruction
+                        // cache), half a part at a time, so that these modes do not set the register count of the straight-line code.
+                        auto decode_by_part = [&]() {
 #pragma unroll 1
-                        for (int h = 0; h < H; ++h) {
-                            const uint32_t row = (h == 0) ? 0u : (p.gdiv((uint32_t)H * (uint32_t)u + (uint32_t)h) - g0);
-                            if (row != cur_row) {
-                                cur_row = row;
-                                load_group(row, c);
+                            for (int h = 0; h < H; ++h) {
+                                const uint32_t at = n.st + WS::kS + col * 2 + group_row(u, n.g0, h) * 256;
+                                const uint32_t s = ptx::lds_u16(at), z = ptx::lds_u16(at + H * 256), zi = hadd2_u(z, kMagic1024);
+                                ColK c;
+                                c.s2 = dup_lo(s);
+                                c.z2 = dup_lo(z);
+                                c.zb = SPARSE ? prmt(zi, zi, 0x0000) : 0u;
+                                const bool fast = !__any_sync(0xFFFFFFFFu, (not_fast_bits<kBound>(s, z, zi) & 0xFFFFu) != 0);
+                                const bool lin = __all_sync(0xFFFFFFFFu, __hge(__ushort_as_half((unsigned short)s), __ushort_as_half(0)));
+#pragma unroll 1
+                                for (int half = 0; half < 2; ++half) {
+                                    uint32_t A[16];
+                                    if (fast) F::template decode<MODE_FAST>(words(n, h), masks(n, h), half, c, A, lut);
+                                    else if (lin) F::template decode<MODE_GENERAL>(words(n, h), masks(n, h), half, c, A, lut);
+                                    else F::template decode<MODE_SLOW>(words(n, h), masks(n, h), half, c, A, lut);
+                                    ptx::tmem_st16(a_cols(n, h) + 16 * half, A);
+                                }
+                                if (h == H - 1) release_weights(n.ws);
                             }
-                            const uint32_t wb = st + WS::kW + h * (F::WROWS * 512) + col * 4;
-                            const uint32_t mb = st + WS::kMask + h * (F::MROWS * 512) + col * 4;
-                            uint32_t A[32];
-                            if (!__any_sync(0xFFFFFFFFu, not_fast_bits(c) != 0)) {
-                                if (SPARSE) c.zb = __half2uint_rz(__ushort_as_half((unsigned short)(c.z2 & 0xFFFFu))) * 0x01010101u;
-                                F::template decode<MODE_FAST>(wb, mb, c, A, lut);
-                            } else {
-                                c.zb = 0;
-                                const bool lin = __hge(__ushort_as_half((unsigned short)(c.s2 & 0xFFFFu)), __ushort_as_half(0));
-                                if (__all_sync(0xFFFFFFFFu, lin)) F::template decode<MODE_GENERAL>(wb, mb, c, A, lut);
-                                else F::template decode<MODE_SLOW>(wb, mb, c, A, lut);
+                        };
+                        if (__builtin_expect(__any_sync(0xFFFFFFFFu, nf != 0), 0)) {
+                            if (!acquire_a_stage(n, false)) { ok = false; break; }
+                            decode_by_part();
+                        } else {
+#pragma unroll
+                            for (int h = 0; h < H; ++h) {
+                                ColK c;
+                                c.s2 = (h & 1) ? dup_hi(sp[h / 2]) : dup_lo(sp[h / 2]);
+                                c.z2 = (h & 1) ? dup_hi(zp[h / 2]) : dup_lo(zp[h / 2]);
+                                c.zb = SPARSE ? prmt(zi[h / 2], zi[h / 2], (h & 1) ? 0x2222 : 0x0000) : 0u;
+                                decode_part<F, MODE_FAST>(words(n, h), masks(n, h), c, A, lut);
+                                if (h == H - 1) release_weights(n.ws);
+                                if (h == 0 && !acquire_a_stage(n, false)) { ok = false; break; }
+                                ptx::tmem_st32(a_cols(n, h), A);
                             }
-                            if (h == H - 1) release_weights();
-                            ptx::tmem_st32(lane_addr + C::kACol0 + as * C::kAStageCols + h * 32, A);
+                        }
+                    } else {
+                        // polled before the first part is decoded, so that the answer costs no latency when it is needed
+                        const bool free_early = ptx::mbar_test_wait(ptx::smem_u32(&bars.ab_free[n.as]), n.aph ^ 1u);
+                        // scale and zero-point of this thread's column in row `row` of the stage's group box, both halves of a register
+                        auto load_group = [&](uint32_t row, ColK& c) {
+                            const uint32_t sz = ptx::lds32(n.st + WS::kS + row * 256 + (col & ~1) * 2) >> (16 * (col & 1));
+                            const uint32_t zz = ptx::lds32(n.st + WS::kZ + row * 256 + (col & ~1) * 2) >> (16 * (col & 1));
+                            c.s2 = prmt(sz, sz, 0x1010);
+                            c.z2 = prmt(zz, zz, 0x1010);
+                            c.zb = 0;
+                        };
+                        auto not_fast = [&](const ColK& c) -> uint32_t {
+                            const uint32_t zr = hadd2_u(hadd2_u(c.z2, kMagic1024), H2_N1024), zlo = c.z2 & 0xFFFFu;
+                            return ((zlo | ((zlo & 0x7FFFu) + kBound) | c.s2) & 0x8000u) | (zr ^ c.z2);
+                        };
+                        auto zero_bytes = [&](ColK& c) {
+                            if (SPARSE) c.zb = __half2uint_rz(__ushort_as_half((unsigned short)(c.z2 & 0xFFFFu))) * 0x01010101u;
+                        };
+                        // The parts are decoded in the fast mode; whether every group of the unit really is in it is voted once, when the last group
+                        // has been read and before the weight stage is released.  If not, the unit is decoded again with a decision per part (the
+                        // stores are simply overwritten).
+                        bool redo = false;
+                        {
+                            ColK c;
+                            uint32_t cur_row = 0xFFFFFFFFu, nf = 0;
+#pragma unroll
+                            for (int h = 0; h < H; ++h) {
+                                // scale and zero-point change only where the group does (warp-uniform)
+                                const uint32_t row = group_row(u, n.g0, h);
+                                if (row != cur_row) {
+                                    cur_row = row;
+                                    load_group(row, c);
+                                    nf |= not_fast(c);
+                                    zero_bytes(c);
+                                }
+                                if (h == H - 1 && __any_sync(0xFFFFFFFFu, nf != 0)) {
+                                    redo = true;
+                                    break;
+                                }
+                                decode_part<F, MODE_FAST>(words(n, h), masks(n, h), c, A, lut);
+                                if (h == H - 1) release_weights(n.ws);
+                                if (h == 0 && !acquire_a_stage(n, free_early)) { ok = false; break; }
+                                ptx::tmem_st32(a_cols(n, h), A);
+                            }
+                        }
+                        if (redo && ok) {
+                            // (rolled loop: three decode bodies in the instruction cache, not three per part)
+                            ptx::tc_wait_st();
+                            ColK c;
+                            uint32_t cur_row = 0xFFFFFFFFu;
+#pragma unroll 1
+                            for (int h = 0; h < H; ++h) {
+                                const uint32_t row = group_row(u, n.g0, h);
+                                if (row != cur_row) {
+                                    cur_row = row;
+                                    load_group(row, c);
+                                }
+                                if (!__any_sync(0xFFFFFFFFu, not_fast(c) != 0)) {
+                                    zero_bytes(c);
+                                    decode_part<F, MODE_FAST>(words(n, h), masks(n, h), c, A, lut);
+                                } else {
+                                    c.zb = 0;
+                                    const bool lin = __hge(__ushort_as_half((unsigned short)(c.s2 & 0xFFFFu)), __ushort_as_half(0));
+                                    if (__all_sync(0xFFFFFFFFu, lin)) decode_part<F, MODE_GENERAL>(words(n, h), masks(n, h), c, A, lut);
+                                    else decode_part<F, MODE_SLOW>(words(n, h), masks(n, h), c, A, lut);
+                                }
+                                if (h == H - 1) release_weights(n.ws);
+                                ptx::tmem_st32(a_cols(n, h), A);
+                            }
                         }
                     }
                     if (!ok) break;
-                    // (not deferred for the warpgroup's first stage: the pipeline is still filling and the MMA warp is waiting)
-                    if (C::kDeferArrive && si >= (uint32_t)C::kWG) pending = (int)as;
-                    else announce((int)as);
+                    announce((int)n.as);
                 }
                 if (!ok) { aborted = true; break; }
-                if (C::kDeferArrive && pending >= 0) { announce(pending); pending = -1; }
                 if (!C::kEpiWarps && wg == 0) ok = epilogue(seg, tile);
                 ++seg;
                 si0 += (uint32_t)(u1 - u0);
