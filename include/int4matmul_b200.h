@@ -63,8 +63,8 @@ int i4mm_last_launch_shape(void);
 
 /*
  * Bytes of device scratch the two multiply entries need.  The scratch holds the per-CTA partial tiles
- * of the split-K reduction (tagged words on the tcgen05 path, plus arrival counters on the streaming
- * path) and a status word.  It must be zero-filled once before its first use; the kernels leave it
+ * of the split-K reduction (on the tcgen05 and few-row paths words that tell by themselves that they have been
+ * written, on the streaming path with arrival counters) and a status word.  It must be zero-filled once before its first use; the kernels leave it
  * all-zero again when they finish, so one buffer can serve every later call on the same stream.
  * Calls that overlap on the device must not share a buffer.  After a call for which
  * i4mm_device_status reported I4MM_ERR_TIMEOUT, zero the buffer again before reusing it.

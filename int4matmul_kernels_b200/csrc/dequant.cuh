@@ -107,39 +107,4 @@ __device__ __forceinline__ void sparse_expand(uint32_t& lo, uint32_t& hi, uint32
     hi = __funnelshift_rc(hi, 0u, used);
 }
 
-// The same with a table of 16-byte entries: selectors of positions 0..3 | (4 * popcount) << 16, of positions 4..7, and the masks of
-// the kept positions, 0xFF each (so the fast mode takes zero-points up to 255).  Fewer instructions, more shared-memory
-// wavefronts; which one is better where: see SparseTable in umma_kernel.cu.
-__device__ __forceinline__ void sparse_table_entry(uint32_t& e, int keep) { e = sparse_selectors(keep); }
-__device__ __forceinline__ void sparse_table_entry(uint4& e, int keep) {
-    const uint32_t sel = sparse_selectors(keep);
-    uint32_t mask[2] = {0, 0};
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-        if (keep & (1 << j)) mask[j >> 2] |= 0xFFu << (8 * (j & 3));
-    e = make_uint4((sel & 0xFFFFu) | (4u * (uint32_t)__popc(keep) << 16), sel >> 16, mask[0], mask[1]);
-}
-template <int MODE>
-__device__ __forceinline__ void sparse_expand(uint32_t& lo, uint32_t& hi, uint32_t m, int step, const uint4* lut, const ColK& c,
-                                              uint32_t (&A)[4]) {
-    const uint4 e = lut[(m >> (8 * step)) & 0xFFu];
-    const uint32_t even = lo & 0x0F0F0F0Fu, odd = (lo >> 4) & 0x0F0F0F0Fu;
-    const uint32_t off = hsub2_u(BASE_1_1, c.z2);
-#pragma unroll
-    for (int q4 = 0; q4 < 2; ++q4) {
-        uint32_t d = prmt(even, odd, q4 ? e.y : e.x);
-        const uint32_t k = q4 ? e.w : e.z;
-        if (MODE == MODE_FAST) d = bit_select(k, d, c.zb);
-        A[2 * q4] = finish<4, MODE>(prmt(d, 0x64646464u, 0x5140), MUL_1_1, BASE_1_1, off, c);
-        A[2 * q4 + 1] = finish<4, MODE>(prmt(d, 0x64646464u, 0x7362), MUL_1_1, BASE_1_1, off, c);
-        if (MODE != MODE_FAST) {
-            A[2 * q4] &= prmt(k, k, 0x1100);
-            A[2 * q4 + 1] &= prmt(k, k, 0x3322);
-        }
-    }
-    const uint32_t used = e.x >> 16;
-    lo = __funnelshift_rc(lo, hi, used);
-    hi = __funnelshift_rc(hi, 0u, used);
-}
-
 }  // namespace i4mm

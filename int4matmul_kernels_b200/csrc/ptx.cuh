@@ -135,6 +135,16 @@ __device__ __forceinline__ void st_relaxed_gpu_u64(unsigned long long* p, unsign
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
+// four 32-bit words, each single-copy atomic by itself
+__device__ __forceinline__ uint4 ld_relaxed_gpu_v4(const uint4* p) {
+    uint4 v;
+    asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_relaxed_gpu_v4(uint4* p, uint4 v) {
+    asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+
 // ---- shared-memory loads by 32-bit shared address -------------------------------------------------------
 __device__ __forceinline__ uint4 lds128(uint32_t addr) {
     uint4 v;

@@ -641,7 +641,9 @@ stream_kernel(const StreamParams p) {
                     float v = 0.f;
                     for (int bb = b_lo; bb <= b_hi; ++bb) {
                         const int which = (bb > b_lo || lo_starts_here) ? 0 : 1;
-                        v += __ldcg(p.partials + ((size_t)bb * 2 + which) * (ROWS * kCTile) + idx);
+                        float* const part = p.partials + ((size_t)bb * 2 + which) * (ROWS * kCTile) + idx;
+                        v += __ldcg(part);
+                        __stcg(part, 0.f);                       // the scratch is left all-zero, as the other kernels need it
                     }
                     if (oc < p.S) {
                         __half* o = p.out + (size_t)m * p.S + oc;

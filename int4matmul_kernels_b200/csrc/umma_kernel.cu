@@ -16,15 +16,15 @@
 //   MMA warp          one elected thread issues 8 (16) x tcgen05.mma (M = 128, N = NT, K = 16) per unit, A from tensor
 //                     memory, B from the swizzled shared-memory tile, and commits to mbarriers that recycle the
 //                     stages; the accumulator never leaves tensor memory until the tile is done
-//   epilogue          reads the accumulator (tcgen05.ld), converts to fp16 and stores: one warpgroup of its own for up to 32
-//                     rows (a CTA's last tile: from 2 rows on the dequant warpgroups as well, see last_epilogue), dequant
-//                     warpgroup 0 for 33..64, two warpgroups of their own (half of the columns each) above
+//   epilogue          reads the accumulator (tcgen05.ld), converts to fp16 and stores: one warpgroup of its own for up to 64
+//                     rows (a CTA's last tile: from 2 rows on the dequant warpgroups as well, see last_epilogue), two warpgroups
+//                     of their own (half of the columns each) above
 //
-// Configurations (Cfg<NT, PAIR>): NT <= 32 rows stream the weights once from HBM - one CTA per SM, 3 dequant warpgroups,
-// 9 weight stages and 3 A / activation stages of 256 k, and the (tile, unit) space cut into equal ranges per CTA
-// (split-K over the whole GPU, partial tiles summed through scratch in a fixed order).  NT = 64: two CTAs per SM, whole tiles.
-// NT >= 128: one CTA per SM, whole tiles, epilogue stores transposed through shared memory; by default launched as
-// clusters of two CTAs that run each MMA together (cta_group::2, M = 256 over two SMs), see PAIR below.
+// Configurations (Cfg<NT, PAIR>), one CTA per SM: NT <= 64 rows stream the weights once from HBM - 3 dequant warpgroups, 9 (6)
+// weight stages and 3 A / activation stages of 256 k, and the (tile, unit) space cut into equal ranges per CTA (split-K over the
+// whole GPU, partial tiles summed through scratch in a fixed order).  NT >= 128: whole tiles, epilogue stores transposed through
+// shared memory; by default launched as clusters of two CTAs that run each MMA together (cta_group::2, M = 256 over two SMs), see
+// PAIR below.
 // Every wait is bounded and reports through the status word instead of hanging.
 #include "../../include/int4matmul_b200.h"
 
@@ -60,7 +60,7 @@ struct UmmaParams {
     int accumulate;
     int overlap;         // weight-side tensors may be read while the kernel before this one is still running
     int kparts;          // > 1: every tile's K range is cut into this many parts, one CTA (pair) each, fp32 partial outputs
-                         // go to the scratch as (part, row, S) and kparts_reduce_kernel sums them (more than 32 rows only)
+                         // go to the scratch as (part, row, S) and kparts_reduce_kernel sums them (more than 64 rows only)
     GroupDiv gdiv;
 };
 
@@ -75,8 +75,8 @@ template <bool PERM>
 struct UFormat<4, false, PERM> {
     static constexpr int WROWS = 8, MROWS = 0;       // packed rows / mask rows per 64-k part
     static constexpr bool kPermutedK = PERM;
-    template <int MODE, class Entry>
-    __device__ static __forceinline__ void decode(uint32_t wbase, uint32_t, int half, const ColK& c, uint32_t* A, const Entry*) {
+    template <int MODE>
+    __device__ static __forceinline__ void decode(uint32_t wbase, uint32_t, int half, const ColK& c, uint32_t* A, const uint32_t*) {
         if (PERM) {
             // nibbles j and j + 4 of a word sit at the same offset of its two 16-bit halves: one LOP3 per pair plants both
             // into the mantissas of (1024, 1024); the odd nibbles come out multiplied by 16
@@ -109,8 +109,8 @@ template <bool PERM>
 struct UFormat<2, false, PERM> {
     static constexpr int WROWS = 4, MROWS = 0;
     static constexpr bool kPermutedK = false;
-    template <int MODE, class Entry>
-    __device__ static __forceinline__ void decode(uint32_t wbase, uint32_t, int half, const ColK& c, uint32_t* A, const Entry*) {
+    template <int MODE>
+    __device__ static __forceinline__ void decode(uint32_t wbase, uint32_t, int half, const ColK& c, uint32_t* A, const uint32_t*) {
         const uint32_t offa = hsub2_u(BASE_1_4, c.z2), offb = hsub2_u(BASE_16_64, c.z2);
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
@@ -132,8 +132,8 @@ template <bool PERM>
 struct UFormat<3, false, PERM> {
     static constexpr int WROWS = 6, MROWS = 0;
     static constexpr bool kPermutedK = false;
-    template <int MODE, class Entry>
-    __device__ static __forceinline__ void decode(uint32_t wbase, uint32_t, int blk, const ColK& c, uint32_t* A, const Entry*) {
+    template <int MODE>
+    __device__ static __forceinline__ void decode(uint32_t wbase, uint32_t, int blk, const ColK& c, uint32_t* A, const uint32_t*) {
         const uint32_t off = hsub2_u(BASE_1_8, c.z2);
         const uint32_t w0 = ptx::lds32(wbase + (3 * blk) * 512), w1 = ptx::lds32(wbase + (3 * blk + 1) * 512), w2 = ptx::lds32(wbase + (3 * blk + 2) * 512);
         // the 96-bit stream in 12-bit chunks: chunk j holds fields 4j .. 4j+3 = pairs (2j, 2j+1)
@@ -159,8 +159,8 @@ template <bool PERM>
 struct UFormat<4, true, PERM> {
     static constexpr int WROWS = 4, MROWS = 2;
     static constexpr bool kPermutedK = false;
-    template <int MODE, class Entry>
-    __device__ static __forceinline__ void decode(uint32_t wbase, uint32_t mbase, int blk, const ColK& c, uint32_t* A, const Entry* lut) {
+    template <int MODE>
+    __device__ static __forceinline__ void decode(uint32_t wbase, uint32_t mbase, int blk, const ColK& c, uint32_t* A, const uint32_t* lut) {
         // a 32-block of this column: the 64-bit word of its 16 kept nibbles (in increasing k) and its keep-mask
         uint32_t lo = ptx::lds32(wbase + (2 * blk) * 512), hi = ptx::lds32(wbase + (2 * blk + 1) * 512);
         const uint32_t m = ptx::lds32(mbase + blk * 512);
@@ -174,8 +174,8 @@ struct UFormat<4, true, PERM> {
     }
 };
 
-template <class F, int MODE, class Entry>
-__device__ __forceinline__ void decode_part(uint32_t wbase, uint32_t mbase, const ColK& c, uint32_t (&A)[32], const Entry* lut) {
+template <class F, int MODE>
+__device__ __forceinline__ void decode_part(uint32_t wbase, uint32_t mbase, const ColK& c, uint32_t (&A)[32], const uint32_t* lut) {
 #pragma unroll
     for (int half = 0; half < 2; ++half) F::template decode<MODE>(wbase, mbase, half, c, A + 16 * half, lut);
 }
@@ -199,26 +199,20 @@ struct WStage {     // one stage of the packed-weight ring: one unit = H parts o
 constexpr int kMaxWStages = 16;
 constexpr int kMaxABStages = 6;
 
-// Look-up table of the 16:32 expansion.  Entries of 4 bytes are the better ones everywhere (96 rows 5120 x 20480: 52.0 us, 56.3 with
-// 16 bytes) but with tiles of 64 rows, where two CTAs on an SM keep the ALU pipe full and what counts is instructions (48 rows
-// 5120 x 20480: 64.2 and 55.6, 20480 x 5120: 47.8 and 44.7).
-// kFastBound: the fast mode takes zero-points up to 127 / 255, whose fp16 bits + kFastBound = 0x7FFF.
-template <bool SPARSE, int NT>
-struct SparseTable {
-    using Entry = uint32_t;
-    static constexpr uint32_t kFastBound = SPARSE ? 0x280Fu : 0x1FFFu;
-};
-template <>
-struct SparseTable<true, 64> {
-    using Entry = uint4;
-    static constexpr uint32_t kFastBound = 0x2407u;
-};
+// The fast mode takes zero-points up to 512 (16:32, whose expansion XORs them into the nibbles: up to 127): kFastBound + the fp16 bits of
+// the largest one = 0x7FFF.
+template <bool SPARSE>
+constexpr uint32_t kFastBound = SPARSE ? 0x280Fu : 0x1FFFu;
 
 template <int NT, bool PAIR>
 struct Cfg {
     // packed-weight ring (128 k per stage).  Few rows: the kernel streams weights from HBM, and the ring has to
     // cover the DRAM latency; many rows: weights are a trickle next to the activation tiles
-    static constexpr bool kStream = NT <= 32;                         // weight-streaming shapes: one CTA per SM with everything doubled
+    // Weight-streaming shapes: one CTA per SM with everything doubled, and K split over the CTAs.  They end at 64 rows.  Rows 33..64 had tiles
+    // of 64 rows at two CTAs an SM, whole or with K cut into parts and a second launch: 48 rows 13824 x 5120 int4 25.7 us, now 18.8,
+    // 16:32 38.1 / 22.0, int3 34.0 / 18.7, int2 33.1 / 17.4; 5120 x 20480 55.8 / 22.9, 53.8 / 29.7, 43.4 / 23.5, 42.7 / 22.4; 16384 x 16384
+    // 66.3 / 44.3, 76.9 / 56.7, 59.9 / 43.5, 62.3 / 39.0; 1024 x 1024 8.9 / 7.8, 9.6 / 8.2, 9.0 / 7.8, 9.0 / 7.8; nothing was faster there.
+    static constexpr bool kStream = NT <= 64;
     // NT = 128..192: an MMA of N <= 192 takes 512..768 cycles per 128 k, the dequantisation of its weights with two
     // warpgroups ~1400, so these shapes get four warpgroups as well, and a deeper weight ring
     // (single CTAs have the shared memory for the 4 A / activation stages that four warpgroups need only at NT = 128)
@@ -234,14 +228,13 @@ struct Cfg {
     // complete, expect_tx + the copy's issue another ~190): at 128 k per stage that alone is ~27 us for 16384 x 16384
     // weights on 148 SMs, so the weight-streaming shapes use 256-k units.
     static constexpr int kHalves = kStream ? 4 : 2;
-    static constexpr int kWStages = kStream ? (NT <= 16 ? 9 : 6) : NT <= 64 ? 8 : kDequantBound ? 6 : 3;
+    static constexpr int kWStages = kStream ? (NT <= 16 ? 9 : 6) : kDequantBound ? 6 : 3;
     // staging slots (units of look-ahead) for activation rows that are reordered on their way into the A / activation
     // stages (umma_kernel's PERM)
     static constexpr int kXStaging = 4;
     static constexpr int kWG = kStream ? 3 : kDequantBound ? 4 : 2;   // dequant warpgroups (4 warps each), taking units in turn
     static constexpr int kABStages = kStream ? 3 : NT == 128 ? 4 : 3;   // ring of (A in tensor memory, activation tile in shared memory) pairs, one unit per stage
     static constexpr bool kWGuard = kWStages % kWG != 0;
-    static constexpr bool kEpiWarps = NT >= 128 || kStream;           // a warpgroup of its own for the epilogue (else dequant warpgroup 0 does it)
     static constexpr bool kEpiTransposed = NT >= 128;                 // epilogue stores go through a shared-memory transposition tile
     static constexpr bool kEpiHandoff = kStream;                      // the MMA warp waits for the accumulator and wakes the epilogue warps (named barrier)
     // many rows: two epilogue warpgroups, each draining half of the accumulator's columns, so that the next tile's
@@ -251,19 +244,16 @@ struct Cfg {
     // thread's loop (wait ~190 cycles, expect_tx + copies ~250) delivers a 16 KB stage per ~500-700 cycles, about
     // 4-5 TB/s over the whole GPU, which is less than the memory system can stream.
     static constexpr int kWProducers = kStream ? 2 : 1;
-    static constexpr int kWarps = 4 * kWG + (kEpiWarps ? 4 * kEpiGroups : 0) + 3 + (kWProducers - 1);  // + weight producer(s), activation producer, MMA issuer
+    static constexpr int kWarps = 4 * kWG + 4 * kEpiGroups + 3 + (kWProducers - 1);  // + weight producer(s), activation producer, MMA issuer
     static constexpr int kThreads = kWarps * 32;
     static constexpr int kDCols = NT < 32 ? 32 : NT;                  // accumulator columns
     static constexpr int kACol0 = kDCols;                             // A stages follow: 32 columns per 64 k
     static constexpr int kAStageCols = 32 * kHalves;
     static constexpr int kColsUsed = kDCols + kAStageCols * kABStages;
     static constexpr int kTmemCols = kColsUsed <= 256 ? 256 : 512;
-    // split-K over CTAs with a scratch reduction: the few-row shapes.  (It was measured at 128 rows with a sum by one warpgroup, one
-    // partner at a time: 15-30 K cycles per tile, which lost more than the better balance gained.  Not measured since the sum is
-    // spread over the warpgroups; more rows cut K into parts, see choose_kparts.)
-    static constexpr bool kSplit = NT <= 32;
-    static constexpr int kSlotElems = NT * 128;                       // 64-bit words of one CTA's partial tile in the scratch
-    static constexpr int kMinBlocks = kStream ? 1 : NT <= 64 ? 2 : 1;
+    // split-K over CTAs with a scratch reduction (more rows cut K into parts, see choose_kparts)
+    static constexpr bool kSplit = kStream;
+    static constexpr int kSlotVecs = NT / 4 * 128;                    // one CTA's partial tile in the scratch: [4 rows][128 columns] of 16 bytes
 };
 
 // A / activation stages.  A CTA of a pair holds only half of each activation tile, which leaves shared memory for as
@@ -306,18 +296,24 @@ __device__ __forceinline__ void store_rows(const OutMap& om, __half* out0, long 
 
 // The epilogue of the weight-streaming shapes (one row tile).  Split-K: the CTAs b_lo .. b_hi share a tile.  b_lo,
 // which owns its first units and reaches them last, adds the others' partial tiles to its own accumulator in CTA order - a fixed
-// order, so results are reproducible; the others wait for nobody.  A partial element is one 64-bit word (fp32 value | tag 1
-// in the high half), written with a single store, so no fence, counter or second round trip is needed; the reader clears
+// order, so results are reproducible; the others wait for nobody.  A partial sum is a 32-bit word that is never zero (share_word), four rows of
+// a column in one 16-byte store, so no fence, counter or second round trip is needed: a reader knows each word by itself, and clears
 // what it has read, which leaves the scratch all-zero for the next launch.  One slot per CTA is enough: a CTA has at most one
 // tile that it shares and does not sum.  A tile that a CTA sums is its last one, so there are two functions.
+// What a thread waits for are its loads, so fewer and wider ones count: with one 64-bit word (value | tag) per row, int4 16 rows 20480 x 5120
+// 22.3 us, now 19.7; 5120 x 5120 13.2 / 10.2; 16384 x 2048 17.0 / 12.4; 32 rows 25.1 / 21.1, 15.6 / 11.7, 20.4 / 14.9; one row 18.4 / 17.7, 10.3 / 9.7,
+// 12.7 / 11.5.
+__device__ __forceinline__ uint32_t share_word(uint32_t v) { return __float_as_uint(__uint_as_float(v) + 0.0f) ^ 0x80000000u; }   // (-0 goes as +0)
+__device__ __forceinline__ float share_value(uint32_t w) { return __uint_as_float(w ^ 0x80000000u); }
 
 // A tile before a CTA's last one, by the epilogue warps: a whole tile, or (share: this lane's column of the CTA's slot) the CTA's share
 // of a tile that another CTA sums.  The next tile's MMAs wait for it.  Not inlined and with its arguments by value: with `p` by
 // reference a call cost ~1 us (1024 x 32768 int4, 5 rows, two or three tiles a CTA: 16.2 us, now 12.9), and inlined it slowed the
 // decode loop (13824 x 5120 int4, 4 rows: 17.4 us, now 16.5).
 // out0: the column's first output; rows / out_rows: rows of the launch, and those that this lane stores.
+template <int NT>
 __device__ __noinline__ bool early_epilogue(const OutMap& om, int n_dst, long long ld, __half* out0, int rows, int out_rows, int accumulate,
-                                            unsigned long long* share, uint32_t tmem_base, uint32_t d_empty, uint32_t s_abort) {
+                                            uint4* share, uint32_t tmem_base, uint32_t d_empty, uint32_t s_abort) {
     const uint32_t lane_addr = tmem_base + ((threadIdx.x & 96u) << 16);
     auto release = [&]() {
         ptx::tc_fence_before_sync();
@@ -344,9 +340,36 @@ __device__ __noinline__ bool early_epilogue(const OutMap& om, int n_dst, long lo
             ptx::tc_wait_ld();
             if (rb + 16 >= rows) release();
 #pragma unroll
-            for (int i = 0; i < 16; ++i)
-                if (rb + i < rows) ptx::st_relaxed_gpu_u64(share + (rb + i) * 128, (1ull << 32) | v[i]);
+            for (int i = 0; i < 16; i += 4)
+                if (rb + i < rows)
+                    ptx::st_relaxed_gpu_v4(share + (rb + i) / 4 * 128, make_uint4(share_word(v[i]), share_word(v[i + 1]), share_word(v[i + 2]), share_word(v[i + 3])));
         }
+        return true;
+    }
+    if (NT > 32 && !accumulate) {
+        // converted and held in registers, so that the accumulator is free before the stores
+        uint32_t h2[NT / 2];
+#pragma unroll
+        for (int rb = 0; rb < NT; rb += 16) {
+            uint32_t v[16];
+            ptx::tmem_ld16(lane_addr + rb, v);
+            ptx::tc_wait_ld();
+#pragma unroll
+            for (int i = 0; i < 16; i += 2)
+                h2[(rb + i) / 2] = h2_as_u32(__floats2half2_rn(__uint_as_float(v[i]), __uint_as_float(v[i + 1])));
+        }
+        release();
+#pragma unroll
+        for (int rb = 0; rb < NT; rb += 16) {
+            __half h[16];
+#pragma unroll
+            for (int i = 0; i < 16; i += 2) {
+                h[i] = __low2half(u32_as_h2(h2[(rb + i) / 2]));
+                h[i + 1] = __high2half(u32_as_h2(h2[(rb + i) / 2]));
+            }
+            store_rows<16>(om, out0 + (size_t)rb * ld, ld, n_dst, h, out_rows - rb);
+        }
+        if (n_dst > 1) __threadfence_system();
         return true;
     }
     auto finish_rows = [&](auto rb_tag, int rb) {
@@ -378,11 +401,11 @@ __device__ __noinline__ bool early_epilogue(const OutMap& om, int n_dst, long lo
 
 // A CTA's last tile: units t0 .. t0 + units - 1.  What bounds it is the number of dependent round trips to L2 (~0.7 us each) between
 // the last MMA and the end of the launch, so the tile can be left to all of the CTA's warpgroups (the dequant warps have nothing
-// else to do by then), `part` of `parts` rows each; a thread has RB x PB partial words in flight, up to 16: with 4 rows and 4
-// partners or 8 rows and 2 partners.  One warpgroup that read 8 rows of one partner at a time took 25.9 us with 16 rows of 16384 x 5120
-// int4 and 34.4 with 32; now 20.8 and 23.2.  (When: see spread_last.)
+// else to do by then), `part` of `parts` of its groups of four rows each; a thread has its groups of up to 4 partners in flight (33..64 rows: of 2,
+// with 4 the registers spill: 48 rows 5120 x 5120 12.9 us, 16.2).
+// (When: see spread_last.)
 // bar_id, bar_threads: the named barrier at which the MMA warp says that the accumulator is complete (once per call, also where this
-// part has no rows).  Inlined, with one pass over at most 8 rows: a call cost ~1 us here as well.
+// part has no rows).  Inlined: a call cost ~1 us here as well.
 template <int NT>
 __device__ __forceinline__ bool last_epilogue(const UmmaParams& p, uint32_t tmem_base, const volatile int* s_abort, long long t0, int units,
                                               int part, int parts, uint32_t bar_id, uint32_t bar_threads) {
@@ -392,17 +415,18 @@ __device__ __forceinline__ bool last_epilogue(const UmmaParams& p, uint32_t tmem
     const long long U = p.U, G = gridDim.x, tile = div_nn(t0, U);
     const int u0 = (int)(t0 - tile * U), u1 = u0 + units;
     const int col = (warp & 3) * 32 + lane, scol = (int)tile * 128 + col;
-    const uint32_t lane_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
     const bool col_ok = scol < p.S;
-    const int me = (int)blockIdx.x, r0 = p.rows * part / parts, n = p.rows * (part + 1) / parts - r0;      // n <= 8
+    const int me = (int)blockIdx.x, groups = (p.rows + 3) / 4, g0 = groups * part / parts, ng = groups * (part + 1) / parts - g0;
+    const int r0 = 4 * g0, n = min(4 * ng, p.rows - r0);                  // this part's rows
+    const uint32_t acc = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + r0;
     int b_lo = me, b_hi = me;
     if (u0 != 0 || u1 != (int)U) {
         const long long T = p.CT * U, lo_t = tile * U;
         b_lo = range_owner(T, G, lo_t);
         b_hi = range_owner(T, G, lo_t + U - 1);
     }
-    unsigned long long* const partials64 = reinterpret_cast<unsigned long long*>(p.partials);
-    auto slot_of = [&](int bb) { return partials64 + (size_t)bb * Cfg<NT, false>::kSlotElems + col; };
+    uint4* const slot0 = reinterpret_cast<uint4*>(p.partials) + g0 * 128 + col;
+    auto slot_of = [&](int bb) { return slot0 + (size_t)bb * Cfg<NT, false>::kSlotVecs; };
     auto wait_accumulator = [&]() -> bool {
         __syncwarp();
         ptx::named_bar_sync(bar_id, bar_threads);      // released by the MMA warp once the accumulator is complete
@@ -410,75 +434,87 @@ __device__ __forceinline__ bool last_epilogue(const UmmaParams& p, uint32_t tmem
         ptx::tc_fence_after_sync();
         return true;
     };
+    constexpr int kMaxGroups = NT <= 32 ? 2 : NT / 16;
     if (me != b_lo) {
         if (!wait_accumulator()) return false;
-        unsigned long long* const mine = slot_of(me) + r0 * 128;
-        uint32_t v[8];
-        ptx::tmem_ld(lane_addr + r0, v);
-        ptx::tc_wait_ld();
+        uint4* const mine = slot_of(me);
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
-            if (i < n) ptx::st_relaxed_gpu_u64(mine + i * 128, (1ull << 32) | v[i]);
+        for (int j = 0; j < kMaxGroups; ++j) {
+            uint32_t v[4];
+            if (j < ng) {
+                ptx::tmem_ld4(acc + 4 * j, v);
+                ptx::tc_wait_ld();
+                ptx::st_relaxed_gpu_v4(mine + j * 128, make_uint4(share_word(v[0]), share_word(v[1]), share_word(v[2]), share_word(v[3])));
+            }
+        }
         return true;
     }
     __half* const out0 = p.om.dst[0] + (col_ok ? p.om.col(scol) : 0) + (size_t)r0 * p.om.ld;
     bool waiting_ok = true;
-    // all of this part's rows (n <= RB), the partners PB at a time: RB x PB loads in flight
-    auto finish_rows = [&](auto rb_tag, auto pb_tag) -> bool {
-        constexpr int RB = decltype(rb_tag)::value, PB = decltype(pb_tag)::value;
-        float sum[RB];
-        __half old[RB];
+    // all of this part's groups (ng <= NG), the partners PB at a time: NG x PB loads in flight
+    auto finish = [&](auto ng_tag, auto pb_tag) -> bool {
+        constexpr int NG = decltype(ng_tag)::value, PB = decltype(pb_tag)::value;
+        float sum[4 * NG];
+        __half old[4 * NG];
 #pragma unroll
-        for (int i = 0; i < RB; ++i) {
+        for (int i = 0; i < 4 * NG; ++i) {
             sum[i] = 0.f;
             old[i] = __ushort_as_half(0);
             if (p.accumulate && i < n && col_ok) old[i] = out0[(size_t)i * p.om.ld];
         }
 #pragma unroll 1
         for (int q = b_lo + 1; q <= b_hi; q += PB) {
-            unsigned long long w[PB][RB];
+            uint4 w[PB][NG];
 #pragma unroll
-            for (int j = 0; j < PB; ++j)
+            for (int k = 0; k < PB; ++k)
 #pragma unroll
-                for (int i = 0; i < RB; ++i)
-                    if (q + j <= b_hi && i < n) w[j][i] = ptx::ld_relaxed_gpu_u64(slot_of(q + j) + (r0 + i) * 128);
+                for (int j = 0; j < NG; ++j)
+                    if (q + k <= b_hi && j < ng) w[k][j] = ptx::ld_relaxed_gpu_v4(slot_of(q + k) + j * 128);
 #pragma unroll
-            for (int j = 0; j < PB; ++j)
+            for (int k = 0; k < PB; ++k)
 #pragma unroll
-                for (int i = 0; i < RB; ++i)
-                    if (q + j <= b_hi && i < n) {
-                        unsigned long long* const at = slot_of(q + j) + (r0 + i) * 128;
-                        for (uint32_t spins = 0; (uint32_t)(w[j][i] >> 32) != 1u && waiting_ok; ++spins) {
+                for (int j = 0; j < NG; ++j)
+                    if (q + k <= b_hi && j < ng) {
+                        uint4& x = w[k][j];
+                        for (uint32_t spins = 0; (x.x == 0u || x.y == 0u || x.z == 0u || x.w == 0u) && waiting_ok; ++spins) {
                             if (spins >= ptx::kSpinLimit) {            // a contributor never delivered: report, stop waiting
                                 atomicExch(p.status, 34);
                                 waiting_ok = false;
                                 break;
                             }
                             __nanosleep(20);
-                            w[j][i] = ptx::ld_relaxed_gpu_u64(at);
+                            x = ptx::ld_relaxed_gpu_v4(slot_of(q + k) + j * 128);
                         }
-                        sum[i] += __uint_as_float((uint32_t)w[j][i]);
-                        ptx::st_relaxed_gpu_u64(at, 0ull);
+                        sum[4 * j] += share_value(x.x);
+                        sum[4 * j + 1] += share_value(x.y);
+                        sum[4 * j + 2] += share_value(x.z);
+                        sum[4 * j + 3] += share_value(x.w);
+                        ptx::st_relaxed_gpu_v4(slot_of(q + k) + j * 128, make_uint4(0, 0, 0, 0));
                     }
         }
         if (!wait_accumulator()) return false;
-        uint32_t v[RB];
-        ptx::tmem_ld(lane_addr + r0, v);
-        ptx::tc_wait_ld();
-        __half h[RB];
+        __half h[4 * NG];
 #pragma unroll
-        for (int i = 0; i < RB; ++i) {
-            float f = __uint_as_float(v[i]) + sum[i];
-            if (p.accumulate) f += __half2float(old[i]);
-            h[i] = __float2half_rn(f);
+        for (int j = 0; j < NG; ++j) {
+            uint32_t v[4] = {0u, 0u, 0u, 0u};
+            if (j < ng) {
+                ptx::tmem_ld4(acc + 4 * j, v);
+                ptx::tc_wait_ld();
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                float f = __uint_as_float(v[i]) + sum[4 * j + i];
+                if (p.accumulate) f += __half2float(old[4 * j + i]);
+                h[4 * j + i] = __float2half_rn(f);
+            }
         }
-        store_rows<RB>(p.om, out0, p.om.ld, p.om.n_dst, h, col_ok ? n : 0);
+        store_rows<4 * NG>(p.om, out0, p.om.ld, p.om.n_dst, h, col_ok ? n : 0);
         return true;
     };
-    if (n <= 4) {
-        if (!finish_rows(std::integral_constant<int, 4>(), std::integral_constant<int, 4>())) return false;
+    if (NT <= 32 && ng <= 1) {
+        if (!finish(std::integral_constant<int, 1>(), std::integral_constant<int, 4>())) return false;
     } else {
-        if (!finish_rows(std::integral_constant<int, 8>(), std::integral_constant<int, 2>())) return false;
+        if (!finish(std::integral_constant<int, kMaxGroups>(), std::integral_constant<int, NT <= 32 ? 4 : 2>())) return false;
     }
     if (p.om.n_dst > 1) __threadfence_system();                // as in umma_kernel's epilogue
     return true;
@@ -489,7 +525,7 @@ __device__ __forceinline__ bool last_epilogue(const UmmaParams& p, uint32_t tmem
 // the activation tile, which halves the L2 -> shared-memory traffic that bounds the many-row shapes.
 // PERM (up to 3 rows of dense int4 only): the cheaper k order of UFormat, with the activations reordered to match.
 template <int BITS, bool SPARSE, int NT, bool PAIR, bool PERM = false>
-__global__ void __launch_bounds__(Cfg<NT, PAIR>::kThreads, Cfg<NT, PAIR>::kMinBlocks)
+__global__ void __launch_bounds__(Cfg<NT, PAIR>::kThreads, 1)
 umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaParams p, const __half* x) {
     using C = Cfg<NT, PAIR>;
     using F = UFormat<BITS, SPARSE, PERM>;
@@ -504,12 +540,12 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
     // single CTAs at NT = 256 have no shared memory left for a second transposition tile: the second epilogue group idles
     constexpr int kEpiGroups = (C::kEpiGroups == 2 && (PAIR || NT < 256)) ? 2 : 1;
     constexpr int kEpiWarp0 = 4 * C::kWG;                           // first epilogue warp (a multiple of 4: lane quarter = warp % 4)
-    constexpr int kWProducer = kEpiWarp0 + (C::kEpiWarps ? 4 * C::kEpiGroups : 0), kBProducer = kWProducer + 1, kMma = kWProducer + 2;
+    constexpr int kWProducer = kEpiWarp0 + 4 * C::kEpiGroups, kBProducer = kWProducer + 1, kMma = kWProducer + 2;
     constexpr int kWProducer2 = kWProducer + 3;                     // only when Cfg::kWProducers == 2
     constexpr int kABStages = ABStages<NT, PAIR>::value;
     extern __shared__ __align__(1024) unsigned char smem[];      // [B ring (1024-aligned tiles)][W ring]
     __shared__ __align__(8) Barriers bars;
-    __shared__ typename SparseTable<SPARSE, NT>::Entry lut[SPARSE ? kSparseLutEntries : 1];
+    __shared__ uint32_t lut[SPARSE ? kSparseLutEntries : 1];
     __shared__ uint32_t tmem_base_smem;
     __shared__ volatile int s_abort;     // set by a warp that gives up on the accumulator (the MMA warp before it releases the epilogue
                                          // warps for the last time; an epilogue warp before its group's next named barrier)
@@ -554,7 +590,7 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
             }
             ptx::fence_mbar_init();
         }
-        if (SPARSE && warp < 8) sparse_table_entry(lut[warp * 32 + lane], warp * 32 + lane);   // (warps 0..7 are dequant warps in every configuration)
+        if (SPARSE && warp < 8) lut[warp * 32 + lane] = sparse_selectors(warp * 32 + lane);   // (warps 0..7 are dequant warps in every configuration)
         if (warp == kMma) {
             if (PAIR) {
                 ptx::tmem_alloc_pair(ptx::smem_u32(&tmem_base_smem), C::kTmemCols);
@@ -615,7 +651,7 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
         spread_last = p.rows > 6 || t_lo > first || range_lo(n_tiles * U, G, b + 2) <= first + U;
     }
     constexpr uint32_t kSpreadThreads = (C::kWG + 1) * 128 + 32;
-    static_assert(!C::kStream || NT <= 8 * (C::kWG + 1), "last_epilogue takes at most 8 rows a warpgroup");
+    static_assert(!C::kStream || NT <= 16 * (C::kWG + 1), "last_epilogue takes at most 4 groups of rows a warpgroup");
 
     if (warp == kWProducer || (C::kWProducers == 2 && warp == kWProducer2)) {
         // =========================== packed weights (+ scales / zeros): one thread per producer warp ===========================
@@ -833,8 +869,8 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
         }
     } else {
         // =========================== dequant warpgroups; epilogue warps ===========================
-        // Accumulator of one finished tile (or K part of one) of the shapes for more than 32 rows -> fp16 rows of `out`, or fp32 rows in
-        // the scratch.  (Up to 32 rows: early_epilogue, last_epilogue.)  Run by 4 warps whose index modulo 4 selects the 32 tensor-memory lanes (= weight columns) they may read.
+        // Accumulator of one finished tile (or K part of one) of the shapes for more than 64 rows -> fp16 rows of `out`, or fp32 rows in
+        // the scratch.  (Up to 64 rows: early_epilogue, last_epilogue.)  Run by 4 warps whose index modulo 4 selects the 32 tensor-memory lanes (= weight columns) they may read.
         bool dependency_waited = false;
         auto epilogue = [&](uint32_t seg, long long tile) -> bool {
             if (!dependency_waited) {
@@ -958,38 +994,6 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                     }
                     ptx::named_bar_sync(bar_id, 128);
                 }
-            } else {
-            constexpr int CH = NT >= 64 ? 32 : 16;          // accumulator columns per tensor-memory load
-#pragma unroll 1
-            for (int j0 = 0; j0 < NT; j0 += CH) {
-                uint32_t v[CH];
-                if (CH == 32) ptx::tmem_ld32(lane_addr + j0, reinterpret_cast<uint32_t(&)[32]>(v));
-                else ptx::tmem_ld16(lane_addr + j0, reinterpret_cast<uint32_t(&)[16]>(v));
-                ptx::tc_wait_ld();
-                if (j0 + CH >= NT) {                       // the last columns are in registers: the accumulator is free again
-                    ptx::tc_fence_before_sync();
-                    __syncwarp();
-                    if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&bars.d_empty));
-                }
-                if (p.kparts > 1) {
-                    put_kpart(v, j0);
-                    continue;
-                }
-                if (col_ok) {
-                    const long long dcol = p.om.col(scol);
-#pragma unroll
-                    for (int j = 0; j < CH; ++j) {
-                        const int m = j0 + j;
-                        if (m < nrows) {
-                            float f = __uint_as_float(v[j]);
-                            const size_t at = (size_t)(row0 + m) * p.om.ld + dcol;
-                            if (p.accumulate) f += __half2float(p.om.dst[0][at]);
-                            const __half h = __float2half_rn(f);
-                            for (int d = 0; d < p.om.n_dst; ++d) p.om.dst[d][at] = h;
-                        }
-                    }
-                }
-            }
             }
             // Stores into other GPUs' buffers: every storing thread makes its own stores visible system-wide before the
             // CTA can finish, so that the hand-shake kernel's flag (written by another SM, possibly over another link)
@@ -1000,9 +1004,9 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
 
         uint32_t seg = 0;
         bool aborted = false;                                              // a wait timed out (weight-streaming shapes)
-        if (C::kEpiWarps && warp >= kEpiWarp0 + 4 * kEpiGroups) {
+        if (warp >= kEpiWarp0 + 4 * kEpiGroups) {
             // (an epilogue warpgroup that this configuration does not use)
-        } else if (C::kEpiWarps && warp >= kEpiWarp0) {
+        } else if (warp >= kEpiWarp0) {
             // ----- dedicated epilogue warps: one pass per segment -----
             for (long long t = t_lo; t < t_hi;) {
                 const long long tile = div_nn(t, U);
@@ -1013,8 +1017,8 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                     ptx::grid_dependency_wait();                       // as in `epilogue`
                     const int col = (int)threadIdx.x & 127, scol = (int)tile * 128 + col;
                     const bool col_ok = scol < p.S;
-                    if (!early_epilogue(p.om, p.om.n_dst, p.om.ld, p.om.dst[0] + (col_ok ? p.om.col(scol) : 0), p.rows, col_ok ? p.rows : 0, p.accumulate,
-                                        u0 == 0 ? nullptr : reinterpret_cast<unsigned long long*>(p.partials) + (size_t)b * C::kSlotElems + col,
+                    if (!early_epilogue<NT>(p.om, p.om.n_dst, p.om.ld, p.om.dst[0] + (col_ok ? p.om.col(scol) : 0), p.rows, col_ok ? p.rows : 0, p.accumulate,
+                                        u0 == 0 ? nullptr : reinterpret_cast<uint4*>(p.partials) + (size_t)b * C::kSlotVecs + col,
                                         tmem_base, ptx::smem_u32(&bars.d_empty), ptx::smem_u32(const_cast<int*>(&s_abort)))) {
                         aborted = true;
                         break;
@@ -1087,9 +1091,9 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                 auto words = [&](const Unit& n, int h) -> uint32_t { return n.st + WS::kW + h * (F::WROWS * 512) + col * 4; };
                 auto masks = [&](const Unit& n, int h) -> uint32_t { return n.st + WS::kMask + h * (F::MROWS * 512) + col * 4; };
                 auto a_cols = [&](const Unit& n, int h) -> uint32_t { return lane_addr + C::kACol0 + n.as * C::kAStageCols + h * 32; };
-                // Fast mode: scale signs clear, zero-points integers in [0, 512] (sparse format: see SparseTable), for every column of the
+                // Fast mode: scale signs clear, zero-points integers in [0, 512] (16:32: see kFastBound), for every column of the
                 // warp in every group of the unit.
-                constexpr uint32_t kBound = SparseTable<SPARSE, NT>::kFastBound;
+                constexpr uint32_t kBound = kFastBound<SPARSE>;
                 // this warpgroup's units of the segment: those whose stage index is congruent to wg modulo kWG
                 for (int u = u0 + (int)(((uint32_t)wg + (uint32_t)C::kWG - si0 % (uint32_t)C::kWG) % (uint32_t)C::kWG); u < u1; u += C::kWG) {
                     Unit n;
@@ -1104,7 +1108,7 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                         // 16:32 52.4, int3 40.5, int2 37.3; now 35.9, 51.5, 39.1, 33.8.  General mode, which decoded twice: 66, 111, 79, 71; now
                         // 53, 86, 62, 63; every second group in the exponent coding: 176, 208, 180, 142; now 181, 194, 179, 126.  Not better: the parts
                         // as a loop of two iterations (36.8, 52.9, 41.6, 36.4); two warpgroups with 128 registers; an MMA warp, an accumulator and
-                        // half-stages for each warpgroup.  The shapes below, which wait for other things, do not gain: NT = 64 loses 2..6 %.)
+                        // half-stages for each warpgroup.  The shapes below, which wait for other things, do not gain.)
                         uint32_t sp[H / 2], zp[H / 2], zi[H / 2], nf = 0;           // two parts' scales, zero-points, zero-points + 1024
 #pragma unroll
                         for (int h = 0; h < H; h += 2) {
@@ -1232,8 +1236,6 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                     announce((int)n.as);
                 }
                 if (!ok) { aborted = true; break; }
-                if (!C::kEpiWarps && wg == 0) ok = epilogue(seg, tile);
-                ++seg;
                 si0 += (uint32_t)(u1 - u0);
                 t += u1 - u0;
             }
@@ -1407,16 +1409,16 @@ bool encode_x_blocks_cached(CUtensorMap* out, const void* base, uint64_t rows, u
     return true;
 }
 
-constexpr long long kPartialWords = 148LL * 4 * 32 * 128;      // 64-bit words of partial tiles in the workspace (capi.cu sizes it)
+constexpr long long kPartialBytes = 148LL * 4 * 32 * 128 * 8;      // for partial sums in the workspace (capi.cu sizes it)
 
-// More than 32 rows and tiles that fill less than half of the GPU: cut K into parts so that
+// More than 64 rows and tiles that fill less than half of the GPU: cut K into parts so that
 // tiles x parts CTAs (pairs) run, as long as every part keeps at least 4 stages and the partial outputs fit the scratch.
 int choose_kparts(long long capacity, long long tiles, int U, long long rows, long long S) {
     if (tiles <= 0 || tiles * 2 > capacity) return 1;
     long long f = capacity / tiles;
     if (f > 8) f = 8;
     if (f > U / 4) f = U / 4;
-    while (f > 1 && f * rows * S * 4 > kPartialWords * 8) --f;
+    while (f > 1 && f * rows * S * 4 > kPartialBytes) --f;
     return f < 2 ? 1 : (int)f;
 }
 
@@ -1466,28 +1468,19 @@ int launch_nt(const UmmaParams& p_in, const __half* x, int n_groups, cudaStream_
                         (!C::kEpiTransposed ? 0 : PAIR ? NT * 256 : 4096 * ((C::kEpiGroups == 2 && NT < 256) ? 2 : 1)) +
                         (PERM ? (size_t)C::kXStaging * kBStageBytes : 0);
     auto kern = umma_kernel<BITS, SPARSE, NT, PAIR, PERM>;
-    // per-device caches; atomics because two host threads may make their first call at once (both then compute the same values)
-    static std::atomic<int> ctas_per_sm[16];
+    // per-device cache; atomic because two host threads may make their first call at once (both then compute the same value)
     static std::atomic<int> sm_count[16];
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) { *cuda_err = e; return I4MM_ERR_LAUNCH; }
     dev &= 15;
-    if (ctas_per_sm[dev] == 0) {
+    if (sm_count[dev] == 0) {
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) { *cuda_err = e; return I4MM_ERR_LAUNCH; }
-        // CTAs per SM: what the launch bounds and the shared-memory budget were sized for, capped by the tensor
-        // memory (512 columns per SM).  The occupancy calculator is not used: it reports 1 for a kernel that
-        // allocates tensor memory, whatever amount the kernel asks for at run time.
-        int n = C::kMinBlocks, sms = 0;
+        int sms = 0;
         e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (e != cudaSuccess) { *cuda_err = e; return I4MM_ERR_LAUNCH; }
-        const int tmem_limit = 512 / C::kTmemCols;
-        if (n > tmem_limit) n = tmem_limit;
-        const int smem_limit = (int)((227 * 1024) / (smem + 2048));
-        if (n > smem_limit) n = smem_limit;
         sm_count[dev] = sms;
-        ctas_per_sm[dev] = n > 0 ? n : 1;
     }
     if (PAIR) {
         // clusters of two CTAs; as many as can be resident at once, each walking its share of the pair tiles
@@ -1530,12 +1523,12 @@ int launch_nt(const UmmaParams& p_in, const __half* x, int n_groups, cudaStream_
         return I4MM_OK;
     }
     const long long n_tiles = (long long)p.MTILES * p.CT;
-    long long grid = (long long)sm_count[dev] * ctas_per_sm[dev];
+    long long grid = sm_count[dev];                     // one CTA per SM: every configuration fills its shared or tensor memory
     if (!C::kSplit && !p.accumulate)
         p.kparts = choose_kparts(grid, n_tiles, p.U, p.rows, p.S);
     const long long work = p.kparts > 1 ? n_tiles * p.kparts : C::kSplit ? n_tiles * p.U : n_tiles;
     if (grid > work || p.kparts > 1) grid = work;
-    if (C::kSplit && grid > kPartialWords / C::kSlotElems) grid = kPartialWords / C::kSlotElems;   // one partial tile per CTA in the scratch
+    if (C::kSplit && grid > kPartialBytes / (C::kSlotVecs * 16)) grid = kPartialBytes / (C::kSlotVecs * 16);   // one partial tile per CTA in the scratch
     {
         // The kernel may start while the kernel before it in the stream is still running: its set-up overlaps that
         // kernel's tail, and with `overlap` so do its copies of the weight-side tensors (which the caller has declared

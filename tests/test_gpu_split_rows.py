@@ -1,4 +1,4 @@
-"""GPU parity tests of the few-row tcgen05 shapes (1..32 rows) where column tiles are shared: the owner of a tile sums its partners'
+"""GPU parity tests of the few-row tcgen05 shapes (1..64 rows) where column tiles are shared: the owner of a tile sums its partners'
 shares, with its epilogue warps alone or with every warpgroup, some rows each (dense int4 with up to 3 rows runs in another k order)."""
 import ctypes
 
@@ -63,7 +63,7 @@ def test_matvec_route_adds_into_outs_of_several_tiles_per_cta(fmt, batch):
     assert_parity(got[..., cols], want, bound, f"accumulate {fmt}")
 
 
-# shared tiles; whole tiles and shared ones; a few-row kernel's call (path 0) and K parts (48 rows), which store on their own
+# shared tiles; whole tiles and shared ones; a few-row kernel's call (path 0)
 @pytest.mark.parametrize("n,s", [(8256, 320), (512, 38400), (2048, 1024)])
 @pytest.mark.parametrize("m", [1, 2, 5, 16, 17, 32, 48])
 @pytest.mark.parametrize("path", [capi.PATH_AUTO, P])
@@ -88,3 +88,77 @@ def test_several_destinations_hold_the_same_bits(fmt, path, m, n, s):
     torch.cuda.synchronize()
     for b in bufs:
         assert torch.equal(b[:, :s], want[0]) and (b[:, s:] == 7.0).all()
+
+
+# 33..64 rows: every number of row groups per warpgroup (groups of 4 rows, ragged last ones), on the same sizes
+@pytest.mark.parametrize("n,s,g", [(16384, 64, 128), (8256, 320, 192), (2048, 2432, -1), (2048, 9536, 64), (512, 38400, 128)])
+@pytest.mark.parametrize("m", [33, 36, 47, 48, 49, 61, 64])
+@pytest.mark.parametrize("fmt", FORMATS, ids=fmt_id)
+def test_shared_tiles_of_33_to_64_rows(fmt, m, n, s, g):
+    bits, sparse = fmt
+    p = oracle.make_packed_problem(bits, n, s, m, g, sparse=sparse, seed=n + s + m)
+    got = run_problem(p, path=P)
+    assert capi.load().i4mm_last_launch_shape() == 64
+    cols = np.unique(np.concatenate([np.arange(64), s - 1 - np.arange(64), np.random.default_rng(m).integers(0, s, 60)]))
+    want, bound = oracle.expected_columns(bits, p["matrix"], p["mask"], p["scales"], p["zeros"], g, p["x"], cols)
+    assert_parity(got[..., cols], want, bound, f"{fmt} m={m} {n}x{s} g{g}")
+    again = run_problem(p, path=P)
+    assert np.array_equal(got.view(np.uint16), again.view(np.uint16))
+    ws = ops.workspace(torch.device("cuda", torch.cuda.current_device()), torch.cuda.current_stream())
+    assert int(ws.count_nonzero()) == 0
+
+
+@pytest.mark.parametrize("n,s", [(512, 38400), (4096, 192)])
+@pytest.mark.parametrize("batch", [33, 50, 64])
+def test_matvec_route_adds_33_to_64_rows_into_outs(batch, n, s):
+    p = oracle.make_packed_problem(4, n, s, 1, 64, batch=batch, seed=43)
+    base = np.random.default_rng(4).standard_normal((batch, 1, s)).astype(np.float16)
+    got = run_problem(p, path=P, outs_in=base, route="vec")
+    cols = np.unique(np.concatenate([np.arange(0, s, 128), np.arange(63, s, 64)]))
+    want, bound = oracle.expected_columns(4, p["matrix"], p["mask"], p["scales"], p["zeros"], 64, p["x"], cols,
+                                          outs_in=np.ascontiguousarray(base[..., cols]))
+    assert_parity(got[..., cols], want, bound, f"accumulate {batch} {n}x{s}")
+
+
+@pytest.mark.parametrize("m", [1, 4, 7, 16, 32, 50])
+def test_partial_sums_of_zero_infinity_and_nan_are_delivered(m):
+    """A shared tile's partial sums travel as words that are never zero: rows of zeros (of either sign), infinities and NaN."""
+    n, s = 8192, 320
+    p = oracle.make_packed_problem(4, n, s, m, 128, seed=m)
+    p["zeros"][:] = 8                                                 # no weight row is all of one sign
+    x = p["x"]
+    for row in range(m):
+        kind = (row + (m == 1)) % 5
+        if kind == 0:
+            x[0, row] = 0.0
+        elif kind == 1:
+            x[0, row] = -0.0
+        elif kind == 2:
+            x[0, row, n // 2] = np.inf
+        elif kind == 3:
+            x[0, row, 3] = np.nan
+    got = run_problem(p, path=P, route="mtx")[0]
+    want, bound = oracle.expected_columns(4, p["matrix"], p["mask"], p["scales"], p["zeros"], 128, x, np.arange(s))
+    for row in range(m):
+        kind = (row + (m == 1)) % 5
+        if kind <= 1:
+            assert not got[row].any()
+        elif kind == 3:
+            assert np.isnan(got[row]).all()
+        elif kind == 2:
+            assert np.array_equal(np.isnan(got[row]), np.isnan(want[0, row])) and np.array_equal(np.isposinf(got[row]), np.isposinf(want[0, row]))
+        else:
+            assert_parity(got[None, row:row + 1], want[:, row:row + 1], bound[:, row:row + 1], f"row {row}")
+    ops.check_device_status()
+    ws = ops.workspace(torch.device("cuda", torch.cuda.current_device()), torch.cuda.current_stream())
+    assert int(ws.count_nonzero()) == 0
+
+
+@pytest.mark.parametrize("m", [1, 5, 32])
+def test_the_streaming_path_leaves_the_scratch_to_the_other_kernels(m):
+    p = oracle.make_packed_problem(4, 8192, 320, m, 128, seed=m)
+    want = run_problem(p, path=P)
+    assert_parity(run_problem(p, path=capi.PATH_STREAM), want, np.full(want.shape, np.abs(want.astype(np.float32)).max()), "streaming path")
+    ws = ops.workspace(torch.device("cuda", torch.cuda.current_device()), torch.cuda.current_stream())
+    assert int(ws.count_nonzero()) == 0
+    assert np.array_equal(run_problem(p, path=P).view(np.uint16), want.view(np.uint16))
