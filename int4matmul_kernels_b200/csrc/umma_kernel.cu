@@ -20,7 +20,7 @@
 //                     rows (a CTA's last tile: from 2 rows on the dequant warpgroups as well, see last_epilogue), two warpgroups
 //                     of their own (half of the columns each) above
 //
-// Configurations (Cfg<NT, PAIR>), one CTA per SM: NT <= 64 rows stream the weights once from HBM - 3 dequant warpgroups, 9 (6)
+// Configurations (Cfg<NT, PAIR, STREAM>), one CTA per SM: NT <= 64 rows stream the weights once from HBM - 3 dequant warpgroups, 9 (6)
 // weight stages and 3 A / activation stages of 256 k, and the (tile, unit) space cut into equal ranges per CTA (split-K over the
 // whole GPU, partial tiles summed through scratch in a fixed order).  NT >= 128: whole tiles, epilogue stores transposed through
 // shared memory; by default launched as clusters of two CTAs that run each MMA together (cta_group::2, M = 256 over two SMs), see
@@ -58,6 +58,7 @@ struct UmmaParams {
     int CT;              // column tiles: ceil(S / 128)
     int MTILES;          // row tiles: ceil(rows / NT)
     int accumulate;
+    int whole_tiles;     // no tile is shared (weight-streaming shapes), nor K cut into parts (the others)
     int overlap;         // weight-side tensors may be read while the kernel before this one is still running
     int kparts;          // > 1: every tile's K range is cut into this many parts, one CTA (pair) each, fp32 partial outputs
                          // go to the scratch as (part, row, S) and kparts_reduce_kernel sums them (more than 64 rows only)
@@ -204,7 +205,7 @@ constexpr int kMaxABStages = 6;
 template <bool SPARSE>
 constexpr uint32_t kFastBound = SPARSE ? 0x280Fu : 0x1FFFu;
 
-template <int NT, bool PAIR>
+template <int NT, bool PAIR, bool STREAM = NT <= 64>
 struct Cfg {
     // packed-weight ring (128 k per stage).  Few rows: the kernel streams weights from HBM, and the ring has to
     // cover the DRAM latency; many rows: weights are a trickle next to the activation tiles
@@ -212,11 +213,11 @@ struct Cfg {
     // of 64 rows at two CTAs an SM, whole or with K cut into parts and a second launch: 48 rows 13824 x 5120 int4 25.7 us, now 18.8,
     // 16:32 38.1 / 22.0, int3 34.0 / 18.7, int2 33.1 / 17.4; 5120 x 20480 55.8 / 22.9, 53.8 / 29.7, 43.4 / 23.5, 42.7 / 22.4; 16384 x 16384
     // 66.3 / 44.3, 76.9 / 56.7, 59.9 / 43.5, 62.3 / 39.0; 1024 x 1024 8.9 / 7.8, 9.6 / 8.2, 9.0 / 7.8, 9.0 / 7.8; nothing was faster there.
-    static constexpr bool kStream = NT <= 64;
+    static constexpr bool kStream = STREAM;
     // NT = 128..192: an MMA of N <= 192 takes 512..768 cycles per 128 k, the dequantisation of its weights with two
     // warpgroups ~1400, so these shapes get four warpgroups as well, and a deeper weight ring
     // (single CTAs have the shared memory for the 4 A / activation stages that four warpgroups need only at NT = 128)
-    static constexpr bool kDequantBound = NT == 128 || (PAIR && NT >= 128 && NT <= 192);
+    static constexpr bool kDequantBound = !STREAM && (NT == 128 || (PAIR && NT >= 128 && NT <= 192));
     // A stage of either ring is waited for by parity, which tells a completed phase only from the one before it.
     // Where the weight stages are not a multiple of the warpgroups, consecutive uses of a stage belong to different
     // warpgroups, and one could poll for a stage's next fill while the previous one, meant for another warpgroup, has
@@ -227,19 +228,19 @@ struct Cfg {
     // whose loops cost ~500 cycles per stage whatever its size (an mbarrier wait ~190 cycles even when it is already
     // complete, expect_tx + the copy's issue another ~190): at 128 k per stage that alone is ~27 us for 16384 x 16384
     // weights on 148 SMs, so the weight-streaming shapes use 256-k units.
-    static constexpr int kHalves = kStream ? 4 : 2;
-    static constexpr int kWStages = kStream ? (NT <= 16 ? 9 : 6) : kDequantBound ? 6 : 3;
+    static constexpr int kHalves = NT <= 64 ? 4 : 2;
+    static constexpr int kWStages = kStream ? (NT <= 16 || NT == 128 ? 9 : 6) : kDequantBound ? 6 : 3;
     // staging slots (units of look-ahead) for activation rows that are reordered on their way into the A / activation
     // stages (umma_kernel's PERM)
     static constexpr int kXStaging = 4;
     static constexpr int kWG = kStream ? 3 : kDequantBound ? 4 : 2;   // dequant warpgroups (4 warps each), taking units in turn
-    static constexpr int kABStages = kStream ? 3 : NT == 128 ? 4 : 3;   // ring of (A in tensor memory, activation tile in shared memory) pairs, one unit per stage
+    static constexpr int kABStages = NT == 128 ? 4 : 3;   // ring of (A in tensor memory, activation tile in shared memory) pairs, one unit per stage
     static constexpr bool kWGuard = kWStages % kWG != 0;
-    static constexpr bool kEpiTransposed = NT >= 128;                 // epilogue stores go through a shared-memory transposition tile
+    static constexpr bool kEpiTransposed = !kStream;                 // epilogue stores go through a shared-memory transposition tile
     static constexpr bool kEpiHandoff = kStream;                      // the MMA warp waits for the accumulator and wakes the epilogue warps (named barrier)
     // many rows: two epilogue warpgroups, each draining half of the accumulator's columns, so that the next tile's
     // MMAs wait half as long for the accumulator
-    static constexpr int kEpiGroups = NT >= 128 ? 2 : 1;
+    static constexpr int kEpiGroups = kStream ? 1 : 2;
     // The weight-streaming shapes have two weight-producer threads (in two warps) that fill the stages in turn: one
     // thread's loop (wait ~190 cycles, expect_tx + copies ~250) delivers a 16 KB stage per ~500-700 cycles, about
     // 4-5 TB/s over the whole GPU, which is less than the memory system can stream.
@@ -247,27 +248,29 @@ struct Cfg {
     static constexpr int kWarps = 4 * kWG + 4 * kEpiGroups + 3 + (kWProducers - 1);  // + weight producer(s), activation producer, MMA issuer
     static constexpr int kThreads = kWarps * 32;
     static constexpr int kDCols = NT < 32 ? 32 : NT;                  // accumulator columns
-    static constexpr int kACol0 = kDCols;                             // A stages follow: 32 columns per 64 k
+    static constexpr int kDBufs = kStream && NT == 128 ? 2 : 1;       // accumulators, used by the tiles in turn
+    static constexpr int kACol0 = kDBufs * kDCols;                             // A stages follow: 32 columns per 64 k
     static constexpr int kAStageCols = 32 * kHalves;
-    static constexpr int kColsUsed = kDCols + kAStageCols * kABStages;
+    static constexpr int kColsUsed = kACol0 + kAStageCols * kABStages;
     static constexpr int kTmemCols = kColsUsed <= 256 ? 256 : 512;
     // split-K over CTAs with a scratch reduction (more rows cut K into parts, see choose_kparts)
     static constexpr bool kSplit = kStream;
     static constexpr int kSlotVecs = NT / 4 * 128;                    // one CTA's partial tile in the scratch: [4 rows][128 columns] of 16 bytes
+    static constexpr int kSlots = NT <= 32 ? 1 : 2;                   // of those per CTA, see last_epilogue
 };
 
 // A / activation stages.  A CTA of a pair holds only half of each activation tile, which leaves shared memory for as
 // many stages as tensor memory has columns for (accumulator + 64 per stage <= 512).
-template <int NT, bool PAIR>
+template <int NT, bool PAIR, bool STREAM>
 struct ABStages {
-    static constexpr int value = !PAIR ? Cfg<NT, false>::kABStages : (Cfg<NT, true>::kDCols + 64 * 5 <= 512 ? 5 : 4);   // pairs: 128-k units
+    static constexpr int value = !PAIR ? Cfg<NT, false, STREAM>::kABStages : (Cfg<NT, true>::kDCols + 64 * 5 <= 512 ? 5 : 4);   // pairs: 128-k units
 };
 
 struct Barriers {
     unsigned long long w_full[kMaxWStages], w_empty[kMaxWStages];
     unsigned long long ab_full[kMaxABStages];  // 4 dequant warps + the activation producer (with its transaction bytes)
     unsigned long long ab_free[kMaxABStages];  // tcgen05.commit: the MMAs that read the stage are done
-    unsigned long long d_full, d_empty;
+    unsigned long long d_full, d_empty[2];     // d_empty: one per accumulator
 };
 
 struct TensorMaps {
@@ -280,7 +283,8 @@ struct TensorMaps {
 };
 
 // Rows 0 .. n - 1 of one column to every destination (out0: the first row in the first one).  The first destination's stores are
-// predicated, without the branch and the loop over destinations per row (5120 x 20480 int4, 32 rows: 24.9 -> 23.5 us).
+// predicated, without the branch and the loop over destinations per row (5120 x 20480 int4, 32 rows: 24.9 -> 23.5 us).  (Rows and columns changing
+// places among eight lanes, so that a store is 16 bytes, was no faster: 72 rows 2048 x 16384 int4 13.2 / 13.1 us, but 16 rows 9.8 / 10.2.)
 template <int RB>
 __device__ __forceinline__ void store_rows(const OutMap& om, __half* out0, long long ld, int n_dst, const __half (&h)[RB], int n) {
 #pragma unroll
@@ -298,8 +302,8 @@ __device__ __forceinline__ void store_rows(const OutMap& om, __half* out0, long 
 // which owns its first units and reaches them last, adds the others' partial tiles to its own accumulator in CTA order - a fixed
 // order, so results are reproducible; the others wait for nobody.  A partial sum is a 32-bit word that is never zero (share_word), four rows of
 // a column in one 16-byte store, so no fence, counter or second round trip is needed: a reader knows each word by itself, and clears
-// what it has read, which leaves the scratch all-zero for the next launch.  One slot per CTA is enough: a CTA has at most one
-// tile that it shares and does not sum.  A tile that a CTA sums is its last one, so there are two functions.
+// what it has read, which leaves the scratch all-zero for the next launch.  A CTA has at most one
+// tile that it shares and goes on from, before its last one, so there are two functions.
 // What a thread waits for are its loads, so fewer and wider ones count: with one 64-bit word (value | tag) per row, int4 16 rows 20480 x 5120
 // 22.3 us, now 19.7; 5120 x 5120 13.2 / 10.2; 16384 x 2048 17.0 / 12.4; 32 rows 25.1 / 21.1, 15.6 / 11.7, 20.4 / 14.9; one row 18.4 / 17.7, 10.3 / 9.7,
 // 12.7 / 11.5.
@@ -313,8 +317,8 @@ __device__ __forceinline__ float share_value(uint32_t w) { return __uint_as_floa
 // out0: the column's first output; rows / out_rows: rows of the launch, and those that this lane stores.
 template <int NT>
 __device__ __noinline__ bool early_epilogue(const OutMap& om, int n_dst, long long ld, __half* out0, int rows, int out_rows, int accumulate,
-                                            uint4* share, uint32_t tmem_base, uint32_t d_empty, uint32_t s_abort) {
-    const uint32_t lane_addr = tmem_base + ((threadIdx.x & 96u) << 16);
+                                            uint4* share, uint32_t acc, uint32_t bar_id, uint32_t d_empty, uint32_t s_abort) {
+    const uint32_t lane_addr = acc + ((threadIdx.x & 96u) << 16);
     auto release = [&]() {
         ptx::tc_fence_before_sync();
         __syncwarp();
@@ -329,7 +333,7 @@ __device__ __noinline__ bool early_epilogue(const OutMap& om, int n_dst, long lo
         }
     };
     if (!share) load_old(0);
-    ptx::named_bar_sync(2, 128 + 32);              // released by the MMA warp once the accumulator is complete
+    ptx::named_bar_sync(bar_id, 128 + 32);         // released by the MMA warp once the accumulator is complete
     if (ptx::lds32(s_abort)) return false;
     ptx::tc_fence_after_sync();
     if (share) {
@@ -346,7 +350,7 @@ __device__ __noinline__ bool early_epilogue(const OutMap& om, int n_dst, long lo
         }
         return true;
     }
-    if (NT > 32 && !accumulate) {
+    if (NT == 64 && !accumulate) {
         // converted and held in registers, so that the accumulator is free before the stores
         uint32_t h2[NT / 2];
 #pragma unroll
@@ -399,142 +403,200 @@ __device__ __noinline__ bool early_epilogue(const OutMap& om, int n_dst, long lo
     return true;
 }
 
-// A CTA's last tile: units t0 .. t0 + units - 1.  What bounds it is the number of dependent round trips to L2 (~0.7 us each) between
-// the last MMA and the end of the launch, so the tile can be left to all of the CTA's warpgroups (the dequant warps have nothing
-// else to do by then), `part` of `parts` of its groups of four rows each; a thread has its groups of up to 4 partners in flight (33..64 rows: of 2,
-// with 4 the registers spill: 48 rows 5120 x 5120 12.9 us, 16.2).
-// (When: see spread_last.)
+// Adds the shares of n partners, PB at a time, to the sums of NG groups of four rows (the first `here` of them are there) and clears them.
+// at(k, j): partner k's words of group j.  NG x PB loads are in flight, and everything that is missing is asked for again at once: word by word
+// each would cost a round trip of its own.
+template <int NG, int PB, class At>
+__device__ __forceinline__ void add_shares(float (&sum)[4 * NG], int n, int here, int* status, bool& waiting_ok, At at) {
+#pragma unroll 1
+    for (int q = 0; q < n; q += PB) {
+        uint4 w[PB][NG];
+        auto missing = [&](int k, int j) -> bool {
+            return q + k < n && j < here && (w[k][j].x == 0u || w[k][j].y == 0u || w[k][j].z == 0u || w[k][j].w == 0u);
+        };
+#pragma unroll
+        for (int k = 0; k < PB; ++k)
+#pragma unroll
+            for (int j = 0; j < NG; ++j) w[k][j] = make_uint4(0, 0, 0, 0);
+        for (uint32_t spins = 0; waiting_ok; ++spins) {
+#pragma unroll
+            for (int k = 0; k < PB; ++k)
+#pragma unroll
+                for (int j = 0; j < NG; ++j)
+                    if (missing(k, j)) w[k][j] = ptx::ld_relaxed_gpu_v4(at(q + k, j));
+            bool any = false;
+#pragma unroll
+            for (int k = 0; k < PB; ++k)
+#pragma unroll
+                for (int j = 0; j < NG; ++j) any |= missing(k, j);
+            if (!any) break;
+            if (spins >= ptx::kSpinLimit) {                    // a contributor never delivered: report, stop waiting
+                atomicExch(status, 34);
+                waiting_ok = false;
+            }
+            __nanosleep(20);
+        }
+#pragma unroll
+        for (int k = 0; k < PB; ++k)
+#pragma unroll
+            for (int j = 0; j < NG; ++j)
+                if (q + k < n && j < here) {
+                    const uint4 x = w[k][j];
+                    sum[4 * j] += share_value(x.x);
+                    sum[4 * j + 1] += share_value(x.y);
+                    sum[4 * j + 2] += share_value(x.z);
+                    sum[4 * j + 3] += share_value(x.w);
+                    ptx::st_relaxed_gpu_v4(at(q + k, j), make_uint4(0, 0, 0, 0));
+                }
+    }
+}
+
+// A CTA's last tile: units t0 .. t0 + units - 1.  What bounds it is the number of dependent round trips to L2 (~0.7 us each) and the words a
+// CTA reads between the last MMA and the end of the launch, so the tile can be left to all of the CTA's warpgroups (the dequant warps
+// have nothing else to do by then), `part` of `parts` of its groups of four rows each.  (When: see spread_last.)
+// Up to 32 rows b_lo sums the tile, with 4 partners' words a thread in flight.  More rows are too many words for one CTA (128 rows
+// 5120 x 5120 int4: the sum took 14 of the launch's 34 K cycles on 40 of the GPU's SMs, now 6 K): there all CTAs whose last tile it is - all that
+// share it but one that goes on to the next tile, whose share came early - sum some groups each; a CTA writes its sums of the others'
+// groups and adds theirs to its own.  (us, b_lo alone / all: int4 48 rows 13824 x 5120 18.3 / 17.3, 128 rows 26.2 / 22.0, 5120 x 5120
+// 19.4 / 15.6; but 16 rows 2048 x 8192 8.7 / 9.3, 5120 x 6976 11.3 / 11.9.)
 // bar_id, bar_threads: the named barrier at which the MMA warp says that the accumulator is complete (once per call, also where this
 // part has no rows).  Inlined: a call cost ~1 us here as well.
+// The CTAs that share it, and how many of them, from b_lo on, sum it
+struct TileCtas {
+    int b_lo, b_hi, members;
+};
 template <int NT>
-__device__ __forceinline__ bool last_epilogue(const UmmaParams& p, uint32_t tmem_base, const volatile int* s_abort, long long t0, int units,
-                                              int part, int parts, uint32_t bar_id, uint32_t bar_threads) {
-    // outputs, old outputs and the scratch may still be in use by the kernel before this one in the stream
-    ptx::grid_dependency_wait();
-    const int warp = (int)(threadIdx.x >> 5), lane = threadIdx.x & 31;
-    const long long U = p.U, G = gridDim.x, tile = div_nn(t0, U);
-    const int u0 = (int)(t0 - tile * U), u1 = u0 + units;
-    const int col = (warp & 3) * 32 + lane, scol = (int)tile * 128 + col;
-    const bool col_ok = scol < p.S;
-    const int me = (int)blockIdx.x, groups = (p.rows + 3) / 4, g0 = groups * part / parts, ng = groups * (part + 1) / parts - g0;
-    const int r0 = 4 * g0, n = min(4 * ng, p.rows - r0);                  // this part's rows
-    const uint32_t acc = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + r0;
-    int b_lo = me, b_hi = me;
-    if (u0 != 0 || u1 != (int)U) {
-        const long long T = p.CT * U, lo_t = tile * U;
-        b_lo = range_owner(T, G, lo_t);
-        b_hi = range_owner(T, G, lo_t + U - 1);
-    }
-    uint4* const slot0 = reinterpret_cast<uint4*>(p.partials) + g0 * 128 + col;
-    auto slot_of = [&](int bb) { return slot0 + (size_t)bb * Cfg<NT, false>::kSlotVecs; };
+__device__ __forceinline__ bool last_epilogue(const OutMap& om, int n_dst, long long ld, __half* out, bool col_ok, int rows, int accumulate, uint4* slots, int* status,
+                                           TileCtas ctas, uint32_t acc, int part, int parts, uint32_t bar_id, uint32_t bar_threads, uint32_t s_abort) {
+    constexpr bool kAll = NT > 32;                             // every CTA whose last tile it is sums some groups
+    const int b_lo = ctas.b_lo, b_hi = ctas.b_hi, members = ctas.members, me = (int)blockIdx.x, groups = (rows + 3) / 4;
+    // A CTA's slot, or two: its share of the tile that it shares and goes on from, and the one of its last tile.
+    auto slot_of = [&](int bb) { return slots + (size_t)(kAll ? 2 * bb + (bb < b_lo + members ? 1 : 0) : bb) * Cfg<NT, false, true>::kSlotVecs; };
     auto wait_accumulator = [&]() -> bool {
         __syncwarp();
         ptx::named_bar_sync(bar_id, bar_threads);      // released by the MMA warp once the accumulator is complete
-        if (*s_abort) return false;
+        if (ptx::lds32(s_abort)) return false;
         ptx::tc_fence_after_sync();
         return true;
     };
-    constexpr int kMaxGroups = NT <= 32 ? 2 : NT / 16;
-    if (me != b_lo) {
-        if (!wait_accumulator()) return false;
-        uint4* const mine = slot_of(me);
-#pragma unroll
-        for (int j = 0; j < kMaxGroups; ++j) {
-            uint32_t v[4];
-            if (j < ng) {
-                ptx::tmem_ld4(acc + 4 * j, v);
-                ptx::tc_wait_ld();
-                ptx::st_relaxed_gpu_v4(mine + j * 128, make_uint4(share_word(v[0]), share_word(v[1]), share_word(v[2]), share_word(v[3])));
-            }
-        }
-        return true;
-    }
-    __half* const out0 = p.om.dst[0] + (col_ok ? p.om.col(scol) : 0) + (size_t)r0 * p.om.ld;
+    auto share_group = [&](const uint32_t* v) { return make_uint4(share_word(v[0]), share_word(v[1]), share_word(v[2]), share_word(v[3])); };
     bool waiting_ok = true;
-    // all of this part's groups (ng <= NG), the partners PB at a time: NG x PB loads in flight
-    auto finish = [&](auto ng_tag, auto pb_tag) -> bool {
+    // groups g .. g + NG - 1 up to g_end: partners' shares + accumulator + old outputs -> outputs
+    auto finish = [&](auto ng_tag, auto pb_tag, int g, int g_end, bool& ready) -> bool {
         constexpr int NG = decltype(ng_tag)::value, PB = decltype(pb_tag)::value;
+        const int here = g_end - g, n = min(4 * here, rows - 4 * g);
+        __half* const out0 = out + (size_t)(4 * g) * ld;
         float sum[4 * NG];
         __half old[4 * NG];
 #pragma unroll
         for (int i = 0; i < 4 * NG; ++i) {
             sum[i] = 0.f;
             old[i] = __ushort_as_half(0);
-            if (p.accumulate && i < n && col_ok) old[i] = out0[(size_t)i * p.om.ld];
+            if (accumulate && i < n && col_ok) old[i] = out0[(size_t)i * ld];
         }
-#pragma unroll 1
-        for (int q = b_lo + 1; q <= b_hi; q += PB) {
-            uint4 w[PB][NG];
-#pragma unroll
-            for (int k = 0; k < PB; ++k)
-#pragma unroll
-                for (int j = 0; j < NG; ++j)
-                    if (q + k <= b_hi && j < ng) w[k][j] = ptx::ld_relaxed_gpu_v4(slot_of(q + k) + j * 128);
-#pragma unroll
-            for (int k = 0; k < PB; ++k)
-#pragma unroll
-                for (int j = 0; j < NG; ++j)
-                    if (q + k <= b_hi && j < ng) {
-                        uint4& x = w[k][j];
-                        for (uint32_t spins = 0; (x.x == 0u || x.y == 0u || x.z == 0u || x.w == 0u) && waiting_ok; ++spins) {
-                            if (spins >= ptx::kSpinLimit) {            // a contributor never delivered: report, stop waiting
-                                atomicExch(p.status, 34);
-                                waiting_ok = false;
-                                break;
-                            }
-                            __nanosleep(20);
-                            x = ptx::ld_relaxed_gpu_v4(slot_of(q + k) + j * 128);
-                        }
-                        sum[4 * j] += share_value(x.x);
-                        sum[4 * j + 1] += share_value(x.y);
-                        sum[4 * j + 2] += share_value(x.z);
-                        sum[4 * j + 3] += share_value(x.w);
-                        ptx::st_relaxed_gpu_v4(slot_of(q + k) + j * 128, make_uint4(0, 0, 0, 0));
-                    }
-        }
-        if (!wait_accumulator()) return false;
+        // (b_lo .. b_hi without this CTA)
+        add_shares<NG, PB>(sum, b_hi - b_lo, here, status, waiting_ok,
+                           [&](int k, int j) { return slot_of(b_lo + k + (!kAll || b_lo + k >= me ? 1 : 0)) + (g + j) * 128; });
+        if (!ready && !wait_accumulator()) return false;
+        ready = true;
         __half h[4 * NG];
 #pragma unroll
         for (int j = 0; j < NG; ++j) {
             uint32_t v[4] = {0u, 0u, 0u, 0u};
-            if (j < ng) {
-                ptx::tmem_ld4(acc + 4 * j, v);
+            if (j < here) {
+                ptx::tmem_ld4(acc + 4 * (g + j), v);
                 ptx::tc_wait_ld();
             }
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 float f = __uint_as_float(v[i]) + sum[4 * j + i];
-                if (p.accumulate) f += __half2float(old[4 * j + i]);
+                if (accumulate) f += __half2float(old[4 * j + i]);
                 h[4 * j + i] = __float2half_rn(f);
             }
         }
-        store_rows<4 * NG>(p.om, out0, p.om.ld, p.om.n_dst, h, col_ok ? n : 0);
+        store_rows<4 * NG>(om, out0, ld, n_dst, h, col_ok ? n : 0);
         return true;
     };
-    if (NT <= 32 && ng <= 1) {
-        if (!finish(std::integral_constant<int, 1>(), std::integral_constant<int, 4>())) return false;
+    using std::integral_constant;
+    if constexpr (!kAll) {
+        const int g = groups * part / parts, g_end = groups * (part + 1) / parts;
+        if (me != b_lo) {
+            if (!wait_accumulator()) return false;
+#pragma unroll
+            for (int j = 0; j < 2; ++j)                        // (NT / 16 groups a part, 2 where the epilogue warps have up to 6 rows)
+                if (g + j < g_end) {
+                    uint32_t v[4];
+                    ptx::tmem_ld4(acc + 4 * (g + j), v);
+                    ptx::tc_wait_ld();
+                    ptx::st_relaxed_gpu_v4(slot_of(me) + (g + j) * 128, share_group(v));
+                }
+            return true;
+        }
+        bool ready = false;
+        if (g_end - g <= 1) {
+            if (!finish(integral_constant<int, 1>(), integral_constant<int, 4>(), g, g_end, ready)) return false;
+        } else {
+            if (!finish(integral_constant<int, 2>(), integral_constant<int, 4>(), g, g_end, ready)) return false;
+        }
     } else {
-        if (!finish(std::integral_constant<int, kMaxGroups>(), std::integral_constant<int, NT <= 32 ? 4 : 2>())) return false;
+        // this CTA's groups [lo, hi); of those, this part's
+        const int rank = me - b_lo, lo = (groups * rank + members - 1) / members, hi = (groups * (rank + 1) + members - 1) / members;
+        const int g_end = lo + (hi - lo) * (part + 1) / parts;
+        int g = lo + (hi - lo) * part / parts;
+        bool ready = false;
+        if (hi - lo < groups) {
+            if (!wait_accumulator()) return false;
+            ready = true;
+            const int end = groups * (part + 1) / parts;
+#pragma unroll 1
+            for (int j = groups * part / parts; j < end; j += 2) {
+                uint32_t v[8];
+                ptx::tmem_ld8(acc + 4 * j, v);
+                ptx::tc_wait_ld();
+#pragma unroll
+                for (int k = 0; k < 2; ++k)
+                    if (j + k < end && (j + k < lo || j + k >= hi)) ptx::st_relaxed_gpu_v4(slot_of(me) + (j + k) * 128, share_group(v + 4 * k));
+            }
+        }
+        // (once at least: every part meets the MMA warp)
+        if (b_hi - b_lo <= 2) {
+            do {
+                if (!finish(integral_constant<int, 4>(), integral_constant<int, 2>(), g, g_end, ready)) return false;
+            } while ((g += 4) < g_end);
+        } else {
+            do {
+                if (!finish(integral_constant<int, 2>(), integral_constant<int, 4>(), g, g_end, ready)) return false;
+            } while ((g += 2) < g_end);
+        }
     }
-    if (p.om.n_dst > 1) __threadfence_system();                // as in umma_kernel's epilogue
+    if (n_dst > 1) __threadfence_system();                // as in umma_kernel's epilogue
     return true;
+}
+
+// The same as a call of its own.  Which form an instance takes is a matter of the decode loop's registers: up to 32 rows it is faster without the
+// inlined form beside it (us, inlined / called: one row 16384 x 16384 16:32 52.7 / 50.5, int3 39.4 / 38.6, 16 rows int4 38.6 / 37.8), but with the
+// permuted k order (one row int4 35.5 / 37.0) and more rows, whose call keeps more registers (48 rows 5120 x 6976 int4 13.3 / 15.5).
+template <int NT>
+__device__ __noinline__ bool last_epilogue_call(const OutMap& om, int n_dst, long long ld, __half* out, bool col_ok, int rows, int accumulate, uint4* slots, int* status,
+                                                TileCtas ctas, uint32_t acc, int part, int parts, uint32_t bar_id, uint32_t bar_threads, uint32_t s_abort) {
+    return last_epilogue<NT>(om, n_dst, ld, out, col_ok, rows, accumulate, slots, status, ctas, acc, part, parts, bar_id, bar_threads, s_abort);
 }
 
 // PAIR: launched as clusters of two CTAs (two SMs) that run every MMA together (cta_group::2, M = 256): the pair's
 // tile is 256 weight columns x NT rows, each CTA dequantises its own 128 columns and loads only half of the rows of
 // the activation tile, which halves the L2 -> shared-memory traffic that bounds the many-row shapes.
 // PERM (up to 3 rows of dense int4 only): the cheaper k order of UFormat, with the activations reordered to match.
-template <int BITS, bool SPARSE, int NT, bool PAIR, bool PERM = false>
-__global__ void __launch_bounds__(Cfg<NT, PAIR>::kThreads, 1)
+template <int BITS, bool SPARSE, int NT, bool PAIR, bool PERM = false, bool STREAM = NT <= 64>
+__global__ void __launch_bounds__(Cfg<NT, PAIR, STREAM>::kThreads, 1)
 umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaParams p, const __half* x) {
-    using C = Cfg<NT, PAIR>;
+    using C = Cfg<NT, PAIR, STREAM>;
     using F = UFormat<BITS, SPARSE, PERM>;
     static_assert(!PERM || (C::kStream && F::kPermutedK), "the permuted k order is for dense int4 weight streaming");
     constexpr int H = C::kHalves;                                    // 64-k parts per unit
     using WS = WStage<F, H>;
     static_assert(!PAIR || (NT >= 128 && !C::kEpiHandoff), "CTA pairs are for the many-row shapes");
     static_assert((2 * C::kWStages) % C::kWG == 0, "every second use of a weight stage must be by the same warpgroup");
-    static_assert(ABStages<NT, PAIR>::value >= C::kWG, "fewer A stages than warpgroups: a parity wait could see the phase before last");
+    static_assert(ABStages<NT, PAIR, STREAM>::value >= C::kWG, "fewer A stages than warpgroups: a parity wait could see the phase before last");
     constexpr int kBHalfBytes = (PAIR ? NT / 2 : NT) * 128;        // one 64-k activation sub-tile held by this CTA
     constexpr int kBStageBytes = H * kBHalfBytes;
     // single CTAs at NT = 256 have no shared memory left for a second transposition tile: the second epilogue group idles
@@ -542,7 +604,7 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
     constexpr int kEpiWarp0 = 4 * C::kWG;                           // first epilogue warp (a multiple of 4: lane quarter = warp % 4)
     constexpr int kWProducer = kEpiWarp0 + 4 * C::kEpiGroups, kBProducer = kWProducer + 1, kMma = kWProducer + 2;
     constexpr int kWProducer2 = kWProducer + 3;                     // only when Cfg::kWProducers == 2
-    constexpr int kABStages = ABStages<NT, PAIR>::value;
+    constexpr int kABStages = ABStages<NT, PAIR, STREAM>::value;
     extern __shared__ __align__(1024) unsigned char smem[];      // [B ring (1024-aligned tiles)][W ring]
     __shared__ __align__(8) Barriers bars;
     __shared__ uint32_t lut[SPARSE ? kSparseLutEntries : 1];
@@ -585,7 +647,8 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
             }
             if (lane == 31) {
                 ptx::mbar_init(ptx::smem_u32(&bars.d_full), 1);
-                ptx::mbar_init(ptx::smem_u32(&bars.d_empty), (PAIR ? 8 : 4) * kEpiGroups);
+                ptx::mbar_init(ptx::smem_u32(&bars.d_empty[0]), (PAIR ? 8 : 4) * kEpiGroups);
+                ptx::mbar_init(ptx::smem_u32(&bars.d_empty[1]), 4);
                 s_abort = 0;
             }
             ptx::fence_mbar_init();
@@ -624,7 +687,7 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
     auto tile_mt = [&](long long tile) -> int { return (int)(tile / CTd); };
     long long t_lo, t_hi;
     const int kpart = p.kparts > 1 ? (int)(b % p.kparts) : 0;
-    if (C::kSplit) {
+    if (C::kSplit && !p.whole_tiles) {
         t_lo = range_lo(n_tiles * U, G, b);
         t_hi = range_lo(n_tiles * U, G, b + 1);
     } else if (p.kparts > 1) {
@@ -651,7 +714,7 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
         spread_last = p.rows > 6 || t_lo > first || range_lo(n_tiles * U, G, b + 2) <= first + U;
     }
     constexpr uint32_t kSpreadThreads = (C::kWG + 1) * 128 + 32;
-    static_assert(!C::kStream || NT <= 16 * (C::kWG + 1), "last_epilogue takes at most 4 groups of rows a warpgroup");
+    static_assert(!C::kStream || C::kWG == 3, "last_epilogue: a warpgroup has at most NT / 16 groups of rows");
 
     if (warp == kWProducer || (C::kWProducers == 2 && warp == kWProducer2)) {
         // =========================== packed weights (+ scales / zeros): one thread per producer warp ===========================
@@ -802,7 +865,8 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                 const int u0 = (int)(t - tile * U);
                 const int u1 = (int)min(U, u0 + (t_hi - t));
                 last = t + (u1 - u0) >= t_hi;
-                if (!ptx::mbar_wait(ptx::smem_u32(&bars.d_empty), (seg & 1u) ^ 1u)) {
+                const uint32_t buf = seg % C::kDBufs, d = tmem_base + buf * C::kDCols;
+                if (!ptx::mbar_wait(ptx::smem_u32(&bars.d_empty[buf]), ((seg / C::kDBufs) & 1u) ^ 1u)) {
                     if (lane == 0) atomicExch(p.status, 21);
                     ok = false;
                     break;
@@ -823,8 +887,8 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                         for (int k = 0; k < 4 * H; ++k) {
                             // K = 16 per instruction: +8 columns of A; B: +32 bytes (2 descriptor units) inside a 64-k sub-tile
                             const uint64_t bd = bdesc + (uint64_t)((k >> 2) * (kBHalfBytes >> 4) + (k & 3) * 2);
-                            if (PAIR) ptx::umma_f16_ts_pair(tmem_base, a0 + k * 8, bd, idesc, (u > u0 || k > 0) ? 1u : 0u);
-                            else ptx::umma_f16_ts(tmem_base, a0 + k * 8, bd, idesc, (u > u0 || k > 0) ? 1u : 0u);
+                            if (PAIR) ptx::umma_f16_ts_pair(d, a0 + k * 8, bd, idesc, (u > u0 || k > 0) ? 1u : 0u);
+                            else ptx::umma_f16_ts(d, a0 + k * 8, bd, idesc, (u > u0 || k > 0) ? 1u : 0u);
                         }
                         if (PAIR) {                                      // the stage comes free in both CTAs
                             ptx::tc_commit_pair(ptx::map_to_cta(ptx::smem_u32(&bars.ab_free[s]), 0));
@@ -855,7 +919,7 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                     }
                     ptx::tc_fence_before_sync();
                     if (spread_last && last) ptx::named_bar_arrive(5, kSpreadThreads);
-                    else ptx::named_bar_arrive(2, 128 + 32);
+                    else ptx::named_bar_arrive(2 + 4 * buf, 128 + 32);
                 }
                 ++seg;
                 t += u1 - u0;
@@ -863,7 +927,7 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
             if (C::kEpiHandoff && !ok) {
                 s_abort = 1;
                 __threadfence_block();
-                if (!spread_last || !last) ptx::named_bar_arrive(2, 128 + 32);
+                if (!spread_last || !last) ptx::named_bar_arrive(2 + 4 * (seg % C::kDBufs), 128 + 32);
                 if (spread_last) ptx::named_bar_arrive(5, kSpreadThreads);      // the last tile's: by every role once, whatever happened
             }
         }
@@ -936,7 +1000,7 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                         if (j0 + 16 >= j_end) {
                             ptx::tc_fence_before_sync();
                             __syncwarp();
-                            if (lane == 0) ptx::mbar_arrive_cluster(ptx::map_to_cta(ptx::smem_u32(&bars.d_empty), 0));
+                            if (lane == 0) ptx::mbar_arrive_cluster(ptx::map_to_cta(ptx::smem_u32(&bars.d_empty[0]), 0));
                         }
                         if (p.kparts > 1) {
                             put_kpart(v, j0);
@@ -969,8 +1033,8 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                         ptx::tc_fence_before_sync();
                         __syncwarp();
                         if (lane == 0) {
-                            if (PAIR) ptx::mbar_arrive_cluster(ptx::map_to_cta(ptx::smem_u32(&bars.d_empty), 0));
-                            else ptx::mbar_arrive(ptx::smem_u32(&bars.d_empty));
+                            if (PAIR) ptx::mbar_arrive_cluster(ptx::map_to_cta(ptx::smem_u32(&bars.d_empty[0]), 0));
+                            else ptx::mbar_arrive(ptx::smem_u32(&bars.d_empty[0]));
                         }
                     }
                     if (p.kparts > 1) {
@@ -1015,11 +1079,12 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                 if constexpr (C::kStream) {
                     if (t + (u1 - u0) >= t_hi) break;                  // the last tile: below
                     ptx::grid_dependency_wait();                       // as in `epilogue`
-                    const int col = (int)threadIdx.x & 127, scol = (int)tile * 128 + col;
+                    const int col = (int)threadIdx.x & 127, scol = tile_ct(tile) * 128 + col, row0 = tile_mt(tile) * NT, rows = min(NT, p.rows - row0);
                     const bool col_ok = scol < p.S;
-                    if (!early_epilogue<NT>(p.om, p.om.n_dst, p.om.ld, p.om.dst[0] + (col_ok ? p.om.col(scol) : 0), p.rows, col_ok ? p.rows : 0, p.accumulate,
-                                        u0 == 0 ? nullptr : reinterpret_cast<uint4*>(p.partials) + (size_t)b * C::kSlotVecs + col,
-                                        tmem_base, ptx::smem_u32(&bars.d_empty), ptx::smem_u32(const_cast<int*>(&s_abort)))) {
+                    const uint32_t buf = seg % C::kDBufs;
+                    if (!early_epilogue<NT>(p.om, p.om.n_dst, p.om.ld, p.om.dst[0] + (size_t)row0 * p.om.ld + (col_ok ? p.om.col(scol) : 0), rows, col_ok ? rows : 0,
+                                        p.accumulate, u0 == 0 ? nullptr : reinterpret_cast<uint4*>(p.partials) + (size_t)(C::kSlots * b) * C::kSlotVecs + col,
+                                        tmem_base + buf * C::kDCols, 2 + 4 * buf, ptx::smem_u32(&bars.d_empty[buf]), ptx::smem_u32(const_cast<int*>(&s_abort)))) {
                         aborted = true;
                         break;
                     }
@@ -1244,9 +1309,26 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
             if (aborted) {
                 if (spread_last) ptx::named_bar_arrive(5, kSpreadThreads);
             } else if (spread_last || (warp >= kEpiWarp0 && t_lo < t_hi)) {
-                const long long t0 = max(t_lo, div_nn(t_hi - 1, U) * U);
-                last_epilogue<NT>(p, tmem_base, &s_abort, t0, (int)(t_hi - t0), spread_last ? warp >> 2 : 0, spread_last ? C::kWG + 1 : 1,
-                                  spread_last ? 5 : 2, spread_last ? kSpreadThreads : 128 + 32);
+                // outputs, old outputs and the scratch may still be in use by the kernel before this one in the stream
+                ptx::grid_dependency_wait();
+                const long long tile = div_nn(t_hi - 1, U), lo_t = tile * U;
+                const uint32_t buf = C::kDBufs == 1 ? 0u : (uint32_t)(tile - div_nn(t_lo, U)) % C::kDBufs;
+                TileCtas ctas{(int)b, (int)b, 1};
+                if (t_lo > lo_t || t_hi < lo_t + U) {
+                    ctas.b_lo = range_owner(n_tiles * U, G, lo_t);
+                    ctas.b_hi = range_owner(n_tiles * U, G, lo_t + U - 1);
+                    if (NT > 32) ctas.members = ctas.b_hi - ctas.b_lo + (range_lo(n_tiles * U, G, ctas.b_hi + 1) == lo_t + U ? 1 : 0);
+                }
+                const int col = (warp & 3) * 32 + lane, scol = tile_ct(tile) * 128 + col, row0 = tile_mt(tile) * NT;
+                const bool col_ok = scol < p.S;
+                auto run = [&](auto epilogue) {
+                    epilogue(p.om, p.om.n_dst, p.om.ld, p.om.dst[0] + (size_t)row0 * p.om.ld + (col_ok ? p.om.col(scol) : 0), col_ok, min(NT, p.rows - row0),
+                             p.accumulate, reinterpret_cast<uint4*>(p.partials) + col, p.status, ctas,
+                             tmem_base + buf * C::kDCols + ((uint32_t)((warp & 3) * 32) << 16), spread_last ? warp >> 2 : 0, spread_last ? C::kWG + 1 : 1,
+                             spread_last ? 5 : 2 + 4 * buf, spread_last ? kSpreadThreads : 128 + 32, ptx::smem_u32(const_cast<int*>(&s_abort)));
+                };
+                if constexpr (NT <= 32 && !PERM) run([](const auto&... a) { last_epilogue_call<NT>(a...); });
+                else run([](const auto&... a) { last_epilogue<NT>(a...); });
             }
         }
     }
@@ -1441,12 +1523,25 @@ int launch_kparts_reduce(const UmmaParams& p, cudaStream_t stream, cudaError_t* 
     return I4MM_OK;
 }
 
-template <int BITS, bool SPARSE, int NT, bool PAIR, bool PERM = false>
+// Weight-streaming shapes: whole tiles, although some SMs then have less to do or nothing, where the units that the busiest CTA has more than
+// with equal ranges cost less than the sums of shared tiles (units: 256 k, from 65 rows on 128 k; us, int4, equal ranges / whole tiles):
+// 16 rows 2048 x 15360 (1.5 units more) 10.9 / 9.6, 5120 x 15360 (3.8) 16.4 / 16.1, 2048 x 7680 (4.8) 8.7 / 8.5, 5120 x 14080 (5.1) 15.5 / 16.1,
+// 2048 x 25600, two tiles a CTA (5.2) 13.9 / 14.8; 64 rows 5120 x 14080 18.3 / 18.0, 8192 x 15360 (6.1) 24.6 / 24.7, 2048 x 25600 17.8 / 16.6;
+// 128 rows 2048 x 9600 (7.9) 14.0 / 12.9, 5120 x 14080 (10.3) 22.8 / 22.1, 5120 x 12800 (13.0) 21.4 / 22.0, 2048 x 25600 (10.4) 25.1 / 22.9;
+// 72 rows 5120 x 14080 21.0 / 21.2.
+bool whole_tiles_better(int nt, long long tiles, int U, long long ctas) {
+    if (tiles % ctas == 0) return false;                       // (equal ranges are whole tiles)
+    const long long w = (tiles + ctas - 1) / ctas;
+    const long long tenths = 10 * (w * U * ctas - tiles * U) / ctas;
+    return tenths < (nt <= 32 ? 45 : nt <= 64 ? (w == 1 ? 55 : 75) : (w == 1 ? 105 : 140));
+}
+
+template <int BITS, bool SPARSE, int NT, bool PAIR, bool PERM = false, bool STREAM = NT <= 64>
 int launch_nt(const UmmaParams& p_in, const __half* x, int n_groups, cudaStream_t stream, cudaError_t* cuda_err) {
     UmmaParams p = p_in;
     p.kparts = 1;
     using F = UFormat<BITS, SPARSE>;
-    using C = Cfg<NT, PAIR>;
+    using C = Cfg<NT, PAIR, STREAM>;
     constexpr int H = C::kHalves;
     p.U = (p.N + 64 * H - 1) / (64 * H);
     constexpr int kBStageBytes = H * (PAIR ? NT / 2 : NT) * 128;
@@ -1464,10 +1559,10 @@ int launch_nt(const UmmaParams& p_in, const __half* x, int n_groups, cudaStream_
     ok = ok && encode_2d_cached(&tm.z, p.zeros, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, n_groups, p.S, H, 128, CU_TENSOR_MAP_SWIZZLE_NONE);
     if (!ok) return I4MM_ERR_DEVICE;
 
-    const size_t smem = 1024 + (size_t)ABStages<NT, PAIR>::value * kBStageBytes + (size_t)C::kWStages * WStage<F, H>::kBytes +
+    const size_t smem = 1024 + (size_t)ABStages<NT, PAIR, STREAM>::value * kBStageBytes + (size_t)C::kWStages * WStage<F, H>::kBytes +
                         (!C::kEpiTransposed ? 0 : PAIR ? NT * 256 : 4096 * ((C::kEpiGroups == 2 && NT < 256) ? 2 : 1)) +
                         (PERM ? (size_t)C::kXStaging * kBStageBytes : 0);
-    auto kern = umma_kernel<BITS, SPARSE, NT, PAIR, PERM>;
+    auto kern = umma_kernel<BITS, SPARSE, NT, PAIR, PERM, STREAM>;
     // per-device cache; atomic because two host threads may make their first call at once (both then compute the same value)
     static std::atomic<int> sm_count[16];
     int dev = 0;
@@ -1510,7 +1605,7 @@ int launch_nt(const UmmaParams& p_in, const __half* x, int n_groups, cudaStream_
         }
         long long clusters = max_clusters[dev];
         const long long tiles2 = (long long)p.MTILES * ((p.CT + 1) / 2);
-        if (!p.accumulate)
+        if (!p.accumulate && !p.whole_tiles)
             p.kparts = choose_kparts(clusters, tiles2, p.U, p.rows, p.S);
         const long long work = tiles2 * p.kparts;
         if (clusters > work || p.kparts > 1) clusters = work;
@@ -1524,11 +1619,18 @@ int launch_nt(const UmmaParams& p_in, const __half* x, int n_groups, cudaStream_
     }
     const long long n_tiles = (long long)p.MTILES * p.CT;
     long long grid = sm_count[dev];                     // one CTA per SM: every configuration fills its shared or tensor memory
-    if (!C::kSplit && !p.accumulate)
+    if (!C::kSplit && !p.accumulate && !p.whole_tiles)
         p.kparts = choose_kparts(grid, n_tiles, p.U, p.rows, p.S);
-    const long long work = p.kparts > 1 ? n_tiles * p.kparts : C::kSplit ? n_tiles * p.U : n_tiles;
+    if (C::kSplit) {
+        p.whole_tiles = whole_tiles_better(NT, n_tiles, p.U, grid);
+        if (p.whole_tiles) {
+            const long long w = (n_tiles + grid - 1) / grid;
+            grid = (n_tiles + w - 1) / w;
+        }
+    }
+    const long long work = p.kparts > 1 ? n_tiles * p.kparts : C::kSplit && !p.whole_tiles ? n_tiles * p.U : n_tiles;
     if (grid > work || p.kparts > 1) grid = work;
-    if (C::kSplit && grid > kPartialBytes / (C::kSlotVecs * 16)) grid = kPartialBytes / (C::kSlotVecs * 16);   // one partial tile per CTA in the scratch
+    if (C::kSplit && grid > kPartialBytes / (C::kSlots * C::kSlotVecs * 16)) grid = kPartialBytes / (C::kSlots * C::kSlotVecs * 16);   // partial tiles in the scratch
     {
         // The kernel may start while the kernel before it in the stream is still running: its set-up overlaps that
         // kernel's tail, and with `overlap` so do its copies of the weight-side tensors (which the caller has declared
@@ -1592,6 +1694,20 @@ int launch_fmt(UmmaParams& p, const __half* x, int n_groups, int pair_mode, int 
     }
     // 128 rows or more (the whole-tile configurations) run as CTA pairs, two SMs per MMA, unless the caller asked for single CTAs
     const bool pair = pair_mode == 0 && (force_nt ? force_nt >= 128 : p.rows >= kPairMinRows);
+    // 65..128 rows: the weight-streaming shape, or whole tiles of the shape that is made for them (its decode does not share the CTA with sums,
+    // and its stores are 16 bytes) where those leave fewer SMs idle than the sums cost.  us, whole tiles / streaming: int4 96 rows 2048 x 16384
+    // 13.2 / 13.7, 16:32 14.7 / 16.0, 5120 x 16384 22.3 / 22.4, 26.0 / 28.0; K parts, as before / streaming: 5120 x 5120 21.4 / 13.8, 22.2 / 14.8,
+    // 13824 x 5120 31.4 / 22.2, 34.7 / 23.6; two waves / streaming: 5120 x 20480 40.3 / 31.4, 47.4 / 37.0.
+    // 128 rows in a CTA pair take 0.85 of the time per unit: pairs / streaming, int4, 5120 x 27648 (68 units to 58, of 128 k) 39.1 / 42.0, 13824 x 15360
+    // (92 to 88) 53.6 / 56.7, 2048 x 20480 (27 to 17) 21.3 / 22.4, 5120 x 11008 (34 to 23) 22.2 / 20.3, 5120 x 20480 (68 to 43) 39.3 / 33.7.
+    if (!force_nt && p.rows > 64 && p.rows <= 128 && p.om.n_dst == 1) {
+        const long long U = (p.N + 127) / 128, w = (p.CT + sms - 1) / sms;
+        p.whole_tiles = p.CT % sms == 0 || (pair ? w * U * 17 * sms < (p.CT * U + 10 * sms) * 20 : whole_tiles_better(128, p.CT, (int)U, sms));
+        if (!p.whole_tiles) {
+            p.MTILES = 1;
+            return launch_nt<BITS, SPARSE, 128, false, false, true>(p, x, n_groups, stream, cuda_err);
+        }
+    }
     // Stores into several GPUs' buffers (the gathering multiply) make the epilogue of a tile last longer than the tile's
     // MMAs.  Under exactly that condition the CTA-pair instances with 224 and 256 rows per tile (two dequant warpgroups,
     // three weight stages) were seen, on 8 GPUs, to produce now and then one wrong block of 32 columns x one row tile

@@ -1,4 +1,4 @@
-"""GPU parity tests of the few-row tcgen05 shapes (1..64 rows) where column tiles are shared: the owner of a tile sums its partners'
+"""GPU parity tests of the few-row tcgen05 shapes (1..128 rows) where column tiles are shared: the owner of a tile sums its partners'
 shares, with its epilogue warps alone or with every warpgroup, some rows each (dense int4 with up to 3 rows runs in another k order)."""
 import ctypes
 
@@ -120,7 +120,7 @@ def test_matvec_route_adds_33_to_64_rows_into_outs(batch, n, s):
     assert_parity(got[..., cols], want, bound, f"accumulate {batch} {n}x{s}")
 
 
-@pytest.mark.parametrize("m", [1, 4, 7, 16, 32, 50])
+@pytest.mark.parametrize("m", [1, 4, 7, 16, 32, 50, 100])
 def test_partial_sums_of_zero_infinity_and_nan_are_delivered(m):
     """A shared tile's partial sums travel as words that are never zero: rows of zeros (of either sign), infinities and NaN."""
     n, s = 8192, 320
@@ -162,3 +162,34 @@ def test_the_streaming_path_leaves_the_scratch_to_the_other_kernels(m):
     ws = ops.workspace(torch.device("cuda", torch.cuda.current_device()), torch.cuda.current_stream())
     assert int(ws.count_nonzero()) == 0
     assert np.array_equal(run_problem(p, path=P).view(np.uint16), want.view(np.uint16))
+
+
+# 65..128 rows: tiles shared by up to 64 and by 3 or 4 CTAs, a CTA that goes on to the next tile, two accumulators in turn (1.35 tiles a
+# CTA), S % 128 = 64; and whole tiles of the other shape (75 tiles of 16 units)
+@pytest.mark.parametrize("n,s,g,m", [(16384, 64, 128, m) for m in (65, 100, 128)] + [(8256, 320, 192, m) for m in (65, 77, 127, 128)] +
+                         [(4096, 5056, -1, m) for m in (66, 96, 128)] + [(8192, 9536, 64, 97), (2048, 9536, 64, 97)] + [(4096, 25600, 128, m) for m in (65, 127)])
+@pytest.mark.parametrize("fmt", FORMATS, ids=fmt_id)
+def test_shared_tiles_of_65_to_128_rows(fmt, n, s, g, m):
+    bits, sparse = fmt
+    p = oracle.make_packed_problem(bits, n, s, m, g, sparse=sparse, seed=n + s + m)
+    got = run_problem(p, path=P)
+    assert capi.load().i4mm_last_launch_shape() == 128
+    cols = np.unique(np.concatenate([np.arange(64), s - 1 - np.arange(64), np.random.default_rng(m).integers(0, s, 60)]))
+    want, bound = oracle.expected_columns(bits, p["matrix"], p["mask"], p["scales"], p["zeros"], g, p["x"], cols)
+    assert_parity(got[..., cols], want, bound, f"{fmt} m={m} {n}x{s} g{g}")
+    again = run_problem(p, path=P)
+    assert np.array_equal(got.view(np.uint16), again.view(np.uint16))
+    ws = ops.workspace(torch.device("cuda", torch.cuda.current_device()), torch.cuda.current_stream())
+    assert int(ws.count_nonzero()) == 0
+
+
+@pytest.mark.parametrize("n,s", [(4096, 25600), (8192, 192)])
+@pytest.mark.parametrize("batch", [65, 128])
+def test_matvec_route_adds_65_to_128_rows_into_outs(batch, n, s):
+    p = oracle.make_packed_problem(4, n, s, 1, 64, batch=batch, seed=47)
+    base = np.random.default_rng(5).standard_normal((batch, 1, s)).astype(np.float16)
+    got = run_problem(p, path=P, outs_in=base, route="vec")
+    cols = np.unique(np.concatenate([np.arange(0, s, 128), np.arange(63, s, 64)]))
+    want, bound = oracle.expected_columns(4, p["matrix"], p["mask"], p["scales"], p["zeros"], 64, p["x"], cols,
+                                          outs_in=np.ascontiguousarray(base[..., cols]))
+    assert_parity(got[..., cols], want, bound, f"accumulate {batch} {n}x{s}")
