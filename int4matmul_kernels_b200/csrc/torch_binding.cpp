@@ -206,36 +206,48 @@ struct Weights {
     }
 };
 
-// `workspaces`: the Python package's dict (device index, raw stream) -> zero-initialised uint8 tensor
-int launch_checked(const Weights& w, bool matvec, int64_t path, void* out, const Tensor& x, int64_t rows, const py::dict& workspaces) {
-    const auto dev = x.device();
-    if (w.bits != 4 && w.bits != 3 && w.bits != 2) return -1;
-    const int64_t in_size = x.size(-1);
-    if (!plain(x, dev, torch::kHalf) || !plain(w.matrix, dev, torch::kInt) || !plain(w.scales, dev, torch::kHalf) ||
-        !plain(w.zeros, dev, torch::kHalf) || w.matrix.dim() != 2 || w.scales.dim() != 2 || w.zeros.dim() != 2)
-        return -1;
+// Whether a multiply of fp16 rows of `in_size` on `dev` by w passes the entries' checks
+bool valid(const Weights& w, const c10::Device& dev, int64_t in_size) {
+    if (w.bits != 4 && w.bits != 3 && w.bits != 2) return false;
+    if (!plain(w.matrix, dev, torch::kInt) || !plain(w.scales, dev, torch::kHalf) || !plain(w.zeros, dev, torch::kHalf) ||
+        w.matrix.dim() != 2 || w.scales.dim() != 2 || w.zeros.dim() != 2)
+        return false;
     const int64_t mtx_in = w.matrix.size(0), out_size = w.matrix.size(1);
-    const bool sparse = w.mask.defined();
-    if (sparse) {
+    if (w.mask.defined()) {
         if (w.bits != 4 || mtx_in * 16 != in_size || mtx_in % 2 || !plain(w.mask, dev, torch::kInt) || w.mask.dim() != 2 ||
             w.mask.size(0) != mtx_in / 2 || w.mask.size(1) != out_size)
-            return -1;
+            return false;
     } else if ((mtx_in * 32) % w.bits || mtx_in * 32 / w.bits != in_size) {
-        return -1;
+        return false;
     }
-    if (w.scales.size(1) != out_size || w.zeros.sizes() != w.scales.sizes()) return -1;
-    if (w.group_size == 0 || (w.group_size > 0 && w.group_size % 64)) return -1;
+    if (w.scales.size(1) != out_size || w.zeros.sizes() != w.scales.sizes()) return false;
+    return w.group_size != 0 && (w.group_size < 0 || w.group_size % 64 == 0);
+}
+
+// the scratch of the current stream of `dev`, from the Python package's dict (device index, raw stream) -> zero-initialised uint8
+// tensor; undefined if there is none yet
+Tensor scratch(const py::dict& workspaces, const c10::Device& dev, cudaStream_t stream) {
+    PyObject* const item = PyDict_GetItem(workspaces.ptr(), py::make_tuple((int)dev.index(), (uint64_t)(uintptr_t)stream).ptr());
+    return item ? py::cast<Tensor>(py::handle(item)) : Tensor();
+}
+
+int launch(const Weights& w, bool matvec, int64_t path, void* out, const void* x, int64_t rows, int64_t in_size, const Tensor& ws, cudaStream_t stream) {
+    return i4mm_quant_matmul((int)w.bits, matvec ? 1 : 0, (int)path, out, w.matrix.data_ptr(), w.mask.defined() ? w.mask.data_ptr() : nullptr,
+                             x, w.scales.data_ptr(), w.zeros.data_ptr(), rows, in_size, w.matrix.size(1), w.scales.size(0),
+                             w.group_size, ws.data_ptr(), (size_t)ws.numel(), (void*)stream);
+}
+
+int launch_checked(const Weights& w, bool matvec, int64_t path, void* out, const Tensor& x, int64_t rows, const py::dict& workspaces) {
+    const auto dev = x.device();
+    if (!plain(x, dev, torch::kHalf) || !valid(w, dev, x.size(-1))) return -1;
     c10::cuda::OptionalCUDAGuard guard;
     if (c10::cuda::current_device() != dev.index()) guard.set_device(dev);
     const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
-    PyObject* const item = PyDict_GetItem(workspaces.ptr(), py::make_tuple((int)dev.index(), (uint64_t)(uintptr_t)stream).ptr());
-    if (!item) return -1;
-    const Tensor ws = py::cast<Tensor>(py::handle(item));
+    const Tensor ws = scratch(workspaces, dev, stream);
+    if (!ws.defined()) return -1;
     // (every tensor is held by a reference of this call's own)
     py::gil_scoped_release release;
-    return i4mm_quant_matmul((int)w.bits, matvec ? 1 : 0, (int)path, out, w.matrix.data_ptr(), sparse ? w.mask.data_ptr() : nullptr,
-                             x.data_ptr(), w.scales.data_ptr(), w.zeros.data_ptr(), rows, in_size, out_size, w.scales.size(0),
-                             w.group_size, ws.data_ptr(), (size_t)ws.numel(), (void*)stream);
+    return launch(w, matvec, path, out, x.data_ptr(), rows, x.size(-1), ws, stream);
 }
 
 // ops._mult; route 0: by seq_len, 1: matmul, 2: matvec
@@ -314,6 +326,73 @@ py::object try_row_norm(int64_t mode, const py::object& a_, const py::object& b,
     }
 }
 
+// One layer of sharding.DecoderStack on one GPU: the data flow of its forward(), the same eight launches (`early`:
+// I4MM_PATH_STATIC_WEIGHTS or 0).  h, x: the residual stream and its normalised rows; returns h, or the pair of the next layer's h and x,
+// a status, or -1 with nothing launched.  A layer of one row is 70 us of work on the GPU; eight calls from Python took longer than that.
+py::object try_layer(const py::object& mats, const py::object& h_, const py::object& x_, bool last, int64_t early, const py::dict& workspaces) {
+    static const char* const kNames[4] = {"qkv", "o", "gate_up", "down"};
+    Tensor h, x;
+    Weights w[4];
+    int64_t columns[4];
+    if (!PyDict_Check(mats.ptr()) || !as_tensor(h_, h) || !as_tensor(x_, x)) return py::int_(-1);
+    for (int i = 0; i < 4; ++i) {
+        PyObject* const m = PyDict_GetItemString(mats.ptr(), kNames[i]);
+        if (!m) return py::int_(-1);
+        const py::handle q(m);
+        const py::object none = py::none();
+        if (!w[i].read(py::getattr(q, "bits", none), py::getattr(q, "matrix", none), py::getattr(q, "scales", none), py::getattr(q, "zeros", none),
+                       py::getattr(q, "group_size", none), py::getattr(q, "mask", none)) ||
+            !as_int(py::getattr(q, "s", none), columns[i]))
+            return py::int_(-1);
+    }
+    try {
+        if (!h.is_cuda()) return py::int_(-1);
+        const auto dev = h.device();
+        if (h.dim() != 2 || h.size(0) == 0 || !plain(h, dev, torch::kHalf) || !plain(x, dev, torch::kHalf) || x.sizes() != h.sizes() ||
+            c10::cuda::current_device() != dev.index())
+            return py::int_(-1);
+        const int64_t rows = h.size(0), width = h.size(1);
+        for (int i = 0; i < 4; ++i)
+            if (w[i].matrix.dim() != 2 || w[i].matrix.size(1) != columns[i]) return py::int_(-1);
+        const int64_t qkv = w[0].matrix.size(1), gate_up = w[2].matrix.size(1), inner = gate_up / 2;
+        if (qkv != 3 * width || w[1].matrix.size(1) != width || gate_up % 2 || inner % 2 || width % 2 || w[3].matrix.size(1) != width ||
+            !valid(w[0], dev, width) || !valid(w[1], dev, width) || !valid(w[2], dev, width) || !valid(w[3], dev, inner))
+            return py::int_(-1);
+        const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+        const Tensor ws = scratch(workspaces, dev, stream);
+        if (!ws.defined()) return py::int_(-1);
+        const auto options = at::TensorOptions().dtype(torch::kHalf).device(dev);
+        const Tensor p = at::empty({rows, qkv}, options), t = at::empty({rows, width}, options), o = at::empty({rows, width}, options),
+                     h2 = at::empty({rows, width}, options), g = at::empty({rows, gate_up}, options), a = at::empty({rows, inner}, options),
+                     d = at::empty({rows, width}, options),
+                     y = last ? at::empty({rows, width}, options) : at::empty({2, rows, width}, options);
+        int status;
+        {
+            py::gil_scoped_release release;
+            const auto col = [](const Tensor& m, int64_t c) -> const void* { return static_cast<const at::Half*>(m.data_ptr()) + c; };
+            const auto norm = [&](int mode, const Tensor& out, const void* a0, const void* b0, const void* c0, int64_t n, int64_t sa, int64_t sb, int64_t sc) {
+                return i4mm_row_norm(mode | (int)early, out.data_ptr(), a0, b0, c0, rows, n, sa, sb, sc, (void*)stream);
+            };
+            const auto mult = [&](int i, const Tensor& out, const Tensor& in) {
+                return launch(w[i], false, early, out.data_ptr(), in.data_ptr(), rows, in.size(1), ws, stream);
+            };
+            status = mult(0, p, x);
+            if (status == I4MM_OK) status = norm(1, t, col(p, 0), col(p, width), col(p, 2 * width), width, qkv, qkv, qkv);
+            if (status == I4MM_OK) status = mult(1, o, t);
+            if (status == I4MM_OK) status = norm(2, h2, h.data_ptr(), o.data_ptr(), nullptr, width, width, width, 0);
+            if (status == I4MM_OK) status = mult(2, g, h2);
+            if (status == I4MM_OK) status = norm(3, a, col(g, 0), col(g, inner), nullptr, inner, gate_up, gate_up, 0);
+            if (status == I4MM_OK) status = mult(3, d, a);
+            if (status == I4MM_OK) status = norm(last ? 2 : 4, y, h2.data_ptr(), d.data_ptr(), nullptr, width, width, width, 0);
+        }
+        if (status != I4MM_OK) return py::int_(status);
+        if (last) return py::cast(y);
+        return py::make_tuple(y.select(0, 0), y.select(0, 1));
+    } catch (const c10::Error&) {
+        return py::int_(-1);                               // (an allocation failed; nothing was launched)
+    }
+}
+
 // Not in the reference (its kernels have no waits): waits for every stream this module has launched on, on the
 // current device, and raises if a kernel gave up on one of its bounded device-side waits since the last check.
 // The multiply entries do not call it themselves, because it synchronises.
@@ -348,6 +427,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
 
     m.def("_try_mult", &try_mult, "ops._mult for arguments that pass its checks: status, or -1");
     m.def("_try_linear", &try_linear, "QuantLinear.forward for arguments that pass its checks: output, status or -1");
+    m.def("_try_layer", &try_layer, "one layer of sharding.DecoderStack on one GPU: h, or (h, x), a status or -1");
     m.def("_try_row_norm", &try_row_norm, "ops.row_norm for arguments that pass its checks: output, status or -1");
 
     m.def("weight_matrix_packing", &weight_matrix_packing, "int4_sparse_pack");

@@ -246,3 +246,14 @@ def row_norm(mode: int, a: torch.Tensor, b: torch.Tensor | None = None, c: torch
     if status != capi.OK:
         raise Int4MatmulError(status, "row_norm")
     return y
+
+
+def stack_layer(mats: dict, h: torch.Tensor, x: torch.Tensor, last: bool):
+    """One layer of `sharding.DecoderStack` as one call of the compiled module: h, or (h, x) for the next layer; None where that
+    module has to leave the layer to the single calls (an argument that they convert, allocate for or refuse)."""
+    done = native()._try_layer(mats, h, x, last, capi.PATH_STATIC_WEIGHTS if _static_weights else 0, _workspaces)
+    if not isinstance(done, int):
+        return done
+    if done > 0:
+        raise Int4MatmulError(done, "stack layer")
+    return None

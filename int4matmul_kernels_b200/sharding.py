@@ -314,10 +314,27 @@ class DecoderStack:
         h = cls.combine(2, a, b)
         return h, cls.combine(0, h)
 
+    def _layer_natively(self):
+        """The compiled module if a layer may be one call of it: one GPU, and nothing of the data flow replaced."""
+        if self.world != 1 or self.multiply is not cuda_multiply or getattr(self, "peer", None) is not None:
+            return False
+        if type(self) is not DecoderStack or any(n in self.__dict__ or DecoderStack.__dict__[n] is not f for n, f in _DATA_FLOW.items()):
+            return False
+        return ops.native()
+
     def forward(self, h: torch.Tensor) -> torch.Tensor:
         comb = self.combine
         x = comb(0, h)
+        native = self._layer_natively() if h.is_cuda else False
         for i, mats in enumerate(self.layers):
+            last = i + 1 == len(self.layers)
+            if native:
+                done = ops.stack_layer(mats, h, x, last)
+                if done is not None:
+                    if last:
+                        return done
+                    h, x = done
+                    continue
             q, k, v = self._linear(mats["qkv"], x, 3, "qkv")
             t = comb(1, q, k, v)
             (o,) = self._linear(mats["o"], t, 1, "o")
@@ -325,8 +342,11 @@ class DecoderStack:
             gate, up = self._linear(mats["gate_up"], h, 2, "gate_up")
             a = comb(3, gate, up)
             (d,) = self._linear(mats["down"], a, 1, "down")
-            if i + 1 < len(self.layers):
-                h, x = self.combine_and_normalise(h, d)
-            else:
+            if last:
                 h = comb(2, h, d)
+            else:
+                h, x = self.combine_and_normalise(h, d)
         return h
+
+
+_DATA_FLOW = {n: DecoderStack.__dict__[n] for n in ("_linear", "combine", "combine_and_normalise")}

@@ -1,5 +1,6 @@
 """The compiled fast path of the Python entries (ops, QuantLinear) against the same calls through ctypes: equal results for
 everything both accept, and the same exceptions for what the entries refuse."""
+import dataclasses
 import threading
 import time
 
@@ -7,7 +8,7 @@ import numpy as np
 import pytest
 import torch
 
-from int4matmul_kernels_b200 import ops, packing
+from int4matmul_kernels_b200 import capi, ops, packing, sharding
 from int4matmul_kernels_b200.quantize import QuantLinear
 
 pytestmark = pytest.mark.gpu
@@ -169,3 +170,83 @@ def test_threads_that_share_a_stream_do_not_mix_their_launches():
         t.join()
     assert not bad, len(bad)
     ops.check_device_status()
+
+
+def small_stack(bits, sparse, rows):
+    """Two layers of 256 (inner width 448) with weights of one format, and rows of activations."""
+    cfg = sharding.StackConfig(hidden=256, mlp=448, layers=2, bits=4, group_size=64)
+    stack = sharding.DecoderStack(cfg, 0, 1, "cuda", layers=0)
+    stack.layers = []
+    for layer in range(2):
+        mats = {}
+        for i, (name, n, s) in enumerate((("qkv", 256, 768), ("o", 256, 256), ("gate_up", 256, 896), ("down", 448, 256))):
+            w = packing.synthetic_weights(bits, n, s, 64, sparse=sparse, seed=10 * layer + i)
+            mats[name] = sharding.QuantWeights(bits, n, s, 64, w["matrix"], w["scales"], w["zeros"], w["mask"])
+        stack.layers.append(mats)
+    return stack, torch.randn((rows, 256), generator=torch.Generator().manual_seed(rows)).half().cuda()
+
+
+@pytest.mark.parametrize("bits,sparse", [(4, False), (3, False), (2, False), (4, True)])
+@pytest.mark.parametrize("rows", [1, 5, 40])
+def test_stack_layers_in_one_call(monkeypatch, bits, sparse, rows):
+    stack, h = small_stack(bits, sparse, rows)
+    stack.forward(h)                                                    # (allocates this stream's scratch)
+    lib = capi.load()
+    for static in (False, True):
+        ops.set_static_weights(static)
+        try:
+            before = lib.i4mm_launch_count()
+            fast, slow = both(monkeypatch, lambda: stack.forward(h))
+            assert lib.i4mm_launch_count() - before == 2 * (1 + 2 * 8)
+        finally:
+            ops.set_static_weights(False)
+        assert torch.equal(fast, slow)
+    side = torch.cuda.Stream()                                          # no scratch there yet: the single calls allocate it
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        outs = [stack.forward(h) for _ in range(2)]
+    side.synchronize()
+    assert all(torch.equal(o, slow) for o in outs)
+
+
+def test_stack_layers_leave_everything_else_to_the_single_calls(monkeypatch):
+    stack, h = small_stack(4, False, 3)
+    want = stack.forward(h)
+    called = []
+    monkeypatch.setattr(ops, "stack_layer", lambda *a: called.append(a))        # (a layer refused: None)
+    assert torch.equal(stack.forward(h), want) and len(called) == 2
+    called.clear()
+    stack.multiply = lambda w, x: sharding.cuda_multiply(w, x)                  # another multiply, a replaced step
+    assert torch.equal(stack.forward(h), want)
+    stack.multiply = sharding.cuda_multiply
+    stack._linear = lambda *a: sharding.DecoderStack._linear(stack, *a)
+    assert torch.equal(stack.forward(h), want) and not called
+    monkeypatch.undo()
+    del stack._linear
+    strided = torch.stack([h, h], dim=-1)[..., 0]
+    for broken in ("scales", "s", "group_size"):
+        mats = dict(stack.layers[1])
+        old = mats["down"]
+        mats["down"] = dataclasses.replace(old, **{broken: {"scales": old.scales.float(), "s": old.s + 64, "group_size": 100}[broken]})
+        other, _ = small_stack(4, False, 3)
+        other.layers = [stack.layers[0], mats]
+        messages = []
+        for native in (True, False):
+            with monkeypatch.context() as m:
+                if not native:
+                    m.setattr(ops, "_native", False)
+                with pytest.raises((ValueError, TypeError, RuntimeError)) as e:
+                    other.forward(h)
+                messages.append((type(e.value), str(e.value)))
+        assert messages[0] == messages[1]
+    with monkeypatch.context() as m:
+        fast = [type(e) for e in (_outcome(stack, strided),)]
+        m.setattr(ops, "_native", False)
+        assert fast == [type(e) for e in (_outcome(stack, strided),)]
+
+
+def _outcome(stack, h):
+    try:
+        return stack.forward(h)
+    except Exception as e:
+        return e
