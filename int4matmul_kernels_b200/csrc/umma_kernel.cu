@@ -1680,6 +1680,26 @@ int choose_tile_rows(int rows, int col_tiles, int sms, int max_nt) {
 
 constexpr int kPairMinRows = 128;
 
+// More than 128 rows in one call: tiles of 128 rows on the weight-streaming shape, or taller ones on CTA pairs.  Pairs decode a weight for up
+// to 256 rows at once and run a tile's MMAs on two SMs, so they win wherever their tiles fill the pairs; the streaming shape hands out single
+// units, so it wins where they do not, and where pairs would cut K into parts that a second kernel adds up.  Both times in 1/100 us (units: 128 k;
+// pairs: a fixed part, a quarter of a row per unit and row of the tile, the adding kernel; streaming: whole tiles, or equal ranges and their
+// sums), fitted to 472 shapes of 130..512 rows (2048 / 5120 / 13824 x 2048..20480) and held against 160 more, drawn from 129..2048 rows and
+// 1024..20480 on both sides: there the chosen one took 0.88 (int4), 0.87 (int3), 0.78 (int2) and 0.91 (16:32) of the time of pairs alone in the
+// mean, within 1 % of always taking the better one, and was in no shape more than 1.5 % slower than pairs.
+// us, pairs / streaming, int4: 13824 x 2048 200 rows 31.2 / 19.5 (K parts), 13824 x 5120 200 rows 48.6 / 34.7, 5120 x 5120 160 rows 24.6 / 18.9;
+// 5120 x 6976 333 rows 27.0 / 32.9 (28 pair tiles of 256 rows twice: every SM busy).
+bool streaming_better(bool sparse, int rows, int CT, int U, long long S, int sms, bool kparts_allowed) {
+    const long long pairs = sms / 2, CT2 = (CT + 1) / 2, tiles = (long long)((rows + 127) / 128) * CT;
+    const long long nt = choose_tile_rows(rows, (int)CT2, (int)pairs, 256), tiles2 = (rows + nt - 1) / nt * CT2;
+    const long long kp = kparts_allowed ? choose_kparts(pairs, tiles2, U, rows, S) : 1;
+    const long long t_pairs = 800 + (tiles2 * kp + pairs - 1) / pairs * ((U + kp - 1) / kp) * nt / 4 + (kp > 1 ? 1100 : 0);
+    const long long w = (tiles + sms - 1) / sms;
+    const long long t_streaming = tiles % sms == 0 || whole_tiles_better(128, tiles, U, sms) ? 800 + (sparse ? 45 : 40) * w * U + 300 * (w - 1)
+                                                                                             : 1000 + (sparse ? 55 : 46) * tiles * U / sms;
+    return t_streaming * 20 < t_pairs * 19;
+}
+
 template <int BITS, bool SPARSE>
 int launch_fmt(UmmaParams& p, const __half* x, int n_groups, int pair_mode, int force_nt, cudaStream_t stream, cudaError_t* cuda_err) {
     static std::atomic<int> sms_of[16];
@@ -1707,6 +1727,10 @@ int launch_fmt(UmmaParams& p, const __half* x, int n_groups, int pair_mode, int 
             p.MTILES = 1;
             return launch_nt<BITS, SPARSE, 128, false, false, true>(p, x, n_groups, stream, cuda_err);
         }
+    }
+    if (!force_nt && pair_mode == 0 && p.rows > 128 && p.om.n_dst == 1 && streaming_better(SPARSE, p.rows, p.CT, (p.N + 127) / 128, p.S, sms, !p.accumulate)) {
+        p.MTILES = (p.rows + 127) / 128;
+        return launch_nt<BITS, SPARSE, 128, false, false, true>(p, x, n_groups, stream, cuda_err);
     }
     // Stores into several GPUs' buffers (the gathering multiply) make the epilogue of a tile last longer than the tile's
     // MMAs.  Under exactly that condition the CTA-pair instances with 224 and 256 rows per tile (two dequant warpgroups,

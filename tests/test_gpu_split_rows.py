@@ -1,4 +1,4 @@
-"""GPU parity tests of the few-row tcgen05 shapes (1..128 rows) where column tiles are shared: the owner of a tile sums its partners'
+"""GPU parity tests of the few-row tcgen05 shapes (1..128 rows a tile) where column tiles are shared: the owner of a tile sums its partners'
 shares, with its epilogue warps alone or with every warpgroup, some rows each (dense int4 with up to 3 rows runs in another k order)."""
 import ctypes
 
@@ -189,6 +189,36 @@ def test_matvec_route_adds_65_to_128_rows_into_outs(batch, n, s):
     p = oracle.make_packed_problem(4, n, s, 1, 64, batch=batch, seed=47)
     base = np.random.default_rng(5).standard_normal((batch, 1, s)).astype(np.float16)
     got = run_problem(p, path=P, outs_in=base, route="vec")
+    cols = np.unique(np.concatenate([np.arange(0, s, 128), np.arange(63, s, 64)]))
+    want, bound = oracle.expected_columns(4, p["matrix"], p["mask"], p["scales"], p["zeros"], 64, p["x"], cols,
+                                          outs_in=np.ascontiguousarray(base[..., cols]))
+    assert_parity(got[..., cols], want, bound, f"accumulate {batch} {n}x{s}")
+
+
+# More than 128 rows: row tiles of 128 beside each other (a ragged last one of 1, 5, 72 and 122 rows), a CTA whose range goes over from
+# one row tile to the next, two and three tiles a CTA; K in one unit and with a last unit that is only partly there
+@pytest.mark.parametrize("n,s,g,m", [(8256, 320, 192, 133), (8192, 2432, -1, 200), (8192, 2432, 64, 257), (4096, 5056, 64, 129), (13824, 2048, 128, 378)])
+@pytest.mark.parametrize("fmt", FORMATS, ids=fmt_id)
+def test_row_tiles_of_the_streaming_shape(fmt, n, s, g, m):
+    bits, sparse = fmt
+    p = oracle.make_packed_problem(bits, n, s, m, g, sparse=sparse, seed=n + s + m)
+    got = run_problem(p, path=P)
+    assert capi.load().i4mm_last_launch_shape() == 128
+    cols = np.unique(np.concatenate([np.arange(32), s - 1 - np.arange(32), np.random.default_rng(m).integers(0, s, 40)]))
+    want, bound = oracle.expected_columns(bits, p["matrix"], p["mask"], p["scales"], p["zeros"], g, p["x"], cols)
+    assert_parity(got[..., cols], want, bound, f"{fmt} m={m} {n}x{s} g{g}")
+    again = run_problem(p, path=P)
+    assert np.array_equal(got.view(np.uint16), again.view(np.uint16))
+    ws = ops.workspace(torch.device("cuda", torch.cuda.current_device()), torch.cuda.current_stream())
+    assert int(ws.count_nonzero()) == 0
+
+
+def test_matvec_route_adds_more_than_128_rows_into_outs():
+    n, s, batch = 13824, 2048, 200
+    p = oracle.make_packed_problem(4, n, s, 1, 64, batch=batch, seed=53)
+    base = np.random.default_rng(6).standard_normal((batch, 1, s)).astype(np.float16)
+    got = run_problem(p, path=P, outs_in=base, route="vec")
+    assert capi.load().i4mm_last_launch_shape() == 128
     cols = np.unique(np.concatenate([np.arange(0, s, 128), np.arange(63, s, 64)]))
     want, bound = oracle.expected_columns(4, p["matrix"], p["mask"], p["scales"], p["zeros"], 64, p["x"], cols,
                                           outs_in=np.ascontiguousarray(base[..., cols]))
