@@ -1536,6 +1536,31 @@ bool whole_tiles_better(int nt, long long tiles, int U, long long ctas) {
     return tenths < (nt <= 32 ? 45 : nt <= 64 ? (w == 1 ? 55 : 75) : (w == 1 ? 105 : 140));
 }
 
+// Weight-streaming shapes: how many CTAs share each tile, the same number for all, or 0: all CTAs have equal ranges and tiles are shared as it
+// comes.  Equal ranges use every SM, but a CTA of them may hold parts of two tiles, one summed after the other, and few tiles have many
+// partners, each of which costs its share of the sums: a smaller grid in which no range crosses a tile is the faster one wherever the
+// units that it adds cost less.  Costs in tenths of a unit's time, fitted to 1366 shapes (int4, int3, 16:32; 1 .. 128 rows; 4 .. 64 tiles of
+// 1024 .. 20480 rows of weights), where the rule takes 0.92 (up to 16 rows), 0.89, 0.90 and 0.86 (65 rows and more) of the time of equal
+// ranges in the mean; none is slower by more than 4 %, three by more than 1.2 %.
+// us, equal ranges / CTAs per tile: int4, 4 rows 3072 x 1024 7.0 / 6.0 (6), 2048 x 2560 6.7 / 6.0 (3), 16 rows 4096 x 1024 8.9 / 6.8 (8), 32 rows
+// 2048 x 2560 8.7 / 7.3 (3), 64 rows 4096 x 1024 11.1 / 8.2 (8), 128 rows 4096 x 8192 17.2 / 14.5 (2), 4096 x 5120 13.7 / 12.5 (3), 2048 x 1024
+// 11.5 / 8.3 (4); not taken: 4 rows 13824 x 2560 11.6 / 11.8 (6), 5120 x 2560 (3) 8.7 / 8.9, 20480 x 5120 19.8 / 21.3 (3).
+int ctas_of_a_tile(int nt, bool sparse, long long tiles, long long U, long long ctas) {
+    const long long partner = nt <= 16 ? (sparse ? 2 : 4) : nt <= 32 ? (sparse ? 4 : 5) : nt <= 64 ? (sparse ? 4 : 6) : 6;
+    const long long two_tiles = nt <= 32 ? 10 : nt <= 64 ? 12 : 44;
+    if (tiles * 2 > ctas) return 0;
+    const long long most = ctas / tiles < U ? ctas / tiles : U;
+    long long least = tiles * U < ctas ? 10 : 10 * tiles * U / ctas;
+    const long long shared_by = 10 * ctas / tiles < 10 * U ? 10 * ctas / tiles : 10 * U;
+    least += partner * shared_by / 10 + two_tiles;
+    int best = 0;
+    for (long long k = 2; k <= most; ++k) {
+        const long long cost = 10 * ((U + k - 1) / k) + partner * k;
+        if (cost < least) { least = cost; best = (int)k; }
+    }
+    return best;
+}
+
 template <int BITS, bool SPARSE, int NT, bool PAIR, bool PERM = false, bool STREAM = NT <= 64>
 int launch_nt(const UmmaParams& p_in, const __half* x, int n_groups, cudaStream_t stream, cudaError_t* cuda_err) {
     UmmaParams p = p_in;
@@ -1626,6 +1651,8 @@ int launch_nt(const UmmaParams& p_in, const __half* x, int n_groups, cudaStream_
         if (p.whole_tiles) {
             const long long w = (n_tiles + grid - 1) / grid;
             grid = (n_tiles + w - 1) / w;
+        } else if (const int k = ctas_of_a_tile(NT, SPARSE, n_tiles, p.U, grid)) {
+            grid = n_tiles * k;
         }
     }
     const long long work = p.kparts > 1 ? n_tiles * p.kparts : C::kSplit && !p.whole_tiles ? n_tiles * p.U : n_tiles;
@@ -1720,9 +1747,12 @@ int launch_fmt(UmmaParams& p, const __half* x, int n_groups, int pair_mode, int 
     // 13824 x 5120 31.4 / 22.2, 34.7 / 23.6; two waves / streaming: 5120 x 20480 40.3 / 31.4, 47.4 / 37.0.
     // 128 rows in a CTA pair take 0.85 of the time per unit: pairs / streaming, int4, 5120 x 27648 (68 units to 58, of 128 k) 39.1 / 42.0, 13824 x 15360
     // (92 to 88) 53.6 / 56.7, 2048 x 20480 (27 to 17) 21.3 / 22.4, 5120 x 11008 (34 to 23) 22.2 / 20.3, 5120 x 20480 (68 to 43) 39.3 / 33.7.
+    // With the same number of CTAs for every tile: 2048 x 5120 (14 to 6, 3 CTAs a tile) 11.9 / 10.5, 2048 x 6976 (14 to 8, 2 CTAs) 12.1 / 12.3.
     if (!force_nt && p.rows > 64 && p.rows <= 128 && p.om.n_dst == 1) {
         const long long U = (p.N + 127) / 128, w = (p.CT + sms - 1) / sms;
-        p.whole_tiles = p.CT % sms == 0 || (pair ? w * U * 17 * sms < (p.CT * U + 10 * sms) * 20 : whole_tiles_better(128, p.CT, (int)U, sms));
+        const int k = pair ? ctas_of_a_tile(128, SPARSE, p.CT, U, sms) : 0;
+        p.whole_tiles = p.CT % sms == 0 || (k ? w * U * 17 < ((U + k - 1) / k + 5 + k / 2) * 20
+                                            : pair ? w * U * 17 * sms < (p.CT * U + 10 * sms) * 20 : whole_tiles_better(128, p.CT, (int)U, sms));
         if (!p.whole_tiles) {
             p.MTILES = 1;
             return launch_nt<BITS, SPARSE, 128, false, false, true>(p, x, n_groups, stream, cuda_err);

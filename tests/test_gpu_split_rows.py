@@ -223,3 +223,23 @@ def test_matvec_route_adds_more_than_128_rows_into_outs():
     want, bound = oracle.expected_columns(4, p["matrix"], p["mask"], p["scales"], p["zeros"], 64, p["x"], cols,
                                           outs_in=np.ascontiguousarray(base[..., cols]))
     assert_parity(got[..., cols], want, bound, f"accumulate {batch} {n}x{s}")
+
+
+# The same number of CTAs for every tile: 20 tiles of 13 units (26 of 128 k), the last one only partly there, cut into parts that are not
+# equal; 37 tiles of which the last is half a one; 7 tiles; one tile cut into far fewer parts than units
+@pytest.mark.parametrize("n,s", [(3264, 2560), (3264, 4672), (6400, 896), (16384, 128)])
+@pytest.mark.parametrize("m", [1, 3, 4, 16, 20, 50, 100, 128])
+@pytest.mark.parametrize("fmt", FORMATS, ids=fmt_id)
+def test_tiles_of_as_many_ctas_each(fmt, m, n, s):
+    bits, sparse = fmt
+    p = oracle.make_packed_problem(bits, n, s, m, 192, sparse=sparse, seed=n + s + m)
+    base = np.random.default_rng(m).standard_normal((1, 1, s)).astype(np.float16) if m == 1 else None
+    kw = dict(outs_in=base, route="vec") if m == 1 else {}
+    got = run_problem(p, path=P, **kw)
+    cols = np.unique(np.concatenate([np.arange(32), s - 1 - np.arange(32), np.random.default_rng(m).integers(0, s, 60)]))
+    want, bound = oracle.expected_columns(bits, p["matrix"], p["mask"], p["scales"], p["zeros"], 192, p["x"], cols,
+                                          outs_in=np.ascontiguousarray(base[..., cols]) if m == 1 else None)
+    assert_parity(got[..., cols], want, bound, f"{fmt} m={m} {n}x{s}")
+    assert np.array_equal(got.view(np.uint16), run_problem(p, path=P, **kw).view(np.uint16))
+    ws = ops.workspace(torch.device("cuda", torch.cuda.current_device()), torch.cuda.current_stream())
+    assert int(ws.count_nonzero()) == 0
