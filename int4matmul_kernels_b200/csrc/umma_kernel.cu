@@ -16,15 +16,15 @@
 //   MMA warp          one elected thread issues 8 (16) x tcgen05.mma (M = 128, N = NT, K = 16) per unit, A from tensor
 //                     memory, B from the swizzled shared-memory tile, and commits to mbarriers that recycle the
 //                     stages; the accumulator never leaves tensor memory until the tile is done
-//   epilogue          reads the accumulator (tcgen05.ld), converts to fp16 and stores: one warpgroup of its own for up to 64
-//                     rows (a CTA's last tile: from 2 rows on the dequant warpgroups as well, see last_epilogue), two warpgroups
-//                     of their own (half of the columns each) above
+//   epilogue          reads the accumulator (tcgen05.ld), converts to fp16 and stores: one warpgroup of its own in the
+//                     weight-streaming shapes (a CTA's last tile: from 2 rows on the dequant warpgroups as well, see last_epilogue),
+//                     two warpgroups of their own (half of the columns each) in the others
 //
-// Configurations (Cfg<NT, PAIR, STREAM>), one CTA per SM: NT <= 64 rows stream the weights once from HBM - 3 dequant warpgroups, 9 (6)
-// weight stages and 3 A / activation stages of 256 k, and the (tile, unit) space cut into equal ranges per CTA (split-K over the
-// whole GPU, partial tiles summed through scratch in a fixed order).  NT >= 128: whole tiles, epilogue stores transposed through
-// shared memory; by default launched as clusters of two CTAs that run each MMA together (cta_group::2, M = 256 over two SMs), see
-// PAIR below.
+// Configurations (Cfg<NT, PAIR, STREAM>), one CTA per SM: up to 64 rows stream the weights once from HBM - 3 dequant warpgroups, 9 (6)
+// weight stages and 3 A / activation stages of 256 k, and the (tile, unit) space cut into ranges of units, one per CTA (split-K over the
+// whole GPU, partial tiles summed through scratch in a fixed order).  More rows: either the same with NT = 128, units of 128 k and two
+// accumulators, or NT >= 128 in whole tiles (or K parts), epilogue stores transposed through shared memory, by default launched as
+// clusters of two CTAs that run each MMA together (cta_group::2, M = 256 over two SMs), see PAIR below; launch_fmt chooses.
 // Every wait is bounded and reports through the status word instead of hanging.
 #include "../../include/int4matmul_b200.h"
 
@@ -209,7 +209,8 @@ template <int NT, bool PAIR, bool STREAM = NT <= 64>
 struct Cfg {
     // packed-weight ring (128 k per stage).  Few rows: the kernel streams weights from HBM, and the ring has to
     // cover the DRAM latency; many rows: weights are a trickle next to the activation tiles
-    // Weight-streaming shapes: one CTA per SM with everything doubled, and K split over the CTAs.  They end at 64 rows.  Rows 33..64 had tiles
+    // Weight-streaming shapes: one CTA per SM with everything doubled, and K split over the CTAs: all of up to 64 rows, and NT = 128 where
+    // launch_fmt takes it.  Rows 33..64 had tiles
     // of 64 rows at two CTAs an SM, whole or with K cut into parts and a second launch: 48 rows 13824 x 5120 int4 25.7 us, now 18.8,
     // 16:32 38.1 / 22.0, int3 34.0 / 18.7, int2 33.1 / 17.4; 5120 x 20480 55.8 / 22.9, 53.8 / 29.7, 43.4 / 23.5, 42.7 / 22.4; 16384 x 16384
     // 66.3 / 44.3, 76.9 / 56.7, 59.9 / 43.5, 62.3 / 39.0; 1024 x 1024 8.9 / 7.8, 9.6 / 8.2, 9.0 / 7.8, 9.0 / 7.8; nothing was faster there.
@@ -227,7 +228,7 @@ struct Cfg {
     // A unit (one stage of every ring) is kHalves parts of 64 k.  The producers and the MMA issuer are single threads
     // whose loops cost ~500 cycles per stage whatever its size (an mbarrier wait ~190 cycles even when it is already
     // complete, expect_tx + the copy's issue another ~190): at 128 k per stage that alone is ~27 us for 16384 x 16384
-    // weights on 148 SMs, so the weight-streaming shapes use 256-k units.
+    // weights on 148 SMs, so the weight-streaming shapes use 256-k units (but NT = 128: 128 k, its activation stages would not fit).
     static constexpr int kHalves = NT <= 64 ? 4 : 2;
     static constexpr int kWStages = kStream ? (NT <= 16 || NT == 128 ? 9 : 6) : kDequantBound ? 6 : 3;
     // staging slots (units of look-ahead) for activation rows that are reordered on their way into the A / activation
@@ -253,7 +254,7 @@ struct Cfg {
     static constexpr int kAStageCols = 32 * kHalves;
     static constexpr int kColsUsed = kACol0 + kAStageCols * kABStages;
     static constexpr int kTmemCols = kColsUsed <= 256 ? 256 : 512;
-    // split-K over CTAs with a scratch reduction (more rows cut K into parts, see choose_kparts)
+    // split-K over CTAs with a scratch reduction (the other shapes cut K into parts, see choose_kparts)
     static constexpr bool kSplit = kStream;
     static constexpr int kSlotVecs = NT / 4 * 128;                    // one CTA's partial tile in the scratch: [4 rows][128 columns] of 16 bytes
     static constexpr int kSlots = NT <= 32 ? 1 : 2;                   // of those per CTA, see last_epilogue
@@ -1163,8 +1164,8 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                 for (int u = u0 + (int)(((uint32_t)wg + (uint32_t)C::kWG - si0 % (uint32_t)C::kWG) % (uint32_t)C::kWG); u < u1; u += C::kWG) {
                     Unit n;
                     if (!next_unit(u, n)) { ok = false; break; }
-                    uint32_t A[32];
                     if constexpr (C::kStream) {
+                        uint32_t A[32];
                         // Few rows are bound by this loop: by its instructions (per unit ~700 a scheduler with the other roles', and the half-precision
                         // pipe alone is busy for 650 cycles) and by the waits between its steps.  So the mode is voted before anything is
                         // decoded, for two groups at a time, the parts are straight-line code without a branch in between, and a unit is
@@ -1241,8 +1242,12 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                             const uint32_t zr = hadd2_u(hadd2_u(c.z2, kMagic1024), H2_N1024), zlo = c.z2 & 0xFFFFu;
                             return ((zlo | ((zlo & 0x7FFFu) + kBound) | c.s2) & 0x8000u) | (zr ^ c.z2);
                         };
+                        // (by a conversion and a multiply, 16:32 2048 rows 5120 x 20480 took 342.9 us, now 339.5)
                         auto zero_bytes = [&](ColK& c) {
-                            if (SPARSE) c.zb = __half2uint_rz(__ushort_as_half((unsigned short)(c.z2 & 0xFFFFu))) * 0x01010101u;
+                            if (SPARSE) {
+                                const uint32_t zi = hadd2_u(c.z2, kMagic1024);         // (integer zero-points: their value in the low bits)
+                                c.zb = prmt(zi, zi, 0x0000);
+                            }
                         };
                         // The parts are decoded in the fast mode; whether every group of the unit really is in it is voted once, when the last group
                         // has been read and before the weight stage is released.  If not, the unit is decoded again with a decision per part (the
@@ -1265,6 +1270,7 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                                     redo = true;
                                     break;
                                 }
+                                uint32_t A[32];
                                 decode_part<F, MODE_FAST>(words(n, h), masks(n, h), c, A, lut);
                                 if (h == H - 1) release_weights(n.ws);
                                 if (h == 0 && !acquire_a_stage(n, free_early)) { ok = false; break; }
@@ -1283,6 +1289,7 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                                     cur_row = row;
                                     load_group(row, c);
                                 }
+                                uint32_t A[32];
                                 if (!__any_sync(0xFFFFFFFFu, not_fast(c) != 0)) {
                                     zero_bytes(c);
                                     decode_part<F, MODE_FAST>(words(n, h), masks(n, h), c, A, lut);
@@ -1493,7 +1500,7 @@ bool encode_x_blocks_cached(CUtensorMap* out, const void* base, uint64_t rows, u
 
 constexpr long long kPartialBytes = 148LL * 4 * 32 * 128 * 8;      // for partial sums in the workspace (capi.cu sizes it)
 
-// More than 64 rows and tiles that fill less than half of the GPU: cut K into parts so that
+// Shapes of whole tiles (more than 64 rows), where these fill less than half of the GPU: cut K into parts so that
 // tiles x parts CTAs (pairs) run, as long as every part keeps at least 4 stages and the partial outputs fit the scratch.
 int choose_kparts(long long capacity, long long tiles, int U, long long rows, long long S) {
     if (tiles <= 0 || tiles * 2 > capacity) return 1;
