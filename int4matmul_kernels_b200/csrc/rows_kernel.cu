@@ -575,10 +575,10 @@ cudaError_t rows_launch_fmt(const RowsParams& p, int sms, int dev, cudaStream_t 
 // (6144) 49.1 -> 51.4, 2048 49.1 -> 48.6, 1536 (4096) 43.1 -> 39.8.
 // Very long columns: the last part adds the sums of hundreds of parts one after the other, 4 rows 65536 x 64 38.8 -> 30.1, 131072 x 64
 // 40.9 -> 57.6, 8 rows 32768 x 64 38.0 -> 31.8, 65536 x 64 42.9 -> 58.0.
-// The lines were drawn when one warpgroup of the tcgen05 kernel summed a shared tile (77, 99 us for the last two sizes above).  Against
-// the present one they hold for layers and lie too far out elsewhere: 4 and 8 rows of long columns (16384 x 1024 12.6 -> 14.4 and
-// 14.1 -> 23.5, 65536 x 256 25.1 -> 35.6 and 27.3 -> 65.8), one row alone of int3 and 16:32 from about 16 Mi weights on (5120^2 10.7 ->
-// 11.8 and 11.9 -> 12.8), of all but int2 from about 40 Mi, and 1984 x 19008 (11.9 -> 14.9).
+// The lines were drawn against an older tcgen05 kernel.  Against the present one (its figure first) they hold up to about 8 Mi weights - one row
+// int4 2688 x 2432 7.3 -> 5.4, int2 4224 x 1024 6.8 -> 5.3, 4 rows 16:32 4480 x 1344 9.2 -> 6.8 - and lie too far out above: one adding row, alone,
+// int4 5120^2 9.5 -> 11.2, int3 9.6 -> 11.8, 16:32 11.1 -> 12.8, 5..8 rows 7680 x 1472 8.8 -> 15.8.  With the zero-fill that an adding row mostly
+// follows, and on a first call with new buffers (tensor maps are encoded then), 5120^2 is level or faster here: 11.3 -> 10.8 in a graph, 28.5 -> 26.8.
 // (The bounds also keep step and tile numbers far inside 32 bits.)
 constexpr long long kMi = 1ll << 20;
 
