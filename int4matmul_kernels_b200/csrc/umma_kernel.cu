@@ -51,6 +51,7 @@ struct UmmaParams {
     const __half* scales;
     const __half* zeros;
     float* partials;
+    unsigned int* present;   // one word per CTA, all-zero between launches (see last_epilogue)
     int* status;
     int rows;            // all activation rows (B * M)
     int N, S;
@@ -299,12 +300,15 @@ __device__ __forceinline__ void store_rows(const OutMap& om, __half* out0, long 
     }
 }
 
-// The epilogue of the weight-streaming shapes (one row tile).  Split-K: the CTAs b_lo .. b_hi share a tile.  b_lo,
+// The epilogue of the weight-streaming shapes.  Split-K: the CTAs b_lo .. b_hi share a tile.  b_lo,
 // which owns its first units and reaches them last, adds the others' partial tiles to its own accumulator in CTA order - a fixed
-// order, so results are reproducible; the others wait for nobody.  A partial sum is a 32-bit word that is never zero (share_word), four rows of
+// order, so results are reproducible.  A partial sum is a 32-bit word that is never zero (share_word), four rows of
 // a column in one 16-byte store, so no fence, counter or second round trip is needed: a reader knows each word by itself, and clears
 // what it has read, which leaves the scratch all-zero for the next launch.  A CTA has at most one
 // tile that it shares and goes on from, before its last one, so there are two functions.
+// CTAs are numbered against the order in which blocks start (CTA b is block G - 1 - b), so b_lo waits only for blocks that started before it:
+// a launch gets through on however few SMs other streams leave it (with b_lo's block starting first, two were needed).  For the waits of more
+// than 32 rows see last_epilogue.
 // What a thread waits for are its loads, so fewer and wider ones count: with one 64-bit word (value | tag) per row, int4 16 rows 20480 x 5120
 // 22.3 us, now 19.7; 5120 x 5120 13.2 / 10.2; 16384 x 2048 17.0 / 12.4; 32 rows 25.1 / 21.1, 15.6 / 11.7, 20.4 / 14.9; one row 18.4 / 17.7, 10.3 / 9.7,
 // 12.7 / 11.5.
@@ -407,6 +411,7 @@ __device__ __noinline__ bool early_epilogue(const OutMap& om, int n_dst, long lo
 // Adds the shares of n partners, PB at a time, to the sums of NG groups of four rows (the first `here` of them are there) and clears them.
 // at(k, j): partner k's words of group j.  NG x PB loads are in flight, and everything that is missing is asked for again at once: word by word
 // each would cost a round trip of its own.
+constexpr uint32_t kShareSpins = 1u << 22;        // seconds: a poll is a round trip to L2
 template <int NG, int PB, class At>
 __device__ __forceinline__ void add_shares(float (&sum)[4 * NG], int n, int here, int* status, bool& waiting_ok, At at) {
 #pragma unroll 1
@@ -431,7 +436,7 @@ __device__ __forceinline__ void add_shares(float (&sum)[4 * NG], int n, int here
 #pragma unroll
                 for (int j = 0; j < NG; ++j) any |= missing(k, j);
             if (!any) break;
-            if (spins >= ptx::kSpinLimit) {                    // a contributor never delivered: report, stop waiting
+            if (spins >= kShareSpins) {                        // a contributor never delivered: report, stop waiting
                 atomicExch(status, 34);
                 waiting_ok = false;
             }
@@ -452,6 +457,45 @@ __device__ __forceinline__ void add_shares(float (&sum)[4 * NG], int n, int here
     }
 }
 
+// The CTAs that share a tile, and how many of them, from b_lo on, sum it
+struct TileCtas {
+    int b_lo, b_hi, members;
+    __device__ __forceinline__ int first_group(int groups, int member) const { return (groups * member + members - 1) / members; }
+};
+constexpr int kLeftWords = 10;                    // (see the assertion in launch_nt)
+constexpr uint32_t kLeaveSpins = 1u << 7;         // ~0.15 ms, far more than the starts of CTAs that do run side by side differ
+// CTA bb's slot, for up to 32 rows one, else two: its share of the tile that it shares and goes on from, and the one of its last tile
+template <int NT>
+__device__ __forceinline__ uint4* share_slot(uint4* slots, const TileCtas& ctas, int bb) {
+    return slots + (size_t)(NT > 32 ? 2 * bb + (bb < ctas.b_lo + ctas.members ? 1 : 0) : bb) * Cfg<NT, false, true>::kSlotVecs;
+}
+
+// The groups of member `r`, which left them to b_lo (see last_epilogue), this part of them: its own share is in its slot; the same sums in the same order.
+template <int NT>
+__device__ __noinline__ bool finish_for(const UmmaParams& p, __half* out, bool col_ok, int rows, uint4* slots, TileCtas ctas, int r, int part, int parts) {
+    bool waiting_ok = true;
+    const int groups = (rows + 3) / 4, lo = ctas.first_group(groups, r), n_groups = ctas.first_group(groups, r + 1) - lo, g_end = lo + n_groups * (part + 1) / parts;
+    const int who = ctas.b_lo + r;
+#pragma unroll 1
+    for (int g = lo + n_groups * part / parts; g < g_end; ++g) {
+        float sum[4] = {0.f, 0.f, 0.f, 0.f}, own[4] = {0.f, 0.f, 0.f, 0.f};
+        add_shares<1, 1>(sum, ctas.b_hi - ctas.b_lo, 1, p.status, waiting_ok,
+                         [&](int k, int) { return share_slot<NT>(slots, ctas, ctas.b_lo + k + (k >= r ? 1 : 0)) + g * 128; });
+        add_shares<1, 1>(own, 1, 1, p.status, waiting_ok, [&](int, int) { return share_slot<NT>(slots, ctas, who) + g * 128; });
+        __half* const out0 = out + (size_t)(4 * g) * p.om.ld;
+        const int n = col_ok ? min(4, rows - 4 * g) : 0;
+        __half h[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float f = own[i] + sum[i];
+            if (p.accumulate && i < n) f += __half2float(out0[(size_t)i * p.om.ld]);
+            h[i] = __float2half_rn(f);
+        }
+        store_rows<4>(p.om, out0, p.om.ld, p.om.n_dst, h, n);
+    }
+    return waiting_ok;
+}
+
 // A CTA's last tile: units t0 .. t0 + units - 1.  What bounds it is the number of dependent round trips to L2 (~0.7 us each) and the words a
 // CTA reads between the last MMA and the end of the launch, so the tile can be left to all of the CTA's warpgroups (the dequant warps
 // have nothing else to do by then), `part` of `parts` of its groups of four rows each.  (When: see spread_last.)
@@ -460,19 +504,18 @@ __device__ __forceinline__ void add_shares(float (&sum)[4 * NG], int n, int here
 // share it but one that goes on to the next tile, whose share came early - sum some groups each; a CTA writes its sums of the others'
 // groups and adds theirs to its own.  (us, b_lo alone / all: int4 48 rows 13824 x 5120 18.3 / 17.3, 128 rows 26.2 / 22.0, 5120 x 5120
 // 19.4 / 15.6; but 16 rows 2048 x 8192 8.7 / 9.3, 5120 x 6976 11.3 / 11.9.)
+// A member but b_lo so needs shares of blocks that start after it, and must not keep its SM from them.  b_lo's block starts last of all, and then
+// writes 1 into the `present` word of each member.  A member that does not find it within kLeaveSpins writes 2 and leaves: the share of its own
+// groups goes into its slot as well, and b_lo, which finds the 2, sums them in its place (finish_for).  Beside each other the CTAs of a tile have
+// settled this long before the last MMA; s_left says what was settled: a member's word 0 whether it leaves, b_lo's bits who has left.
 // bar_id, bar_threads: the named barrier at which the MMA warp says that the accumulator is complete (once per call, also where this
 // part has no rows).  Inlined: a call cost ~1 us here as well.
-// The CTAs that share it, and how many of them, from b_lo on, sum it
-struct TileCtas {
-    int b_lo, b_hi, members;
-};
 template <int NT>
 __device__ __forceinline__ bool last_epilogue(const OutMap& om, int n_dst, long long ld, __half* out, bool col_ok, int rows, int accumulate, uint4* slots, int* status,
-                                           TileCtas ctas, uint32_t acc, int part, int parts, uint32_t bar_id, uint32_t bar_threads, uint32_t s_abort) {
+                                           TileCtas ctas, const UmmaParams& p, const volatile uint32_t* s_left, uint32_t acc, int part, int parts, uint32_t bar_id, uint32_t bar_threads, uint32_t s_abort) {
     constexpr bool kAll = NT > 32;                             // every CTA whose last tile it is sums some groups
-    const int b_lo = ctas.b_lo, b_hi = ctas.b_hi, members = ctas.members, me = (int)blockIdx.x, groups = (rows + 3) / 4;
-    // A CTA's slot, or two: its share of the tile that it shares and goes on from, and the one of its last tile.
-    auto slot_of = [&](int bb) { return slots + (size_t)(kAll ? 2 * bb + (bb < b_lo + members ? 1 : 0) : bb) * Cfg<NT, false, true>::kSlotVecs; };
+    const int b_lo = ctas.b_lo, b_hi = ctas.b_hi, members = ctas.members, me = (int)(gridDim.x - 1 - blockIdx.x), groups = (rows + 3) / 4;
+    auto slot_of = [&](int bb) { return share_slot<NT>(slots, ctas, bb); };
     auto wait_accumulator = [&]() -> bool {
         __syncwarp();
         ptx::named_bar_sync(bar_id, bar_threads);      // released by the MMA warp once the accumulator is complete
@@ -541,13 +584,14 @@ __device__ __forceinline__ bool last_epilogue(const OutMap& om, int n_dst, long 
         }
     } else {
         // this CTA's groups [lo, hi); of those, this part's
-        const int rank = me - b_lo, lo = (groups * rank + members - 1) / members, hi = (groups * (rank + 1) + members - 1) / members;
+        const int rank = me - b_lo, lo = ctas.first_group(groups, rank), hi = ctas.first_group(groups, rank + 1);
         const int g_end = lo + (hi - lo) * (part + 1) / parts;
         int g = lo + (hi - lo) * part / parts;
         bool ready = false;
-        if (hi - lo < groups) {
+        if (members > 1) {
             if (!wait_accumulator()) return false;
             ready = true;
+            const bool leave = rank > 0 && s_left[0] != 0u;
             const int end = groups * (part + 1) / parts;
 #pragma unroll 1
             for (int j = groups * part / parts; j < end; j += 2) {
@@ -556,8 +600,9 @@ __device__ __forceinline__ bool last_epilogue(const OutMap& om, int n_dst, long 
                 ptx::tc_wait_ld();
 #pragma unroll
                 for (int k = 0; k < 2; ++k)
-                    if (j + k < end && (j + k < lo || j + k >= hi)) ptx::st_relaxed_gpu_v4(slot_of(me) + (j + k) * 128, share_group(v + 4 * k));
+                    if (j + k < end && (leave || j + k < lo || j + k >= hi)) ptx::st_relaxed_gpu_v4(slot_of(me) + (j + k) * 128, share_group(v + 4 * k));
             }
+            if (leave) return true;
         }
         // (once at least: every part meets the MMA warp)
         if (b_hi - b_lo <= 2) {
@@ -569,6 +614,11 @@ __device__ __forceinline__ bool last_epilogue(const OutMap& om, int n_dst, long 
                 if (!finish(integral_constant<int, 2>(), integral_constant<int, 4>(), g, g_end, ready)) return false;
             } while ((g += 2) < g_end);
         }
+        if (rank == 0) {
+#pragma unroll 1
+            for (int r = 1; r < members && waiting_ok; ++r)
+                if (s_left[r / 32] >> (r % 32) & 1u) waiting_ok = finish_for<NT>(p, out, col_ok, rows, slots, ctas, r, part, parts);
+        }
     }
     if (n_dst > 1) __threadfence_system();                // as in umma_kernel's epilogue
     return true;
@@ -579,8 +629,8 @@ __device__ __forceinline__ bool last_epilogue(const OutMap& om, int n_dst, long 
 // permuted k order (one row int4 35.5 / 37.0) and more rows, whose call keeps more registers (48 rows 5120 x 6976 int4 13.3 / 15.5).
 template <int NT>
 __device__ __noinline__ bool last_epilogue_call(const OutMap& om, int n_dst, long long ld, __half* out, bool col_ok, int rows, int accumulate, uint4* slots, int* status,
-                                                TileCtas ctas, uint32_t acc, int part, int parts, uint32_t bar_id, uint32_t bar_threads, uint32_t s_abort) {
-    return last_epilogue<NT>(om, n_dst, ld, out, col_ok, rows, accumulate, slots, status, ctas, acc, part, parts, bar_id, bar_threads, s_abort);
+                                                TileCtas ctas, const UmmaParams& p, const volatile uint32_t* s_left, uint32_t acc, int part, int parts, uint32_t bar_id, uint32_t bar_threads, uint32_t s_abort) {
+    return last_epilogue<NT>(om, n_dst, ld, out, col_ok, rows, accumulate, slots, status, ctas, p, s_left, acc, part, parts, bar_id, bar_threads, s_abort);
 }
 
 // PAIR: launched as clusters of two CTAs (two SMs) that run every MMA together (cta_group::2, M = 256): the pair's
@@ -610,6 +660,8 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
     __shared__ __align__(8) Barriers bars;
     __shared__ uint32_t lut[SPARSE ? kSparseLutEntries : 1];
     __shared__ uint32_t tmem_base_smem;
+    __shared__ struct { TileCtas ctas; int ct, mt; uint32_t buf; } s_last;      // (weight-streaming shapes)
+    __shared__ volatile uint32_t s_left[C::kStream && NT > 32 ? kLeftWords : 1];
     __shared__ volatile int s_abort;     // set by a warp that gives up on the accumulator (the MMA warp before it releases the epilogue
                                          // warps for the last time; an epilogue warp before its group's next named barrier)
 
@@ -680,7 +732,8 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
     const long long U = p.U;
     const int CTd = PAIR ? (p.CT + 1) / 2 : p.CT;                  // column tiles of a CTA, or column-tile pairs of a CTA pair
     const long long n_tiles = (long long)p.MTILES * CTd;
-    const long long G = PAIR ? gridDim.x / 2 : gridDim.x, b = PAIR ? blockIdx.x / 2 : blockIdx.x;
+    // (weight-streaming shapes: numbered against the order in which blocks start, see early_epilogue)
+    const long long G = PAIR ? gridDim.x / 2 : gridDim.x, b = PAIR ? blockIdx.x / 2 : C::kStream ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
     // tile index -> this CTA's column tile (may lie past the last one in a pair: loads are zero-filled, stores masked) and row tile
     // Column tiles vary fastest.  (Row tiles fastest would read each packed-weight tile from HBM only once, but then every
     // SM asks L2 for the same activation lines at the same moment, and that hot spot cost 3-25 % when measured.)
@@ -1067,12 +1120,53 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
             return true;
         };
 
+        // Weight-streaming shapes: where this CTA's last tile is and who shares it, by one warp while nothing has arrived yet.  (It is ~1500 cycles of
+        // divisions.  Done by every warp before its last tile it cost up to 1 us where that tile is short: int4 16 rows 5120 x 5120 10.2 us, now 9.7,
+        // 16:32 5120 x 20480 26.2 / 24.6, int4 48 rows 2048 x 8192 9.9 / 9.4, 128 rows 5120 x 20480 33.4 / 31.9.)
+        if constexpr (C::kStream) {
+            if (warp == kEpiWarp0 && t_lo < t_hi) {
+                const long long tile = div_nn(t_hi - 1, U), lo_t = tile * U;
+                TileCtas ctas{(int)b, (int)b, 1};
+                if (t_lo > lo_t || t_hi < lo_t + U) {
+                    ctas.b_lo = range_owner(n_tiles * U, G, lo_t);
+                    ctas.b_hi = range_owner(n_tiles * U, G, lo_t + U - 1);
+                    if (NT > 32) ctas.members = ctas.b_hi - ctas.b_lo + (range_lo(n_tiles * U, G, ctas.b_hi + 1) == lo_t + U ? 1 : 0);
+                }
+                if (lane == 0) s_last = {ctas, tile_ct(tile), tile_mt(tile), C::kDBufs == 1 ? 0u : (uint32_t)(tile - div_nn(t_lo, U)) % C::kDBufs};
+            }
+            ptx::named_bar_sync(7, (C::kWG + 1) * 128);
+        }
+        // One warp of every CTA that sums a shared tile with others; b_lo as it starts, the other members before their last tile
+        auto settle_presence = [&](bool start) {
+            if (warp != kEpiWarp0 || t_lo >= t_hi) return;
+            const TileCtas ctas = s_last.ctas;
+            if (ctas.members <= 1 || start != (b == ctas.b_lo)) return;
+            ptx::grid_dependency_wait();                   // (the words may still be in use by the kernel before this one)
+            if (start) {
+#pragma unroll 1
+                for (int r0 = 0; r0 < ctas.members; r0 += 32) {
+                    const int r = r0 + lane;
+                    const bool gone = r > 0 && r < ctas.members && atomicExch(p.present + b + r, 1u) == 2u;
+                    if (gone) atomicExch(p.present + b + r, 0u);
+                    const uint32_t bits = __ballot_sync(0xFFFFFFFFu, gone);
+                    if (lane == 0) s_left[r0 / 32] = bits;
+                }
+            } else if (lane == 0) {
+                uint32_t seen;
+                for (uint32_t spins = 0; (seen = atomicCAS(p.present + b, 0u, spins < kLeaveSpins ? 0u : 2u)) == 0u && spins < kLeaveSpins; ++spins) __nanosleep(500);
+                if (seen != 0u) atomicExch(p.present + b, 0u);
+                s_left[0] = seen == 0u;
+            }
+            __syncwarp();
+        };
+
         uint32_t seg = 0;
         bool aborted = false;                                              // a wait timed out (weight-streaming shapes)
         if (warp >= kEpiWarp0 + 4 * kEpiGroups) {
             // (an epilogue warpgroup that this configuration does not use)
         } else if (warp >= kEpiWarp0) {
             // ----- dedicated epilogue warps: one pass per segment -----
+            if constexpr (C::kStream && NT > 32) settle_presence(true);
             for (long long t = t_lo; t < t_hi;) {
                 const long long tile = div_nn(t, U);
                 const int u0 = (int)(t - tile * U);
@@ -1092,6 +1186,9 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                 } else if (!epilogue(seg, tile)) break;
                 ++seg;
                 t += u1 - u0;
+            }
+            if constexpr (C::kStream && NT > 32) {
+                if (!aborted) settle_presence(false);
             }
         } else {
             // ----- dequant warps -----
@@ -1318,19 +1415,13 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
             } else if (spread_last || (warp >= kEpiWarp0 && t_lo < t_hi)) {
                 // outputs, old outputs and the scratch may still be in use by the kernel before this one in the stream
                 ptx::grid_dependency_wait();
-                const long long tile = div_nn(t_hi - 1, U), lo_t = tile * U;
-                const uint32_t buf = C::kDBufs == 1 ? 0u : (uint32_t)(tile - div_nn(t_lo, U)) % C::kDBufs;
-                TileCtas ctas{(int)b, (int)b, 1};
-                if (t_lo > lo_t || t_hi < lo_t + U) {
-                    ctas.b_lo = range_owner(n_tiles * U, G, lo_t);
-                    ctas.b_hi = range_owner(n_tiles * U, G, lo_t + U - 1);
-                    if (NT > 32) ctas.members = ctas.b_hi - ctas.b_lo + (range_lo(n_tiles * U, G, ctas.b_hi + 1) == lo_t + U ? 1 : 0);
-                }
-                const int col = (warp & 3) * 32 + lane, scol = tile_ct(tile) * 128 + col, row0 = tile_mt(tile) * NT;
+                const TileCtas ctas = s_last.ctas;
+                const uint32_t buf = C::kDBufs == 1 ? 0u : s_last.buf;
+                const int col = (warp & 3) * 32 + lane, scol = s_last.ct * 128 + col, row0 = s_last.mt * NT;
                 const bool col_ok = scol < p.S;
                 auto run = [&](auto epilogue) {
                     epilogue(p.om, p.om.n_dst, p.om.ld, p.om.dst[0] + (size_t)row0 * p.om.ld + (col_ok ? p.om.col(scol) : 0), col_ok, min(NT, p.rows - row0),
-                             p.accumulate, reinterpret_cast<uint4*>(p.partials) + col, p.status, ctas,
+                             p.accumulate, reinterpret_cast<uint4*>(p.partials) + col, p.status, ctas, p, s_left,
                              tmem_base + buf * C::kDCols + ((uint32_t)((warp & 3) * 32) << 16), spread_last ? warp >> 2 : 0, spread_last ? C::kWG + 1 : 1,
                              spread_last ? 5 : 2 + 4 * buf, spread_last ? kSpreadThreads : 128 + 32, ptx::smem_u32(const_cast<int*>(&s_abort)));
                 };
@@ -1664,6 +1755,7 @@ int launch_nt(const UmmaParams& p_in, const __half* x, int n_groups, cudaStream_
     }
     const long long work = p.kparts > 1 ? n_tiles * p.kparts : C::kSplit && !p.whole_tiles ? n_tiles * p.U : n_tiles;
     if (grid > work || p.kparts > 1) grid = work;
+    static_assert(NT <= 32 || !C::kSplit || kPartialBytes / (C::kSlots * C::kSlotVecs * 16) <= 32 * kLeftWords, "last_epilogue: a bit per CTA");
     if (C::kSplit && grid > kPartialBytes / (C::kSlots * C::kSlotVecs * 16)) grid = kPartialBytes / (C::kSlots * C::kSlotVecs * 16);   // partial tiles in the scratch
     {
         // The kernel may start while the kernel before it in the stream is still running: its set-up overlaps that
@@ -1827,6 +1919,7 @@ int umma_launch(int bits, bool sparse, const StreamParams& sp, int total_rows, i
     p.scales = sp.scales;
     p.zeros = sp.zeros;
     p.partials = sp.partials;
+    p.present = sp.counters;
     p.status = sp.status;
     p.rows = total_rows;
     p.N = sp.N;
