@@ -614,10 +614,12 @@ __device__ __forceinline__ bool last_epilogue(const OutMap& om, int n_dst, long 
                 if (!finish(integral_constant<int, 2>(), integral_constant<int, 4>(), g, g_end, ready)) return false;
             } while ((g += 2) < g_end);
         }
-        if (rank == 0) {
+        if (rank == 0 && members > 1) {                // (s_left is written then)
 #pragma unroll 1
-            for (int r = 1; r < members && waiting_ok; ++r)
-                if (s_left[r / 32] >> (r % 32) & 1u) waiting_ok = finish_for<NT>(p, out, col_ok, rows, slots, ctas, r, part, parts);
+            for (int r0 = 0; r0 < members; r0 += 32)
+#pragma unroll 1
+                for (uint32_t left = s_left[r0 / 32]; left != 0u && waiting_ok; left &= left - 1u)
+                    waiting_ok = finish_for<NT>(p, out, col_ok, rows, slots, ctas, r0 + __ffs((int)left) - 1, part, parts);
         }
     }
     if (n_dst > 1) __threadfence_system();                // as in umma_kernel's epilogue
