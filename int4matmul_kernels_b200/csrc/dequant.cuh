@@ -6,7 +6,8 @@
 
 namespace i4mm {
 
-enum : int { MODE_FAST = 0, MODE_GENERAL = 1, MODE_SLOW = 2 };
+// MODE_WIDE: 16:32 only, the fast mode for zero-points up to 255
+enum : int { MODE_FAST = 0, MODE_GENERAL = 1, MODE_SLOW = 2, MODE_WIDE = 3 };
 
 // (mask & a) | (~mask & b)
 __device__ __forceinline__ uint32_t bit_select(uint32_t mask, uint32_t a, uint32_t b) {
@@ -35,7 +36,7 @@ struct ColK {
 // v = (1024 + q_lo * 2^a, 1024 + q_hi * 2^b) -> the two fp16 weights.  mul / base undo the two shifts exactly.
 template <int BITS, int MODE>
 __device__ __forceinline__ uint32_t finish(uint32_t v, uint32_t mul, uint32_t base, uint32_t off, const ColK& c) {
-    if (MODE == MODE_FAST) return hmul2_u(hfma2_u(v, mul, off), c.s2);         // off = base - zero
+    if (MODE == MODE_FAST || MODE == MODE_WIDE) return hmul2_u(hfma2_u(v, mul, off), c.s2);         // off = base - zero
     const uint32_t q = hfma2_u(v, mul, base);                                  // exact integers
     if (MODE == MODE_GENERAL) return hmul2_u(hsub2_u(q, c.z2), c.s2);
     const __half2 qh = u32_as_h2(q);
@@ -87,19 +88,24 @@ __device__ __forceinline__ void sparse_expand(uint32_t& lo, uint32_t& hi, uint32
     // instructions of five per 4 positions: one row 16384 x 16384 57.3 -> 54.4 us, 2048 rows 5120 x 20480 350.5 -> 340.4; few-row
     // kernel 2048 x 5632 1 row 8.4 -> 8.1, 8 rows 11.6 -> 11.4, of 24 sizes only 2048 x 2048 with 5..8 rows is slower, 8.0 -> 8.1)
     const uint32_t flip = MODE == MODE_FAST ? c.zb : 0u;
-    const uint32_t even = and_xor(lo, 0x0F0F0F0Fu, flip), odd = and_xor(lo >> 4, 0x0F0F0F0Fu, flip);
+    uint32_t even = and_xor(lo, 0x0F0F0F0Fu, flip), odd = and_xor(lo >> 4, 0x0F0F0F0Fu, flip), pick = sel;
     const uint32_t off = hsub2_u(BASE_1_1, c.z2);
+    if (MODE == MODE_WIDE) {
+        // No XOR brings both a kept byte (below 128) and a dropped one right here.  But where a position is dropped, the eighth nibble is not
+        // used: the zero-point takes its place, and dropped positions select it instead of 8.
+        odd = prmt(odd, c.zb, byte4 == 0x3FCu ? 0x3210u : 0x4210u);
+        pick = sel - ((sel >> 3) & 0x11111111u);
+    }
 #pragma unroll
     for (int q4 = 0; q4 < 2; ++q4) {
-        const uint32_t s = q4 ? sel >> 16 : sel;                                         // (PRMT reads the low 16 bits)
+        const uint32_t s = q4 ? pick >> 16 : pick;                                       // (PRMT reads the low 16 bits)
         const uint32_t d = prmt(even, odd, s) ^ flip;
         A[2 * q4] = finish<4, MODE>(prmt(d, 0x64646464u, 0x5140), MUL_1_1, BASE_1_1, off, c);
         A[2 * q4 + 1] = finish<4, MODE>(prmt(d, 0x64646464u, 0x7362), MUL_1_1, BASE_1_1, off, c);
-        if (MODE != MODE_FAST) {                                                         // exact zeros at dropped positions
-            const uint32_t keep = prmt(0x7F7F7F7Fu, 0x7F7F7F7Fu, s);
-            const uint32_t k = keep * 2u + (keep & 0x01010101u);                         // 0x7F -> 0xFF
-            A[2 * q4] &= prmt(k, k, 0x1100);
-            A[2 * q4 + 1] &= prmt(k, k, 0x3322);
+        if (MODE == MODE_GENERAL || MODE == MODE_SLOW) {                                 // exact zeros at dropped positions
+            const uint32_t k = prmt(0x7F7F7F7Fu, 0x7F7F7F7Fu, s) << 1;                   // kept 0xFE, dropped 0x00: the sign says which
+            A[2 * q4] &= prmt(k, k, 0x9988);
+            A[2 * q4 + 1] &= prmt(k, k, 0xBBAA);
         }
     }
     const uint32_t used = 4u * (uint32_t)__popc(byte4);                                  // bits of the stream, up to 32

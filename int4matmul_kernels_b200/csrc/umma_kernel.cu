@@ -205,6 +205,7 @@ constexpr int kMaxABStages = 6;
 // the largest one = 0x7FFF.
 template <bool SPARSE>
 constexpr uint32_t kFastBound = SPARSE ? 0x280Fu : 0x1FFFu;
+constexpr uint32_t kWideBound = 0x2407u;          // MODE_WIDE: up to 255
 
 template <int NT, bool PAIR, bool STREAM = NT <= 64>
 struct Cfg {
@@ -1256,7 +1257,7 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                 auto words = [&](const Unit& n, int h) -> uint32_t { return n.st + WS::kW + h * (F::WROWS * 512) + col * 4; };
                 auto masks = [&](const Unit& n, int h) -> uint32_t { return n.st + WS::kMask + h * (F::MROWS * 512) + col * 4; };
                 auto a_cols = [&](const Unit& n, int h) -> uint32_t { return lane_addr + C::kACol0 + n.as * C::kAStageCols + h * 32; };
-                // Fast mode: scale signs clear, zero-points integers in [0, 512] (16:32: see kFastBound), for every column of the
+                // Fast mode: scale signs clear, zero-points integers in [0, 512] (16:32: see kFastBound and kWideBound), for every column of the
                 // warp in every group of the unit.
                 constexpr uint32_t kBound = kFastBound<SPARSE>;
                 // this warpgroup's units of the segment: those whose stage index is congruent to wg modulo kWG
@@ -1287,7 +1288,9 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                             nf |= not_fast_bits<kBound>(sp[i], zp[i], zi[i]);
                         }
                         // A unit that is not in the fast mode, with a decision per part: rolled (one body of each mode in the instruction
-                        // cache), half a part at a time, so that these modes do not set the register count of the straight-line code.
+                        // cache), half a part at a time, so that these modes do not set the register count of the straight-line code.  Its fast mode
+                        // of 16:32 is the wide one.  (us, zero-points 128..255 by the general mode / by this one: 48 rows 16384 x 16384 85 / 71, 13824 x 5120
+                        // 28.9 / 25.3, one row 16384 x 16384 80 / 68.)
                         auto decode_by_part = [&]() {
 #pragma unroll 1
                             for (int h = 0; h < H; ++h) {
@@ -1297,12 +1300,12 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                                 c.s2 = dup_lo(s);
                                 c.z2 = dup_lo(z);
                                 c.zb = SPARSE ? prmt(zi, zi, 0x0000) : 0u;
-                                const bool fast = !__any_sync(0xFFFFFFFFu, (not_fast_bits<kBound>(s, z, zi) & 0xFFFFu) != 0);
+                                const bool fast = !__any_sync(0xFFFFFFFFu, (not_fast_bits<SPARSE ? kWideBound : kBound>(s, z, zi) & 0xFFFFu) != 0);
                                 const bool lin = __all_sync(0xFFFFFFFFu, __hge(__ushort_as_half((unsigned short)s), __ushort_as_half(0)));
 #pragma unroll 1
                                 for (int half = 0; half < 2; ++half) {
                                     uint32_t A[16];
-                                    if (fast) F::template decode<MODE_FAST>(words(n, h), masks(n, h), half, c, A, lut);
+                                    if (fast) F::template decode<SPARSE ? MODE_WIDE : MODE_FAST>(words(n, h), masks(n, h), half, c, A, lut);
                                     else if (lin) F::template decode<MODE_GENERAL>(words(n, h), masks(n, h), half, c, A, lut);
                                     else F::template decode<MODE_SLOW>(words(n, h), masks(n, h), half, c, A, lut);
                                     ptx::tmem_st16(a_cols(n, h) + 16 * half, A);
