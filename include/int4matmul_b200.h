@@ -15,8 +15,9 @@
  *   scales  fp16  (n_groups, S)      scale >= 0: W = (q - zero) * scale, both steps rounded to fp16
  *   zeros   fp16  (n_groups, S)      scale <  0: W = fma(+-2^(q & (2^(bits-1)-1)), -scale, zero)
  *                                    Any zero-point is exact.  The fastest decode takes scales >= 0 with integer zero-points
- *                                    0 .. 512 (16:32: 0 .. 127); with others >= 0 a call takes up to 1.6 times as long (one row
- *                                    16384^2: int4 35 and 52 us; 16:32 51 and 80, with integers up to 255 68).
+ *                                    0 .. 512 (16:32: 0 .. 127).  With others up to about 128 rows take up to 1.6 times as long (one
+ *                                    row 16384^2: int4 35 and 52 us; 16:32 51 and 78, with integers up to 255 67), with scales < 0
+ *                                    up to twice (every second group: 70 and 94); 512 rows int4 1.1 and 3 times.
  *   out     fp16  (rows, S)
  *   group_size  positive multiple of 64, or negative for "one group over all of N"
  *   N, S multiples of 64.  sparse is only defined for bits == 4.

@@ -6,8 +6,9 @@
 
 namespace i4mm {
 
-// MODE_WIDE: 16:32 only, the fast mode for zero-points up to 255
-enum : int { MODE_FAST = 0, MODE_GENERAL = 1, MODE_SLOW = 2, MODE_WIDE = 3 };
+// MODE_WIDE: 16:32 only, the fast mode for zero-points up to 255.  MODE_SLOW, MODE_EITHER: either coding by the column, the first by conversions, weight
+// by weight.
+enum : int { MODE_FAST = 0, MODE_GENERAL = 1, MODE_SLOW = 2, MODE_WIDE = 3, MODE_EITHER = 4 };
 
 // (mask & a) | (~mask & b)
 __device__ __forceinline__ uint32_t bit_select(uint32_t mask, uint32_t a, uint32_t b) {
@@ -39,6 +40,14 @@ __device__ __forceinline__ uint32_t finish(uint32_t v, uint32_t mul, uint32_t ba
     if (MODE == MODE_FAST || MODE == MODE_WIDE) return hmul2_u(hfma2_u(v, mul, off), c.s2);         // off = base - zero
     const uint32_t q = hfma2_u(v, mul, base);                                  // exact integers
     if (MODE == MODE_GENERAL) return hmul2_u(hsub2_u(q, c.z2), c.s2);
+    if (MODE == MODE_EITHER) {
+        // dequant_dynamic for both halves, +-2^(q & EXP) put together from its bits
+        constexpr uint32_t SGN = 0x10001u << (BITS - 1), EXP = SGN - 0x10001u;
+        const uint32_t qi = hadd2_u(q, kMagic1024);                            // q in the low bits
+        const uint32_t power = (((qi & EXP) << 10) + 0x3C003C00u) | ((qi & SGN) << (16 - BITS));
+        const uint32_t lin = hmul2_u(hsub2_u(q, c.z2), c.s2), expo = hfma2_u(power, c.s2 ^ 0x80008000u, c.z2);
+        return __hge(__ushort_as_half((unsigned short)(c.s2 & 0xFFFFu)), __ushort_as_half(0)) ? lin : expo;
+    }
     const __half2 qh = u32_as_h2(q);
     const __half s = __ushort_as_half((unsigned short)(c.s2 & 0xFFFFu));
     const __half z = __ushort_as_half((unsigned short)(c.z2 & 0xFFFFu));
@@ -102,7 +111,7 @@ __device__ __forceinline__ void sparse_expand(uint32_t& lo, uint32_t& hi, uint32
         const uint32_t d = prmt(even, odd, s) ^ flip;
         A[2 * q4] = finish<4, MODE>(prmt(d, 0x64646464u, 0x5140), MUL_1_1, BASE_1_1, off, c);
         A[2 * q4 + 1] = finish<4, MODE>(prmt(d, 0x64646464u, 0x7362), MUL_1_1, BASE_1_1, off, c);
-        if (MODE == MODE_GENERAL || MODE == MODE_SLOW) {                                 // exact zeros at dropped positions
+        if (MODE != MODE_FAST && MODE != MODE_WIDE) {                                    // exact zeros at dropped positions
             const uint32_t k = prmt(0x7F7F7F7Fu, 0x7F7F7F7Fu, s) << 1;                   // kept 0xFE, dropped 0x00: the sign says which
             A[2 * q4] &= prmt(k, k, 0x9988);
             A[2 * q4 + 1] &= prmt(k, k, 0xBBAA);

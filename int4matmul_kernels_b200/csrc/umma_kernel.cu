@@ -1271,10 +1271,10 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                         // decoded, for two groups at a time, the parts are straight-line code without a branch in between, and a unit is
                         // announced as soon as it is written.  (With a branch per part on a new group, the vote at the last part, the other modes'
                         // 32 registers beside it, and the announcement put off to the warpgroup's next unit: one row 16384 x 16384 int4 37.2 us,
-                        // 16:32 52.4, int3 40.5, int2 37.3; now 35.9, 51.5, 39.1, 33.8.  General mode, which decoded twice: 66, 111, 79, 71; now
-                        // 53, 86, 62, 63; every second group in the exponent coding: 176, 208, 180, 142; now 181, 194, 179, 126.  Not better: the parts
-                        // as a loop of two iterations (36.8, 52.9, 41.6, 36.4); two warpgroups with 128 registers; an MMA warp, an accumulator and
-                        // half-stages for each warpgroup.  The shapes below, which wait for other things, do not gain.)
+                        // 16:32 52.4, int3 40.5, int2 37.3; now 35.4, 51.0, 39.1, 33.0.  General mode, which decoded twice: 66, 111, 79, 71; now
+                        // 52, 78, 60, 57.  Not better: the parts as a loop of two iterations (36.8, 52.9, 41.6, 36.4, with 35.9, 51.5, 39.1, 33.8 at the
+                        // time); two warpgroups with 128 registers; an MMA warp, an accumulator and half-stages for each warpgroup.  The shapes below,
+                        // which wait for other things, do not gain.)
                         uint32_t sp[H / 2], zp[H / 2], zi[H / 2], nf = 0;           // two parts' scales, zero-points, zero-points + 1024
 #pragma unroll
                         for (int h = 0; h < H; h += 2) {
@@ -1291,6 +1291,9 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                         // cache), half a part at a time, so that these modes do not set the register count of the straight-line code.  Its fast mode
                         // of 16:32 is the wide one.  (us, zero-points 128..255 by the general mode / by this one: 48 rows 16384 x 16384 85 / 71, 13824 x 5120
                         // 28.9 / 25.3, one row 16384 x 16384 80 / 68.)
+                        // Every second group in the exponent coding, one row 16384 x 16384: by conversions int4 180, 16:32 192, int3 179, int2 126, now
+                        // 70, 94, 76, 72.  (The other shapes keep the conversions: beside this mode their general one takes longer, int4 512 rows
+                        // 5120 x 20480 106.6 / 109.6, int3 124.5 / 133.6.)
                         auto decode_by_part = [&]() {
 #pragma unroll 1
                             for (int h = 0; h < H; ++h) {
@@ -1307,7 +1310,7 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                                     uint32_t A[16];
                                     if (fast) F::template decode<SPARSE ? MODE_WIDE : MODE_FAST>(words(n, h), masks(n, h), half, c, A, lut);
                                     else if (lin) F::template decode<MODE_GENERAL>(words(n, h), masks(n, h), half, c, A, lut);
-                                    else F::template decode<MODE_SLOW>(words(n, h), masks(n, h), half, c, A, lut);
+                                    else F::template decode<MODE_EITHER>(words(n, h), masks(n, h), half, c, A, lut);
                                     ptx::tmem_st16(a_cols(n, h) + 16 * half, A);
                                 }
                                 if (h == H - 1) release_weights(n.ws);
