@@ -51,7 +51,6 @@ struct UmmaParams {
     const __half* scales;
     const __half* zeros;
     float* partials;
-    unsigned int* present;   // one word per CTA, all-zero between launches (see last_epilogue)
     int* status;
     int rows;            // all activation rows (B * M)
     int N, S;
@@ -59,11 +58,13 @@ struct UmmaParams {
     int CT;              // column tiles: ceil(S / 128)
     int MTILES;          // row tiles: ceil(rows / NT)
     int accumulate;
-    int whole_tiles;     // no tile is shared (weight-streaming shapes), nor K cut into parts (the others)
     int overlap;         // weight-side tensors may be read while the kernel before this one is still running
     int kparts;          // > 1: every tile's K range is cut into this many parts, one CTA (pair) each, fp32 partial outputs
                          // go to the scratch as (part, row, S) and kparts_reduce_kernel sums them (more than 64 rows only)
     GroupDiv gdiv;
+    // (last: where they lay before gdiv, 128 rows on CTA pairs took 2..3 % longer in int4 and int3, 5120 x 27648 39.4 us, now 38.2)
+    int whole_tiles;     // no tile is shared (weight-streaming shapes), nor K cut into parts (the others)
+    unsigned int* present;   // one word per CTA, all-zero between launches (see last_epilogue)
 };
 
 // ---- formats: one 64-k part of one column -> 32 registers of fp16 pairs -----------------------------------------
