@@ -30,10 +30,10 @@ bool umma_supported(int bits, bool sparse, int total_rows, int N, int S);
 
 namespace {
 
-constexpr size_t kCounterBytes = 256 * 1024;          // column-tile counters; the last 64 bytes hold the status word
-constexpr size_t kStatusOffset = kCounterBytes - 64;
-constexpr int kMaxStreamCtas = 148 * 4;               // upper bound on the CTAs of the streaming kernel (sizes the scratch)
-constexpr size_t kPartialBytes = (size_t)kMaxStreamCtas * 2 * 32 * 128 * sizeof(float);
+using i4mm::kCounterBytes;
+using i4mm::kMaxStreamCtas;
+using i4mm::kPartialBytes;
+using i4mm::kStatusOffset;
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 

@@ -14,6 +14,12 @@ namespace i4mm {
 
 constexpr int kSingleGroup = 0x0FFFFFFF;   // group_size < 0 (matmul_kernel.cu:379-381)
 
+// ---- the workspace: [column-tile counters, with the status word in their last 64 bytes][partial sums] --------
+constexpr size_t kCounterBytes = 256 * 1024;
+constexpr size_t kStatusOffset = kCounterBytes - 64;
+constexpr int kMaxStreamCtas = 148 * 4;               // upper bound on the CTAs of the streaming kernel, two slots of 32 x 128 sums each
+constexpr size_t kPartialBytes = (size_t)kMaxStreamCtas * 2 * 32 * 128 * sizeof(float);
+
 // ---- raw half2 arithmetic on 32-bit registers ------------------------------------------------
 __device__ __forceinline__ uint32_t h2_as_u32(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
 __device__ __forceinline__ __half2 u32_as_h2(uint32_t u) { return *reinterpret_cast<__half2*>(&u); }

@@ -1598,8 +1598,6 @@ bool encode_x_blocks_cached(CUtensorMap* out, const void* base, uint64_t rows, u
     return true;
 }
 
-constexpr long long kPartialBytes = 148LL * 4 * 32 * 128 * 8;      // for partial sums in the workspace (capi.cu sizes it)
-
 // Shapes of whole tiles (more than 64 rows), where these fill less than half of the GPU: cut K into parts so that
 // tiles x parts CTAs (pairs) run, as long as every part keeps at least 4 stages and the partial outputs fit the scratch.
 int choose_kparts(long long capacity, long long tiles, int U, long long rows, long long S) {
@@ -1607,7 +1605,7 @@ int choose_kparts(long long capacity, long long tiles, int U, long long rows, lo
     long long f = capacity / tiles;
     if (f > 8) f = 8;
     if (f > U / 4) f = U / 4;
-    while (f > 1 && f * rows * S * 4 > kPartialBytes) --f;
+    while (f > 1 && f * rows * S * 4 > (long long)kPartialBytes) --f;
     return f < 2 ? 1 : (int)f;
 }
 
@@ -1764,8 +1762,10 @@ int launch_nt(const UmmaParams& p_in, const __half* x, int n_groups, cudaStream_
     }
     const long long work = p.kparts > 1 ? n_tiles * p.kparts : C::kSplit && !p.whole_tiles ? n_tiles * p.U : n_tiles;
     if (grid > work || p.kparts > 1) grid = work;
-    static_assert(NT <= 32 || !C::kSplit || kPartialBytes / (C::kSlots * C::kSlotVecs * 16) <= 32 * kLeftWords, "last_epilogue: a bit per CTA");
-    if (C::kSplit && grid > kPartialBytes / (C::kSlots * C::kSlotVecs * 16)) grid = kPartialBytes / (C::kSlots * C::kSlotVecs * 16);   // partial tiles in the scratch
+    constexpr long long kMostCtas = kPartialBytes / (C::kSlots * C::kSlotVecs * 16);       // those whose shares the scratch holds
+    static_assert(!C::kSplit || kMostCtas >= 148, "every SM of the GPU has its slots");
+    static_assert(NT <= 32 || !C::kSplit || (kMostCtas <= 32 * kLeftWords && kMostCtas * 4 <= kStatusOffset), "last_epilogue: a bit and a word per CTA");
+    if (C::kSplit && grid > kMostCtas) grid = kMostCtas;
     {
         // The kernel may start while the kernel before it in the stream is still running: its set-up overlaps that
         // kernel's tail, and with `overlap` so do its copies of the weight-side tensors (which the caller has declared
