@@ -1509,6 +1509,18 @@ EncodeTiledFn encode_tiled_fn() {
     return fn;
 }
 
+// The encoder needs a context that is current in the calling thread, which the first CUDA call of a new thread may find missing.
+template <class Encode>
+bool encode_with_context(Encode encode) {
+    if (encode() == CUDA_SUCCESS) return true;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    return encode() == CUDA_SUCCESS;
+}
+
 // 2-D row-major tensor (rows, cols) of `elem_bytes` elements, box (box_rows, box_cols)
 bool encode_2d(CUtensorMap* out, const void* base, CUtensorMapDataType dt, int elem_bytes, uint64_t rows, uint64_t cols,
                uint32_t box_rows, uint32_t box_cols, CUtensorMapSwizzle swz) {
@@ -1518,8 +1530,10 @@ bool encode_2d(CUtensorMap* out, const void* base, CUtensorMapDataType dt, int e
     const cuuint64_t strides[1] = {(cuuint64_t)cols * elem_bytes};
     const cuuint32_t box[2] = {box_cols, box_rows};
     const cuuint32_t estr[2] = {1, 1};
-    return enc(out, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
-               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    return encode_with_context([&] {
+        return enc(out, dt, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    });
 }
 
 // what the last tcgen05 launch of this host thread chose: tile rows + 1000 if CTA pairs + 10000 * K parts (tests read it)
@@ -1588,8 +1602,10 @@ bool encode_x_blocks_cached(CUtensorMap* out, const void* base, uint64_t rows, u
     const cuuint64_t strides[2] = {(cuuint64_t)n * 2, 128};
     const cuuint32_t box[3] = {64, box_rows, blocks};
     const cuuint32_t estr[3] = {1, 1, 1};
-    if (enc(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    if (!encode_with_context([&] {
+            return enc(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                       CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        }))
         return false;
     std::lock_guard<std::mutex> lock(g_map_mutex);
     slot.key = key;

@@ -172,6 +172,29 @@ def test_threads_that_share_a_stream_do_not_mix_their_launches():
     ops.check_device_status()
 
 
+@pytest.mark.parametrize("rows", [1, 40, 300])
+def test_the_first_cuda_call_of_a_thread_may_be_a_multiply(rows):
+    """With weights that no call has seen, so that tensor maps are encoded, which needs the thread to have a CUDA context."""
+    m, s, z, _ = weights(4, 5120, 3072, 128)
+    x = torch.randn((1, rows, 5120), generator=torch.Generator().manual_seed(rows)).half().cuda()
+    out, results = torch.empty((1, rows, 3072), dtype=torch.float16, device="cuda"), []
+    ops.workspace(torch.device("cuda", torch.cuda.current_device()), torch.cuda.current_stream())
+    torch.cuda.synchronize()
+
+    def run():
+        try:
+            results.append(ops.quant_int4_linear_mult_mtx(out, m, x, s, z, 128, None, path=capi.PATH_TCGEN05))
+        except Exception as e:
+            results.append(e)
+    thread = threading.Thread(target=run)
+    thread.start()
+    thread.join()
+    assert results == [None]
+    want = torch.empty_like(out)
+    ops.quant_int4_linear_mult_mtx(want, m, x, s, z, 128, None, path=capi.PATH_TCGEN05)
+    assert torch.equal(out, want)
+
+
 def small_stack(bits, sparse, rows):
     """Two layers of 256 (inner width 448) with weights of one format, and rows of activations."""
     cfg = sharding.StackConfig(hidden=256, mlp=448, layers=2, bits=4, group_size=64)
