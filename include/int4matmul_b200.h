@@ -61,6 +61,15 @@ unsigned long long i4mm_launch_count(void);
  * few-row kernel (up to 8 rows of a small matrix, path 0); 0 after a call that took the streaming path.  For tests that
  * must know which kernel instance they exercised; no reference counterpart. */
 int i4mm_last_launch_shape(void);
+/* How that launch spread the work over the GPU: 0 not the tcgen05 path; whole tiles of the shapes that are made for them; K parts (a
+ * second kernel adds them); or the weight-streaming shape (any row count up to 64, tiles of 128 rows above) with equal ranges of units
+ * for all CTAs, with whole tiles, or with the same number k of CTAs for every tile (I4MM_SCHEDULE_STREAM_CTAS_PER_TILE + k). */
+#define I4MM_SCHEDULE_WHOLE_TILES 1
+#define I4MM_SCHEDULE_K_PARTS 2
+#define I4MM_SCHEDULE_STREAM_EQUAL_RANGES 3
+#define I4MM_SCHEDULE_STREAM_WHOLE_TILES 4
+#define I4MM_SCHEDULE_STREAM_CTAS_PER_TILE 1000
+int i4mm_last_launch_schedule(void);
 
 /*
  * Bytes of device scratch the two multiply entries need.  The scratch holds the per-CTA partial tiles

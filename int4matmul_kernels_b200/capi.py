@@ -17,6 +17,9 @@ ERR_WORKSPACE, ERR_LAUNCH, ERR_MASK, ERR_DEVICE, ERR_TIMEOUT, ERR_TOO_LARGE = 6,
 PATH_AUTO, PATH_STREAM, PATH_TCGEN05, PATH_TCGEN05_SINGLE_CTA = 0, 1, 2, 3
 PATH_STATIC_WEIGHTS = 0x100000      # I4MM_PATH_STATIC_WEIGHTS: or-ed into a path (see the header)
 
+# i4mm_last_launch_schedule
+WHOLE_TILES, K_PARTS, STREAM_EQUAL_RANGES, STREAM_WHOLE_TILES, STREAM_CTAS_PER_TILE = 1, 2, 3, 4, 1000
+
 # every symbol the header declares, with its ctypes signature
 _SIGNATURES = {
     "i4mm_status_string": (ctypes.c_char_p, [ctypes.c_int]),
@@ -24,6 +27,7 @@ _SIGNATURES = {
     "i4mm_version": (ctypes.c_int, []),
     "i4mm_launch_count": (ctypes.c_ulonglong, []),
     "i4mm_last_launch_shape": (ctypes.c_int, []),
+    "i4mm_last_launch_schedule": (ctypes.c_int, []),
     "i4mm_workspace_bytes": (ctypes.c_size_t, []),
     "i4mm_quant_matmul": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, ctypes.c_int,
                                          ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,

@@ -14,6 +14,7 @@ void count_launch(int n) { g_launches.fetch_add((unsigned long long)n); }
 static thread_local int g_last_cuda_error = 0;        // what i4mm_last_cuda_error returns; every entry point records here
 void record_cuda_error(int e) { g_last_cuda_error = e; }
 int umma_last_shape();
+int umma_last_schedule();
 void set_last_shape(int shape);
 cudaError_t stream_launch(int bits, bool sparse, StreamParams p, int total_rows, int ctas, cudaStream_t stream);
 cudaError_t sparse_pack_launch(void* wt_out, void* msk_out, const void* wt_in, const void* msk_in,
@@ -67,6 +68,8 @@ const char* i4mm_status_string(int status) {
 int i4mm_last_cuda_error(void) { return i4mm::g_last_cuda_error; }
 
 int i4mm_last_launch_shape(void) { return i4mm::umma_last_shape(); }
+
+int i4mm_last_launch_schedule(void) { return i4mm::umma_last_schedule(); }
 
 int i4mm_version(void) { return 100; }
 

@@ -1538,6 +1538,7 @@ bool encode_2d(CUtensorMap* out, const void* base, CUtensorMapDataType dt, int e
 
 // what the last tcgen05 launch of this host thread chose: tile rows + 1000 if CTA pairs + 10000 * K parts (tests read it)
 thread_local int g_last_shape = 0;
+thread_local int g_last_schedule = 0;             // i4mm_last_launch_schedule
 
 // Encoded tensor maps are a pure function of (base address, shape, box, swizzle): callers multiply with the same
 // weight tensors over and over, so the maps are kept in a small direct-mapped table instead of being encoded by the
@@ -1760,11 +1761,13 @@ int launch_nt(const UmmaParams& p_in, const __half* x, int n_groups, cudaStream_
         if (e != cudaSuccess) { *cuda_err = e; return I4MM_ERR_LAUNCH; }
         count_launch();
         g_last_shape = NT + 1000 + 10000 * (p.kparts > 1 ? p.kparts : 0);
+        g_last_schedule = p.kparts > 1 ? I4MM_SCHEDULE_K_PARTS : I4MM_SCHEDULE_WHOLE_TILES;
         if (p.kparts > 1) return launch_kparts_reduce(p, stream, cuda_err);
         return I4MM_OK;
     }
     const long long n_tiles = (long long)p.MTILES * p.CT;
     long long grid = sm_count[dev];                     // one CTA per SM: every configuration fills its shared or tensor memory
+    int schedule = I4MM_SCHEDULE_STREAM_EQUAL_RANGES;
     if (!C::kSplit && !p.accumulate && !p.whole_tiles)
         p.kparts = choose_kparts(grid, n_tiles, p.U, p.rows, p.S);
     if (C::kSplit) {
@@ -1772,8 +1775,10 @@ int launch_nt(const UmmaParams& p_in, const __half* x, int n_groups, cudaStream_
         if (p.whole_tiles) {
             const long long w = (n_tiles + grid - 1) / grid;
             grid = (n_tiles + w - 1) / w;
+            schedule = I4MM_SCHEDULE_STREAM_WHOLE_TILES;
         } else if (const int k = ctas_of_a_tile(NT, SPARSE, n_tiles, p.U, grid)) {
             grid = n_tiles * k;
+            schedule = I4MM_SCHEDULE_STREAM_CTAS_PER_TILE + k;
         }
     }
     const long long work = p.kparts > 1 ? n_tiles * p.kparts : C::kSplit && !p.whole_tiles ? n_tiles * p.U : n_tiles;
@@ -1803,6 +1808,7 @@ int launch_nt(const UmmaParams& p_in, const __half* x, int n_groups, cudaStream_
     if (e != cudaSuccess) { *cuda_err = e; return I4MM_ERR_LAUNCH; }
     count_launch();
     g_last_shape = NT + 10000 * (p.kparts > 1 ? p.kparts : 0);
+    g_last_schedule = p.kparts > 1 ? I4MM_SCHEDULE_K_PARTS : C::kStream ? schedule : I4MM_SCHEDULE_WHOLE_TILES;
     if (p.kparts > 1) return launch_kparts_reduce(p, stream, cuda_err);
     return I4MM_OK;
 }
@@ -1927,7 +1933,11 @@ int launch_fmt(UmmaParams& p, const __half* x, int n_groups, int pair_mode, int 
 }  // namespace
 
 int umma_last_shape() { return g_last_shape; }
-void set_last_shape(int shape) { g_last_shape = shape; }
+int umma_last_schedule() { return g_last_schedule; }
+void set_last_shape(int shape) {
+    g_last_shape = shape;
+    g_last_schedule = 0;
+}
 
 bool umma_supported(int bits, bool sparse, int total_rows, int N, int S) {
     (void)bits; (void)sparse; (void)S;

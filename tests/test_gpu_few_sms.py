@@ -45,7 +45,7 @@ def hold():
 
 # one tile cut into parts; three tiles; more tiles than half of the CTAs, with CTAs that go on to a next tile; two accumulators in turn; row tiles
 # beside each other; old outputs.  (Rows up to 32: one CTA of a tile waits for the others; above: those that sum wait for each other.)
-@pytest.mark.parametrize("n,s,m", [(16384, 64, 1), (16384, 128, 16), (2048, 9536, 5), (16384, 64, 33), (16384, 128, 64), (2048, 9536, 48), (16384, 128, 65),
+@pytest.mark.parametrize("n,s,m", [(16384, 64, 1), (16384, 128, 16), (4096, 9536, 5), (16384, 64, 33), (16384, 128, 64), (4096, 9536, 48), (16384, 128, 65),
                                    (8256, 320, 100), (4096, 5056, 128), (4096, 25600, 127), (13824, 2048, 378)])
 @pytest.mark.parametrize("free", [1, 5])
 def test_a_launch_gets_through_beside_a_kernel_that_holds_the_other_sms(hold, free, n, s, m):
@@ -59,6 +59,7 @@ def test_a_launch_gets_through_beside_a_kernel_that_holds_the_other_sms(hold, fr
             out, w["matrix"], w["x"], w["scales"], w["zeros"], 192, None, path=capi.PATH_TCGEN05)
         return out
     quiet = multiply(base.clone() if m == 1 else torch.empty((1, m, s), dtype=torch.float16, device=dev))
+    assert capi.load().i4mm_last_launch_schedule() == capi.STREAM_EQUAL_RANGES or capi.load().i4mm_last_launch_schedule() > capi.STREAM_CTAS_PER_TILE
     beside = base.clone() if m == 1 else torch.empty_like(quiet)
     torch.cuda.synchronize()
     cols = np.unique(np.concatenate([np.arange(16), s - 1 - np.arange(16)]))

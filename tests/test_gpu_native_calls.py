@@ -149,26 +149,42 @@ def test_other_threads_run_while_a_launch_waits_for_room_in_the_queue():
 
 
 def test_threads_that_share_a_stream_do_not_mix_their_launches():
-    """Multiplies cut into K parts are two launches with sums in the stream's scratch between them."""
+    """Multiplies cut into K parts are two launches with sums in the stream's scratch between them (tiles of 128 and 160 rows: this
+    matrix fills few pairs); beside them one-launch multiplies that share tiles through the same scratch."""
     problems = []
-    for i, rows in enumerate((40, 48, 64, 8)):
-        m, s, z, _ = weights(4, 4096, 512, 128)
-        layer = QuantLinear(4, 4096, 512, 128, m, s, z)
+    lib = capi.load()
+    m, s, z, _ = weights(4, 4096, 512, 128)
+    layer = QuantLinear(4, 4096, 512, 128, m, s, z)
+    for i, (rows, height) in enumerate(((40, 128), (100, 128), (150, 160), (300, 160), (48, 0), (8, 0))):
         x = torch.randn((rows, 4096), generator=torch.Generator().manual_seed(i)).half().cuda()
-        problems.append((layer, x, layer(x)))
+
+        def multiply(x=x, rows=rows, height=height):
+            if not height:
+                return layer(x)
+            out = torch.empty((1, rows, 512), dtype=torch.float16, device="cuda")
+            ops.quant_int4_linear_mult_mtx(out, m, x.unsqueeze(0), s, z, 128, None, path=capi.PATH_TCGEN05 | (height << 8))
+            return out[0]
+        before = lib.i4mm_launch_count()
+        want = multiply()
+        assert lib.i4mm_launch_count() - before == (2 if height else 1)
+        assert (lib.i4mm_last_launch_schedule() == capi.K_PARTS) == bool(height)
+        problems.append((multiply, want))
     torch.cuda.synchronize()
     bad = []
 
-    def run(layer, x, want):
-        outs = [layer(x) for _ in range(300)]
-        torch.cuda.synchronize()
-        bad.extend(i for i, o in enumerate(outs) if not torch.equal(o, want))
+    def run(multiply, want):
+        try:
+            outs = [multiply() for _ in range(300)]
+            torch.cuda.synchronize()
+            bad.extend(i for i, o in enumerate(outs) if not torch.equal(o, want))
+        except Exception as e:
+            bad.append(e)
     threads = [threading.Thread(target=run, args=p) for p in problems]
     for t in threads:
         t.start()
     for t in threads:
         t.join()
-    assert not bad, len(bad)
+    assert not bad, (len(bad), bad[0])
     ops.check_device_status()
 
 
@@ -262,14 +278,14 @@ def test_stack_layers_leave_everything_else_to_the_single_calls(monkeypatch):
                     other.forward(h)
                 messages.append((type(e.value), str(e.value)))
         assert messages[0] == messages[1]
-    with monkeypatch.context() as m:
-        fast = [type(e) for e in (_outcome(stack, strided),)]
-        m.setattr(ops, "_native", False)
-        assert fast == [type(e) for e in (_outcome(stack, strided),)]
-
-
-def _outcome(stack, h):
-    try:
-        return stack.forward(h)
-    except Exception as e:
-        return e
+    rows_apart = torch.cat([h, h], dim=1)[:, :h.shape[1]]                        # a row stride: taken by the single calls
+    fast, slow = both(monkeypatch, lambda: stack.forward(rows_apart))
+    assert torch.equal(fast, want) and torch.equal(slow, want)
+    messages = []                                                               # an element stride: refused
+    for native in (ops.native(), False):
+        with monkeypatch.context() as m:
+            m.setattr(ops, "_native", native)
+            with pytest.raises(ValueError) as e:
+                stack.forward(strided)
+            messages.append(str(e.value))
+    assert messages[0] == messages[1]

@@ -14,6 +14,8 @@ from test_gpu_stream import FORMATS, fmt_id
 
 pytestmark = pytest.mark.gpu
 P = capi.PATH_TCGEN05
+# schedules of the weight-streaming shape (up to 148 CTAs a tile)
+STREAMED = (capi.STREAM_EQUAL_RANGES, capi.STREAM_WHOLE_TILES, *range(capi.STREAM_CTAS_PER_TILE + 2, capi.STREAM_CTAS_PER_TILE + 149))
 
 
 # By the CTAs of 148 SMs: one 256-k unit per CTA and as many partners as units (16384 x 64); a last unit that is only partly there
@@ -174,6 +176,8 @@ def test_shared_tiles_of_65_to_128_rows(fmt, n, s, g, m):
     p = oracle.make_packed_problem(bits, n, s, m, g, sparse=sparse, seed=n + s + m)
     got = run_problem(p, path=P)
     assert capi.load().i4mm_last_launch_shape() == 128
+    whole = (n, s) == (2048, 9536)                     # 75 tiles of 16 units: whole ones of the other shape
+    assert capi.load().i4mm_last_launch_schedule() in ((capi.WHOLE_TILES,) if whole else STREAMED)
     cols = np.unique(np.concatenate([np.arange(64), s - 1 - np.arange(64), np.random.default_rng(m).integers(0, s, 60)]))
     want, bound = oracle.expected_columns(bits, p["matrix"], p["mask"], p["scales"], p["zeros"], g, p["x"], cols)
     assert_parity(got[..., cols], want, bound, f"{fmt} m={m} {n}x{s} g{g}")
@@ -203,7 +207,7 @@ def test_row_tiles_of_the_streaming_shape(fmt, n, s, g, m):
     bits, sparse = fmt
     p = oracle.make_packed_problem(bits, n, s, m, g, sparse=sparse, seed=n + s + m)
     got = run_problem(p, path=P)
-    assert capi.load().i4mm_last_launch_shape() == 128
+    assert capi.load().i4mm_last_launch_shape() == 128 and capi.load().i4mm_last_launch_schedule() in STREAMED
     cols = np.unique(np.concatenate([np.arange(32), s - 1 - np.arange(32), np.random.default_rng(m).integers(0, s, 40)]))
     want, bound = oracle.expected_columns(bits, p["matrix"], p["mask"], p["scales"], p["zeros"], g, p["x"], cols)
     assert_parity(got[..., cols], want, bound, f"{fmt} m={m} {n}x{s} g{g}")
@@ -236,6 +240,7 @@ def test_tiles_of_as_many_ctas_each(fmt, m, n, s):
     base = np.random.default_rng(m).standard_normal((1, 1, s)).astype(np.float16) if m == 1 else None
     kw = dict(outs_in=base, route="vec") if m == 1 else {}
     got = run_problem(p, path=P, **kw)
+    assert capi.load().i4mm_last_launch_schedule() > capi.STREAM_CTAS_PER_TILE
     cols = np.unique(np.concatenate([np.arange(32), s - 1 - np.arange(32), np.random.default_rng(m).integers(0, s, 60)]))
     want, bound = oracle.expected_columns(bits, p["matrix"], p["mask"], p["scales"], p["zeros"], 192, p["x"], cols,
                                           outs_in=np.ascontiguousarray(base[..., cols]) if m == 1 else None)

@@ -41,18 +41,26 @@ def test_row_norm_modes_match_the_fp32_expression(rows, width):
     assert torch.equal(both[0], got[2]) and torch.equal(both[1], ops.row_norm(0, got[2]))
 
 
-@pytest.mark.parametrize("rows", [5, 40, 200])
-def test_row_norm_launched_behind_a_multiply_reads_its_finished_output(rows):
+# (rows, tile height, schedule): weight streaming, in one row tile and in two, as the calls are; K parts and CTA pairs by their tile height
+@pytest.mark.parametrize("rows,height,schedule", [(5, 0, capi.STREAM_EQUAL_RANGES), (40, 0, capi.STREAM_EQUAL_RANGES), (200, 0, capi.STREAM_EQUAL_RANGES),
+                                                  (40, 128, capi.K_PARTS), (600, 256, capi.WHOLE_TILES)])
+def test_row_norm_launched_behind_a_multiply_reads_its_finished_output(rows, height, schedule):
     """The glue kernels are launched so that they may start while the kernel before them is still running (and so is
     the reduce kernel of a multiply whose K range was cut into parts); what they read must be that kernel's finished
     output.  Chains launched back to back without a synchronisation against the same chains with one, at the sizes of
-    the 13B-class stack (a 13824 -> 5120 multiply: K parts at 40 rows, CTA pairs at 200), ordinary launches and
-    launches that may overlap."""
+    the 13B-class stack (a 13824 -> 5120 multiply), ordinary launches and launches that may overlap."""
     cfg = sharding.StackConfig(hidden=5120, mlp=13824, layers=1, bits=4, group_size=64)
     w = sharding.synthetic_stack_matrix(cfg, 0, "down", 13824, 5120, torch.device("cuda"))
     g = torch.Generator().manual_seed(rows)
     xs = [torch.randn((rows, w.n), generator=g).to(torch.float16).cuda() for _ in range(3)]
     h = torch.randn((rows, w.s), generator=g).to(torch.float16).cuda()
+
+    def multiply(x):
+        if not height:
+            return sharding.cuda_multiply(w, x)
+        out = torch.empty((1, rows, w.s), dtype=torch.float16, device=x.device)
+        ops.quant_int4_linear_mult_mtx(out, w.matrix, x.unsqueeze(0), w.scales, w.zeros, w.group_size, None, path=2 | (height << 8))
+        return out[0]
 
     def glue(mode, d):
         return ops.row_norm(mode, d) if mode == 0 else ops.row_norm(mode, d, h, d) if mode == 1 else ops.row_norm(mode, h, d)
@@ -61,13 +69,14 @@ def test_row_norm_launched_behind_a_multiply_reads_its_finished_output(rows):
         for mode in range(5):
             refs = []
             for x in xs:
-                d = sharding.cuda_multiply(w, x)
+                d = multiply(x)
+                assert capi.load().i4mm_last_launch_schedule() == schedule
                 torch.cuda.synchronize()
                 refs.append(glue(mode, d))
                 torch.cuda.synchronize()
             ops.set_static_weights(static)
             try:
-                outs = [glue(mode, sharding.cuda_multiply(w, xs[i % 3])) for i in range(24)]
+                outs = [glue(mode, multiply(xs[i % 3])) for i in range(24)]
                 torch.cuda.synchronize()
             finally:
                 ops.set_static_weights(False)

@@ -113,24 +113,32 @@ def test_single_cta_path_matches_cta_pairs_bit_for_bit(fmt, m):
 @pytest.mark.parametrize("s", [128, 256, 640, 1152])
 def test_cta_pairs_with_odd_and_even_column_tile_counts(s):
     p = oracle.make_problem(4, 1024, s, 520, 128, seed=s)
-    got = run_problem(p, path=P)
     want, _, bound = oracle.expected(p)
-    assert_parity(got, want, bound, f"pairs S={s}")
+    assert_parity(run_problem(p, path=P), want, bound, f"S={s}")
+    assert_parity(run_problem(p, path=P | (192 << 8)), want, bound, f"pairs S={s}")       # (tiles of 192 rows run on pairs whatever the shape)
+    assert capi.load().i4mm_last_launch_shape() % 10000 == 1192
 
 
 @pytest.mark.parametrize("fmt", FORMATS, ids=fmt_id)
 @pytest.mark.parametrize("m", [40, 64, 100, 128, 300, 520])
 @pytest.mark.parametrize("path", [P, capi.PATH_TCGEN05_SINGLE_CTA])
 def test_k_parts_for_shapes_with_few_column_tiles(fmt, m, path):
-    """More than 32 rows and few tiles: K is cut into parts (one CTA or CTA pair each) whose fp32 partial outputs a
-    second kernel sums in part order; afterwards the few-row split-K path must still find its scratch all-zero."""
+    """Few tiles of the whole-tile shapes: K is cut into parts (one CTA or CTA pair each) whose fp32 partial outputs a
+    second kernel sums in part order; afterwards the split-K path must still find its scratch all-zero.  The tile height is
+    fixed for that, with the shape that the call takes by itself beside it."""
     bits, sparse = fmt
     p = oracle.make_problem(bits, 2048, 320, m, 128, sparse=sparse, seed=700 + m)
-    got = run_problem(p, path=path)
     want, _, bound = oracle.expected(p)
-    assert_parity(got, want, bound, f"k-parts rows={m} {fmt}")
-    again = run_problem(p, path=path)
-    assert np.array_equal(got.view(np.uint16), again.view(np.uint16))
+    for height in (0, 128 if m <= 128 else 160):
+        got = run_problem(p, path=path | (height << 8))
+        if height:
+            assert capi.load().i4mm_last_launch_shape() == 40000 + height + (1000 if path == P else 0)
+            assert capi.load().i4mm_last_launch_schedule() == capi.K_PARTS
+        assert_parity(got, want, bound, f"k-parts rows={m} {fmt} height {height}")
+        again = run_problem(p, path=path | (height << 8))
+        assert np.array_equal(got.view(np.uint16), again.view(np.uint16))
+        ws = ops.workspace(torch.device("cuda", torch.cuda.current_device()), torch.cuda.current_stream())
+        assert int(ws.count_nonzero()) == 0
     p1 = oracle.make_problem(bits, 2048, 320, 1, 128, sparse=sparse, seed=800 + m)
     got1 = run_problem(p1, path=P)
     want1, _, bound1 = oracle.expected(p1, outs_in=np.zeros((1, 1, 320), np.float16))
