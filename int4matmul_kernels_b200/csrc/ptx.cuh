@@ -35,7 +35,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 // Bounded wait.  kSpinLimit polls of try_wait (each of which may suspend for up to ~20 us) are seconds of
-// wall clock: far beyond any legitimate wait here.
+// wall clock: far beyond any legitimate wait here.  (As many polls of a word in global memory are a quarter of a second.)
 constexpr uint32_t kSpinLimit = 1u << 18;
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
     for (uint32_t i = 0; i < kSpinLimit; ++i)

@@ -212,11 +212,10 @@ template <int NT, bool PAIR, bool STREAM = NT <= 64>
 struct Cfg {
     // packed-weight ring (128 k per stage).  Few rows: the kernel streams weights from HBM, and the ring has to
     // cover the DRAM latency; many rows: weights are a trickle next to the activation tiles
-    // Weight-streaming shapes: one CTA per SM with everything doubled, and K split over the CTAs: all of up to 64 rows, and NT = 128 where
-    // launch_fmt takes it.  Rows 33..64 had tiles
-    // of 64 rows at two CTAs an SM, whole or with K cut into parts and a second launch: 48 rows 13824 x 5120 int4 25.7 us, now 18.8,
-    // 16:32 38.1 / 22.0, int3 34.0 / 18.7, int2 33.1 / 17.4; 5120 x 20480 55.8 / 22.9, 53.8 / 29.7, 43.4 / 23.5, 42.7 / 22.4; 16384 x 16384
-    // 66.3 / 44.3, 76.9 / 56.7, 59.9 / 43.5, 62.3 / 39.0; 1024 x 1024 8.9 / 7.8, 9.6 / 8.2, 9.0 / 7.8, 9.0 / 7.8; nothing was faster there.
+    // Weight-streaming shapes: everything doubled, K split over the CTAs with a scratch reduction, an epilogue from registers that the MMA warp
+    // wakes (named barrier): all of up to 64 rows, and NT = 128 where launch_fmt takes it.  The others: whole tiles, or K parts (choose_kparts),
+    // and epilogue stores that go through a shared-memory transposition tile.  (33..64 rows in whole tiles of 64 rows, two CTAs an SM, or K parts:
+    // 48 rows 13824 x 5120 int4 26.6 us, now 17.4, 16:32 37.8 / 20.8; 5120 x 20480 57.1 / 23.0, 54.9 / 29.3; 1024 x 1024 8.9 / 6.5, 9.6 / 7.6.)
     static constexpr bool kStream = STREAM;
     // NT = 128..192: an MMA of N <= 192 takes 512..768 cycles per 128 k, the dequantisation of its weights with two
     // warpgroups ~1400, so these shapes get four warpgroups as well, and a deeper weight ring
@@ -240,8 +239,6 @@ struct Cfg {
     static constexpr int kWG = kStream ? 3 : kDequantBound ? 4 : 2;   // dequant warpgroups (4 warps each), taking units in turn
     static constexpr int kABStages = NT == 128 ? 4 : 3;   // ring of (A in tensor memory, activation tile in shared memory) pairs, one unit per stage
     static constexpr bool kWGuard = kWStages % kWG != 0;
-    static constexpr bool kEpiTransposed = !kStream;                 // epilogue stores go through a shared-memory transposition tile
-    static constexpr bool kEpiHandoff = kStream;                      // the MMA warp waits for the accumulator and wakes the epilogue warps (named barrier)
     // many rows: two epilogue warpgroups, each draining half of the accumulator's columns, so that the next tile's
     // MMAs wait half as long for the accumulator
     static constexpr int kEpiGroups = kStream ? 1 : 2;
@@ -257,8 +254,6 @@ struct Cfg {
     static constexpr int kAStageCols = 32 * kHalves;
     static constexpr int kColsUsed = kACol0 + kAStageCols * kABStages;
     static constexpr int kTmemCols = kColsUsed <= 256 ? 256 : 512;
-    // split-K over CTAs with a scratch reduction (the other shapes cut K into parts, see choose_kparts)
-    static constexpr bool kSplit = kStream;
     static constexpr int kSlotVecs = NT / 4 * 128;                    // one CTA's partial tile in the scratch: [4 rows][128 columns] of 16 bytes
     static constexpr int kSlots = NT <= 32 ? 1 : 2;                   // of those per CTA, see last_epilogue
 };
@@ -649,7 +644,7 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
     static_assert(!PERM || (C::kStream && F::kPermutedK), "the permuted k order is for dense int4 weight streaming");
     constexpr int H = C::kHalves;                                    // 64-k parts per unit
     using WS = WStage<F, H>;
-    static_assert(!PAIR || (NT >= 128 && !C::kEpiHandoff), "CTA pairs are for the many-row shapes");
+    static_assert(!PAIR || (NT >= 128 && !C::kStream), "CTA pairs are for the many-row shapes");
     static_assert((2 * C::kWStages) % C::kWG == 0, "every second use of a weight stage must be by the same warpgroup");
     static_assert(ABStages<NT, PAIR, STREAM>::value >= C::kWG, "fewer A stages than warpgroups: a parity wait could see the phase before last");
     constexpr int kBHalfBytes = (PAIR ? NT / 2 : NT) * 128;        // one 64-k activation sub-tile held by this CTA
@@ -745,7 +740,7 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
     auto tile_mt = [&](long long tile) -> int { return (int)(tile / CTd); };
     long long t_lo, t_hi;
     const int kpart = p.kparts > 1 ? (int)(b % p.kparts) : 0;
-    if (C::kSplit && !p.whole_tiles) {
+    if (C::kStream && !p.whole_tiles) {
         t_lo = range_lo(n_tiles * U, G, b);
         t_hi = range_lo(n_tiles * U, G, b + 1);
     } else if (p.kparts > 1) {
@@ -968,7 +963,7 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                     }
                 }
                 __syncwarp();
-                if (C::kEpiHandoff) {
+                if (C::kStream) {
                     // the epilogue warps sleep on a hardware barrier instead of polling for the whole segment
                     if (!ptx::mbar_wait(ptx::smem_u32(&bars.d_full), seg & 1u)) {
                         if (lane == 0) atomicExch(p.status, 23);
@@ -982,7 +977,7 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                 ++seg;
                 t += u1 - u0;
             }
-            if (C::kEpiHandoff && !ok) {
+            if (C::kStream && !ok) {
                 s_abort = 1;
                 __threadfence_block();
                 if (!spread_last || !last) ptx::named_bar_arrive(2 + 4 * (seg % C::kDBufs), 128 + 32);
@@ -991,8 +986,9 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
         }
     } else {
         // =========================== dequant warpgroups; epilogue warps ===========================
-        // Accumulator of one finished tile (or K part of one) of the shapes for more than 64 rows -> fp16 rows of `out`, or fp32 rows in
-        // the scratch.  (Up to 64 rows: early_epilogue, last_epilogue.)  Run by 4 warps whose index modulo 4 selects the 32 tensor-memory lanes (= weight columns) they may read.
+        // Accumulator of one finished tile (or K part of one) of the whole-tile shapes -> fp16 rows of `out`, or fp32 rows in the scratch.
+        // (Weight streaming: early_epilogue, last_epilogue.)  Run by 4 warps whose index modulo 4 selects the 32 tensor-memory lanes
+        // (= weight columns) they may read.
         bool dependency_waited = false;
         auto epilogue = [&](uint32_t seg, long long tile) -> bool {
             if (!dependency_waited) {
@@ -1018,13 +1014,11 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
             };
             bool got = ptx::mbar_wait(ptx::smem_u32(&bars.d_full), seg & 1u);
             if (!got && lane == 0) atomicExch(p.status, 33);
-            if (C::kEpiTransposed) {
-                // the four warps of an epilogue group meet at named barriers further down: a give-up has to be
-                // the whole group's decision, or the warps that went on would wait there for ever
-                if (!got) s_abort = 1;
-                ptx::named_bar_sync(1 + 3 * ((warp - kEpiWarp0) >> 2), 128);
-                got = s_abort == 0;
-            }
+            // the four warps of an epilogue group meet at named barriers further down: a give-up has to be
+            // the whole group's decision, or the warps that went on would wait there for ever
+            if (!got) s_abort = 1;
+            ptx::named_bar_sync(1 + 3 * ((warp - kEpiWarp0) >> 2), 128);
+            got = s_abort == 0;
             if (!got) return false;
             ptx::tc_fence_after_sync();
             // matvec route with more than 64 rows (a batch of one-row products): the caller's old values of rows
@@ -1036,64 +1030,28 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                     if (j0 + j < nrows)
                         v[j] = __float_as_uint(__uint_as_float(v[j]) + __half2float(p.om.dst[0][(size_t)(row0 + j0 + j) * p.om.ld + p.om.col(scol)]));
             };
-            if (C::kEpiTransposed) {
-                // 16 accumulator columns (= 16 output rows) at a time: transposed through a 4 KB shared-memory tile so that
-                // the global stores are 16-byte rows instead of one 2-byte element per lane
-                const int eg = (warp - kEpiWarp0) >> 2;                     // epilogue warpgroup: its share of the accumulator columns
-                const uint32_t stage_tile = epi_tile + eg * 4096;          // [16 rows][128 columns] fp16
-                const uint32_t bar_id = 1 + 3 * eg;                         // named barriers 1 and 4
-                const int t128 = (warp & 3) * 32 + lane;
-                constexpr int kShare = NT / kEpiGroups;
-                const int j_end = (eg + 1) * kShare;
-                if (PAIR) {
-                    // A CTA of a pair has the shared memory to stage its whole share as fp16 ([kShare rows][128 columns]):
-                    // the accumulator is released after the tensor-memory loads and conversions alone, and the global
-                    // stores run while the next tile's MMAs are already under way.
-                    const uint32_t stage = epi_tile + eg * (kShare * 256);
-#pragma unroll 1
-                    for (int j0 = eg * kShare; j0 < j_end; j0 += 16) {
-                        uint32_t v[16];
-                        ptx::tmem_ld16(lane_addr + j0, v);
-                        ptx::tc_wait_ld();
-                        if (j0 + 16 >= j_end) {
-                            ptx::tc_fence_before_sync();
-                            __syncwarp();
-                            if (lane == 0) ptx::mbar_arrive_cluster(ptx::map_to_cta(ptx::smem_u32(&bars.d_empty[0]), 0));
-                        }
-                        if (p.kparts > 1) {
-                            put_kpart(v, j0);
-                            continue;
-                        }
-                        if (p.accumulate) add_old_outs(v, j0);
-#pragma unroll
-                        for (int j = 0; j < 16; ++j)
-                            ptx::sts16(stage + (j0 - eg * kShare + j) * 256 + col * 2,
-                                       __half_as_ushort(__float2half_rn(__uint_as_float(v[j]))));
-                    }
-                    ptx::named_bar_sync(bar_id, 128);
-#pragma unroll 1
-                    for (int idx = t128; idx < (p.kparts > 1 ? 0 : kShare * 16); idx += 128) {   // 16-byte chunks: row = idx / 16, chunk = idx % 16
-                        const int m = eg * kShare + (idx >> 4), c8 = (idx & 15) * 8;
-                        if (m < nrows && ct * 128 + c8 < p.S) {
-                            const uint4 q = ptx::lds128(stage + (idx >> 4) * 256 + c8 * 2);
-                            const size_t at = (size_t)(row0 + m) * p.om.ld + p.om.col(ct * 128 + c8);   // (a chunk of 8 columns never straddles parts)
-                            for (int d = 0; d < p.om.n_dst; ++d) *reinterpret_cast<uint4*>(p.om.dst[d] + at) = q;
-                        }
-                    }
-                    ptx::named_bar_sync(bar_id, 128);                       // the staging area may be written again
-                } else
+            // 16 accumulator columns (= 16 output rows) at a time: transposed through a 4 KB shared-memory tile so that
+            // the global stores are 16-byte rows instead of one 2-byte element per lane
+            const int eg = (warp - kEpiWarp0) >> 2;                     // epilogue warpgroup: its share of the accumulator columns
+            const uint32_t stage_tile = epi_tile + eg * 4096;          // [16 rows][128 columns] fp16
+            const uint32_t bar_id = 1 + 3 * eg;                         // named barriers 1 and 4
+            const int t128 = (warp & 3) * 32 + lane;
+            constexpr int kShare = NT / kEpiGroups;
+            const int j_end = (eg + 1) * kShare;
+            if (PAIR) {
+                // A CTA of a pair has the shared memory to stage its whole share as fp16 ([kShare rows][128 columns]):
+                // the accumulator is released after the tensor-memory loads and conversions alone, and the global
+                // stores run while the next tile's MMAs are already under way.
+                const uint32_t stage = epi_tile + eg * (kShare * 256);
 #pragma unroll 1
                 for (int j0 = eg * kShare; j0 < j_end; j0 += 16) {
                     uint32_t v[16];
                     ptx::tmem_ld16(lane_addr + j0, v);
                     ptx::tc_wait_ld();
-                    if (j0 + 16 >= j_end) {                // this group's last columns are in registers: its share of the accumulator is free
+                    if (j0 + 16 >= j_end) {
                         ptx::tc_fence_before_sync();
                         __syncwarp();
-                        if (lane == 0) {
-                            if (PAIR) ptx::mbar_arrive_cluster(ptx::map_to_cta(ptx::smem_u32(&bars.d_empty[0]), 0));
-                            else ptx::mbar_arrive(ptx::smem_u32(&bars.d_empty[0]));
-                        }
+                        if (lane == 0) ptx::mbar_arrive_cluster(ptx::map_to_cta(ptx::smem_u32(&bars.d_empty[0]), 0));
                     }
                     if (p.kparts > 1) {
                         put_kpart(v, j0);
@@ -1102,20 +1060,51 @@ umma_kernel(const __grid_constant__ TensorMaps tm, const __grid_constant__ UmmaP
                     if (p.accumulate) add_old_outs(v, j0);
 #pragma unroll
                     for (int j = 0; j < 16; ++j)
-                        ptx::sts16(stage_tile + j * 256 + col * 2, __half_as_ushort(__float2half_rn(__uint_as_float(v[j]))));
-                    ptx::named_bar_sync(bar_id, 128);
-#pragma unroll
-                    for (int r = 0; r < 2; ++r) {
-                        const int idx = t128 + r * 128;                     // 256 chunks of 16 bytes: row = idx / 16, chunk = idx % 16
-                        const int m = j0 + (idx >> 4), c8 = (idx & 15) * 8;
-                        if (m < nrows && ct * 128 + c8 < p.S) {
-                            const uint4 q = ptx::lds128(stage_tile + (idx >> 4) * 256 + c8 * 2);
-                            const size_t at = (size_t)(row0 + m) * p.om.ld + p.om.col(ct * 128 + c8);
-                            for (int d = 0; d < p.om.n_dst; ++d) *reinterpret_cast<uint4*>(p.om.dst[d] + at) = q;
-                        }
-                    }
-                    ptx::named_bar_sync(bar_id, 128);
+                        ptx::sts16(stage + (j0 - eg * kShare + j) * 256 + col * 2,
+                                   __half_as_ushort(__float2half_rn(__uint_as_float(v[j]))));
                 }
+                ptx::named_bar_sync(bar_id, 128);
+#pragma unroll 1
+                for (int idx = t128; idx < (p.kparts > 1 ? 0 : kShare * 16); idx += 128) {   // 16-byte chunks: row = idx / 16, chunk = idx % 16
+                    const int m = eg * kShare + (idx >> 4), c8 = (idx & 15) * 8;
+                    if (m < nrows && ct * 128 + c8 < p.S) {
+                        const uint4 q = ptx::lds128(stage + (idx >> 4) * 256 + c8 * 2);
+                        const size_t at = (size_t)(row0 + m) * p.om.ld + p.om.col(ct * 128 + c8);   // (a chunk of 8 columns never straddles parts)
+                        for (int d = 0; d < p.om.n_dst; ++d) *reinterpret_cast<uint4*>(p.om.dst[d] + at) = q;
+                    }
+                }
+                ptx::named_bar_sync(bar_id, 128);                       // the staging area may be written again
+            } else
+#pragma unroll 1
+            for (int j0 = eg * kShare; j0 < j_end; j0 += 16) {
+                uint32_t v[16];
+                ptx::tmem_ld16(lane_addr + j0, v);
+                ptx::tc_wait_ld();
+                if (j0 + 16 >= j_end) {                // this group's last columns are in registers: its share of the accumulator is free
+                    ptx::tc_fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&bars.d_empty[0]));
+                }
+                if (p.kparts > 1) {
+                    put_kpart(v, j0);
+                    continue;
+                }
+                if (p.accumulate) add_old_outs(v, j0);
+#pragma unroll
+                for (int j = 0; j < 16; ++j)
+                    ptx::sts16(stage_tile + j * 256 + col * 2, __half_as_ushort(__float2half_rn(__uint_as_float(v[j]))));
+                ptx::named_bar_sync(bar_id, 128);
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    const int idx = t128 + r * 128;                     // 256 chunks of 16 bytes: row = idx / 16, chunk = idx % 16
+                    const int m = j0 + (idx >> 4), c8 = (idx & 15) * 8;
+                    if (m < nrows && ct * 128 + c8 < p.S) {
+                        const uint4 q = ptx::lds128(stage_tile + (idx >> 4) * 256 + c8 * 2);
+                        const size_t at = (size_t)(row0 + m) * p.om.ld + p.om.col(ct * 128 + c8);
+                        for (int d = 0; d < p.om.n_dst; ++d) *reinterpret_cast<uint4*>(p.om.dst[d] + at) = q;
+                    }
+                }
+                ptx::named_bar_sync(bar_id, 128);
             }
             // Stores into other GPUs' buffers: every storing thread makes its own stores visible system-wide before the
             // CTA can finish, so that the hand-shake kernel's flag (written by another SM, possibly over another link)
@@ -1707,7 +1696,7 @@ int launch_nt(const UmmaParams& p_in, const __half* x, int n_groups, cudaStream_
     if (!ok) return I4MM_ERR_DEVICE;
 
     const size_t smem = 1024 + (size_t)ABStages<NT, PAIR, STREAM>::value * kBStageBytes + (size_t)C::kWStages * WStage<F, H>::kBytes +
-                        (!C::kEpiTransposed ? 0 : PAIR ? NT * 256 : 4096 * ((C::kEpiGroups == 2 && NT < 256) ? 2 : 1)) +
+                        (C::kStream ? 0 : PAIR ? NT * 256 : 4096 * ((C::kEpiGroups == 2 && NT < 256) ? 2 : 1)) +
                         (PERM ? (size_t)C::kXStaging * kBStageBytes : 0);
     auto kern = umma_kernel<BITS, SPARSE, NT, PAIR, PERM, STREAM>;
     // per-device cache; atomic because two host threads may make their first call at once (both then compute the same value)
@@ -1768,9 +1757,9 @@ int launch_nt(const UmmaParams& p_in, const __half* x, int n_groups, cudaStream_
     const long long n_tiles = (long long)p.MTILES * p.CT;
     long long grid = sm_count[dev];                     // one CTA per SM: every configuration fills its shared or tensor memory
     int schedule = I4MM_SCHEDULE_STREAM_EQUAL_RANGES;
-    if (!C::kSplit && !p.accumulate && !p.whole_tiles)
+    if (!C::kStream && !p.accumulate && !p.whole_tiles)
         p.kparts = choose_kparts(grid, n_tiles, p.U, p.rows, p.S);
-    if (C::kSplit) {
+    if (C::kStream) {
         p.whole_tiles = whole_tiles_better(NT, n_tiles, p.U, grid);
         if (p.whole_tiles) {
             const long long w = (n_tiles + grid - 1) / grid;
@@ -1781,12 +1770,12 @@ int launch_nt(const UmmaParams& p_in, const __half* x, int n_groups, cudaStream_
             schedule = I4MM_SCHEDULE_STREAM_CTAS_PER_TILE + k;
         }
     }
-    const long long work = p.kparts > 1 ? n_tiles * p.kparts : C::kSplit && !p.whole_tiles ? n_tiles * p.U : n_tiles;
+    const long long work = p.kparts > 1 ? n_tiles * p.kparts : C::kStream && !p.whole_tiles ? n_tiles * p.U : n_tiles;
     if (grid > work || p.kparts > 1) grid = work;
     constexpr long long kMostCtas = kPartialBytes / (C::kSlots * C::kSlotVecs * 16);       // those whose shares the scratch holds
-    static_assert(!C::kSplit || kMostCtas >= 148, "every SM of the GPU has its slots");
-    static_assert(NT <= 32 || !C::kSplit || (kMostCtas <= 32 * kLeftWords && kMostCtas * 4 <= kStatusOffset), "last_epilogue: a bit and a word per CTA");
-    if (C::kSplit && grid > kMostCtas) grid = kMostCtas;
+    static_assert(!C::kStream || kMostCtas >= 148, "every SM of the GPU has its slots");
+    static_assert(NT <= 32 || !C::kStream || (kMostCtas <= 32 * kLeftWords && kMostCtas * 4 <= kStatusOffset), "last_epilogue: a bit and a word per CTA");
+    if (C::kStream && grid > kMostCtas) grid = kMostCtas;
     {
         // The kernel may start while the kernel before it in the stream is still running: its set-up overlaps that
         // kernel's tail, and with `overlap` so do its copies of the weight-side tensors (which the caller has declared
@@ -1845,7 +1834,9 @@ constexpr int kPairMinRows = 128;
 // 1024..20480 on both sides: there the chosen one took 0.88 (int4), 0.87 (int3), 0.78 (int2) and 0.91 (16:32) of the time of pairs alone in the
 // mean, within 1 % of always taking the better one, and was in no shape more than 1.5 % slower than pairs.
 // us, pairs / streaming, int4: 13824 x 2048 200 rows 31.2 / 19.5 (K parts), 13824 x 5120 200 rows 48.6 / 34.7, 5120 x 5120 160 rows 24.6 / 18.9;
-// 5120 x 6976 333 rows 27.0 / 32.9 (28 pair tiles of 256 rows twice: every SM busy).
+// 5120 x 6976 333 rows 27.0 / 32.9 (56 pair tiles of 192 rows leave 18 of 74 pairs idle, and are the faster ones all the same: the streaming shape
+// decodes every weight three times).  (Where launch_nt then takes the same number of CTAs for every tile, it does so because that is faster than
+// the equal ranges reckoned with here.)
 bool streaming_better(bool sparse, int rows, int CT, int U, long long S, int sms, bool kparts_allowed) {
     const long long pairs = sms / 2, CT2 = (CT + 1) / 2, tiles = (long long)((rows + 127) / 128) * CT;
     const long long nt = choose_tile_rows(rows, (int)CT2, (int)pairs, 256), tiles2 = (rows + nt - 1) / nt * CT2;
