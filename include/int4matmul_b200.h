@@ -74,8 +74,9 @@ int i4mm_last_launch_schedule(void);
 /*
  * Bytes of device scratch the two multiply entries need.  The scratch holds the per-CTA partial tiles
  * of the split-K reduction (on the tcgen05 and few-row paths words that tell by themselves that they have been
- * written, on the streaming path with arrival counters) and a status word.  It must be zero-filled once before its first use; the kernels leave it
- * all-zero again when they finish, so one buffer can serve every later call on the same stream.
+ * written, on the streaming path with arrival counters), a word per CTA and a status word.  It must be zero-filled once
+ * before its first use; the kernels leave it all-zero again when they finish, so one buffer can serve every later call on
+ * the same stream.
  * Calls that overlap on the device must not share a buffer.  After a call for which
  * i4mm_device_status reported I4MM_ERR_TIMEOUT, zero the buffer again before reusing it.
  */
@@ -90,6 +91,9 @@ size_t i4mm_workspace_bytes(void);
  *   accumulate != 0  ->  out = half(float(out) + x.W): what the reference's matvec route does to the
  *                        caller's `outs` (matvec_kernel.cu:351, 263, 381-382)
  *   accumulate == 0  ->  out is overwritten, as the reference's matmul route does (matmul_kernel.cu:299-332)
+ *
+ * A multiply gets through on however few SMs the kernels of other streams leave it, with the same result: no block waits for
+ * one that the GPU starts after it (blocks start in the order of their numbers), or gives that up after ~0.15 ms.
  *
  * rows = B*M may be any value >= 0 (rows == 0 returns I4MM_OK without a launch).  The entry picks the few-row kernel
  * for up to 8 rows of a small matrix and the tcgen05 tensor-core kernel for everything else; `path` forces one:
