@@ -92,6 +92,29 @@ def test_several_destinations_hold_the_same_bits(fmt, path, m, n, s):
         assert torch.equal(b[:, :s], want[0]) and (b[:, s:] == 7.0).all()
 
 
+# more than 64 rows with several destinations: the whole-tile shapes, in K parts (8256 x 320) and in whole tiles (512 x 38400), single CTAs and pairs
+@pytest.mark.parametrize("n,s,schedule", [(8256, 320, capi.K_PARTS), (512, 38400, capi.WHOLE_TILES)])
+@pytest.mark.parametrize("m", [100, 300])
+def test_several_destinations_of_many_rows(m, n, s, schedule):
+    p = oracle.make_packed_problem(4, n, s, m, 64, seed=n + m)
+    w = {k: to_dev(p[k]) for k in ("matrix", "scales", "zeros", "x")}
+    lib, ld, stream = capi.load(), s + 64, torch.cuda.current_stream()
+    bufs = [torch.full((m, ld), 7.0, dtype=torch.float16, device="cuda") for _ in range(3)]
+    ws = ops.workspace(torch.device("cuda", torch.cuda.current_device()), stream)
+    status = lib.i4mm_quant_matmul_gather(4, P, (ctypes.c_void_p * 3)(*[b.data_ptr() for b in bufs]), 3, ld, 1, 0, 1, w["matrix"].data_ptr(), None,
+                                          w["x"].data_ptr(), w["scales"].data_ptr(), w["zeros"].data_ptr(), m, n, s, p["scales"].shape[0], 64,
+                                          ws.data_ptr(), ws.numel(), stream.cuda_stream)
+    assert status == capi.OK and lib.i4mm_last_launch_schedule() == schedule
+    assert (lib.i4mm_last_launch_shape() % 10000 > 1000) == (m >= 128)
+    torch.cuda.synchronize()
+    cols = np.unique(np.concatenate([np.arange(64), s - 1 - np.arange(64), np.random.default_rng(m).integers(0, s, 60)]))
+    want, bound = oracle.expected_columns(4, p["matrix"], None, p["scales"], p["zeros"], 64, p["x"], cols)
+    assert_parity(bufs[0][:, :s].cpu().numpy()[None, :, cols], want, bound, f"{n}x{s} m={m}")
+    for b in bufs:
+        assert torch.equal(b[:, :s], bufs[0][:, :s]) and (b[:, s:] == 7.0).all()
+    assert int(ws.count_nonzero()) == 0
+
+
 # 33..64 rows: every number of row groups per warpgroup (groups of 4 rows, ragged last ones), on the same sizes
 @pytest.mark.parametrize("n,s,g", [(16384, 64, 128), (8256, 320, 192), (2048, 2432, -1), (2048, 9536, 64), (512, 38400, 128)])
 @pytest.mark.parametrize("m", [33, 36, 47, 48, 49, 61, 64])

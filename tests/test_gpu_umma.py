@@ -7,7 +7,7 @@ import torch
 from int4matmul_kernels_b200 import capi, ops
 from oracle import reference_oracle as oracle
 
-from helpers import assert_parity, run_problem, to_dev
+from helpers import assert_parity, device_problem, run_problem, to_dev
 from test_gpu_stream import FORMATS, fmt_id, one_hot_problem
 
 pytestmark = pytest.mark.gpu
@@ -143,6 +143,30 @@ def test_k_parts_for_shapes_with_few_column_tiles(fmt, m, path):
     got1 = run_problem(p1, path=P)
     want1, _, bound1 = oracle.expected(p1, outs_in=np.zeros((1, 1, 320), np.float16))
     assert_parity(got1, want1, bound1, f"matvec after k-parts {fmt}")
+
+
+def test_k_parts_that_the_shape_rules_choose():
+    """A few hundred rows of a long K on CTA pairs, behind and before multiplies that share tiles through the same scratch, without a synchronisation."""
+    n, s, m = 18368, 2176, 148
+    p = oracle.make_packed_problem(4, n, s, m, 64, seed=9)
+    few = oracle.make_packed_problem(4, 8256, 320, 20, 64, seed=10)
+    cols = np.unique(np.concatenate([np.arange(32), s - 1 - np.arange(32), np.random.default_rng(1).integers(0, s, 40)]))
+    want, bound = oracle.expected_columns(4, p["matrix"], None, p["scales"], p["zeros"], 64, p["x"], cols)
+    alone, few_alone = run_problem(p, path=P), run_problem(few, path=P)
+    d, e = device_problem(p), device_problem(few)
+    outs = [torch.empty((1, m, s), dtype=torch.float16, device="cuda") for _ in range(4)]
+    few_outs = [torch.empty((1, 20, 320), dtype=torch.float16, device="cuda") for _ in range(4)]
+    torch.cuda.synchronize()
+    for out, few_out in zip(outs, few_outs):
+        ops.quant_matmul(4, out, d["matrix"], d["x"], d["scales"], d["zeros"], 64, None, path=P)
+        assert capi.load().i4mm_last_launch_schedule() == capi.K_PARTS and capi.load().i4mm_last_launch_shape() % 10000 == 1160
+        ops.quant_matmul(4, few_out, e["matrix"], e["x"], e["scales"], e["zeros"], 64, None, path=P)
+    torch.cuda.synchronize()
+    assert_parity(alone[..., cols], want, bound, "k-parts")
+    assert all(np.array_equal(o.cpu().numpy().view(np.uint16), alone.view(np.uint16)) for o in outs)
+    assert all(np.array_equal(o.cpu().numpy().view(np.uint16), few_alone.view(np.uint16)) for o in few_outs)
+    ws = ops.workspace(torch.device("cuda", torch.cuda.current_device()), torch.cuda.current_stream())
+    assert int(ws.count_nonzero()) == 0
 
 
 def test_no_device_timeouts_recorded():
